@@ -52,6 +52,7 @@
 #include <vector>
 
 #include "apsp.h"
+#include "apsp_sparse.h"
 #include "common.cuh"
 
 namespace nsg {
@@ -160,33 +161,6 @@ hedetniemi_step_kernel(const float* __restrict__ X, const float* __restrict__ Ap
     if (__syncthreads_or(diff) && tid == 0) changed[step] = 1;
 }
 
-// Properties of A that decide whether repeated squaring applies:
-// flags bit 0 asymmetric, bit 1 non-zero diagonal, bit 2 a negative weight or
-// NaN, bit 3 a finite weight that is not an integer; *wmax = the largest
-// finite weight (as non-negative float bits, so integer max orders them).
-__global__ void analyze_kernel(const float* __restrict__ A, int n, int* flags, int* wmax) {
-    int f = 0, w = 0;
-    const size_t nn = (size_t)n * n;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nn;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        const int i = static_cast<int>(idx / n), j = static_cast<int>(idx % n);
-        const float a = __ldg(A + idx);
-        if (__float_as_int(a) != __float_as_int(__ldg(A + (size_t)j * n + i))) f |= 1;
-        if (i == j && a != 0.f) f |= 2;
-        if (!(a >= 0.f)) f |= 4;
-        if (a >= 0.f && a < __int_as_float(0x7f800000)) {
-            if (a != rintf(a)) f |= 8;
-            w = max(w, __float_as_int(a));
-        }
-    }
-    f = __reduce_or_sync(0xffffffffu, f);
-    w = __reduce_max_sync(0xffffffffu, w);
-    if ((threadIdx.x & 31) == 0) {
-        if (f) atomicOr(flags, f);
-        atomicMax(wmax, w);
-    }
-}
-
 // dst (P x P) = src (n x n, stride n) or its transpose, +inf outside n x n.
 __global__ void pad_copy_kernel(const float* __restrict__ src, float* __restrict__ dst, int n, int P,
                                 int transpose) {
@@ -291,7 +265,11 @@ struct DevMem {
     void* p = nullptr;
     cudaStream_t s;
     DevMem(size_t bytes, cudaStream_t st) : s(st) {
-        NSG_CUDA(cudaMallocAsync(&p, bytes > 0 ? bytes : 1, st));
+        if (bytes) alloc(bytes, st);
+    }
+    void alloc(size_t bytes, cudaStream_t st) {
+        s = st;
+        NSG_CUDA(cudaMallocAsync(&p, bytes, st));
     }
     ~DevMem() { if (p) cudaFreeAsync(p, s); }
     DevMem(const DevMem&) = delete;
@@ -318,28 +296,101 @@ struct Iterates {
 
 std::atomic<int> g_method{-1};
 
-// Whether repeated squaring gives this solve's result (see the file comment):
-// 0 no, 1 exactly (integer weights), 2 within rounding (requested on float
-// weights).
-int use_squaring(const float* A, int n, int max_path_length, cudaStream_t s) {
-    const int method = g_method.load();
-    if (method == 0 || n < 2 || max_path_length < n - 1) return 0;
-    DevMem info(2 * sizeof(int), s);
-    int* d = static_cast<int*>(info.p);
-    NSG_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(int), s));
-    const size_t nn = (size_t)n * n;
-    const int blocks = static_cast<int>(std::min<size_t>((nn + 255) / 256, 4096));
-    analyze_kernel<<<blocks, 256, 0, s>>>(A, n, d, d + 1);
-    NSG_CUDA(cudaGetLastError());
-    int h[2] = {0, 0};
-    NSG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
+// Seconds of a dense step: P^3 terms at 16e12 per second (measured at
+// N = 2000), and what a step of a small matrix takes anyway.
+double dense_step_seconds(int n) {
+    const double P = (n + kPad - 1) / kPad * kPad;
+    return 4e-6 + P * P * P / 16e12;
+}
+
+// A and how a solve of it runs.
+struct Graph {
+    int squaring = 0;  // repeated squaring reaches the result: 1 exactly, 2 within rounding (requested)
+    bool symmetric = false;
+    bool sparse = false;
+    long long width = 0;
+    DevMem words, edges;  // GraphInfo, counts, slice offsets; the entries
+    SellView rows{};
+
+    // unbounded: every shortest path may be taken (maxPathLength >= n - 1)
+    Graph(const float* A, int n, bool unbounded, cudaStream_t s)
+        : words(sizeof(GraphInfo) + sizeof(int) * (2 * (size_t)n + 2), s), edges(0, nullptr) {
+        const int method = g_method.load();
+        const bool may_square = method != 0 && n >= 2 && unbounded;
+        GraphInfo* info = static_cast<GraphInfo*>(words.p);
+        int* counts = reinterpret_cast<int*>(info + 1);
+        int* ptr = counts + n;
+        NSG_CUDA(cudaMemsetAsync(words.p, 0, sizeof(GraphInfo) + sizeof(int) * (size_t)n, s));
+        sparse_analyze(A, n, info, counts, ptr, s);
+        GraphInfo h{};
+        NSG_CUDA(cudaMemcpyAsync(&h, info, sizeof(h), cudaMemcpyDeviceToHost, s));
+        NSG_CUDA(cudaStreamSynchronize(s));
+        symmetric = !(h.flags & 1);
+        width = h.width;
+        if (may_square && !(h.flags & 7)) {
+            float wmax;
+            std::memcpy(&wmax, &h.wmax, sizeof(float));
+            // integer weights with every path sum (at most n-1 edges) exact in float
+            if (!(h.flags & 8) && static_cast<double>(wmax) * (n - 1) < 16777216.0) squaring = 1;
+            else if (method == 1) squaring = 2;  // squaring requested on any weights
+        }
+        sparse = n <= kSparseMaxN && sparse_step_seconds(width, n) < dense_step_seconds(n);
+        if (!sparse) return;
+        edges.alloc(sizeof(int2) * kSellRows * (size_t)std::max<long long>(1, width), s);
+        sparse_fill(A, n, n, ptr, static_cast<int2*>(edges.p), s);
+        rows = {static_cast<const int2*>(edges.p), ptr, sell_slices(n)};
+    }
+};
+
+// Jacobi steps launched in chunks; the last step's flag is read between
+// chunks, so long runs stop shortly after the fixed point (steps past it
+// return at once) and the later chunks, which hide a read each, are longer.
+// launch(t) enqueues step t. Returns the steps run up to and including the
+// one that changed nothing, *launched the steps enqueued, *converged whether
+// there was such a step.
+template <class F>
+int run_steps(int most, int* changed, cudaStream_t s, F&& launch, int* launched, bool* converged) {
+    int chunk = 8, t = 0, last_flag = 1;
+    while (t < most && last_flag) {
+        const int end = t + std::min(most - t, chunk);
+        for (; t < end; ++t) launch(t);
+        NSG_CUDA(cudaMemcpyAsync(&last_flag, changed + (t - 1), sizeof(int), cudaMemcpyDeviceToHost, s));
+        NSG_CUDA(cudaStreamSynchronize(s));
+        chunk = std::min(2 * chunk, 64);
+    }
+    *launched = t;
+    *converged = last_flag == 0;
+    if (last_flag) return t;
+    std::vector<int> flags(t);
+    NSG_CUDA(cudaMemcpyAsync(flags.data(), changed, sizeof(int) * t, cudaMemcpyDeviceToHost, s));
     NSG_CUDA(cudaStreamSynchronize(s));
-    if (h[0] & 7) return 0;                // asymmetric, diagonal, negative or NaN
-    float wmax;
-    std::memcpy(&wmax, &h[1], sizeof(float));
-    // integer weights with every path sum (at most n-1 edges) exact in float
-    if (!(h[0] & 8) && static_cast<double>(wmax) * (n - 1) < 16777216.0) return 1;
-    return method == 1 ? 2 : 0;            // squaring requested on any weights
+    int q = 0;
+    while (flags[q]) ++q;
+    return q + 1;
+}
+
+bool overlap(const float* a, const float* b, size_t nn) { return a < b + nn && b < a + nn; }
+
+int ceil_log2(int v) {
+    int b = 0;
+    while ((1 << b) < v) ++b;
+    return b;
+}
+
+// Sparse Jacobi steps between H and a second matrix, the first one reading A
+// itself. Returns as run_steps; *at is the iterate after *launched steps.
+int sparse_steps(const Graph& g, const float* A, float* H, float* T, int n, int most, cudaStream_t s, int* launched,
+                 bool* converged, float** at) {
+    DevMem changed(sizeof(int) * most, s);
+    NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * most, s));
+    int* ch = static_cast<int*>(changed.p);
+    const int steps = run_steps(most, ch, s, [&](int t) {
+        sparse_step(g.rows, t == 0 ? A : (t & 1) ? H : T, (t & 1) ? T : H, n, ch, t, false, s);
+    }, launched, converged);
+    // step t writes H for even t; after a step that changed nothing both
+    // matrices hold the fixed point (or H alone, if it was the first)
+    *at = *converged || (*launched & 1) ? H : T;
+    return steps;
 }
 
 }  // namespace
@@ -356,63 +407,76 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         NSG_CUDA(cudaMemcpyAsync(H, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
         return 0;
     }
-    if (const int sq = use_squaring(A, n, max_path_length, s)) {
-        // A symmetric: X = A^T = A; each product X <- X (x) X
+    Graph g(A, n, max_path_length >= n - 1, s);
+    const bool sparse = g.sparse && g.squaring != 2;
+    DevMem T(sparse ? nn * sizeof(float) : 0, s), copy(sparse && overlap(A, H, nn) ? nn * sizeof(float) : 0, s);
+    if (copy.p) {
+        NSG_CUDA(cudaMemcpyAsync(copy.p, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        A = static_cast<const float*>(copy.p);
+    }
+    int launched = 0, first = 0;
+    bool converged = false;
+    float* at = nullptr;
+    if (g.squaring) {
+        // A symmetric: X = A^T = A; each product X <- X (x) X.
+        // Exact sums on a sparse A: every A^(t+1) is the same matrix whichever
+        // way it is reached, so the powers are taken one sparse step at a
+        // time while 2^first - 1 of those cost less than `first` products.
+        // A fixed point at step h (the hop diameter) is the one that
+        // ceil(log2 h) products reach and one more confirms.
+        if (sparse) {
+            const double step = sparse_step_seconds(g.width, n), product = dense_step_seconds(n);
+            const int most = ceil_log2(n);
+            while (first < most && ((2 << first) - 1) * step <= (first + 1) * product) ++first;
+            if (first > 0) {
+                const int h = sparse_steps(g, A, H, static_cast<float*>(T.p), n, (1 << first) - 1, s, &launched,
+                                           &converged, &at);
+                if (converged) {
+                    NSG_CUDA(cudaStreamSynchronize(s));
+                    return ceil_log2(h) + 1;
+                }
+                A = at;  // A^(2^first)
+            }
+        }
         Iterates it(A, n, s);
-        int log2n = 0;
-        while ((1 << log2n) < n) ++log2n;
         // Exact sums: powers up to 2^t >= n - 1, then the product that changes
         // nothing. Rounded sums: once every shortest path is covered, a product
         // can still lower an entry by an ulp through another split of a path's
         // sum; those descents are bounded and short, and products that find
         // nothing to change return at once.
-        const int cap = sq == 1 ? log2n + 2 : log2n + 64;
+        const int cap = g.squaring == 1 ? ceil_log2(n) + 2 : ceil_log2(n) + 64;
         DevMem changed(sizeof(int) * cap, s);
         NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * cap, s));
         int* ch = static_cast<int*>(changed.p);
-        for (int t = 0; t < cap; ++t) launch_step(it.X[t & 1], it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
-        std::vector<int> flags(cap);
-        NSG_CUDA(cudaMemcpyAsync(flags.data(), ch, sizeof(int) * cap, cudaMemcpyDeviceToHost, s));
+        const int products = cap - first;
+        for (int t = 0; t < products; ++t)
+            launch_step(it.X[t & 1], it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
+        std::vector<int> flags(products);
+        NSG_CUDA(cudaMemcpyAsync(flags.data(), ch, sizeof(int) * products, cudaMemcpyDeviceToHost, s));
         NSG_CUDA(cudaStreamSynchronize(s));
-        int products = cap;
-        for (int q = 0; q < cap; ++q) {
-            if (flags[q] == 0) {
-                products = q + 1;
-                break;
-            }
-        }
-        if (products == cap && flags[cap - 1]) fail(NSG_ERR_CUDA, "shortest-path squaring did not converge");
-        launch_unpad(it.X[cap & 1], H, n, it.P, s);
+        int q = 0;
+        while (q < products && flags[q]) ++q;
+        if (q == products) fail(NSG_ERR_CUDA, "shortest-path squaring did not converge");
+        launch_unpad(it.X[products & 1], H, n, it.P, s);
         NSG_CUDA(cudaStreamSynchronize(s));
-        return products;
+        return first + q + 1;
+    }
+    if (sparse) {
+        const int steps = sparse_steps(g, A, H, static_cast<float*>(T.p), n, max_path_length, s, &launched,
+                                       &converged, &at);
+        if (at != H) NSG_CUDA(cudaMemcpyAsync(H, at, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        NSG_CUDA(cudaStreamSynchronize(s));
+        return steps;
     }
     Iterates it(A, n, s);
     DevMem changed(sizeof(int) * max_path_length, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * max_path_length, s));
     int* ch = static_cast<int*>(changed.p);
-    // Launch in chunks; read the last step's flag between chunks so long runs
-    // stop shortly after the fixed point instead of queueing empty steps.
-    const int chunk = 8;
-    int t = 0;
-    int last_flag = 1;
-    while (t < max_path_length && last_flag) {
-        const int end = std::min(max_path_length, t + chunk);
-        for (; t < end; ++t) launch_step(it.Ap, it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
-        NSG_CUDA(cudaMemcpyAsync(&last_flag, ch + (t - 1), sizeof(int), cudaMemcpyDeviceToHost, s));
-        NSG_CUDA(cudaStreamSynchronize(s));
-    }
-    std::vector<int> flags(t);
-    NSG_CUDA(cudaMemcpyAsync(flags.data(), ch, sizeof(int) * t, cudaMemcpyDeviceToHost, s));
-    NSG_CUDA(cudaStreamSynchronize(s));
-    int steps = t;
-    for (int q = 0; q < t; ++q) {
-        if (flags[q] == 0) {
-            steps = q + 1;
-            break;
-        }
-    }
-    // The result lives in X[t & 1]; when converged both buffers hold it.
-    launch_unpad(it.X[t & 1], H, n, it.P, s);
+    const int steps = run_steps(max_path_length, ch, s, [&](int t) {
+        launch_step(it.Ap, it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
+    }, &launched, &converged);
+    // The result lives in X[launched & 1]; when converged both buffers hold it.
+    launch_unpad(it.X[launched & 1], H, n, it.P, s);
     NSG_CUDA(cudaStreamSynchronize(s));
     return steps;
 }
@@ -423,20 +487,52 @@ void apsp_paths(const float* A, float* H, int* paths, int n, int L, float tolera
     const size_t nn = (size_t)n * n;
     NSG_CUDA(cudaMemsetAsync(paths, 0xff, sizeof(int) * nn * L, s));  // -1
     if (n == 0) return;
-    Iterates it(A, n, s);
-    DevMem snaps(nn * L * sizeof(float), s);
+    Graph g(A, n, false, s);
+    DevMem snaps(nn * (L + 1) * sizeof(float), s);  // H before each step, and after the last
     DevMem changed(sizeof(int) * L, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * L, s));
     float* Hi = static_cast<float*>(snaps.p);
+    int* ch = static_cast<int*>(changed.p);
+    float* last = Hi + nn * L;
+    if (g.sparse) {
+        NSG_CUDA(cudaMemcpyAsync(Hi, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        for (int p = 0; p < L; ++p) sparse_step(g.rows, Hi + nn * p, Hi + nn * (p + 1), n, ch, p, true, s);
+        SellView cols = g.rows;
+        DevMem words(0, s), edges(0, s);
+        DevMem At(0, s);
+        if (!g.symmetric) {
+            // the columns of A as rows of its transpose
+            const int P = (n + kPad - 1) / kPad * kPad;
+            At.alloc(sizeof(float) * (size_t)P * P, s);
+            float* at = static_cast<float*>(At.p);
+            launch_pad(A, at, n, P, true, s);
+            words.alloc(sizeof(GraphInfo) + sizeof(int) * (2 * (size_t)n + 2), s);
+            GraphInfo* info = static_cast<GraphInfo*>(words.p);
+            int* counts = reinterpret_cast<int*>(info + 1);
+            sparse_count(at, P, n, info, counts, counts + n, s);
+            GraphInfo h{};
+            NSG_CUDA(cudaMemcpyAsync(&h, info, sizeof(h), cudaMemcpyDeviceToHost, s));
+            NSG_CUDA(cudaStreamSynchronize(s));
+            edges.alloc(sizeof(int2) * kSellRows * (size_t)std::max(1, h.width), s);
+            sparse_fill(at, P, n, counts + n, static_cast<int2*>(edges.p), s);
+            cols = {static_cast<const int2*>(edges.p), counts + n, sell_slices(n)};
+        }
+        sparse_walk(cols, last, Hi, paths, tolerance, n, L, s);
+        NSG_CUDA(cudaMemcpyAsync(H, last, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        NSG_CUDA(cudaStreamSynchronize(s));
+        return;
+    }
+    Iterates it(A, n, s);
     for (int p = 0; p < L; ++p) {
         launch_unpad(it.X[p & 1], Hi + nn * p, n, it.P, s);  // H before step p
-        launch_step(it.Ap, it.X[p & 1], it.X[(p + 1) & 1], n, it.P, static_cast<int*>(changed.p), p, s);
+        launch_step(it.Ap, it.X[p & 1], it.X[(p + 1) & 1], n, it.P, ch, p, s);
     }
-    launch_unpad(it.X[L & 1], H, n, it.P, s);
+    launch_unpad(it.X[L & 1], last, n, it.P, s);
     dim3 block(32, 8);
     dim3 grid((n + 31) / 32, (n + 7) / 8);
-    hedetniemi_walk_kernel<<<grid, block, 0, s>>>(H, Hi, A, paths, tolerance, n, L);
+    hedetniemi_walk_kernel<<<grid, block, 0, s>>>(last, Hi, A, paths, tolerance, n, L);
     NSG_CUDA(cudaGetLastError());
+    NSG_CUDA(cudaMemcpyAsync(H, last, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
     NSG_CUDA(cudaStreamSynchronize(s));
 }
 

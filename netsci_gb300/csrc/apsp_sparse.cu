@@ -1,0 +1,336 @@
+// Hedetniemi steps on sparse weight matrices.
+//
+// A step is Hn[i][j] = min_k fl(A[j][k] + H[k][i]) (apsp.cu). An entry
+// A[j][k] = +inf adds +inf or a NaN, neither of which lowers a minimum that
+// starts at +inf, so only the other entries of row j are visited: the result
+// is the dense step's bit for bit, in whatever order they come. Contact
+// graphs and geometric graphs hold about a dozen entries per row, where the
+// dense product visits n.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "apsp_sparse.h"
+#include "common.cuh"
+
+namespace nsg {
+namespace {
+
+constexpr int kInfBits = 0x7f800000;
+
+// Flags, largest weight and entries per row, one 32 x 32 tile of A and its
+// mirror tile per CTA (32 x 8 threads), so that both are read in rows.
+__global__ void analyze_kernel(const float* __restrict__ A, int n, GraphInfo* info, int* counts) {
+    if (blockIdx.x < blockIdx.y) return;
+    __shared__ float t1[32][33], t2[32][33];
+    const float inf = __int_as_float(kInfBits);
+    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, lane = threadIdx.x;
+    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+        t1[y][lane] = (r0 + y < n && c0 + lane < n) ? __ldg(A + (size_t)(r0 + y) * n + c0 + lane) : inf;
+        t2[y][lane] = (c0 + y < n && r0 + lane < n) ? __ldg(A + (size_t)(c0 + y) * n + r0 + lane) : inf;
+    }
+    __syncthreads();
+    int f = 0, w = 0;
+    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            if (side && r0 == c0) break;
+            const float a = side ? t2[y][lane] : t1[y][lane];
+            const int row = (side ? c0 : r0) + y, col = (side ? r0 : c0) + lane;
+            const bool in = row < n && col < n;
+            const unsigned keep = __ballot_sync(0xffffffffu, in && __float_as_int(a) != kInfBits);
+            if (lane == 0 && keep) atomicAdd(counts + row, __popc(keep));
+            if (!in) continue;
+            if (__float_as_int(a) != __float_as_int(side ? t1[lane][y] : t2[lane][y])) f |= 1;
+            if (row == col && a != 0.f) f |= 2;
+            if (!(a >= 0.f)) f |= 4;
+            if (a >= 0.f && a < inf) {
+                if (a != rintf(a)) f |= 8;
+                w = max(w, __float_as_int(a));
+            }
+        }
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    w = __reduce_max_sync(0xffffffffu, w);
+    if (lane == 0) {
+        if (f) atomicOr(&info->flags, f);
+        atomicMax(&info->wmax, w);
+    }
+}
+
+// Entries per row of a matrix of row stride ld, one warp per row.
+__global__ void count_kernel(const float* __restrict__ A, int ld, int n, int* counts) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= n) return;
+    int c = 0;
+    for (int k = lane; k < n; k += 32) c += __float_as_int(__ldg(A + (size_t)row * ld + k)) != kInfBits;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) counts[row] = c;
+}
+
+// Slice widths (the longest row of each slice) and their exclusive prefix;
+// one CTA of 1024 threads.
+__global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ counts, int n, int nslices, int* ptr,
+                                                     GraphInfo* info) {
+    __shared__ int s_warp[32];
+    const int t = threadIdx.x, lane = t & 31;
+    int base = 0;
+    for (int s0 = 0; s0 < nslices; s0 += 1024) {
+        const int s = s0 + t;
+        int w = 0;
+        for (int r = 0; r < kSellRows; ++r) {
+            const int row = s * kSellRows + r;
+            if (s < nslices && row < n) w = max(w, counts[row]);
+        }
+        int x = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_warp[t >> 5] = x;
+        __syncthreads();
+        int before = base, all = base;
+        for (int q = 0; q < 32; ++q) {
+            if (q < (t >> 5)) before += s_warp[q];
+            all += s_warp[q];
+        }
+        if (s < nslices) ptr[s] = before + x - w;
+        base = all;
+        __syncthreads();
+    }
+    if (t == 0) {
+        ptr[nslices] = base;
+        info->width = base;
+    }
+}
+
+// One warp per row (of whole slices): its entries in ascending columns, then
+// the padding up to the slice's width.
+__global__ void fill_kernel(const float* __restrict__ A, int ld, int n, int nslices, const int* __restrict__ ptr,
+                            int2* __restrict__ edges) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= nslices * kSellRows) return;
+    const int s = row / kSellRows, r = row % kSellRows;
+    const int end = ptr[s + 1];
+    int e = ptr[s];
+    if (row < n) {
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + lane;
+            const float a = k < n ? __ldg(A + (size_t)row * ld + k) : __int_as_float(kInfBits);
+            const bool keep = __float_as_int(a) != kInfBits;
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int at = e + __popc(mask & ((1u << lane) - 1u));
+                edges[(size_t)at * kSellRows + r] = make_int2(k, __float_as_int(a));
+            }
+            e += __popc(mask);
+        }
+    }
+    for (int p = e + lane; p < end; p += 32) edges[(size_t)p * kSellRows + r] = make_int2(0, kInfBits);
+}
+
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem, int bytes16) {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    if (bytes16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gmem) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem) : "memory");
+}
+
+// One step. A CTA owns the C columns i0 .. i0+C-1 of H, staged in shared
+// memory once (all n rows: n * C floats), and a range of slices; every
+// neighbour row read is then a shared-memory read. C/4 lanes take a row,
+// four columns each, so 32/(C/4) rows are reduced per warp at a time and the
+// entries of a slice arrive as one 64-byte load per entry index. Results go
+// out transposed (Hn[i][j], j along the lanes). The compare against H stops
+// reading H once a difference was seen in the CTA.
+template <int C>
+__global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const float* __restrict__ H,
+                                                           float* __restrict__ Hn, int n, int per_split, int vec,
+                                                           int* changed, int step, int fill) {
+    extern __shared__ __align__(16) float hs[];
+    __shared__ int s_diff;
+    constexpr int kLanes = C / 4;           // lanes per row
+    constexpr int kRows = 32 / kLanes;      // rows per warp
+    constexpr int kSlices = kRows / kSellRows;
+    const float inf = __int_as_float(kInfBits);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int i0 = blockIdx.x * C;
+    const int first = blockIdx.y * per_split, last = min(g.nslices, first + per_split);
+    if (step > 0 && changed[step - 1] == 0) {  // fixed point reached earlier
+        if (!fill) return;
+        const int j0 = first * kSellRows, w = min(n, last * kSellRows) - j0;
+        for (int idx = tid; idx < C * w; idx += blockDim.x) {
+            const int i = i0 + idx / w, j = j0 + idx % w;
+            if (i < n) Hn[(size_t)i * n + j] = H[(size_t)i * n + j];
+        }
+        return;
+    }
+    if (tid == 0) s_diff = 0;
+    if (vec && i0 + C <= n) {
+        for (int idx = tid; idx < n * kLanes; idx += blockDim.x) {
+            const int k = idx / kLanes, q = idx % kLanes;
+            cp_async(hs + 4 * idx, H + (size_t)k * n + i0 + 4 * q, 1);
+        }
+    } else {
+        for (int idx = tid; idx < n * C; idx += blockDim.x) {
+            const int k = idx / C, c = idx % C;
+            if (i0 + c < n) cp_async(hs + idx, H + (size_t)k * n + i0 + c, 0);
+            else hs[idx] = inf;
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float4* h4 = reinterpret_cast<const float4*>(hs);
+    const int q = lane % kLanes, rw = lane / kLanes, r = rw % kSellRows;
+    const int stride = (blockDim.x >> 5) * kSlices;
+    bool diff = false;
+    for (int s0 = first + (tid >> 5) * kSlices; s0 < last; s0 += stride) {
+        const int s = s0 + rw / kSellRows;
+        if (s >= last) continue;
+        const int end = __ldg(g.ptr + s + 1);
+        int e = __ldg(g.ptr + s);
+        float acc[4] = {inf, inf, inf, inf};
+        const int2* ed = g.edges + r;
+        for (; e + 1 < end; e += 2) {
+            const int2 p0 = __ldg(ed + (size_t)e * kSellRows), p1 = __ldg(ed + (size_t)(e + 1) * kSellRows);
+            const float4 v0 = h4[p0.x * kLanes + q], v1 = h4[p1.x * kLanes + q];
+            const float a0 = __int_as_float(p0.y), a1 = __int_as_float(p1.y);
+            acc[0] = nsg_min3(acc[0], __fadd_rn(a0, v0.x), __fadd_rn(a1, v1.x));
+            acc[1] = nsg_min3(acc[1], __fadd_rn(a0, v0.y), __fadd_rn(a1, v1.y));
+            acc[2] = nsg_min3(acc[2], __fadd_rn(a0, v0.z), __fadd_rn(a1, v1.z));
+            acc[3] = nsg_min3(acc[3], __fadd_rn(a0, v0.w), __fadd_rn(a1, v1.w));
+        }
+        if (e < end) {
+            const int2 p0 = __ldg(ed + (size_t)e * kSellRows);
+            const float4 v0 = h4[p0.x * kLanes + q];
+            const float a0 = __int_as_float(p0.y);
+            acc[0] = fminf(acc[0], __fadd_rn(a0, v0.x));
+            acc[1] = fminf(acc[1], __fadd_rn(a0, v0.y));
+            acc[2] = fminf(acc[2], __fadd_rn(a0, v0.z));
+            acc[3] = fminf(acc[3], __fadd_rn(a0, v0.w));
+        }
+        const int j = s * kSellRows + r;
+        if (j >= n) continue;
+        const bool look = !diff && *reinterpret_cast<volatile int*>(&s_diff) == 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + 4 * q + u;
+            if (i >= n) break;
+            const size_t o = (size_t)i * n + j;
+            if (look && __float_as_int(acc[u]) != __float_as_int(H[o])) diff = true;
+            Hn[o] = acc[u];
+        }
+        if (diff) s_diff = 1;
+    }
+    if (__syncthreads_or(diff) && tid == 0) changed[step] = 1;
+}
+
+// The back-walk of netcalc/src/hedetniemi_gpu.cu:70-107, as
+// hedetniemi_walk_kernel (apsp.cu): the first q (ascending, q != j) with
+// H_p[i][q] + A[q][k] - len < tolerance. An entry A[q][k] = +inf never
+// passes that test, so only the other entries of column k are looked at.
+__global__ void sparse_walk_kernel(SellView cols, const float* __restrict__ H, const float* __restrict__ Hi,
+                                   int* __restrict__ paths, float tolerance, int n, int L) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= n || j >= n) return;
+    int* cell = paths + (size_t)i * L * n + (size_t)j * L;
+    if (i == j) {
+        for (int p = 0; p < L; ++p) cell[p] = i;
+        return;
+    }
+    float len = H[(size_t)i * n + j];
+    int k = j;
+    for (int p = L - 1; p >= 0; --p) {
+        const float* hp = Hi + (size_t)p * n * n + (size_t)i * n;
+        const int s = k / kSellRows;
+        const int end = __ldg(cols.ptr + s + 1);
+        const int2* ed = cols.edges + k % kSellRows;
+        for (int e = __ldg(cols.ptr + s); e < end; ++e) {
+            const int2 c = __ldg(ed + (size_t)e * kSellRows);
+            if (c.x == j) continue;
+            const float a = __int_as_float(c.y);
+            if (__fsub_rn(__fadd_rn(hp[c.x], a), len) < tolerance) {
+                len = __fsub_rn(len, a);
+                k = c.x;
+                break;
+            }
+        }
+        cell[p] = k;
+    }
+}
+
+int sm_count_now() {
+    int dev = 0, sms = 0;
+    NSG_CUDA(cudaGetDevice(&dev));
+    NSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms;
+}
+
+template <int C>
+void launch_step(const SellView& g, const float* H, float* Hn, int n, int* changed, int step, bool fill,
+                 cudaStream_t s) {
+    static_assert(C % 4 == 0 && 32 / (C / 4) >= kSellRows, "whole slices per warp");
+    constexpr int kSlices = 32 / (C / 4) / kSellRows;
+    const size_t smem = (size_t)n * C * sizeof(float);
+    // set on every launch: the attribute belongs to the current device
+    NSG_CUDA(cudaFuncSetAttribute(sparse_step_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+    const int blocks = (n + C - 1) / C;
+    // slices split over CTAs until there is one per SM, at least one warp's worth each
+    const int splits = std::max(1, std::min(sm_count_now() / blocks, g.nslices / (4 * kSlices)));
+    const int per = (g.nslices + splits - 1) / splits;
+    const int warps = std::min(32, std::max(4, (per + kSlices - 1) / kSlices));
+    const int vec = (n % 4 == 0) && (reinterpret_cast<uintptr_t>(H) % 16 == 0);
+    sparse_step_kernel<C><<<dim3(blocks, (g.nslices + per - 1) / per), 32 * warps, smem, s>>>(
+        g, H, Hn, n, per, vec, changed, step, fill ? 1 : 0);
+    NSG_CUDA(cudaGetLastError());
+}
+
+// Columns per CTA: 16 while n rows of them fit in shared memory, then 8 and 4.
+constexpr int kMax16 = 3500, kMax8 = 7000;
+static_assert(kMax16 * 16 * 4 <= 224 << 10 && kMax8 * 8 * 4 <= 224 << 10 && kSparseMaxN * 4 * 4 <= 224 << 10,
+              "a column block fits in shared memory");
+
+}  // namespace
+
+void sparse_analyze(const float* A, int n, GraphInfo* info, int* counts, int* ptr, cudaStream_t s) {
+    const int t = (n + 31) / 32;
+    analyze_kernel<<<dim3(t, t), dim3(32, 8), 0, s>>>(A, n, info, counts);
+    slice_kernel<<<1, 1024, 0, s>>>(counts, n, sell_slices(n), ptr, info);
+    NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_count(const float* A, int ld, int n, GraphInfo* info, int* counts, int* ptr, cudaStream_t s) {
+    count_kernel<<<(n + 7) / 8, 256, 0, s>>>(A, ld, n, counts);
+    slice_kernel<<<1, 1024, 0, s>>>(counts, n, sell_slices(n), ptr, info);
+    NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_fill(const float* A, int ld, int n, const int* ptr, int2* edges, cudaStream_t s) {
+    const int ns = sell_slices(n);
+    fill_kernel<<<ns, 32 * kSellRows, 0, s>>>(A, ld, n, ns, ptr, edges);
+    NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_step(const SellView& g, const float* H, float* Hn, int n, int* changed, int step, bool fill,
+                 cudaStream_t s) {
+    if (n <= kMax16) launch_step<16>(g, H, Hn, n, changed, step, fill, s);
+    else if (n <= kMax8) launch_step<8>(g, H, Hn, n, changed, step, fill, s);
+    else launch_step<4>(g, H, Hn, n, changed, step, fill, s);
+}
+
+double sparse_step_seconds(long long width, int n) {
+    return 3e-6 + 8.0 * static_cast<double>(width) * n / 6e12;
+}
+
+void sparse_walk(const SellView& cols, const float* H, const float* Hi, int* paths, float tolerance, int n, int L,
+                 cudaStream_t s) {
+    dim3 block(32, 8);
+    dim3 grid((n + 31) / 32, (n + 7) / 8);
+    sparse_walk_kernel<<<grid, block, 0, s>>>(cols, H, Hi, paths, tolerance, n, L);
+    NSG_CUDA(cudaGetLastError());
+}
+
+}  // namespace nsg

@@ -68,8 +68,8 @@ __global__ void count_kernel(const float* __restrict__ A, int ld, int n, int* co
     if (lane == 0) counts[row] = c;
 }
 
-// Slice widths (the longest row of each slice) and their exclusive prefix;
-// one CTA of 1024 threads.
+// Slice widths (the longest row of each slice, in whole groups of
+// kSellUnroll) and their exclusive prefix; one CTA of 1024 threads.
 __global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ counts, int n, int nslices, int* ptr,
                                                      GraphInfo* info) {
     __shared__ int s_warp[32];
@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ cou
             const int row = s * kSellRows + r;
             if (s < nslices && row < n) w = max(w, counts[row]);
         }
+        w = (w + kSellUnroll - 1) / kSellUnroll * kSellUnroll;
         int x = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -184,42 +185,57 @@ __global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const flo
     const float4* h4 = reinterpret_cast<const float4*>(hs);
     const int q = lane % kLanes, rw = lane / kLanes, r = rw % kSellRows;
     const int stride = (blockDim.x >> 5) * kSlices;
+    // this lane's columns: rows i0 + 4q .. of the transposed result
+    const int cols = n - (i0 + 4 * q);
+    float* out = Hn + (size_t)(i0 + 4 * q) * n;
+    const float* old = H + (size_t)(i0 + 4 * q) * n;
     bool diff = false;
     for (int s0 = first + (tid >> 5) * kSlices; s0 < last; s0 += stride) {
         const int s = s0 + rw / kSellRows;
         if (s >= last) continue;
-        const int end = __ldg(g.ptr + s + 1);
-        int e = __ldg(g.ptr + s);
+        const int e0 = __ldg(g.ptr + s);
+        int groups = (__ldg(g.ptr + s + 1) - e0) / kSellUnroll;
         float acc[4] = {inf, inf, inf, inf};
-        const int2* ed = g.edges + r;
-        for (; e + 1 < end; e += 2) {
-            const int2 p0 = __ldg(ed + (size_t)e * kSellRows), p1 = __ldg(ed + (size_t)(e + 1) * kSellRows);
-            const float4 v0 = h4[p0.x * kLanes + q], v1 = h4[p1.x * kLanes + q];
-            const float a0 = __int_as_float(p0.y), a1 = __int_as_float(p1.y);
-            acc[0] = nsg_min3(acc[0], __fadd_rn(a0, v0.x), __fadd_rn(a1, v1.x));
-            acc[1] = nsg_min3(acc[1], __fadd_rn(a0, v0.y), __fadd_rn(a1, v1.y));
-            acc[2] = nsg_min3(acc[2], __fadd_rn(a0, v0.z), __fadd_rn(a1, v1.z));
-            acc[3] = nsg_min3(acc[3], __fadd_rn(a0, v0.w), __fadd_rn(a1, v1.w));
+        const int2* ed = g.edges + (size_t)e0 * kSellRows + r;
+        int2 p[kSellUnroll];
+        if (groups > 0) {
+#pragma unroll
+            for (int e = 0; e < kSellUnroll; ++e) p[e] = __ldg(ed + e * kSellRows);
         }
-        if (e < end) {
-            const int2 p0 = __ldg(ed + (size_t)e * kSellRows);
-            const float4 v0 = h4[p0.x * kLanes + q];
-            const float a0 = __int_as_float(p0.y);
-            acc[0] = fminf(acc[0], __fadd_rn(a0, v0.x));
-            acc[1] = fminf(acc[1], __fadd_rn(a0, v0.y));
-            acc[2] = fminf(acc[2], __fadd_rn(a0, v0.z));
-            acc[3] = fminf(acc[3], __fadd_rn(a0, v0.w));
+        for (; groups > 0; --groups) {
+            float4 v[kSellUnroll];
+            float a[kSellUnroll];
+#pragma unroll
+            for (int e = 0; e < kSellUnroll; ++e) {
+                v[e] = h4[p[e].x * kLanes + q];
+                a[e] = __int_as_float(p[e].y);
+            }
+            ed += kSellUnroll * kSellRows;
+            if (groups > 1) {  // the next entries load while these are reduced
+#pragma unroll
+                for (int e = 0; e < kSellUnroll; ++e) p[e] = __ldg(ed + e * kSellRows);
+            }
+#pragma unroll
+            for (int e = 0; e < kSellUnroll; e += 2) {
+                acc[0] = nsg_min3(acc[0], __fadd_rn(a[e], v[e].x), __fadd_rn(a[e + 1], v[e + 1].x));
+                acc[1] = nsg_min3(acc[1], __fadd_rn(a[e], v[e].y), __fadd_rn(a[e + 1], v[e + 1].y));
+                acc[2] = nsg_min3(acc[2], __fadd_rn(a[e], v[e].z), __fadd_rn(a[e + 1], v[e + 1].z));
+                acc[3] = nsg_min3(acc[3], __fadd_rn(a[e], v[e].w), __fadd_rn(a[e + 1], v[e + 1].w));
+            }
         }
         const int j = s * kSellRows + r;
         if (j >= n) continue;
         const bool look = !diff && *reinterpret_cast<volatile int*>(&s_diff) == 0;
+        float* on = out + j;
+        const float* oh = old + j;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int i = i0 + 4 * q + u;
-            if (i >= n) break;
-            const size_t o = (size_t)i * n + j;
-            if (look && __float_as_int(acc[u]) != __float_as_int(H[o])) diff = true;
-            Hn[o] = acc[u];
+            if (u < cols) {
+                if (look && __float_as_int(acc[u]) != __float_as_int(*oh)) diff = true;
+                *on = acc[u];
+            }
+            on += n;
+            oh += n;
         }
         if (diff) s_diff = 1;
     }

@@ -9,8 +9,10 @@ namespace nsg {
 // Rows of a matrix in slices of kSellRows rows: slice s holds
 // ptr[s+1] - ptr[s] entries per row, entry e of row r of the slice at
 // edges[(ptr[s] + e) * kSellRows + r] as (column, weight bits), columns
-// ascending. Shorter rows are padded with (0, +inf).
+// ascending. Widths are multiples of kSellUnroll; shorter rows are padded
+// with (0, +inf).
 constexpr int kSellRows = 8;
+constexpr int kSellUnroll = 4;
 struct SellView {
     const int2* edges;
     const int* ptr;

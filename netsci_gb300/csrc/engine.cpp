@@ -11,6 +11,7 @@
 #include <string>
 
 #include "errors.h"
+#include "ksg_bits.h"
 #include "ksg_grid.h"
 #include "ksg_registry.cuh"
 
@@ -622,12 +623,19 @@ struct KsgPlan::GridState {
     DeviceBuffer gps, pair_arena;         // GridPair per plan pair; pair grids of one batch
     std::vector<int> batch_maxm;          // largest m of each batch
     std::vector<char> batch_order;        // whether each batch builds query orders
-    bool node_est = false;                // some batch does: nodes need scale estimates
+    bool split_nodes = false;             // an ordered batch: many nodes, three kernels
+    bool node_est = false;                // a batch needs the nodes' scale estimates
+    std::vector<BitsConfig> batch_bits;   // bitmap search where ok, else the scan on pair grids
+    int max_m = 0;
     DeviceBuffer wprefix;                 // per batch: npairs+1 prefix of ceil(m/32)
     std::vector<long long> wprefix_off;   // offset of each batch's prefix
     DeviceBuffer groups, gprefix;         // count groups and their item prefix, per batch
     std::vector<long long> group_off, gprefix_off;
     std::vector<int> ngroups;
+    DeviceBuffer ranks, rprefix, refs;    // rank nodes, item prefix and variables, per batch
+    std::vector<long long> rank_off, rprefix_off, ref_off;
+    std::vector<int> nranks, rank_items;
+    DeviceBuffer rank_emax;               // nranks x largest m of an ordered batch
     DeviceBuffer corder;                  // count-query order: ngroups x largest m of a batch
     DeviceBuffer eps_a, eps_b, cnt_a, cnt_b;
     DeviceBuffer evals;                   // 3 counters per run (see GridArgs::evals)
@@ -674,7 +682,8 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
     g->node_arena.reset(std::max<size_t>(arena, 16));
     unsigned char* base = g->node_arena.as<unsigned char>();
     for (size_t i = 0; i < nodes.size(); ++i) {
-        nodes[i] = grid_node_at(base + node_off[i], nodes[i].x, nodes[i].ld, nodes[i].m);
+        nodes[i] = grid_node_at(base + node_off[i], nodes[i].x, nodes[i].ld, nodes[i].m, d_);
+        g->max_m = std::max(g->max_m, nodes[i].m);
     }
     g->nodes.reset(nodes.size() * sizeof(GridNode));
     NSG_CUDA(cudaMemcpy(g->nodes.get(), nodes.data(), nodes.size() * sizeof(GridNode),
@@ -691,49 +700,63 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
             maxm = std::max(maxm, descs[p].m);
             wpre.push_back(acc);
             acc += (descs[p].m + 31) / 32;
-            off = grid_pair_place(gps[p], off, descs[p].m, d_);
         }
+        g->batch_bits.push_back(bits_config(d_, k_, maxm));
+        const bool bits = g->batch_bits.back().ok;
+        for (int p = b.pair0; p < b.pair0 + b.npairs && !bits; ++p) off = grid_pair_place(gps[p], off, descs[p].m, d_);
         wpre.push_back(acc);
         g->batch_maxm.push_back(maxm);
         const int forced = ksg_forced_orders();
         const bool order = forced >= 0 ? forced == 1 : grid_orders_pay(acc, sm_count());
         g->batch_order.push_back(order ? 1 : 0);
-        g->node_est = g->node_est || order;
+        g->node_est = g->node_est || order || bits;
+        g->split_nodes = g->split_nodes || order;
         pair_arena = std::max(pair_arena, off);
     }
     g->pair_arena.reset(std::max<size_t>(pair_arena, 16));
     for (auto& gp : gps) grid_pair_rebase(gp, g->pair_arena.get());
-    // count groups: pairs of a batch that count the same node's variable
+    // count groups and rank nodes: variables of a batch on the same node
     {
         std::vector<CountGroup> groups;
-        std::vector<int> gpre;
-        for (const Batch& b : batches_) {
+        std::vector<RankNode> ranks;
+        std::vector<int> gpre, rpre;
+        std::vector<long long> refs;
+        size_t corder = 0, emax = 0;
+        for (size_t bi = 0; bi < batches_.size(); ++bi) {
+            const Batch& b = batches_[bi];
+            const bool order = g->batch_order[bi] != 0;
+            const CountWork w = count_work(gps.data() + b.pair0, descs.data() + b.pair0, b.npairs,
+                                           order ? kRankMinVars : 1);
             g->group_off.push_back(static_cast<long long>(groups.size()));
             g->gprefix_off.push_back(static_cast<long long>(gpre.size()));
-            const size_t first = groups.size();
-            append_count_groups(gps.data() + b.pair0, b.npairs, groups);
-            int acc = 0;
-            for (size_t gi = first; gi < groups.size(); ++gi) {
-                gpre.push_back(acc);
-                acc += (nodes[groups[gi].node].m + kCountQueries - 1) / kCountQueries;
+            g->rank_off.push_back(static_cast<long long>(ranks.size()));
+            g->rprefix_off.push_back(static_cast<long long>(rpre.size()));
+            g->ref_off.push_back(static_cast<long long>(refs.size()));
+            g->ngroups.push_back(static_cast<int>(w.groups.size()));
+            g->nranks.push_back(static_cast<int>(w.ranks.size()));
+            g->rank_items.push_back(w.rprefix.back());
+            groups.insert(groups.end(), w.groups.begin(), w.groups.end());
+            gpre.insert(gpre.end(), w.gprefix.begin(), w.gprefix.end());
+            ranks.insert(ranks.end(), w.ranks.begin(), w.ranks.end());
+            rpre.insert(rpre.end(), w.rprefix.begin(), w.rprefix.end());
+            refs.insert(refs.end(), w.refs.begin(), w.refs.end());
+            if (order) {
+                corder = std::max(corder, w.groups.size() * static_cast<size_t>(g->batch_maxm[bi]));
+                emax = std::max(emax, w.ranks.size() * static_cast<size_t>(g->batch_maxm[bi]));
             }
-            gpre.push_back(acc);
-            g->ngroups.push_back(static_cast<int>(groups.size() - first));
         }
-        size_t corder = 0;
-        for (size_t bi = 0; bi < batches_.size(); ++bi) {
-            if (g->batch_order[bi]) {
-                corder = std::max(corder, static_cast<size_t>(g->ngroups[bi]) * g->batch_maxm[bi]);
-            }
-        }
-        g->corder.reset(std::max<size_t>(1, corder) * sizeof(int));
-        g->groups.reset(std::max<size_t>(1, groups.size()) * sizeof(CountGroup));
-        if (!groups.empty()) {
-            NSG_CUDA(cudaMemcpy(g->groups.get(), groups.data(), groups.size() * sizeof(CountGroup),
-                                cudaMemcpyHostToDevice));
-        }
-        g->gprefix.reset(gpre.size() * sizeof(int));
-        NSG_CUDA(cudaMemcpy(g->gprefix.get(), gpre.data(), gpre.size() * sizeof(int), cudaMemcpyHostToDevice));
+        auto upload = [](DeviceBuffer& dst, const auto& v) {
+            if (v.empty()) return;
+            dst.reset(v.size() * sizeof(v[0]));
+            NSG_CUDA(cudaMemcpy(dst.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+        };
+        g->corder.reset(corder * sizeof(int));
+        g->rank_emax.reset(emax * sizeof(float));
+        upload(g->groups, groups);
+        upload(g->gprefix, gpre);
+        upload(g->ranks, ranks);
+        upload(g->rprefix, rpre);
+        upload(g->refs, refs);
     }
     g->gps.reset(gps.size() * sizeof(GridPair));
     NSG_CUDA(cudaMemcpy(g->gps.get(), gps.data(), gps.size() * sizeof(GridPair), cudaMemcpyHostToDevice));
@@ -756,15 +779,17 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
     GridState& g = *grid_;
     NSG_CUDA(cudaMemsetAsync(g.evals.get(), 0, 3 * sizeof(unsigned long long), s));
     grid_launch_gather(gather_rows_.as<GatherRow>(), ngather_, d_, fault_.as<int>(), s);
-    grid_launch_nodes(g.nodes.as<GridNode>(), g.nnodes, d_, g.node_est, s);
+    grid_launch_nodes(g.nodes.as<GridNode>(), g.nnodes, d_, g.split_nodes, s);
+    if (g.node_est) bits_launch_est(g.nodes.as<GridNode>(), g.nnodes, g.max_m, d_, s);
     for (size_t bi = 0; bi < batches_.size(); ++bi) {
         const Batch& b = batches_[bi];
         int* ctr = counters_.as<int>() + kCounters * bi;
         KsgPairDesc* bp = pairs_dev_.as<KsgPairDesc>() + b.pair0;
         GridPair* bg = g.gps.as<GridPair>() + b.pair0;
         const bool order = g.batch_order[bi] != 0;
+        const BitsConfig& bits = g.batch_bits[bi];
         const int search_order =
-            grid_launch_pairs(bp, bg, g.nodes.as<GridNode>(), b.npairs, g.batch_maxm[bi], d_, order, s);
+            bits.ok ? 0 : grid_launch_pairs(bp, bg, g.nodes.as<GridNode>(), b.npairs, g.batch_maxm[bi], d_, order, s);
         GridArgs a{};
         a.search_order = search_order;
         a.pairs = bp;
@@ -774,6 +799,13 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         a.groups = g.groups.as<CountGroup>() + g.group_off[bi];
         a.gprefix = g.gprefix.as<int>() + g.gprefix_off[bi];
         a.ngroups = g.ngroups[bi];
+        a.ranks = g.ranks.as<RankNode>() + g.rank_off[bi];
+        a.rprefix = g.rprefix.as<int>() + g.rprefix_off[bi];
+        a.refs = g.refs.as<long long>() + g.ref_off[bi];
+        a.nranks = g.nranks[bi];
+        a.rank_items = g.rank_items[bi];
+        a.rank_emax = order ? g.rank_emax.as<float>() : nullptr;
+        a.rank_ld = g.batch_maxm[bi];
         a.npairs = b.npairs;
         a.pair_base = b.pair0;
         a.k = k_;
@@ -794,7 +826,11 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         a.corder_ld = g.batch_maxm[bi];
         cudaEvent_t* ev = events_.data() + kEventsPerBatch * bi;
         if (timing_) record_event(ev[0], s);
-        grid_launch_search(a, d_, kmax_, g.search_grid, bootstrap_, s);
+        if (bits.ok) {
+            bits_launch_search(a, bits, g.batch_maxm[bi], d_, s);
+        } else {
+            grid_launch_search(a, d_, kmax_, g.search_grid, bootstrap_, s);
+        }
         if (timing_) record_event(ev[1], s);
         a.counter = ctr + 1;
         const GridArgs c = grid_launch_count_order(a, s);
@@ -841,13 +877,19 @@ int KsgPlan::launches() const {
     const int nb = static_cast<int>(batches_.size());
     if (search_ != 1) return 3 * nb;
     if (!nb) return 0;
-    // node grids (+ scale estimates), gather; per batch: pair grids, search,
-    // counts, combine, ties, final sums (+ search and count orders)
-    int n = 1 + (ngather_ ? 1 : 0) + 6 * nb;
+    // node grids (+ scale estimates), gather; per batch: search, combine,
+    // ties, final sums, group and rank counts (+ pair grids where the search
+    // scans them; in batches with orders + search order, count order, the
+    // rank nodes' largest eps)
+    int n = 1 + (ngather_ ? 1 : 0) + 4 * nb;
     if (grid_) {
+        if (grid_->split_nodes) n += 2;
         if (grid_->node_est) ++n;
         for (size_t bi = 0; bi < grid_->batch_order.size(); ++bi) {
-            if (grid_->batch_order[bi] && grid_->batch_maxm[bi] <= kOrderMaxM) n += 2;
+            const bool order = grid_->batch_order[bi] != 0, short_m = grid_->batch_maxm[bi] <= kOrderMaxM;
+            if (!grid_->batch_bits[bi].ok) n += order && short_m ? 2 : 1;
+            if (grid_->ngroups[bi]) n += order && short_m ? 2 : 1;
+            if (grid_->nranks[bi]) n += order ? 2 : 1;
         }
     }
     return n;

@@ -1,0 +1,116 @@
+// Instantiations and launch of the bitmap search (ksg_bits.cuh).
+#include "ksg_bits.cuh"
+
+#include <algorithm>
+
+#include "engine.h"
+#include "errors.h"
+
+namespace nsg {
+
+BitsConfig bits_config(int d, int k, int max_m) {
+    BitsConfig c;
+    if (d < 1 || d > 3 || max_m < 1 || max_m > kBitMaxM) return c;
+    // Shared memory of an SM, and what a CTA takes beside its dynamic part.
+    constexpr size_t kSm = 228 << 10, kStatic = 2048, kReserved = 1024;
+    const int nc = 2 * d - 1, ws = bit_row_words(max_m);
+    c.keep = k <= 12 ? 1 : 3;
+    c.perm_words = ((max_m + 1) / 2 + 3) & ~3;
+    auto fits = [&](int step, int threads, int ctas) {
+        c.step = step;
+        c.threads = threads;
+        c.ctas_per_sm = ctas;
+        c.rows = (kBitBins + step - 1) / step + 1;
+        c.rows_words = nc * c.rows * ws;
+        c.smem = sizeof(unsigned) * (static_cast<size_t>(c.rows_words) + c.perm_words +
+                                     static_cast<size_t>(threads / 32) * bit_warp_words(d, c.keep));
+        c.ok = ctas * (c.smem + kStatic + kReserved) <= kSm;
+        return c.ok;
+    };
+    // two bins per row, as many CTAs per SM as fit (1024 threads in all)
+    for (int n : {8, 4, 2, 1}) {
+        if (fits(2, 1024 / n, n)) return c;
+    }
+    // long rows or lists: fewer warps, then four and six bins per row (wider
+    // intervals, more candidates)
+    for (int step : {2, 4, 6}) {
+        for (int threads : {1024, 768, 512}) {
+            if (fits(step, threads, 1)) return c;
+        }
+    }
+    return c;
+}
+
+namespace {
+
+template <int D, int N>
+void launch(const BitsArgs& a, const BitsConfig& c, int grid, cudaStream_t s) {
+    // set on every launch: the attribute belongs to the current device
+    NSG_CUDA(cudaFuncSetAttribute(ksg_bits_search_kernel<D, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(c.smem)));
+    ksg_bits_search_kernel<D, N><<<grid, c.threads, c.smem, s>>>(a);
+    NSG_CUDA(cudaGetLastError());
+}
+
+template <int D>
+void launch(const BitsArgs& a, const BitsConfig& c, int grid, cudaStream_t s) {
+    if (c.keep == 1) launch<D, 1>(a, c, grid, s);
+    else launch<D, 3>(a, c, grid, s);
+}
+
+}  // namespace
+
+void bits_launch_est(const GridNode* nodes, int nnodes, int max_m, int d, cudaStream_t s) {
+    if (nnodes <= 0) return;
+    max_m = std::min(max_m, kBitMaxM);  // longer nodes take neither bitmaps nor orders (kOrderMaxM)
+    const size_t most = 200 << 10;
+    int step = 1;
+    size_t smem = 0;
+    for (;; step *= 2) {
+        smem = sizeof(unsigned) * (d - 1) * ((kBitBins + step - 1) / step + 1) * static_cast<size_t>(bit_row_words(max_m));
+        if (smem <= most) break;
+    }
+    // a node's frames split over CTAs until there are two per SM
+    const int parts = std::max(1, std::min((2 * sm_count() + nnodes - 1) / nnodes, max_m / 256));
+    const dim3 grid(nnodes, parts);
+    switch (d) {
+        case 1: bits_est_kernel<1><<<grid, kEstThreads, 0, s>>>(nodes, step); break;
+        case 2:
+            NSG_CUDA(cudaFuncSetAttribute(bits_est_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(most)));
+            bits_est_kernel<2><<<grid, kEstThreads, smem, s>>>(nodes, step);
+            break;
+        case 3:
+            NSG_CUDA(cudaFuncSetAttribute(bits_est_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(most)));
+            bits_est_kernel<3><<<grid, kEstThreads, smem, s>>>(nodes, step);
+            break;
+        default: invalid("d must be 1, 2 or 3");
+    }
+    NSG_CUDA(cudaGetLastError());
+}
+
+void bits_launch_search(const GridArgs& g, const BitsConfig& c, int max_m, int d, cudaStream_t s) {
+    if (g.npairs <= 0) return;
+    BitsArgs a{};
+    a.g = g;
+    a.rows = c.rows;
+    a.step = c.step;
+    a.rows_words = c.rows_words;
+    a.perm_words = c.perm_words;
+    // Pairs are split while there are fewer than four items per resident CTA:
+    // every share builds the pair's rows again.
+    const int slots = sm_count() * c.ctas_per_sm;
+    const int most = std::max(1, max_m / (2 * (c.threads / 32)));
+    a.chunks = g.npairs >= 4 * slots ? 1 : std::min(most, (4 * slots + g.npairs - 1) / g.npairs);
+    const long long items = static_cast<long long>(g.npairs) * a.chunks;
+    const int grid = static_cast<int>(std::min<long long>(items, slots));
+    switch (d) {
+        case 1: launch<1>(a, c, grid, s); break;
+        case 2: launch<2>(a, c, grid, s); break;
+        case 3: launch<3>(a, c, grid, s); break;
+        default: invalid("d must be 1, 2 or 3");
+    }
+}
+
+}  // namespace nsg

@@ -1,0 +1,706 @@
+// KSG joint search on rank bitmaps: the same results as the other searches,
+// one warp per query, 32 frames per logic instruction.
+//
+// Every frame a query accepts lies within U (its k-th distance) of it in
+// each of the 2d coordinates. Each node splits every coordinate's range at
+// kBitBins - 1 quantile edges; for a pair, row t of a coordinate is the
+// bitmap of the frames whose bin is below t. The frames that may lie within h
+// of the query in that coordinate are then row[hi + 1] ^ row[lo], with lo and
+// hi the first and last bin the interval can reach (exact: rounding is
+// monotone, see ksg_grid.cuh), and the AND over the coordinates leaves the few
+// frames that can lie within h in all of them: at m = 10000, d = 3, about 12
+// for h = U and 25 to 45 for the h used. Only those are evaluated.
+//
+//   * Rows of a pair live in shared memory, over the frames in the order of
+//     node a's bins of its widest coordinate, so that coordinate needs no
+//     rows: its interval is a range of words (a third of them, typically).
+//     One CTA owns one pair at a time (or a share of its queries) and builds
+//     the rows with ballots: 2% of its time at m = 10000.
+//   * A warp takes a few queries at a time: one lane per query and
+//     coordinate finds the bins its interval reaches. Then, query by query,
+//     each lane ANDs four (or eight) words of 2d - 1 row pairs, finds the set
+//     bit of its rank, and evaluates that frame exactly (one 16-byte gather
+//     per node); the frames within h are listed in shared memory with their
+//     distances. A lane per listed frame counts the smaller distances;
+//     the frames with at most k smaller ones are the query and its k nearest
+//     (and whatever ties with the k-th), and warp reductions over them give
+//     the k-th distance, eps and the tie test.
+//   * h comes from the two nodes' scale estimates: sqrt(est_a est_b) follows
+//     the k-th joint distance with a spread of 8 to 14%. Each warp scales it
+//     so that about one query in ten finds fewer than k frames within h and
+//     tries again with a larger h; whatever h is, the accepted set is complete
+//     (every frame within h was evaluated, and at least k others were).
+//   * A full list of frames within h gives a smaller h, its own k-th distance.
+//     Queries that do not settle (heavy ties, no usable estimate, non-finite
+//     coordinates) scan all frames (scan_all).
+//
+// Ties come out exactly: all frames at the k-th distance are among those
+// evaluated. What bounds the kernel: the shared-memory and gather traffic of
+// a query (about 40 + 50 wavefronts) beside about 300 instructions; the scan
+// it replaces spent about 2000 per query at m = 10000.
+#pragma once
+
+#include "common.cuh"
+#include "ksg.cuh"
+#include "ksg_bits.h"
+#include "ksg_grid.h"
+
+namespace nsg {
+namespace bitk {
+
+constexpr unsigned kFull = 0xffffffffu;
+
+__device__ __forceinline__ float inf_f() { return __int_as_float(0x7f800000); }
+
+template <int D>
+__device__ __forceinline__ float dist(const float (&q)[D], const float (&x)[D]) {
+    if constexpr (D == 1) return fabsf(q[0] - x[0]);
+    else if constexpr (D == 2) return fmaxf(fabsf(q[0] - x[0]), fabsf(q[1] - x[1]));
+    else return nsg_max3(fabsf(q[0] - x[0]), fabsf(q[1] - x[1]), fabsf(q[2] - x[2]));
+}
+
+// Frame j of a node's coordinates as stored by the node kernel (1, 2 or 4
+// floats per frame).
+template <int D>
+__device__ __forceinline__ void load_frame(const float* __restrict__ aos, int j, float (&x)[D]) {
+    if constexpr (D == 1) {
+        x[0] = __ldg(aos + j);
+    } else if constexpr (D == 2) {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(aos) + j);
+        x[0] = v.x;
+        x[1] = v.y;
+    } else {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(aos) + j);
+        x[0] = v.x;
+        x[1] = v.y;
+        x[2] = v.z;
+    }
+}
+
+struct Found {
+    float ea, eb, wk;
+    bool tie;  // frames at wk with different marginals: the reference's order decides
+};
+
+// The first part of [q - h, q + h] and one past its last among the parts
+// that 63 ascending edges e (padded with +inf) cut an axis into.
+__device__ __forceinline__ void reach(const float* e, float q, float h, int& lo, int& hi) {
+    lo = hi = 0;
+#pragma unroll
+    for (int s = 32; s > 0; s >>= 1) {
+        if (__fsub_rn(q, e[lo + s - 1]) > h) lo += s;
+        if (__fsub_rn(e[hi + s - 1], q) <= h) hi += s;
+    }
+    ++hi;
+}
+
+// Inclusive prefix sum over the lanes.
+__device__ __forceinline__ int lane_prefix(int v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+            "shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t"
+            "@p add.s32 %0, %0, t;\n\t}"
+            : "+r"(v)
+            : "r"(o));
+    }
+    return v;
+}
+
+// Position of the bit of rank win + lane among the set bits of the lanes'
+// words (lane order, then word order): word g of a lane covers positions
+// base + 32 g for g < 4 and base + 4096 + 32 (g - 4) above. off: set bits of
+// the lanes before; cnt: of this lane; table: 32 words of shared memory.
+// Lanes whose rank does not exist get an arbitrary position.
+template <int W>
+__device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int off, int cnt, int win, int lane,
+                                           unsigned* table) {
+    // lanes with a bit in the window, in order, and where their bits start in it
+    const int first = off - win;
+    const bool here = cnt > 0 && first < 32 && first + cnt > 0;
+    const unsigned owners = __ballot_sync(kFull, here);
+    const unsigned starts = __reduce_or_sync(kFull, here ? 1u << max(first, 0) : 0u);
+    if (here) table[__popc(owners & ((1u << lane) - 1u))] = static_cast<unsigned>(lane);
+    __syncwarp();
+    const int src = static_cast<int>(table[__popc(starts & (kFull >> (31 - lane))) - 1] & 31u);
+    int r = win + lane - __shfl_sync(kFull, off, src);  // rank within the owner's words
+    unsigned bits = 0;
+    int pos = __shfl_sync(kFull, base, src);
+#pragma unroll
+    for (int g = 0; g < W; ++g) {
+        const unsigned x = __shfl_sync(kFull, w[g], src);
+        const int c = __popc(x);
+        if (g == W - 1 || r < c) {
+            if (bits == 0) {
+                bits = x;
+                pos += 32 * (g & 3) + (g >> 2) * 4096;
+            }
+        }
+        if (bits == 0) r -= c;
+    }
+    for (; r > 0; --r) bits &= bits - 1;
+    __syncwarp();
+    return pos + __ffs(bits) - 1;
+}
+
+// Rows of one coordinate for frames 32 w .. 32 w + 31 (one bin per lane,
+// above every bin where there is no frame): lane t keeps the ballot of row t.
+__device__ __forceinline__ void build_rows(unsigned* rows, int WS, int w, int R, int step, unsigned bin, int lane) {
+    for (int r0 = 0; r0 < R; r0 += 32) {
+        unsigned mine = 0;
+        const int top = min(32, R - r0);
+        for (int t = 0; t < top; ++t) {
+            const unsigned x = __ballot_sync(kFull, bin < static_cast<unsigned>(min((r0 + t) * step, kBitBins)));
+            if (lane == t) mine = x;
+        }
+        if (lane < top) rows[(r0 + lane) * WS + w] = mine;
+    }
+}
+
+// (k+1)-th smallest key over the lanes (at least k + 1 of them below kFull).
+__device__ __forceinline__ unsigned kth_lane(unsigned u, int k) {
+    unsigned last = 0;
+    int cnt = 0;
+    for (;;) {
+        const unsigned mn = __reduce_min_sync(kFull, u > last || cnt == 0 ? u : kFull);
+        cnt += __popc(__ballot_sync(kFull, u == mn));
+        if (cnt > k || mn == kFull) return mn;
+        last = mn;
+    }
+}
+
+// From the first n listed frames within h (n <= 32 N, n > k): the (k+1)-th
+// smallest distance (the query itself is listed, at distance 0), eps over
+// the frames at or below it, and whether frames beyond the k-th tie with it.
+// Lane i of part c counts the distances smaller than that of entry 32 c + i;
+// v holds +inf up to the next multiple of four entries.
+template <int N>
+__device__ __forceinline__ Found select_nearest(const float* v, const float* da, const float* db, int n, int k, int lane) {
+    float x[N];
+    int less[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        x[c] = 32 * c + lane < n ? v[32 * c + lane] : inf_f();
+        less[c] = 0;
+    }
+    for (int t = 0; t < n; t += 4) {
+        const float4 y = *reinterpret_cast<const float4*>(v + t);
+#pragma unroll
+        for (int c = 0; c < N; ++c)
+            less[c] += (y.x < x[c]) + (y.y < x[c]) + (y.z < x[c]) + (y.w < x[c]);
+    }
+    unsigned wk = 0, ea = 0, eb = 0;
+    int le = 0;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        const bool in = 32 * c + lane < n && less[c] <= k;
+        le += __popc(__ballot_sync(kFull, in));
+        if (in) {
+            wk = max(wk, __float_as_uint(x[c]));
+            ea = max(ea, __float_as_uint(da[32 * c + lane]));
+            eb = max(eb, __float_as_uint(db[32 * c + lane]));
+        }
+    }
+    Found r;
+    wk = __reduce_max_sync(kFull, wk);
+    r.wk = __uint_as_float(wk);
+    r.ea = __uint_as_float(__reduce_max_sync(kFull, ea));
+    r.eb = __uint_as_float(__reduce_max_sync(kFull, eb));
+    r.tie = false;
+    if (le > k + 1 && wk != 0) {
+        unsigned alo = kFull, ahi = 0, blo = kFull, bhi = 0;
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            if (32 * c + lane >= n || __float_as_uint(x[c]) != wk) continue;
+            const unsigned a = __float_as_uint(da[32 * c + lane]), b = __float_as_uint(db[32 * c + lane]);
+            alo = min(alo, a);
+            ahi = max(ahi, a);
+            blo = min(blo, b);
+            bhi = max(bhi, b);
+        }
+        alo = __reduce_min_sync(kFull, alo);
+        ahi = __reduce_max_sync(kFull, ahi);
+        blo = __reduce_min_sync(kFull, blo);
+        bhi = __reduce_max_sync(kFull, bhi);
+        r.tie = alo != ahi || blo != bhi;
+    }
+    return r;
+}
+
+// Keeps the entries that are not beyond the (k+1)-th smallest (n > k) and
+// returns how many; *wk is that distance.
+template <int N>
+__device__ __forceinline__ int keep_nearest(float* v, float* da, float* db, int n, int k, int lane, float* wk) {
+    if (lane < 4) v[n + lane] = inf_f();
+    __syncwarp();
+    const float w = select_nearest<N>(v, da, db, n, k, lane).wk;
+    int kept = 0;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        const int t = 32 * c + lane;
+        const bool in = t < n && v[t] <= w;
+        const float x = in ? v[t] : 0.f, a = in ? da[t] : 0.f, b = in ? db[t] : 0.f;
+        const unsigned mask = __ballot_sync(kFull, in);
+        __syncwarp();
+        if (in) {
+            const int to = kept + __popc(mask & ((1u << lane) - 1u));
+            v[to] = x;
+            da[to] = a;
+            db[to] = b;
+        }
+        kept += __popc(mask);
+        __syncwarp();
+    }
+    *wk = w;
+    return kept;
+}
+
+// The same over all m frames: the k + 1 smallest distances in a list spread
+// over the lanes (two entries each), then a second pass for eps and ties.
+template <int D>
+__device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float* __restrict__ xb, int m, int k,
+                                       int query, int lane) {
+    float qa[D], qb[D];
+    load_frame<D>(xa, query, qa);
+    load_frame<D>(xb, query, qb);
+    float l0 = inf_f(), l1 = inf_f();
+    float U = inf_f();
+    for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + lane;
+        float v = inf_f();
+        if (j < m) {
+            float a[D], b[D];
+            load_frame<D>(xa, j, a);
+            load_frame<D>(xb, j, b);
+            v = fmaxf(dist<D>(qa, a), dist<D>(qb, b));
+        }
+        unsigned todo = __ballot_sync(kFull, v < U);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const float x = __shfl_sync(kFull, v, src);
+            float p0 = __shfl_up_sync(kFull, l0, 1), p1 = __shfl_up_sync(kFull, l1, 1);
+            const float top = __shfl_sync(kFull, l0, 31);
+            if (lane == 0) {
+                p0 = -inf_f();
+                p1 = top;
+            }
+            if (l0 > x) l0 = fmaxf(p0, x);
+            if (l1 > x) l1 = fmaxf(p1, x);
+        }
+        U = k < 32 ? __shfl_sync(kFull, l0, k) : __shfl_sync(kFull, l1, k - 32);
+    }
+    float ea = 0.f, eb = 0.f, alo = inf_f(), ahi = -1.f, blo = inf_f(), bhi = -1.f;
+    int le = 0;
+    for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + lane;
+        if (j >= m) break;
+        float a[D], b[D];
+        load_frame<D>(xa, j, a);
+        load_frame<D>(xb, j, b);
+        const float da = dist<D>(qa, a), db = dist<D>(qb, b), v = fmaxf(da, db);
+        if (v <= U) {
+            ++le;
+            ea = fmaxf(ea, da);
+            eb = fmaxf(eb, db);
+        }
+        if (v == U) {
+            alo = fminf(alo, da);
+            ahi = fmaxf(ahi, da);
+            blo = fminf(blo, db);
+            bhi = fmaxf(bhi, db);
+        }
+    }
+    le = __reduce_add_sync(kFull, le);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ea = fmaxf(ea, __shfl_xor_sync(kFull, ea, o));
+        eb = fmaxf(eb, __shfl_xor_sync(kFull, eb, o));
+        alo = fminf(alo, __shfl_xor_sync(kFull, alo, o));
+        ahi = fmaxf(ahi, __shfl_xor_sync(kFull, ahi, o));
+        blo = fminf(blo, __shfl_xor_sync(kFull, blo, o));
+        bhi = fmaxf(bhi, __shfl_xor_sync(kFull, bhi, o));
+    }
+    return Found{ea, eb, U, le > k + 1 && U > 0.f && (alo != ahi || blo != bhi)};
+}
+
+}  // namespace bitk
+
+// A work item is a pair and a share of its queries (B.chunks shares per
+// pair). Dynamic shared memory: rows, node a's frame order, then per warp its
+// queries, their bins and the two lists (bits_config sizes it for the batch's
+// largest m). Up to 32 N frames within h are kept.
+template <int D, int N>
+__global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
+    using namespace bitk;
+    const GridArgs& A = B.g;
+    constexpr int NC = 2 * D - 1;  // coordinates with rows: a's other D - 1, b's D
+    constexpr int Q = bit_queries(D);
+    constexpr int kKeep = 32 * N;
+    extern __shared__ __align__(16) unsigned s_dyn[];
+    __shared__ int s_start[64];
+    __shared__ float s_edge[2 * D][65];
+    __shared__ int s_item, s_next;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int nwarps = blockDim.x >> 5;
+    unsigned short* s_perm = reinterpret_cast<unsigned short*>(s_dyn + B.rows_words);
+    float* s_query = reinterpret_cast<float*>(s_dyn + B.rows_words + B.perm_words) + wid * bit_warp_words(D, N);
+    float* s_v = s_query + Q * 8;                  // distances within h, +inf up to a multiple of four
+    float* s_da = s_v + kKeep + 4;
+    float* s_db = s_da + kKeep;
+    unsigned* s_bins = reinterpret_cast<unsigned*>(s_db + kKeep);
+    unsigned* s_table = s_bins + Q * 2 * D;
+    const int R = B.rows, step = B.step, k = A.k;
+    int cur_a = -1;
+    float scale = 1.f;               // this warp's share in h, see the file comment
+    unsigned long long evals = 0;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) {
+            s_item = atomicAdd(A.counter, 1);
+            s_next = 0;
+        }
+        __syncthreads();
+        const int item = s_item;
+        if (item >= A.npairs * B.chunks) break;
+        const int p = item / B.chunks, ch = item - p * B.chunks;
+        const KsgPairDesc* P = A.pairs + p;
+        const int m = P->m;
+        const int share = ((m + B.chunks - 1) / B.chunks + Q - 1) / Q * Q;
+        const int qlo = ch * share, qhi = min(m, qlo + share);
+        if (qlo >= qhi) continue;
+        const int na_id = A.gp[p].a, nb_id = A.gp[p].b;
+        const GridNode* na = A.nodes + na_id;
+        const GridNode* nb = A.nodes + nb_id;
+        const float* __restrict__ xa = na->aos;
+        const float* __restrict__ xb = nb->aos;
+        const int WS = bit_row_words(m);
+        const bool new_a = na_id != cur_a;
+        cur_a = na_id;
+        if (new_a) {
+            for (int q = tid; q < m; q += blockDim.x) s_perm[q] = __ldg(na->order + q);
+            if (tid < 64) s_start[tid] = __ldg(na->ostart + tid);
+            __syncthreads();
+        }
+        // the edges between whole steps of bins (the first coordinate's: all)
+        for (int e = tid; e < 128 * D; e += blockDim.x) {
+            const int c = e >> 6, t = ((e & 63) + 1) * (c == 0 ? 1 : step);
+            const float* edges = c < D ? na->bedges + c * 64 : nb->bedges + (c - D) * 64;
+            s_edge[c][e & 63] = t < kBitBins ? __ldg(edges + t) : inf_f();
+        }
+        // rows: lane t keeps the ballot of row t
+        {
+            const unsigned* __restrict__ ba = na->bins;
+            const unsigned* __restrict__ bb = nb->bins;
+            for (int w = wid; w < WS; w += nwarps) {
+                const int pos = 32 * w + lane;
+                unsigned va = kFull, vb = kFull;
+                if (pos < m) {
+                    const int j = s_perm[pos];
+                    if (D > 1 && new_a) va = __ldg(ba + j);
+                    vb = __ldg(bb + j);
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (c < D - 1 && !new_a) continue;
+                    const unsigned bin = c < D - 1 ? (va >> (8 * (c + 1)) & 0xffu) : (vb >> (8 * (c - (D - 1))) & 0xffu);
+                    build_rows(s_dyn + c * R * WS, WS, w, R, step, bin, lane);
+                }
+            }
+        }
+        const bool bad = __ldg(na->ostart + 63) != 0 || __ldg(nb->ostart + 63) != 0;
+        // ratio of the k-th joint distance to the geometric mean of the scale
+        // estimates for independent nodes of uniform density; scale follows the rest
+        const float rank = est_rank(m);
+        const float base = exp2f(__log2f(static_cast<float>(k) * m / (rank * rank)) * (0.5f / D) + 0.3f);
+        __syncthreads();
+        const uint4* rows = reinterpret_cast<const uint4*>(s_dyn);
+        // bins of coordinate c of query t, packed: c = 0 the range of uint4
+        // columns, else the offsets of its two rows (in uint4)
+        auto set_bins = [&](int t, int c) {
+            int lo, hi;
+            reach(s_edge[c], s_query[8 * t + (c < D ? c : 4 + c - D)], s_query[8 * t + 3], lo, hi);
+            if (c == 0) {
+                lo = s_start[lo] >> 7;
+                hi = (s_start[hi] + 127) >> 7;
+            } else {
+                lo = ((c - 1) * R + lo) * (WS / 4);
+                hi = ((c - 1) * R + hi) * (WS / 4);
+            }
+            s_bins[2 * D * t + c] = static_cast<unsigned>(hi) << 16 | static_cast<unsigned>(lo);
+        };
+        for (;;) {
+            int q0 = 0;
+            if (lane == 0) q0 = atomicAdd(&s_next, Q);
+            q0 = __shfl_sync(kFull, q0, 0) + qlo;
+            if (q0 >= qhi) break;
+            const int nq = min(Q, qhi - q0);
+            __syncwarp();
+            if (lane < 2 * Q && lane % Q < nq) {
+                const int t = lane % Q, i = q0 + t;
+                float x[D];
+                load_frame<D>(lane < Q ? xa : xb, i, x);
+                float* dst = s_query + 8 * t + (lane < Q ? 0 : 4);
+#pragma unroll
+                for (int c = 0; c < D; ++c) dst[c] = x[c];
+                if (lane < Q) dst[3] = sqrtf(__ldg(na->est + i) * __ldg(nb->est + i)) * (base * scale);
+            }
+            __syncwarp();
+            if (lane < 2 * D * nq) set_bins(lane / (2 * D), lane % (2 * D));
+            __syncwarp();
+            float ra = 0.f, rb = 0.f, rw = 0.f;  // lane t keeps query t's results
+            unsigned tmask = 0;
+            for (int t = 0; t < nq; ++t) {
+                const float4 fa = *reinterpret_cast<const float4*>(s_query + 8 * t);
+                const float4 fb = *reinterpret_cast<const float4*>(s_query + 8 * t + 4);
+                float qa[D], qb[D];
+                qa[0] = fa.x;
+                qb[0] = fb.x;
+                if constexpr (D > 1) {
+                    qa[1] = fa.y;
+                    qb[1] = fb.y;
+                }
+                if constexpr (D > 2) {
+                    qa[2] = fa.z;
+                    qb[2] = fb.z;
+                }
+                float h = fa.w;
+                Found r;
+                bool done = false;
+                for (int tries = 0; tries < kBitTries && !bad && h > 0.f && h < 1e30f; ++tries) {
+                    const unsigned* bins = s_bins + 2 * D * t;
+                    const int x0 = bins[0] & 0xffffu, x1 = bins[0] >> 16;
+                    int inside = 0;
+                    bool stuck = false;
+                    // the AND of the row pairs over one uint4 column
+                    auto column = [&](int x) {
+                        uint4 acc = make_uint4(0, 0, 0, 0);
+                        if (x < x1) {
+#pragma unroll
+                            for (int c = 0; c < NC; ++c) {
+                                const unsigned o = bins[c + 1];
+                                const uint4 u = rows[(o >> 16) + x];
+                                const uint4 v = rows[(o & 0xffffu) + x];
+                                if (c == 0) {
+                                    acc = make_uint4(u.x ^ v.x, u.y ^ v.y, u.z ^ v.z, u.w ^ v.w);
+                                } else {
+                                    acc.x &= u.x ^ v.x;
+                                    acc.y &= u.y ^ v.y;
+                                    acc.z &= u.z ^ v.z;
+                                    acc.w &= u.w ^ v.w;
+                                }
+                            }
+                        }
+                        return acc;
+                    };
+                    // Evaluates the frames of the set bits, 32 at a time; false: too many ties.
+                    auto consume = [&](auto& w, int base, int cnt, bool last) {
+                        const int incl = lane_prefix(cnt);
+                        const int n = __shfl_sync(kFull, incl, 31);
+                        if (last && inside + n <= k) {  // too few whatever their distances
+                            inside += n;
+                            return true;
+                        }
+                        evals += n;
+                        for (int win = 0; win < n; win += 32) {
+                            const int pos = bit_of_rank(w, base, incl - cnt, cnt, win, lane, s_table);
+                            float da = 0.f, db = 0.f, v = inf_f();
+                            if (win + lane < n) {
+                                const int j = s_perm[pos];
+                                float a[D], b[D];
+                                load_frame<D>(xa, j, a);
+                                load_frame<D>(xb, j, b);
+                                da = dist<D>(qa, a);
+                                db = dist<D>(qb, b);
+                                v = fmaxf(da, db);
+                            }
+                            unsigned in = __ballot_sync(kFull, v <= h);
+                            if (inside + __popc(in) > kKeep) {
+                                // k others lie within a smaller h
+                                if (inside > k) inside = keep_nearest<N>(s_v, s_da, s_db, inside, k, lane, &h);
+                                else h = __uint_as_float(kth_lane(v <= h ? __float_as_uint(v) : kFull, k));
+                                in = __ballot_sync(kFull, v <= h);
+                                if (inside + __popc(in) > kKeep) return false;
+                            }
+                            if (v <= h) {
+                                const int slot = inside + __popc(in & ((1u << lane) - 1u));
+                                s_v[slot] = v;
+                                s_da[slot] = da;
+                                s_db[slot] = db;
+                            }
+                            inside += __popc(in);
+                            __syncwarp();
+                        }
+                        return true;
+                    };
+                    for (int xf = x0; xf < x1 && !stuck; xf += 64) {
+                        const int x = xf + lane;
+                        const uint4 u = column(x);
+                        if (xf + 32 >= x1) {
+                            const unsigned w[4] = {u.x, u.y, u.z, u.w};
+                            const int cnt = __popc(u.x) + __popc(u.y) + __popc(u.z) + __popc(u.w);
+                            stuck = !consume(w, 128 * x, cnt, true);
+                        } else {
+                            const uint4 v = column(x + 32);
+                            const unsigned w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                            int cnt = 0;
+#pragma unroll
+                            for (int g = 0; g < 8; ++g) cnt += __popc(w[g]);
+                            stuck = !consume(w, 128 * x, cnt, xf + 64 >= x1);
+                        }
+                    }
+                    if (stuck) break;
+                    if (inside > k) {
+                        if (lane < 4) s_v[inside + lane] = inf_f();
+                        __syncwarp();
+                        r = select_nearest<N>(s_v, s_da, s_db, inside, k, lane);
+                        __syncwarp();
+                        if (tries == 0) scale *= 0.995f;
+                        done = true;
+                        break;
+                    }
+                    if (tries == 0) scale *= 1.05f;
+                    h *= fminf(2.f, exp2f(__log2f(2.f * (k + 1) / (inside + 0.5f)) * (0.5f / D)));
+                    if (lane == 0) s_query[8 * t + 3] = h;
+                    __syncwarp();
+                    if (lane < 2 * D) set_bins(t, lane);
+                    __syncwarp();
+                }
+                if (!done) {
+                    r = scan_all<D>(xa, xb, m, k, q0 + t, lane);
+                    evals += m;
+                }
+                if (lane == t) {
+                    ra = r.ea;
+                    rb = r.eb;
+                    rw = r.wk;
+                }
+                if (r.tie) tmask |= 1u << t;
+            }
+            if (lane < nq) {
+                const long long o = P->scratch + q0 + lane;
+                A.eps_a[o] = ra;
+                A.eps_b[o] = rb;
+                if (A.eps_x) A.eps_x[o] = ra;
+                if (A.eps_y) A.eps_y[o] = rb;
+                if (A.kdist) A.kdist[o] = rw;
+            }
+            if (tmask) {
+                // tied samples of the block take consecutive slots of the tie list
+                int slot = 0;
+                if (lane == 0) slot = atomicAdd(A.tie_count, __popc(tmask));
+                slot = __shfl_sync(kFull, slot, 0);
+                if (tmask >> lane & 1u) {
+                    slot += __popc(tmask & ((1u << lane) - 1u));
+                    if (slot < A.tie_cap) A.ties[slot] = KsgTie{A.pair_base + p, q0 + lane};
+                    else atomicOr(A.fault, FAULT_TIE_OVERFLOW);
+                }
+            }
+        }
+    }
+    if (A.evals && lane == 0 && evals) atomicAdd(A.evals, evals);
+}
+
+// Scale estimates of one node's frames (GridNode::est), a share of them per
+// CTA (blockIdx.y). The width of the bins around a frame gives each
+// coordinate's density, and their product a first radius that would hold
+// R = est_rank(m) frames if the coordinates were independent; the frames
+// within that radius, counted on the node's own rows (in whole bins and
+// words: a few percent of the radius), correct it. With one coordinate the
+// density alone is the estimate. In a CPU model of m = 10000 trajectories the
+// geometric mean of two nodes' estimates follows the k-th joint distance to
+// 8% (nearly independent coordinates) and 12% (correlated ones), as well as
+// the exact 64th-neighbour distances do.
+constexpr int kEstThreads = 512;
+
+template <int D>
+__global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* nodes, int step) {
+    using namespace bitk;
+    extern __shared__ __align__(16) unsigned s_dyn[];
+    __shared__ float s_edge[D][65];
+    __shared__ float s_whole[D][64];
+    __shared__ int s_start[64];
+    const GridNode nd = nodes[blockIdx.x];
+    const int m = nd.m;
+    if (m > kBitMaxM) return;
+    const int share = (m + gridDim.y - 1) / gridDim.y;
+    const int lo = blockIdx.y * share, hi = min(m, lo + share);
+    if (lo >= hi) return;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
+    const int R = (kBitBins + step - 1) / step + 1;
+    const int WS = bit_row_words(m);
+    for (int e = tid; e < 64 * D; e += blockDim.x) {
+        const int c = e >> 6, t = e & 63;
+        s_edge[c][t] = __ldg(nd.bedges + e);
+        s_whole[c][t] = (t + 1) * step < kBitBins ? __ldg(nd.bedges + c * 64 + (t + 1) * step) : inf_f();
+    }
+    if (tid < 64) s_start[tid] = __ldg(nd.ostart + tid);
+    if constexpr (D > 1) {
+        for (int w = wid; w < WS; w += nwarps) {
+            const int pos = 32 * w + lane;
+            const unsigned v = pos < m ? __ldg(nd.bins + __ldg(nd.order + pos)) : kFull;
+#pragma unroll
+            for (int c = 1; c < D; ++c)
+                build_rows(s_dyn + (c - 1) * R * WS, WS, w, R, step, v >> (8 * c) & 0xffu, lane);
+        }
+    }
+    __syncthreads();
+    const float rank = est_rank(m);
+    // lane 4 t + c: coordinate c of the warp's query t
+    for (int q0 = lo + 8 * wid; q0 < hi; q0 += 8 * nwarps) {
+        const int t = lane >> 2, c = lane & 3;
+        const int i = min(q0 + t, hi - 1);
+        float x = 0.f, width = 1.f;
+        if (c < D) {
+            float f[D];
+            load_frame<D>(nd.aos, i, f);
+            x = f[0];
+            if constexpr (D > 1) x = c == 1 ? f[1] : x;
+            if constexpr (D > 2) x = c == 2 ? f[2] : x;
+            const int b = __ldg(nd.bins + i) >> (8 * c) & 0xffu;
+            const int b0 = max(b - 2, 0), b1 = min(b + 3, kBitBins);
+            width = fmaxf((s_edge[c][b1] - s_edge[c][b0]) * (static_cast<float>(kBitBins) / (b1 - b0)),
+                          2e-3f * (s_edge[c][kBitBins] - s_edge[c][0]));
+        }
+        width *= __shfl_xor_sync(kFull, width, 1);
+        width *= __shfl_xor_sync(kFull, width, 2);
+        float est = 0.5f * exp2f(__log2f(width * rank / m) / D);
+        if constexpr (D > 1) {
+            // first and one past the last whole bin within est, as in the search
+            unsigned pack = 0;
+            if (c < D) {
+                int a = 0, b = 0;
+#pragma unroll
+                for (int s = 32; s > 0; s >>= 1) {
+                    if (__fsub_rn(x, s_whole[c][a + s - 1]) > est) a += s;
+                    if (__fsub_rn(s_whole[c][b + s - 1], x) <= est) b += s;
+                }
+                ++b;
+                if (c == 0) {
+                    a = s_start[min(a * step, kBitBins)] >> 5;
+                    b = (s_start[min(b * step, kBitBins)] + 31) >> 5;
+                }
+                pack = static_cast<unsigned>(b) << 16 | static_cast<unsigned>(a);
+            }
+            float within = 0.f;
+            for (int u = 0; u < 8; ++u) {
+                const unsigned range = __shfl_sync(kFull, pack, 4 * u);
+                const unsigned r1 = __shfl_sync(kFull, pack, 4 * u + 1);
+                const unsigned r2 = __shfl_sync(kFull, pack, 4 * u + 2);
+                int n = 0;
+                for (int w = static_cast<int>(range & 0xffffu) + lane; w < static_cast<int>(range >> 16); w += 32) {
+                    unsigned bits = s_dyn[(r1 >> 16) * WS + w] ^ s_dyn[(r1 & 0xffffu) * WS + w];
+                    if constexpr (D > 2) bits &= s_dyn[(R + (r2 >> 16)) * WS + w] ^ s_dyn[(R + (r2 & 0xffffu)) * WS + w];
+                    n += __popc(bits);
+                }
+                n = __reduce_add_sync(kFull, n);
+                if (t == u) within = static_cast<float>(n);
+            }
+            est *= exp2f(__log2f(rank / fmaxf(within, 1.f)) / D);
+        }
+        if (c == 0 && q0 + t < hi) nd.est[i] = est;
+    }
+}
+
+}  // namespace nsg

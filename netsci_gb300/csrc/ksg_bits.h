@@ -1,0 +1,46 @@
+// KSG joint search on rank bitmaps (ksg_bits.cuh): launch configuration.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "ksg_grid.h"
+
+namespace nsg {
+
+constexpr int kBitTries = 6;      // search radii tried before a query scans all frames
+// Queries a warp takes at a time: a lane per query and coordinate.
+__host__ __device__ constexpr int bit_queries(int d) { return d == 3 ? 4 : 8; }
+// Shared words per warp: queries, the 32 n nearest frames' distances, bins, bit_of_rank's table.
+__host__ __device__ constexpr int bit_warp_words(int d, int n) {
+    return bit_queries(d) * 8 + 96 * n + 4 + bit_queries(d) * 2 * d + 32;
+}
+
+// Words of one bitmap row over m frames: whole 16-byte groups, an odd number
+// of them, so that the lanes that store one word each of successive rows
+// spread over the banks.
+__host__ __device__ inline int bit_row_words(int m) { return ((((m + 31) / 32 + 3) / 4) | 1) * 4; }
+
+struct BitsArgs {
+    GridArgs g;
+    int chunks;                 // work items: g.npairs * chunks
+    int rows, step;             // rows per coordinate, bins per row
+    int rows_words, perm_words; // shared-memory layout (words)
+};
+
+struct BitsConfig {
+    bool ok = false;
+    int keep = 0;               // frames within the search radius a query keeps, in 32s
+    int threads = 0, ctas_per_sm = 0;
+    int rows = 0, step = 0, rows_words = 0, perm_words = 0;
+    size_t smem = 0;
+};
+// Shared-memory layout and CTA size for pairs of up to max_m frames; not ok
+// where the rows of such a pair do not fit.
+BitsConfig bits_config(int d, int k, int max_m);
+// Scale estimates of node grids (grid_launch_nodes) of up to max_m frames.
+void bits_launch_est(const GridNode* nodes, int nnodes, int max_m, int d, cudaStream_t s);
+// The search of a batch whose largest m is max_m (the nodes carry scale
+// estimates); takes what grid_launch_search takes but no pair grids.
+void bits_launch_search(const GridArgs& g, const BitsConfig& c, int max_m, int d, cudaStream_t s);
+
+}  // namespace nsg

@@ -107,51 +107,59 @@ __device__ void build_query_order(const int* cnt, int G, int* start, int* tmp1, 
     for (int c = t; c <= G * G; c += blockDim.x) qstart[c] = tmp2[c];
 }
 
-// One CTA per node: axes, quantile edges, cells, counting sort by cell.
+// Quantiles of coordinate c of a node (kQuantFloats) from a sorted sample;
+// v: kSample floats of shared memory.
+__device__ void node_quantiles(const GridNode& nd, int c, float* v, float* out) {
+    for (int s = threadIdx.x; s < kSample; s += blockDim.x) {
+        const int j = static_cast<int>((static_cast<long long>(s) * nd.m) / kSample);
+        v[s] = __ldg(nd.x + static_cast<long long>(c) * nd.ld + j);
+    }
+    bitonic_sort(v);
+    const int t = threadIdx.x;
+    if (t < kGridMaxG) out[t] = t < nd.G - 1 ? v[((t + 1) * kSample) / nd.G] : __int_as_float(0x7f800000);
+    if (t < 64) out[kGridMaxG + t] = v[min((t * kSample) / kBitBins, kSample - 1)];
+    if (t == 0) out[kGridMaxG + 64] = v[(kSample * 9) / 10] - v[kSample / 10];
+    __syncthreads();
+}
+
+// Coordinates by their spread: the widest, the second widest (-1 if none),
+// and the other one.
 template <int D>
-__global__ void __launch_bounds__(kPrepThreads) grid_node_kernel(GridNode* nodes) {
-    __shared__ float s_val[D][kSample];
+__device__ __forceinline__ void node_axes(const float* quant, int (&axis)[3]) {
+    float w[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) w[c] = quant[c * kQuantFloats + kGridMaxG + 64];
+    int c1 = 0;
+    for (int c = 1; c < D; ++c)
+        if (w[c] > w[c1]) c1 = c;
+    int c2 = -1;
+    for (int c = 0; c < D; ++c)
+        if (c != c1 && (c2 < 0 || w[c] > w[c2])) c2 = c;
+    axis[0] = c1;
+    axis[1] = c2;
+    axis[2] = D == 3 ? 3 - c1 - c2 : 0;
+}
+
+// Cells of a node's grid, counting sort by cell.
+template <int D>
+__device__ void node_cells(GridNode* node, const GridNode& nd, const float* quant) {
     __shared__ float s_e1[kGridMaxG], s_e2[kGridMaxG];
     __shared__ int s_cnt[kGridMaxG * kGridMaxG];
     __shared__ int s_start[kGridMaxG * kGridMaxG + 1];
     __shared__ int s_tmp1[kGridMaxG * kGridMaxG], s_tmp2[kGridMaxG * kGridMaxG + 1];
-    __shared__ int s_axis[2];
-    GridNode nd = nodes[blockIdx.x];
     const int m = nd.m, G = nd.G, t = threadIdx.x;
-    const int S = kSample;
-    for (int s = t; s < S; s += blockDim.x) {
-        const int j = static_cast<int>((static_cast<long long>(s) * m) / S);
-#pragma unroll
-        for (int c = 0; c < D; ++c) s_val[c][s] = __ldg(nd.x + static_cast<long long>(c) * nd.ld + j);
-    }
-#pragma unroll
-    for (int c = 0; c < D; ++c) bitonic_sort(s_val[c]);
-    if (t == 0) {
-        // widest and second-widest coordinates by their 10-90% spread
-        float w[D];
-#pragma unroll
-        for (int c = 0; c < D; ++c) w[c] = s_val[c][(S * 9) / 10] - s_val[c][S / 10];
-        int c1 = 0;
-        for (int c = 1; c < D; ++c)
-            if (w[c] > w[c1]) c1 = c;
-        int c2 = -1;
-        for (int c = 0; c < D; ++c)
-            if (c != c1 && (c2 < 0 || w[c] > w[c2])) c2 = c;
-        s_axis[0] = c1;
-        s_axis[1] = c2;
-    }
-    __syncthreads();
-    const int c1 = s_axis[0], c2 = s_axis[1];
+    int axis[3];
+    node_axes<D>(quant, axis);
+    const int c1 = axis[0], c2 = axis[1];
     if (t < kGridMaxG) {
-        const float inf = __int_as_float(0x7f800000);
-        s_e1[t] = t < G - 1 ? s_val[c1][((t + 1) * S) / G] : inf;
-        s_e2[t] = (c2 >= 0 && t < G - 1) ? s_val[c2][((t + 1) * S) / G] : inf;
+        s_e1[t] = quant[c1 * kQuantFloats + t];
+        s_e2[t] = c2 >= 0 ? quant[c2 * kQuantFloats + t] : __int_as_float(0x7f800000);
         nd.e1[t] = s_e1[t];
         nd.e2[t] = s_e2[t];
     }
     if (t == 0) {
-        nodes[blockIdx.x].c1 = c1;
-        nodes[blockIdx.x].c2 = c2;
+        node->c1 = c1;
+        node->c2 = c2;
     }
     for (int c = t; c < G * G; c += blockDim.x) s_cnt[c] = 0;
     __syncthreads();
@@ -182,41 +190,89 @@ __global__ void __launch_bounds__(kPrepThreads) grid_node_kernel(GridNode* nodes
     build_query_order(s_cnt, G, nd.start, s_tmp1, s_tmp2);
 }
 
-// One CTA per node, after grid_node_kernel: the scale estimate of every
-// frame (GridNode::est), from the frames of the 3 x 3 cells around its own.
-// Consecutive threads take consecutive positions, mostly of one cell, so
-// they read the same neighbour frames.
+// What the bitmaps are built from: frames, bins, order by c1 bin.
 template <int D>
-__global__ void __launch_bounds__(kPrepThreads) grid_node_est_kernel(const GridNode* nodes) {
-    const GridNode nd = nodes[blockIdx.x];
-    const int m = nd.m, G = nd.G;
-    const long long st = m;
-    for (int pos = threadIdx.x; pos < m; pos += blockDim.x) {
-        const int j = __ldg(nd.perm + pos);
-        const int c = __ldg(nd.cell + j);
-        const int row = c / G, col = c - (c / G) * G;
-        float q[D];
-#pragma unroll
-        for (int cc = 0; cc < D; ++cc) q[cc] = __ldg(nd.sx + cc * st + pos);
-        float bd[kEstRank];
-        int bj[kEstRank];
-#pragma unroll
-        for (int s = 0; s < kEstRank; ++s) {
-            bd[s] = __int_as_float(0x7f800000);
-            bj[s] = -1;
-        }
-        const int c0 = max(col - 1, 0), c1 = min(col + 1, G - 1);
-        for (int r = max(row - 1, 0); r <= min(row + 1, G - 1); ++r) {
-            const int lo = __ldg(nd.start + r * G + c0), hi = __ldg(nd.start + r * G + c1 + 1);
-            for (int f = lo; f < hi; ++f) {
-                float dm = 0.f;
-#pragma unroll
-                for (int cc = 0; cc < D; ++cc) dm = fmaxf(dm, fabsf(q[cc] - __ldg(nd.sx + cc * st + f)));
-                if (f != pos && dm < bd[kEstRank - 1]) ksgk::list_insert<kEstRank>(bd, bj, dm, f);
-            }
-        }
-        nd.est[j] = bd[kEstRank - 1];
+__device__ void node_frames(const GridNode& nd, const float* quant) {
+    __shared__ float s_be[D][64];
+    __shared__ int s_ocnt[64], s_ostart[65];
+    __shared__ int s_bad;
+    const int m = nd.m, t = threadIdx.x;
+    int axis[3];
+    node_axes<D>(quant, axis);
+    for (int e = t; e < 64 * D; e += blockDim.x) {
+        const int c = e >> 6;
+        const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
+        const float v = quant[ax * kQuantFloats + kGridMaxG + (e & 63)];
+        s_be[c][e & 63] = v;
+        nd.bedges[e] = v;
     }
+    if (t < 64) s_ocnt[t] = 0;
+    if (t == 0) s_bad = 0;
+    __syncthreads();
+    bool bad = false;
+    for (int j = t; j < m; j += blockDim.x) {
+        float x[D];
+        unsigned bins = 0;
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
+            x[c] = __ldg(nd.x + static_cast<long long>(ax) * nd.ld + j);
+            bad |= !isfinite(x[c]);
+            bins |= static_cast<unsigned>(bin_of(s_be[c] + 1, kBitBins - 1, x[c])) << (8 * c);
+        }
+        if constexpr (D == 1) nd.aos[j] = x[0];
+        else if constexpr (D == 2) reinterpret_cast<float2*>(nd.aos)[j] = make_float2(x[0], x[1]);
+        else reinterpret_cast<float4*>(nd.aos)[j] = make_float4(x[0], x[1], x[2], 0.f);
+        nd.bins[j] = bins;
+        atomicAdd(&s_ocnt[bins & 0xffu], 1);
+    }
+    if (bad) s_bad = 1;
+    __syncthreads();
+    block_scan(s_ocnt, s_ostart, 64);
+    if (t < 64) {
+        nd.ostart[t] = t < 63 ? s_ostart[t] : s_bad;
+        s_ocnt[t] = 0;
+    }
+    __syncthreads();
+    if (m > kBitMaxM) return;
+    for (int j = t; j < m; j += blockDim.x) {
+        const int b = nd.bins[j] & 0xffu;
+        nd.order[s_ostart[b] + atomicAdd(&s_ocnt[b], 1)] = static_cast<unsigned short>(j);
+    }
+}
+
+// One CTA per node: quantiles, cells, bitmap frames.
+template <int D>
+__global__ void __launch_bounds__(kPrepThreads) grid_node_kernel(GridNode* nodes) {
+    __shared__ float s_val[kSample];
+    __shared__ float s_quant[D * kQuantFloats];
+    const GridNode nd = nodes[blockIdx.x];
+    for (int c = 0; c < D; ++c) node_quantiles(nd, c, s_val, s_quant + c * kQuantFloats);
+    node_cells<D>(nodes + blockIdx.x, nd, s_quant);
+    node_frames<D>(nd, s_quant);
+}
+
+// The same in three kernels for plans of many nodes: the sort waits on
+// barriers and the counting sorts on atomics, and small CTAs of one kind
+// overlap better than 1024 threads doing one after the other.
+constexpr int kSplitThreads = 512;
+
+__global__ void __launch_bounds__(kSplitThreads) node_quantiles_kernel(const GridNode* nodes) {
+    __shared__ float s_val[kSample];
+    const GridNode nd = nodes[blockIdx.x];
+    node_quantiles(nd, blockIdx.y, s_val, nd.quant + blockIdx.y * kQuantFloats);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kPrepThreads) node_cells_kernel(GridNode* nodes) {
+    const GridNode nd = nodes[blockIdx.x];
+    node_cells<D>(nodes + blockIdx.x, nd, nd.quant);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kSplitThreads) node_frames_kernel(const GridNode* nodes) {
+    const GridNode nd = nodes[blockIdx.x];
+    node_frames<D>(nd, nd.quant);
 }
 
 // One CTA per pair of the batch: cells over (bin of a on its c1, bin of b on
@@ -440,7 +496,6 @@ __global__ void __launch_bounds__(kOrderThreads) grid_count_order_kernel(GridArg
     __shared__ float s_t[2][16];
     const CountGroup grp = A.groups[blockIdx.x];
     const GridNode nd = A.nodes[grp.node];
-    const float* eps = grp.side ? A.eps_b : A.eps_a;
     const int m = nd.m;
     if (threadIdx.x < 32) {
         const int L = threadIdx.x & 15;
@@ -448,22 +503,40 @@ __global__ void __launch_bounds__(kOrderThreads) grid_count_order_kernel(GridArg
         s_t[threadIdx.x >> 4][L] = L < 15 ? e[2 * L + 1] : __int_as_float(0x7fc00000);
     }
     __syncthreads();
-    long long o[kCountGroup];
+    const float* eps[kCountGroup];
 #pragma unroll
-    for (int p = 0; p < kCountGroup; ++p) o[p] = A.pairs[grp.pairs[p]].scratch;  // unused slots repeat pairs[0]
+    for (int p = 0; p < kCountGroup; ++p) {  // unused slots repeat the first variable
+        const int v = grp.vars[p];
+        eps[p] = (v & 1 ? A.eps_b : A.eps_a) + A.pairs[v >> 1].scratch;
+    }
     // the grid's coordinates in storage order (coalesced)
     const float* x1 = nd.sx + static_cast<long long>(nd.c1) * m;
     const float* x2 = nd.c2 >= 0 ? nd.sx + static_cast<long long>(nd.c2) * m : nullptr;
     for (int pos = threadIdx.x; pos < m; pos += blockDim.x) {
         const int j = __ldg(nd.perm + pos);
-        float e = __ldg(eps + o[0] + j);
+        float e = __ldg(eps[0] + j);
 #pragma unroll
-        for (int p = 1; p < kCountGroup; ++p) e = fmaxf(e, __ldg(eps + o[p] + j));
+        for (int p = 1; p < kCountGroup; ++p)
+            if (p < grp.nvars) e = fmaxf(e, __ldg(eps[p] + j));
         s_key[pos] = box_key(s_t[0], s_t[1], __ldg(x1 + pos), x2 ? __ldg(x2 + pos) : 0.f, e);
     }
     __syncthreads();
     write_key_order(s_key, m, A.corder + static_cast<long long>(blockIdx.x) * A.corder_ld,
                     sort_low ? s_key + A.corder_ld : nullptr);
+}
+
+// Largest eps of every frame of the rank nodes over the node's variables:
+// one CTA per node and block of frames, so that eps are read in rows.
+__global__ void __launch_bounds__(256) rank_emax_kernel(GridArgs A) {
+    const RankNode rn = A.ranks[blockIdx.x];
+    const int i = blockIdx.y * blockDim.x + threadIdx.x;
+    if (i >= rn.m) return;
+    float e = 0.f;
+    for (int p = 0; p < rn.count; ++p) {
+        const long long ref = __ldg(A.refs + rn.first + p);
+        e = fmaxf(e, __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i));
+    }
+    A.rank_emax[static_cast<long long>(blockIdx.x) * A.rank_ld + i] = e;
 }
 
 // Search order: cells in kOrderBlock x kOrderBlock blocks, blocks in Z
@@ -560,25 +633,47 @@ void launch_pass1(const GridArgs& a, int kmax, int grid, cudaStream_t st) {
 
 }  // namespace
 
-void append_count_groups(const GridPair* gps, int npairs, std::vector<CountGroup>& out) {
-    for (int side = 0; side < 2; ++side) {
-        // pairs by node, in first-appearance order of the nodes
-        std::vector<std::pair<int, int>> keyed(npairs);
-        for (int p = 0; p < npairs; ++p) keyed[p] = {side ? gps[p].b : gps[p].a, p};
-        std::stable_sort(keyed.begin(), keyed.end(),
-                         [](const std::pair<int, int>& x, const std::pair<int, int>& y) { return x.first < y.first; });
-        for (size_t s = 0; s < keyed.size();) {
-            CountGroup g{};
-            g.node = keyed[s].first;
-            g.side = side;
-            while (s < keyed.size() && keyed[s].first == g.node && g.npairs < kCountGroup) {
-                g.pairs[g.npairs++] = keyed[s].second;
-                ++s;
+CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, int min_rank) {
+    CountWork w;
+    // variables by node, in first-appearance order within a node
+    std::vector<std::pair<int, int>> keyed(2 * static_cast<size_t>(npairs));
+    for (int p = 0; p < npairs; ++p) {
+        keyed[p] = {gps[p].a, 2 * p};
+        keyed[static_cast<size_t>(npairs) + p] = {gps[p].b, 2 * p + 1};
+    }
+    std::stable_sort(keyed.begin(), keyed.end(),
+                     [](const std::pair<int, int>& x, const std::pair<int, int>& y) { return x.first < y.first; });
+    int gitems = 0, ritems = 0;
+    for (size_t s = 0; s < keyed.size();) {
+        size_t e = s;
+        while (e < keyed.size() && keyed[e].first == keyed[s].first) ++e;
+        const int node = keyed[s].first, m = descs[keyed[s].second >> 1].m;
+        if (static_cast<int>(e - s) >= min_rank) {
+            w.ranks.push_back({node, static_cast<int>(w.refs.size()), static_cast<int>(e - s), m});
+            w.rprefix.push_back(ritems);
+            ritems += (m + kRankWarps - 1) / kRankWarps;
+            for (; s < e; ++s) {
+                const int v = keyed[s].second;
+                w.refs.push_back(descs[v >> 1].scratch * 2 + (v & 1));
             }
-            for (int q = g.npairs; q < kCountGroup; ++q) g.pairs[q] = g.pairs[0];
-            out.push_back(g);
+        }
+        while (s < e) {
+            // the rest in groups of equal size (8 variables: 4 + 4)
+            const int left = static_cast<int>(e - s);
+            const int take = (left + (left + kCountGroup - 1) / kCountGroup - 1) / ((left + kCountGroup - 1) / kCountGroup);
+            CountGroup g{};
+            g.node = node;
+            g.nvars = take;
+            for (int q = 0; q < kCountGroup; ++q) g.vars[q] = keyed[s + (q < take ? q : 0)].second;
+            s += take;
+            w.groups.push_back(g);
+            w.gprefix.push_back(gitems);
+            gitems += (m + kCountQueries - 1) / kCountQueries;
         }
     }
+    w.gprefix.push_back(gitems);
+    w.rprefix.push_back(ritems);
+    return w;
 }
 
 int grid_cells_per_axis(int m) {
@@ -587,24 +682,30 @@ int grid_cells_per_axis(int m) {
     return g;
 }
 
-void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool est, cudaStream_t st) {
-    if (nnodes <= 0) return;
-    switch (d) {
-        case 1:
-            grid_node_kernel<1><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            if (est) grid_node_est_kernel<1><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            break;
-        case 2:
-            grid_node_kernel<2><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            if (est) grid_node_est_kernel<2><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            break;
-        case 3:
-            grid_node_kernel<3><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            if (est) grid_node_est_kernel<3><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-            break;
-        default: invalid("d must be 1, 2 or 3");
+namespace {
+
+template <int D>
+void launch_nodes(GridNode* nodes, int nnodes, bool split, cudaStream_t st) {
+    if (split) {
+        node_quantiles_kernel<<<dim3(nnodes, D), kSplitThreads, 0, st>>>(nodes);
+        node_cells_kernel<D><<<nnodes, kPrepThreads, 0, st>>>(nodes);
+        node_frames_kernel<D><<<nnodes, kSplitThreads, 0, st>>>(nodes);
+    } else {
+        grid_node_kernel<D><<<nnodes, kPrepThreads, 0, st>>>(nodes);
     }
     NSG_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool split, cudaStream_t st) {
+    if (nnodes <= 0) return;
+    switch (d) {
+        case 1: launch_nodes<1>(nodes, nnodes, split, st); break;
+        case 2: launch_nodes<2>(nodes, nnodes, split, st); break;
+        case 3: launch_nodes<3>(nodes, nnodes, split, st); break;
+        default: invalid("d must be 1, 2 or 3");
+    }
 }
 
 bool grid_orders_pay(long long search_warps, int sms) {
@@ -616,10 +717,14 @@ size_t grid_node_bytes(int m, int d) {
     const size_t mm = static_cast<size_t>(m);
     return a16(2 * kGridMaxG * sizeof(float)) + grid_index_bytes(grid_cells_per_axis(m)) +
            a16(mm * sizeof(unsigned short)) + a16(mm * sizeof(int)) + a16(mm * sizeof(float)) +
-           a16(static_cast<size_t>(d) * mm * sizeof(float));
+           a16(static_cast<size_t>(d) * mm * sizeof(float)) +
+           // bitmap search: frames, bins, order, edges, starts
+           a16((d == 3 ? 4 : d) * mm * sizeof(float)) + a16(mm * sizeof(unsigned)) +
+           a16(mm * sizeof(unsigned short)) + static_cast<size_t>(d) * (64 + kQuantFloats) * sizeof(float) +
+           64 * sizeof(int);
 }
 
-GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m) {
+GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m, int d) {
     auto a16 = [](size_t b) { return (b + 15) & ~size_t(15); };
     const size_t mm = static_cast<size_t>(m);
     GridNode n{};
@@ -639,6 +744,16 @@ GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m) {
     n.est = reinterpret_cast<float*>(base);
     base += a16(mm * sizeof(float));
     n.sx = reinterpret_cast<float*>(base);
+    base += a16(static_cast<size_t>(d) * mm * sizeof(float));
+    n.aos = reinterpret_cast<float*>(base);
+    base += a16((d == 3 ? 4 : d) * mm * sizeof(float));
+    n.bins = reinterpret_cast<unsigned*>(base);
+    base += a16(mm * sizeof(unsigned));
+    n.order = reinterpret_cast<unsigned short*>(base);
+    base += a16(mm * sizeof(unsigned short));
+    n.bedges = reinterpret_cast<float*>(base);
+    n.quant = n.bedges + 64 * d;
+    n.ostart = reinterpret_cast<int*>(n.quant + kQuantFloats * d);
     return n;
 }
 
@@ -734,18 +849,36 @@ GridArgs grid_launch_count_order(const GridArgs& a, cudaStream_t st) {
     } else {
         c.corder = nullptr;
     }
+    if (c.rank_emax && c.nranks > 0) {
+        rank_emax_kernel<<<dim3(c.nranks, (c.rank_ld + 255) / 256), 256, 0, st>>>(c);
+        NSG_CUDA(cudaGetLastError());
+    }
     return c;
 }
 
+namespace {
+
+template <int D>
+void launch_counts(const GridArgs& c, int grid, cudaStream_t st) {
+    if (c.ngroups > 0) {
+        ksg_grid_count_kernel<D><<<grid, 32 * kGridWarps, 0, st>>>(c);
+        NSG_CUDA(cudaGetLastError());
+    }
+    if (c.nranks > 0) {
+        ksg_grid_rank_kernel<D><<<c.rank_items, 32 * kRankWarps, 0, st>>>(c);
+        NSG_CUDA(cudaGetLastError());
+    }
+}
+
+}  // namespace
+
 void grid_launch_count_kernel(const GridArgs& c, int d, int grid, cudaStream_t st) {
-    const dim3 b(32 * kGridWarps);
     switch (d) {
-        case 1: ksg_grid_count_kernel<1><<<grid, b, 0, st>>>(c); break;
-        case 2: ksg_grid_count_kernel<2><<<grid, b, 0, st>>>(c); break;
-        case 3: ksg_grid_count_kernel<3><<<grid, b, 0, st>>>(c); break;
+        case 1: launch_counts<1>(c, grid, st); break;
+        case 2: launch_counts<2>(c, grid, st); break;
+        case 3: launch_counts<3>(c, grid, st); break;
         default: invalid("d must be 1, 2 or 3");
     }
-    NSG_CUDA(cudaGetLastError());
 }
 
 void grid_launch_counts(const GridArgs& a, int d, int grid, cudaStream_t st) {

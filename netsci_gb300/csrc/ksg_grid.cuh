@@ -274,19 +274,19 @@ __device__ __forceinline__ void pass1_chunk(const float* tile, const int* jt, in
     }
 }
 
-// Counts over a staged chunk for up to kCountGroup pairs at once: one
-// distance per frame, compared with each pair's eps (unused slots hold -inf).
+// Counts over a staged chunk for P variables at once: one distance per
+// frame, compared with each variable's eps (unused slots hold -inf).
 // Two lanes share a query: the lane of parity `half` takes frames 4g + 2*half
 // and 4g + 2*half + 1 of each group of four. The chunk's counts (at most 64
 // per lane) add up in floats, exactly, from nsg_le_f32: 46-51 against 57-64
-// ms per 8192-pair batch at m = 10000 for integer selects and adds.
-template <int D>
+// ms per 8192-pair batch at m = 10000 for integer selects and adds (P = 4).
+template <int D, int P>
 __device__ __forceinline__ void count_chunk(const float* tile, int n, int half, const float (&q)[D],
-                                            const float (&e)[kCountGroup], int (&cnt)[kCountGroup]) {
+                                            const float (&e)[P], int (&cnt)[P]) {
     const int ngroups = (n + 3) >> 2;
-    float cf[kCountGroup];
+    float cf[P];
 #pragma unroll
-    for (int p = 0; p < kCountGroup; ++p) cf[p] = 0.f;
+    for (int p = 0; p < P; ++p) cf[p] = 0.f;
     for (int g = 0; g < ngroups; ++g) {
         float dq0[D], dq1[D];
 #pragma unroll
@@ -298,10 +298,10 @@ __device__ __forceinline__ void count_chunk(const float* tile, int n, int half, 
         }
         const float d0 = max_of<D>(dq0), d1 = max_of<D>(dq1);
 #pragma unroll
-        for (int p = 0; p < kCountGroup; ++p) cf[p] += nsg_le_f32(d0, e[p]) + nsg_le_f32(d1, e[p]);
+        for (int p = 0; p < P; ++p) cf[p] += nsg_le_f32(d0, e[p]) + nsg_le_f32(d1, e[p]);
     }
 #pragma unroll
-    for (int p = 0; p < kCountGroup; ++p) cnt[p] += static_cast<int>(cf[p]);
+    for (int p = 0; p < P; ++p) cnt[p] += static_cast<int>(cf[p]);
 }
 
 // Tie check over a staged chunk (2d planes): the range of each marginal over
@@ -581,19 +581,94 @@ __global__ void __launch_bounds__(32 * kGridWarps, (KMAX <= 8 ? 4 : 1)) ksg_grid
 }
 
 // ---- pass 2: marginal counts on a node grid -------------------------------------
-// A work item is a count group (up to kCountGroup pairs that count the same
-// node's variable) and a block of kCountQueries queries consecutive in the
-// group's count order (A.corder, else the node grid's query order), two
-// lanes per query. The warp visits the union of the queries' boxes for the
-// largest of the pairs' eps, row by row over the columns of the boxes that
-// hold the row, and counts every pair from one distance per frame.
+// One work item of a count group of up to P variables: a block of
+// kCountQueries queries consecutive in the group's count order (A.corder,
+// else the node grid's query order), two lanes per query. The warp visits the
+// union of the queries' boxes for the largest of the variables' eps, row by
+// row over the columns of the boxes that hold the row, and counts every
+// variable from one distance per frame.
+template <int D, int P>
+__device__ __forceinline__ void count_item(const GridArgs& A, const CountGroup& grp, int gi, int blk, float* tile, int lane) {
+    using namespace gridk;
+    const GridNode& nd = A.nodes[grp.node];
+    const int m = nd.m, G = nd.G;
+    const long long st = m;
+    const int half = lane & 1;  // two lanes per query
+    const int qi = blk * kCountQueries + (lane >> 1);  // query rank in the group's count order
+    const bool valid = qi < m;
+    const int r = !valid ? 0
+                  : A.corder ? __ldg(A.corder + static_cast<long long>(gi) * A.corder_ld + qi)
+                             : query_position(nd.start, G, qi);
+    const int i = valid ? __ldg(nd.perm + r) : 0;
+    const float* sx = nd.sx;
+    float q[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) q[c] = valid ? __ldg(sx + c * st + r) : 0.f;
+    float e[P];
+    float emax = -inf_f();
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const int v = grp.vars[p];
+        const float* eps = v & 1 ? A.eps_b : A.eps_a;
+        e[p] = (valid && p < grp.nvars) ? __ldg(eps + A.pairs[v >> 1].scratch + i) : -inf_f();
+        emax = fmaxf(emax, e[p]);
+    }
+    const float q1 = q[nd.c1];
+    const float q2 = nd.c2 >= 0 ? q[nd.c2] : 0.f;
+    // each query's box of rows [qrlo, qrhi] and columns [qclo, qchi];
+    // a row is scanned over the columns of the queries whose box holds it
+    int qrlo = G, qrhi = -1, qclo = G, qchi = -1;
+    if (valid) {
+        bin_range(nd.e1, G, q1, emax, qrlo, qrhi);
+        bin_range(nd.e2, G, q2, emax, qclo, qchi);
+    }
+    const int rlo = __reduce_min_sync(0xffffffffu, qrlo);
+    const int rhi = __reduce_max_sync(0xffffffffu, qrhi);
+    const int* start = nd.start;
+    int cnt[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) cnt[p] = 0;
+    long long scanned = 0;
+    for (int cx = rlo; cx <= rhi; ++cx) {
+        const bool in_row = cx >= qrlo && cx <= qrhi;
+        const int clo = __reduce_min_sync(0xffffffffu, in_row ? qclo : G);
+        const int chi = __reduce_max_sync(0xffffffffu, in_row ? qchi : -1);
+        if (clo > chi) continue;
+        const int lo = __ldg(start + cx * G + clo);
+        const int hi = __ldg(start + cx * G + chi + 1);
+        scanned += hi - lo;
+        for (int base = lo; base < hi; base += kGridChunk) {
+            const int n = min(kGridChunk, hi - base);
+            __syncwarp();
+            stage<D, false>(tile, nullptr, sx, st, nullptr, base, n, lane);
+            __syncwarp();
+            count_chunk<D, P>(tile, n, half, q, e, cnt);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) cnt[p] += __shfl_xor_sync(0xffffffffu, cnt[p], 1);
+    if (valid && half == 0) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int v = grp.vars[p];
+            if (p < grp.nvars) (v & 1 ? A.cnt_b : A.cnt_a)[A.pairs[v >> 1].scratch + i] = cnt[p];
+        }
+    }
+    if (A.evals && lane == 0) {
+        // one distance per (query, frame), compared with every variable's eps
+        const unsigned long long ev =
+            static_cast<unsigned long long>(scanned) * min(kCountQueries, m - blk * kCountQueries);
+        atomicAdd(A.evals + 1, ev);
+        atomicAdd(A.evals + 2, ev * grp.nvars);
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(32 * kGridWarps, 4) ksg_grid_count_kernel(GridArgs A) {
     using namespace gridk;
     __shared__ __align__(16) float s_tile[kGridWarps][D * kGridChunk];
     const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    float* tile = s_tile[wid];
+    float* tile = s_tile[threadIdx.x >> 5];
     const int total = __ldg(A.gprefix + A.ngroups);
     for (;;) {
         int t = 0;
@@ -602,74 +677,166 @@ __global__ void __launch_bounds__(32 * kGridWarps, 4) ksg_grid_count_kernel(Grid
         if (t >= total) return;
         int gi, blk;
         item_of(A.gprefix, A.ngroups, t, gi, blk);
-        const CountGroup grp = A.groups[gi];
-        const GridNode nd = A.nodes[grp.node];
-        const float* eps = grp.side ? A.eps_b : A.eps_a;
-        int* out = grp.side ? A.cnt_b : A.cnt_a;
-        const int m = nd.m, G = nd.G;
-        const long long st = m;
-        const int half = lane & 1;  // two lanes per query
-        const int qi = blk * kCountQueries + (lane >> 1);  // query rank in the group's count order
-        const bool valid = qi < m;
-        const int r = !valid ? 0
-                      : A.corder ? __ldg(A.corder + static_cast<long long>(gi) * A.corder_ld + qi)
-                                 : query_position(nd.start, G, qi);
-        const int i = valid ? __ldg(nd.perm + r) : 0;
-        float q[D];
+        const CountGroup& grp = A.groups[gi];
+        if (grp.nvars <= 4) count_item<D, 4>(A, grp, gi, blk, tile, lane);
+        else count_item<D, kCountGroup>(A, grp, gi, blk, tile, lane);
+    }
+}
+
+// ---- pass 2 by rank: nodes with many variables in the batch -------------------------
+// One warp per query of a rank node: the distances of the frames in the
+// query's box for the largest eps (the cells it overlaps, read in rows
+// straight from the grid) are listed in shared memory and counting-sorted
+// into kRankBuckets buckets of equal width; each lane then takes one
+// variable, and its count is the frames of the buckets below its eps's plus
+// those of that bucket that pass the exact comparison (the bucket index is a
+// monotone function of the distance). A few variables are counted while the
+// frames go by. A list that fills up is counted and starts again.
+constexpr int kRankList = 1024;
+constexpr int kRankBuckets = 128;
+constexpr int kRankDirect = 4;
+
+template <int D>
+__global__ void __launch_bounds__(32 * kRankWarps) ksg_grid_rank_kernel(GridArgs A) {
+    using namespace gridk;
+    __shared__ float s_list[kRankWarps][kRankList];
+    __shared__ float s_sort[kRankWarps][kRankList];
+    __shared__ __align__(16) int s_end[kRankWarps][kRankBuckets];
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int ri, blk;
+    item_of(A.rprefix, A.nranks, blockIdx.x, ri, blk);
+    const RankNode rn = A.ranks[ri];
+    const int i = blk * kRankWarps + wid;
+    if (i >= rn.m) return;  // whole warps; no CTA-wide waits below
+    const GridNode& nd = A.nodes[rn.node];
+    const long long* refs = A.refs + rn.first;
+    const int m = nd.m, G = nd.G, P = rn.count;
+    float q[D];
 #pragma unroll
-        for (int c = 0; c < D; ++c) q[c] = valid ? __ldg(nd.sx + c * st + r) : 0.f;
-        float e[kCountGroup];
-        float emax = -inf_f();
+    for (int c = 0; c < D; ++c) q[c] = __ldg(nd.x + static_cast<long long>(c) * nd.ld + i);
+    auto eps_of = [&](int p) {
+        const long long ref = __ldg(refs + p);
+        return __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i);
+    };
+    float emax = 0.f;  // eps are not negative
+    if (A.rank_emax) {
+        emax = __ldg(A.rank_emax + static_cast<long long>(ri) * A.rank_ld + i);
+    } else {
+        for (int p = lane; p < P; p += 32) emax = fmaxf(emax, eps_of(p));
 #pragma unroll
-        for (int p = 0; p < kCountGroup; ++p) {
-            e[p] = (valid && p < grp.npairs) ? __ldg(eps + A.pairs[grp.pairs[p]].scratch + i) : -inf_f();
-            emax = fmaxf(emax, e[p]);
+        for (int o = 16; o > 0; o >>= 1) emax = fmaxf(emax, __shfl_xor_sync(kFull, emax, o));
+    }
+    int rlo, rhi, clo, chi;
+    bin_range(nd.e1, G, q[nd.c1], emax, rlo, rhi);
+    bin_range(nd.e2, G, nd.c2 >= 0 ? q[nd.c2] : 0.f, emax, clo, chi);
+    // row r's range of positions in lane r - rlo
+    int lo = 0, hi = 0;
+    if (lane <= rhi - rlo && clo <= chi) {
+        lo = __ldg(nd.start + (rlo + lane) * G + clo);
+        hi = __ldg(nd.start + (rlo + lane) * G + chi + 1);
+    }
+    const int nrows = clo <= chi ? rhi - rlo + 1 : 0;
+    const float* sx = nd.sx;
+    auto distance = [&](int pos) {
+        float dq[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) dq[c] = fabsf(q[c] - __ldg(sx + static_cast<long long>(c) * m + pos));
+        return max_of<D>(dq);
+    };
+    const unsigned long long scanned = __reduce_add_sync(kFull, hi - lo);
+    if (P <= kRankDirect) {
+        float e[kRankDirect];
+        int cnt[kRankDirect];
+#pragma unroll
+        for (int p = 0; p < kRankDirect; ++p) {
+            e[p] = p < P ? eps_of(p) : -inf_f();
+            cnt[p] = 0;
         }
-        const float q1 = q[nd.c1];
-        const float q2 = nd.c2 >= 0 ? q[nd.c2] : 0.f;
-        // each query's box of rows [qrlo, qrhi] and columns [qclo, qchi];
-        // a row is scanned over the columns of the queries whose box holds it
-        int qrlo = G, qrhi = -1, qclo = G, qchi = -1;
-        if (valid) {
-            bin_range(nd.e1, G, q1, emax, qrlo, qrhi);
-            bin_range(nd.e2, G, q2, emax, qclo, qchi);
-        }
-        const int rlo = __reduce_min_sync(0xffffffffu, qrlo);
-        const int rhi = __reduce_max_sync(0xffffffffu, qrhi);
-        int cnt[kCountGroup];
+        for (int r = 0; r < nrows; ++r) {
+            const int b = __shfl_sync(kFull, lo, r), t = __shfl_sync(kFull, hi, r);
+            for (int pos = b + lane; pos < t; pos += 32) {
+                const float dm = distance(pos);
 #pragma unroll
-        for (int p = 0; p < kCountGroup; ++p) cnt[p] = 0;
-        long long scanned = 0;
-        for (int cx = rlo; cx <= rhi; ++cx) {
-            const bool in_row = cx >= qrlo && cx <= qrhi;
-            const int clo = __reduce_min_sync(0xffffffffu, in_row ? qclo : G);
-            const int chi = __reduce_max_sync(0xffffffffu, in_row ? qchi : -1);
-            if (clo > chi) continue;
-            const int lo = __ldg(nd.start + cx * G + clo);
-            const int hi = __ldg(nd.start + cx * G + chi + 1);
-            scanned += hi - lo;
-            for (int base = lo; base < hi; base += kGridChunk) {
-                const int n = min(kGridChunk, hi - base);
-                __syncwarp();
-                stage<D, false>(tile, nullptr, nd.sx, st, nullptr, base, n, lane);
-                __syncwarp();
-                count_chunk<D>(tile, n, half, q, e, cnt);
+                for (int p = 0; p < kRankDirect; ++p) cnt[p] += dm <= e[p];
             }
         }
 #pragma unroll
-        for (int p = 0; p < kCountGroup; ++p) cnt[p] += __shfl_xor_sync(0xffffffffu, cnt[p], 1);
-        if (valid && half == 0) {
+        for (int p = 0; p < kRankDirect; ++p) {
+            const int n = __reduce_add_sync(kFull, cnt[p]);
+            if (p < P && lane == 0) {
+                const long long ref = __ldg(refs + p);
+                (ref & 1 ? A.cnt_b : A.cnt_a)[(ref >> 1) + i] = n;
+            }
+        }
+    } else {
+        float* list = s_list[wid];
+        float* sorted = s_sort[wid];
+        int* end = s_end[wid];
+        // bucket of a distance or eps up to emax
+        const float inv = emax > 0.f ? kRankBuckets / emax : 0.f;
+        auto bucket = [&](float v) { return min(kRankBuckets - 1, static_cast<int>(v * inv)); };
+        int n = 0;
+        bool first = true;
+        auto flush = [&]() {
+            int4* e4 = reinterpret_cast<int4*>(end);
+            static_assert(kRankBuckets == 128, "four buckets per lane");
+            e4[lane] = make_int4(0, 0, 0, 0);
+            __syncwarp();
+            for (int t = lane; t < n; t += 32) atomicAdd(end + bucket(list[t]), 1);
+            __syncwarp();
+            int4 c = e4[lane];
+            const int sum = c.x + c.y + c.z + c.w;
+            int base = sum;
 #pragma unroll
-            for (int p = 0; p < kCountGroup; ++p)
-                if (p < grp.npairs) out[A.pairs[grp.pairs[p]].scratch + i] = cnt[p];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, base, o);
+                if (lane >= o) base += y;
+            }
+            base -= sum;
+            e4[lane] = make_int4(base, base + c.x, base + c.x + c.y, base + c.x + c.y + c.z);
+            __syncwarp();
+            for (int t = lane; t < n; t += 32) {
+                const float v = list[t];
+                sorted[atomicAdd(end + bucket(v), 1)] = v;
+            }
+            __syncwarp();
+            // end[b] is now the end of bucket b
+            for (int p = lane; p < P; p += 32) {
+                const long long ref = __ldg(refs + p);
+                const float e = __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i);
+                const int b = bucket(e);
+                const int t0 = b ? end[b - 1] : 0, t1 = end[b];
+                int cnt = t0;
+                for (int t = t0; t < t1; ++t) cnt += sorted[t] <= e;
+                int* out = (ref & 1 ? A.cnt_b : A.cnt_a) + (ref >> 1) + i;
+                *out = first ? cnt : *out + cnt;
+            }
+            __syncwarp();
+            first = false;
+            n = 0;
+        };
+        for (int r = 0; r < nrows; ++r) {
+            const int b = __shfl_sync(kFull, lo, r), t = __shfl_sync(kFull, hi, r);
+            for (int p0 = b; p0 < t; p0 += 32) {
+                const int pos = p0 + lane;
+                const float dm = pos < t ? distance(pos) : inf_f();
+                const bool in = pos < t && dm <= emax;
+                const unsigned mask = __ballot_sync(kFull, in);
+                if (in) list[n + __popc(mask & ((1u << lane) - 1u))] = dm;
+                n += __popc(mask);
+                if (n > kRankList - 32) {
+                    __syncwarp();
+                    flush();
+                }
+            }
         }
-        if (A.evals && lane == 0) {
-            // one distance per (query, frame), compared with every pair's eps
-            const unsigned long long ev =
-                static_cast<unsigned long long>(scanned) * min(kCountQueries, m - blk * kCountQueries);
-            atomicAdd(A.evals + 1, ev);
-            atomicAdd(A.evals + 2, ev * grp.npairs);
-        }
+        __syncwarp();
+        if (n > 0 || first) flush();
+    }
+    if (A.evals && lane == 0) {
+        atomicAdd(A.evals + 1, scanned);
+        atomicAdd(A.evals + 2, scanned * P);
     }
 }
 

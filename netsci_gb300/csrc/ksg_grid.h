@@ -39,13 +39,28 @@ struct GridNode {
     int* perm;             // [m] frames in cell order
     int* start;            // cell index (grid_index_bytes(G)), see above
     float* sx;             // [d][m] coordinates in cell order (plane stride m)
-    // [m] local scale of frame j: the distance to its kEstRank-th nearest
-    // frame among those of the 3 x 3 cells around its own (+inf if fewer)
+    // [m] local scale of frame j: about the distance to its est_rank(m)-th
+    // nearest frame (bits_launch_est)
     float* est;
+    // For the bitmap search (ksg_bits.cuh), coordinates in the order c1, c2,
+    // the other one:
+    float* aos;             // [m] frames of 1, 2 or 4 floats (d = 1, 2, 3)
+    unsigned* bins;         // [m] bin of each coordinate, one byte each
+    unsigned short* order;  // [m] frames by their bin of c1 (m <= 65536)
+    float* bedges;          // [d][64] least sampled value, the kBitBins - 1 edges, largest one
+    float* quant;           // [d][kQuantFloats] quantiles of each coordinate (grid_launch_nodes)
+    int* ostart;            // [64] first position of each c1 bin, then m; [63]: a coordinate is not finite
 };
+// Bins per coordinate of the bitmaps, and their largest m (positions are
+// 16-bit).
+constexpr int kBitBins = 54;
+constexpr int kBitMaxM = 65535;
+// Quantiles of one coordinate: kGridMaxG cell edges, 64 bitmap edges (least
+// sampled value, kBitBins - 1 edges, largest), 10-90% spread.
+constexpr int kQuantFloats = kGridMaxG + 64 + 16;
 
 // Neighbour rank of the node scale estimate (GridNode::est).
-constexpr int kEstRank = 6;
+__host__ __device__ inline float est_rank(int m) { return m < 64 ? 4.f : m < 1024 ? m / 16.f : 64.f; }
 
 // Pair grid of one pair of a batch (device descriptor).
 struct GridPair {
@@ -56,17 +71,36 @@ struct GridPair {
     int* qpos;             // [m] search order: position of the query of each rank
 };
 
-// Pairs of a batch that count the same variable (node grid): their counts
-// share every distance evaluation.
-constexpr int kCountGroup = 4;
+// Counts of a batch. A pair's variable is counted on its node's grid, and
+// all variables of a batch on one node share the node's distances:
+//   * a few of them (up to kCountGroup) form a count group: a warp takes 16
+//     queries and compares every distance with each variable's eps;
+//   * more of them form a rank node: a warp takes one query, sorts the
+//     distances up to the largest eps into buckets once, and each lane finds
+//     the rank of one variable's eps.
+constexpr int kCountGroup = 7;
 // Queries per warp in the counts: two lanes per query, each taking every
 // other frame, so the union of the warp's query boxes is that of 16 queries.
 constexpr int kCountQueries = 16;
+// A variable: twice the batch-relative pair index, plus 1 for variable b.
 struct CountGroup {
     int node;                      // node grid
-    int side;                      // 0: variable a of the pairs, 1: variable b
-    int npairs;                    // 1..kCountGroup
-    int pairs[kCountGroup];        // batch-relative pair indices
+    int nvars;                     // 1..kCountGroup
+    int vars[kCountGroup];         // unused ones repeat vars[0]
+};
+struct RankNode {
+    int node;
+    int first, count;              // its variables in CountWork::refs
+    int m;
+};
+// Queries a rank CTA takes, one per warp.
+constexpr int kRankWarps = 4;
+struct CountWork {
+    std::vector<CountGroup> groups;
+    std::vector<int> gprefix;      // [groups + 1] prefix of ceil(m / kCountQueries)
+    std::vector<RankNode> ranks;
+    std::vector<int> rprefix;      // [ranks + 1] prefix of ceil(m / kRankWarps)
+    std::vector<long long> refs;   // variables of the rank nodes: scratch offset * 2 + side
 };
 
 struct GridArgs {
@@ -75,8 +109,16 @@ struct GridArgs {
     const GridNode* nodes;
     const int* wprefix;         // [npairs+1] prefix of ceil(m/32) over the batch (search items)
     const CountGroup* groups;   // count groups of the batch
-    const int* gprefix;         // [ngroups+1] prefix of ceil(m/32) over the groups (count items)
+    const int* gprefix;         // [ngroups+1] prefix of their items (CountWork::gprefix)
     int ngroups;
+    const RankNode* ranks;      // rank nodes of the batch
+    const int* rprefix;         // [nranks+1] prefix of their items
+    const long long* refs;      // their variables
+    int nranks, rank_items;
+    // [nranks][rank_ld] largest eps of each rank node's frames, filled by
+    // grid_launch_count_order; nullptr: the rank kernel finds them itself
+    float* rank_emax;
+    int rank_ld;
     int npairs;
     int pair_base;              // index of pairs[0] in the plan's pair array (tie entries)
     int k;
@@ -136,24 +178,28 @@ struct GatherRow {
     int ld, m, ld_out;
 };
 
-// Appends the count groups of npairs pairs (descriptors with node indices a,
-// b; pair indices relative to gps): for each side, the pairs that count the
-// same node, in order, kCountGroup at a time.
-void append_count_groups(const GridPair* gps, int npairs, std::vector<CountGroup>& out);
+// The counts of npairs pairs (node indices in gps, scratch offsets and m in
+// descs): nodes with at least min_rank variables become rank nodes.
+CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, int min_rank);
+// Variables from which a node's counts are cheaper by rank: a query's ranks
+// cost about as much as six groups' distances whatever their number. Batches
+// that build no orders are latency-bound and rank every node: a warp per query.
+constexpr int kRankMinVars = 8;
 
 // Cells per axis for m samples (about ten frames per cell, at most kGridMaxG).
 int grid_cells_per_axis(int m);
 // Bytes of one node grid's buffers, and its descriptor with the buffers at
 // `base` (16-byte aligned) for row x (stride ld) of m samples.
 size_t grid_node_bytes(int m, int d);
-GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m);
+GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m, int d);
 // Places a pair grid's buffers at byte offset `off` of a batch arena
 // (pointers hold offsets until grid_pair_rebase) and returns the end offset.
 size_t grid_pair_place(GridPair& g, size_t off, int m, int d);
 void grid_pair_rebase(GridPair& g, const void* base);
-// Node grids (nodes: device array whose x, ld, m, G and buffers are set),
-// with their scale estimates when `est` (needed by the search orders).
-void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool est, cudaStream_t st);
+// Node grids (nodes: device array whose x, ld, m, G and buffers are set), in
+// one kernel, or, with `split`, in three: quantiles (a CTA per node and
+// coordinate), cells, bitmap frames.
+void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool split, cudaStream_t st);
 // Pair grids of a batch (pairs, gps: device arrays of npairs) and, when
 // `order` (the nodes carry scale estimates), their search orders. max_m: the
 // largest m of the pairs (sizes the shared-memory staging). Returns
@@ -169,8 +215,9 @@ void grid_launch_search(const GridArgs& a, int d, int kmax, int grid, bool tie_r
 void grid_launch_search_rec(const GridArgs& a, int d, int kmax, int grid, cudaStream_t st);
 void grid_launch_counts(const GridArgs& a, int d, int grid, cudaStream_t st);
 // The two halves of grid_launch_counts: the count-order kernel (when the
-// args carry a count order; returns the args the count kernel takes), then
-// the count kernel itself.
+// args carry a count order and there are groups) and the rank nodes' largest
+// eps (when they carry a buffer); returns the args the count kernels take.
+// Then the group and rank kernels (each where it has work).
 GridArgs grid_launch_count_order(const GridArgs& a, cudaStream_t st);
 void grid_launch_count_kernel(const GridArgs& c, int d, int grid, cudaStream_t st);
 void grid_launch_combine(const KsgPairDesc* pairs, int npairs, const int* cnt_a, const int* cnt_b,

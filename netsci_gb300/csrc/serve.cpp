@@ -9,6 +9,7 @@
 
 #include "apsp.h"
 #include "errors.h"
+#include "ksg_bits.h"
 #include "ksg_registry.cuh"
 
 namespace nsg {
@@ -167,11 +168,12 @@ int Server::register_trajectory(const float* X, int N, int m, int d) {
         const size_t row = static_cast<size_t>(d) * t->ld;
         for (int a = 0; a < N; ++a) {
             nodes[a] = grid_node_at(t->grid_arena.as<unsigned char>() + per * a, t->X.as<float>() + a * row,
-                                    t->ld, m);
+                                    t->ld, m, d);
         }
         GridNode* dst = d_gnodes_.as<GridNode>() + t->slot0;
         NSG_CUDA(cudaMemcpy(dst, nodes.data(), sizeof(GridNode) * N, cudaMemcpyHostToDevice));
-        grid_launch_nodes(dst, N, d, true, nullptr);
+        grid_launch_nodes(dst, N, d, false, nullptr);
+        bits_launch_est(dst, N, m, d, nullptr);
         NSG_CUDA(cudaDeviceSynchronize());
         next_node_slot_ += N;
     } else {
@@ -325,12 +327,13 @@ bool Server::try_admit_locked(Job& j) {
             GridNode nodes[2];
             for (int r = 0; r < 2; ++r) {
                 nodes[r] = grid_node_at(j.grid_arena.as<unsigned char>() + per * r,
-                                        j.dx.as<float>() + static_cast<size_t>(r) * j.d * j.ld, j.ld, j.n);
+                                        j.dx.as<float>() + static_cast<size_t>(r) * j.d * j.ld, j.ld, j.n, j.d);
             }
             GridNode* dst = d_gnodes_.as<GridNode>() + j.mi_slot;
             NSG_CUDA(cudaMemcpyAsync(dst, nodes, sizeof(nodes), cudaMemcpyHostToDevice, ksg_stream_));
             NSG_CUDA(cudaStreamSynchronize(ksg_stream_));  // the host descriptors go out of scope
-            grid_launch_nodes(dst, 2, j.d, true, ksg_stream_);
+            grid_launch_nodes(dst, 2, j.d, false, ksg_stream_);
+            bits_launch_est(dst, 2, j.n, j.d, ksg_stream_);
             j.slots.push_back({j.mi_slot, j.mi_slot + 1});
         }
     }
@@ -398,13 +401,14 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
             GridPair& g = h_gpairs_[p];
             g.a = j->slots[q].first;
             g.b = j->slots[q].second;
-            arena = grid_pair_place(g, arena, pr.m, d);
             h_wpre_[p] = static_cast<int>(wacc);
             wacc += (pr.m + 31) / 32;
             maxm = std::max(maxm, pr.m);
         }
     }
     h_wpre_[np] = static_cast<int>(wacc);
+    const BitsConfig bits = bits_config(d, k, maxm);
+    for (long long i = 0; i < np && !bits.ok; ++i) arena = grid_pair_place(h_gpairs_[i], arena, h_pairs_[i].m, d);
     cudaStream_t s = ksg_stream_;
     // buffers grow on demand (by a quarter more than asked, to grow rarely)
     auto ensure = [&](DeviceBuffer& b, size_t bytes) {
@@ -418,27 +422,30 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     ensure(d_eps_b_, sizeof(float) * samples);
     ensure(d_cnt_a_, sizeof(int) * samples);
     ensure(d_cnt_b_, sizeof(int) * samples);
-    for (long long i = 0; i < np; ++i) grid_pair_rebase(h_gpairs_[i], d_garena_.get());
+    for (long long i = 0; i < np && !bits.ok; ++i) grid_pair_rebase(h_gpairs_[i], d_garena_.get());
     NSG_CUDA(cudaMemcpyAsync(d_pairs_.get(), h_pairs_, sizeof(KsgPairDesc) * np, cudaMemcpyHostToDevice, s));
     NSG_CUDA(cudaMemcpyAsync(d_gpairs_.get(), h_gpairs_, sizeof(GridPair) * np, cudaMemcpyHostToDevice, s));
     NSG_CUDA(cudaMemcpyAsync(d_wpre_.get(), h_wpre_, sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
-    // count groups: pairs of the tick that count the same node's variable
-    std::vector<CountGroup> groups;
-    append_count_groups(h_gpairs_, static_cast<int>(np), groups);
-    std::vector<int> gpre(groups.size() + 1, 0);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        gpre[gi + 1] = gpre[gi] + (h_pairs_[groups[gi].pairs[0]].m + kCountQueries - 1) / kCountQueries;
-    }
+    // count groups and rank nodes: variables of the tick on the same node
     const bool order = grid_orders_pay(wacc, sm_count());  // query orders for this tick
+    const CountWork work_list = count_work(h_gpairs_, h_pairs_, static_cast<int>(np), order ? kRankMinVars : 1);
+    const auto& groups = work_list.groups;
     if (order) ensure(d_corder_, sizeof(int) * std::max<size_t>(1, groups.size() * static_cast<size_t>(maxm)));
-    NSG_CUDA(cudaMemcpyAsync(d_groups_.get(), groups.data(), sizeof(CountGroup) * groups.size(),
-                             cudaMemcpyHostToDevice, s));
-    NSG_CUDA(cudaMemcpyAsync(d_gpre_.get(), gpre.data(), sizeof(int) * gpre.size(), cudaMemcpyHostToDevice, s));
+    auto put = [&](DeviceBuffer& b, const auto& v) {
+        if (v.empty()) return;
+        ensure(b, v.size() * sizeof(v[0]));
+        NSG_CUDA(cudaMemcpyAsync(b.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s));
+    };
+    put(d_groups_, groups);
+    put(d_gpre_, work_list.gprefix);
+    put(d_ranks_, work_list.ranks);
+    put(d_rpre_, work_list.rprefix);
+    put(d_refs_, work_list.refs);
     NSG_CUDA(cudaMemsetAsync(d_counters_.get(), 0, sizeof(int) * 4, s));
     int* ctr = d_counters_.as<int>();
     KsgPairDesc* dp = d_pairs_.as<KsgPairDesc>();
-    const int search_order = grid_launch_pairs(dp, d_gpairs_.as<GridPair>(), d_gnodes_.as<GridNode>(),
-                                               static_cast<int>(np), maxm, d, order, s);
+    const int search_order = bits.ok ? 0 : grid_launch_pairs(dp, d_gpairs_.as<GridPair>(), d_gnodes_.as<GridNode>(),
+                                                             static_cast<int>(np), maxm, d, order, s);
     GridArgs a{};
     a.search_order = search_order;
     a.pairs = dp;
@@ -448,6 +455,11 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     a.groups = d_groups_.as<CountGroup>();
     a.gprefix = d_gpre_.as<int>();
     a.ngroups = static_cast<int>(groups.size());
+    a.ranks = d_ranks_.as<RankNode>();
+    a.rprefix = d_rpre_.as<int>();
+    a.refs = d_refs_.as<long long>();
+    a.nranks = static_cast<int>(work_list.ranks.size());
+    a.rank_items = work_list.rprefix.back();
     a.npairs = static_cast<int>(np);
     a.pair_base = 0;
     a.k = k;
@@ -463,7 +475,8 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     a.corder = order ? d_corder_.as<int>() : nullptr;
     a.corder_ld = maxm;
     const int sms = sm_count();
-    grid_launch_search(a, d, kmax, sms * grid_search_ctas_per_sm(d, kmax), false, s);
+    if (bits.ok) bits_launch_search(a, bits, maxm, d, s);
+    else grid_launch_search(a, d, kmax, sms * grid_search_ctas_per_sm(d, kmax), false, s);
     a.counter = ctr + 1;
     grid_launch_counts(a, d, sms * grid_count_ctas_per_sm(d), s);
     grid_launch_combine(dp, static_cast<int>(np), a.cnt_a, a.cnt_b, psi_->as<float>(), d_scratch_.as<float>(),

@@ -173,8 +173,9 @@ constexpr int kGridMinSamples = 1000;
 // 0.72 ms at m = 10000.
 constexpr int kGridFewPairs = 8;
 constexpr int kGridMinSamplesFew = 4000;
-// per batch: work-queue heads (two for the grid search), tie count, tie-kernel counter
-constexpr int kCounters = 4;
+// per batch: work-queue heads (two for the grid search), tie count,
+// tie-kernel counter, rank-count queue head
+constexpr int kCounters = 5;
 }  // namespace
 
 std::shared_ptr<const DeviceBuffer> device_psi(int n) {
@@ -623,7 +624,7 @@ struct KsgPlan::GridState {
     DeviceBuffer gps, pair_arena;         // GridPair per plan pair; pair grids of one batch
     std::vector<int> batch_maxm;          // largest m of each batch
     std::vector<char> batch_order;        // whether each batch builds query orders
-    bool split_nodes = false;             // an ordered batch: many nodes, three kernels
+    bool split_nodes = false;             // an ordered batch: many nodes, four kernels
     bool node_est = false;                // a batch needs the nodes' scale estimates
     std::vector<BitsConfig> batch_bits;   // bitmap search where ok, else the scan on pair grids
     int max_m = 0;
@@ -635,7 +636,6 @@ struct KsgPlan::GridState {
     DeviceBuffer ranks, rprefix, refs;    // rank nodes, item prefix and variables, per batch
     std::vector<long long> rank_off, rprefix_off, ref_off;
     std::vector<int> nranks, rank_items;
-    DeviceBuffer rank_emax;               // nranks x largest m of an ordered batch
     DeviceBuffer corder;                  // count-query order: ngroups x largest m of a batch
     DeviceBuffer eps_a, eps_b, cnt_a, cnt_b;
     DeviceBuffer evals;                   // 3 counters per run (see GridArgs::evals)
@@ -721,7 +721,7 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
         std::vector<RankNode> ranks;
         std::vector<int> gpre, rpre;
         std::vector<long long> refs;
-        size_t corder = 0, emax = 0;
+        size_t corder = 0;
         for (size_t bi = 0; bi < batches_.size(); ++bi) {
             const Batch& b = batches_[bi];
             const bool order = g->batch_order[bi] != 0;
@@ -742,7 +742,6 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
             refs.insert(refs.end(), w.refs.begin(), w.refs.end());
             if (order) {
                 corder = std::max(corder, w.groups.size() * static_cast<size_t>(g->batch_maxm[bi]));
-                emax = std::max(emax, w.ranks.size() * static_cast<size_t>(g->batch_maxm[bi]));
             }
         }
         auto upload = [](DeviceBuffer& dst, const auto& v) {
@@ -751,7 +750,6 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
             NSG_CUDA(cudaMemcpy(dst.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
         };
         g->corder.reset(corder * sizeof(int));
-        g->rank_emax.reset(emax * sizeof(float));
         upload(g->groups, groups);
         upload(g->gprefix, gpre);
         upload(g->ranks, ranks);
@@ -804,8 +802,7 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         a.refs = g.refs.as<long long>() + g.ref_off[bi];
         a.nranks = g.nranks[bi];
         a.rank_items = g.rank_items[bi];
-        a.rank_emax = order ? g.rank_emax.as<float>() : nullptr;
-        a.rank_ld = g.batch_maxm[bi];
+        a.rank_counter = ctr + 4;
         a.npairs = b.npairs;
         a.pair_base = b.pair0;
         a.k = k_;
@@ -837,7 +834,7 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         if (timing_) record_event(ev[2], s);
         grid_launch_count_kernel(c, d_, g.count_grid, s);
         if (timing_) record_event(ev[3], s);
-        grid_launch_combine(bp, b.npairs, g.cnt_a.as<int>(), g.cnt_b.as<int>(), psi_->as<float>(),
+        grid_launch_combine(bp, b.npairs, g.batch_maxm[bi], g.cnt_a.as<int>(), g.cnt_b.as<int>(), psi_->as<float>(),
                             scratch_.as<float>(), out_.nx, out_.ny, s);
         KsgTieArgs t{};
         t.pairs = pairs_dev_.as<KsgPairDesc>();
@@ -879,17 +876,16 @@ int KsgPlan::launches() const {
     if (!nb) return 0;
     // node grids (+ scale estimates), gather; per batch: search, combine,
     // ties, final sums, group and rank counts (+ pair grids where the search
-    // scans them; in batches with orders + search order, count order, the
-    // rank nodes' largest eps)
+    // scans them; in batches with orders + search and count orders)
     int n = 1 + (ngather_ ? 1 : 0) + 4 * nb;
     if (grid_) {
-        if (grid_->split_nodes) n += 2;
+        if (grid_->split_nodes) n += 3;
         if (grid_->node_est) ++n;
         for (size_t bi = 0; bi < grid_->batch_order.size(); ++bi) {
             const bool order = grid_->batch_order[bi] != 0, short_m = grid_->batch_maxm[bi] <= kOrderMaxM;
             if (!grid_->batch_bits[bi].ok) n += order && short_m ? 2 : 1;
             if (grid_->ngroups[bi]) n += order && short_m ? 2 : 1;
-            if (grid_->nranks[bi]) n += order ? 2 : 1;
+            if (grid_->nranks[bi]) ++n;
         }
     }
     return n;

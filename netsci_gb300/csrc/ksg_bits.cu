@@ -103,6 +103,9 @@ void bits_launch_search(const GridArgs& g, const BitsConfig& c, int max_m, int d
     const int slots = sm_count() * c.ctas_per_sm;
     const int most = std::max(1, max_m / (2 * (c.threads / 32)));
     a.chunks = g.npairs >= 4 * slots ? 1 : std::min(most, (4 * slots + g.npairs - 1) / g.npairs);
+    // a share of few queries is spread over all warps
+    const int per_warp = max_m / (a.chunks * (c.threads / 32));
+    a.grab = std::max(1, std::min(bit_queries(d), per_warp));
     const long long items = static_cast<long long>(g.npairs) * a.chunks;
     const int grid = static_cast<int>(std::min<long long>(items, slots));
     switch (d) {

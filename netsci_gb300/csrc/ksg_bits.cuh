@@ -27,7 +27,7 @@
 //     the k-th distance, eps and the tie test.
 //   * h comes from the two nodes' scale estimates: sqrt(est_a est_b) follows
 //     the k-th joint distance with a spread of 8 to 14%. Each warp scales it
-//     so that about one query in ten finds fewer than k frames within h and
+//     so that about one query in fifteen finds fewer than k frames within h and
 //     tries again with a larger h; whatever h is, the accepted set is complete
 //     (every frame within h was evaluated, and at least k others were).
 //   * A full list of frames within h gives a smaller h, its own k-th distance.
@@ -144,17 +144,28 @@ __device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int
     return pos + __ffs(bits) - 1;
 }
 
-// Rows of one coordinate for frames 32 w .. 32 w + 31 (one bin per lane,
-// above every bin where there is no frame): lane t keeps the ballot of row t.
-__device__ __forceinline__ void build_rows(unsigned* rows, int WS, int w, int R, int step, unsigned bin, int lane) {
-    for (int r0 = 0; r0 < R; r0 += 32) {
-        unsigned mine = 0;
-        const int top = min(32, R - r0);
-        for (int t = 0; t < top; ++t) {
-            const unsigned x = __ballot_sync(kFull, bin < static_cast<unsigned>(min((r0 + t) * step, kBitBins)));
-            if (lane == t) mine = x;
+// Rows of one coordinate for frames 32 w .. 32 w + 31: lane l holds the bin
+// of frame 32 w + l where `frame` says that there is one, and then writes
+// rows l and 32 + l, the frames whose bin is below that row's. The six bits
+// of the bins become six ballots, and each lane compares them with its row's
+// limit bit by bit (a ballot per row took three times the instructions).
+__device__ __forceinline__ void build_rows(unsigned* rows, int WS, int w, int R, int step, unsigned bin, bool frame,
+                                           int lane) {
+    static_assert(kBitBins < 64, "bins and limits have six bits");
+    unsigned plane[6];
+#pragma unroll
+    for (int b = 0; b < 6; ++b) plane[b] = __ballot_sync(kFull, bin >> b & 1u);
+    const unsigned have = __ballot_sync(kFull, frame);
+    for (int r = lane; r < R; r += 32) {
+        const int limit = min(r * step, kBitBins);
+        unsigned below = 0, equal = have;
+#pragma unroll
+        for (int b = 5; b >= 0; --b) {
+            const unsigned bit = limit >> b & 1 ? kFull : 0u;
+            below |= equal & bit & ~plane[b];
+            equal &= ~(bit ^ plane[b]);
         }
-        if (lane < top) rows[(r0 + lane) * WS + w] = mine;
+        rows[r * WS + w] = below;
     }
 }
 
@@ -367,7 +378,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
         const int p = item / B.chunks, ch = item - p * B.chunks;
         const KsgPairDesc* P = A.pairs + p;
         const int m = P->m;
-        const int share = ((m + B.chunks - 1) / B.chunks + Q - 1) / Q * Q;
+        const int share = ((m + B.chunks - 1) / B.chunks + B.grab - 1) / B.grab * B.grab;
         const int qlo = ch * share, qhi = min(m, qlo + share);
         if (qlo >= qhi) continue;
         const int na_id = A.gp[p].a, nb_id = A.gp[p].b;
@@ -389,23 +400,31 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
             const float* edges = c < D ? na->bedges + c * 64 : nb->bedges + (c - D) * 64;
             s_edge[c][e & 63] = t < kBitBins ? __ldg(edges + t) : inf_f();
         }
-        // rows: lane t keeps the ballot of row t
+        // rows
         {
+            // the next word's bins load while this one's rows are made
             const unsigned* __restrict__ ba = na->bins;
             const unsigned* __restrict__ bb = nb->bins;
-            for (int w = wid; w < WS; w += nwarps) {
+            unsigned va = 0, vb = 0;
+            auto fetch = [&](int w) {
                 const int pos = 32 * w + lane;
-                unsigned va = kFull, vb = kFull;
-                if (pos < m) {
+                va = vb = 0;
+                if (w < WS && pos < m) {
                     const int j = s_perm[pos];
                     if (D > 1 && new_a) va = __ldg(ba + j);
                     vb = __ldg(bb + j);
                 }
+            };
+            fetch(wid);
+            for (int w = wid; w < WS; w += nwarps) {
+                const bool frame = 32 * w + lane < m;
+                const unsigned ca = va, cb = vb;
+                fetch(w + nwarps);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     if (c < D - 1 && !new_a) continue;
-                    const unsigned bin = c < D - 1 ? (va >> (8 * (c + 1)) & 0xffu) : (vb >> (8 * (c - (D - 1))) & 0xffu);
-                    build_rows(s_dyn + c * R * WS, WS, w, R, step, bin, lane);
+                    const unsigned bin = c < D - 1 ? ca >> (8 * (c + 1)) : cb >> (8 * (c - (D - 1)));
+                    build_rows(s_dyn + c * R * WS, WS, w, R, step, bin, frame, lane);
                 }
             }
         }
@@ -432,10 +451,10 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
         };
         for (;;) {
             int q0 = 0;
-            if (lane == 0) q0 = atomicAdd(&s_next, Q);
+            if (lane == 0) q0 = atomicAdd(&s_next, B.grab);
             q0 = __shfl_sync(kFull, q0, 0) + qlo;
             if (q0 >= qhi) break;
-            const int nq = min(Q, qhi - q0);
+            const int nq = min(B.grab, qhi - q0);
             __syncwarp();
             if (lane < 2 * Q && lane % Q < nq) {
                 const int t = lane % Q, i = q0 + t;
@@ -472,6 +491,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                     const unsigned* bins = s_bins + 2 * D * t;
                     const int x0 = bins[0] & 0xffffu, x1 = bins[0] >> 16;
                     int inside = 0;
+                    int crowd = 0;
                     bool stuck = false;
                     // the AND of the row pairs over one uint4 column
                     auto column = [&](int x) {
@@ -502,6 +522,11 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                             inside += n;
                             return true;
                         }
+                        if (n > kCrowd * (k + 1) && tries == 0) {
+                            // another look at the rows is cheaper than that many frames
+                            crowd = n;
+                            return true;
+                        }
                         evals += n;
                         for (int win = 0; win < n; win += 32) {
                             const int pos = bit_of_rank(w, base, incl - cnt, cnt, win, lane, s_table);
@@ -518,10 +543,15 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                             unsigned in = __ballot_sync(kFull, v <= h);
                             if (inside + __popc(in) > kKeep) {
                                 // k others lie within a smaller h
-                                if (inside > k) inside = keep_nearest<N>(s_v, s_da, s_db, inside, k, lane, &h);
-                                else h = __uint_as_float(kth_lane(v <= h ? __float_as_uint(v) : kFull, k));
-                                in = __ballot_sync(kFull, v <= h);
-                                if (inside + __popc(in) > kKeep) return false;
+                                if (inside > k) {
+                                    inside = keep_nearest<N>(s_v, s_da, s_db, inside, k, lane, &h);
+                                    in = __ballot_sync(kFull, v <= h);
+                                }
+                                if (inside + __popc(in) > kKeep) {
+                                    if (__popc(in) > k) h = __uint_as_float(kth_lane(v <= h ? __float_as_uint(v) : kFull, k));
+                                    in = __ballot_sync(kFull, v <= h);
+                                    if (inside + __popc(in) > kKeep) return false;
+                                }
                             }
                             if (v <= h) {
                                 const int slot = inside + __popc(in & ((1u << lane) - 1u));
@@ -534,7 +564,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                         }
                         return true;
                     };
-                    for (int xf = x0; xf < x1 && !stuck; xf += 64) {
+                    for (int xf = x0; xf < x1 && !stuck && !crowd; xf += 64) {
                         const int x = xf + lane;
                         const uint4 u = column(x);
                         if (xf + 32 >= x1) {
@@ -551,17 +581,21 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                         }
                     }
                     if (stuck) break;
-                    if (inside > k) {
+                    if (crowd) {
+                        scale *= 0.9985f;
+                        h *= exp2f(__log2f(0.5f * kCrowd * (k + 1) / crowd) * (0.5f / D));
+                    } else if (inside > k) {
                         if (lane < 4) s_v[inside + lane] = inf_f();
                         __syncwarp();
                         r = select_nearest<N>(s_v, s_da, s_db, inside, k, lane);
                         __syncwarp();
-                        if (tries == 0) scale *= 0.995f;
+                        if (tries == 0) scale *= 0.9985f;
                         done = true;
                         break;
+                    } else {
+                        if (tries == 0) scale *= 1.02f;
+                        h *= fminf(2.f, exp2f(__log2f(2.f * (k + 1) / (inside + 0.5f)) * (0.5f / D)));
                     }
-                    if (tries == 0) scale *= 1.05f;
-                    h *= fminf(2.f, exp2f(__log2f(2.f * (k + 1) / (inside + 0.5f)) * (0.5f / D)));
                     if (lane == 0) s_query[8 * t + 3] = h;
                     __syncwarp();
                     if (lane < 2 * D) set_bins(t, lane);
@@ -612,7 +646,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
 // geometric mean of two nodes' estimates follows the k-th joint distance to
 // 8% (nearly independent coordinates) and 12% (correlated ones), as well as
 // the exact 64th-neighbour distances do.
-constexpr int kEstThreads = 512;
+constexpr int kEstThreads = 1024;
 
 template <int D>
 __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* nodes, int step) {
@@ -637,12 +671,19 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
     }
     if (tid < 64) s_start[tid] = __ldg(nd.ostart + tid);
     if constexpr (D > 1) {
+        // the next word's bins load while this one's rows are made
+        auto bins_of = [&](int w) {
+            const int pos = 32 * w + lane;
+            return w < WS && pos < m ? __ldg(nd.bins + __ldg(nd.order + pos)) : 0u;
+        };
+        unsigned next = bins_of(wid);
         for (int w = wid; w < WS; w += nwarps) {
             const int pos = 32 * w + lane;
-            const unsigned v = pos < m ? __ldg(nd.bins + __ldg(nd.order + pos)) : kFull;
+            const unsigned v = next;
+            next = bins_of(w + nwarps);
 #pragma unroll
             for (int c = 1; c < D; ++c)
-                build_rows(s_dyn + (c - 1) * R * WS, WS, w, R, step, v >> (8 * c) & 0xffu, lane);
+                build_rows(s_dyn + (c - 1) * R * WS, WS, w, R, step, v >> (8 * c), pos < m, lane);
         }
     }
     __syncthreads();

@@ -8,7 +8,9 @@
 namespace nsg {
 
 constexpr int kBitTries = 6;      // search radii tried before a query scans all frames
-// Queries a warp takes at a time: a lane per query and coordinate.
+// Bitmap hits per wanted frame from which a first radius is cut back unseen.
+constexpr int kCrowd = 10;
+// Queries a warp takes at a time, at most: a lane per query and coordinate.
 __host__ __device__ constexpr int bit_queries(int d) { return d == 3 ? 4 : 8; }
 // Shared words per warp: queries, the 32 n nearest frames' distances, bins, bit_of_rank's table.
 __host__ __device__ constexpr int bit_warp_words(int d, int n) {
@@ -23,6 +25,7 @@ __host__ __device__ inline int bit_row_words(int m) { return ((((m + 31) / 32 + 
 struct BitsArgs {
     GridArgs g;
     int chunks;                 // work items: g.npairs * chunks
+    int grab;                   // queries a warp takes at a time (at most bit_queries)
     int rows, step;             // rows per coordinate, bins per row
     int rows_words, perm_words; // shared-memory layout (words)
 };

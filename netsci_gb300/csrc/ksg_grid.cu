@@ -11,6 +11,13 @@
 namespace nsg {
 namespace {
 
+int device_sms() {
+    int dev = 0, sms = 0;
+    NSG_CUDA(cudaGetDevice(&dev));
+    NSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms;
+}
+
 constexpr int kPrepThreads = 1024;
 constexpr int kSample = 2048;       // frames sampled per coordinate for the quantiles
 
@@ -140,38 +147,67 @@ __device__ __forceinline__ void node_axes(const float* quant, int (&axis)[3]) {
     axis[2] = D == 3 ? 3 - c1 - c2 : 0;
 }
 
-// Cells of a node's grid, counting sort by cell.
+// Cell and bitmap bins of frames [lo, hi) of a node, and their coordinates in
+// the bitmap search's layout.
 template <int D>
-__device__ void node_cells(GridNode* node, const GridNode& nd, const float* quant) {
+__device__ void node_bins(GridNode* node, const GridNode& nd, const float* quant, int lo, int hi) {
     __shared__ float s_e1[kGridMaxG], s_e2[kGridMaxG];
-    __shared__ int s_cnt[kGridMaxG * kGridMaxG];
-    __shared__ int s_start[kGridMaxG * kGridMaxG + 1];
-    __shared__ int s_tmp1[kGridMaxG * kGridMaxG], s_tmp2[kGridMaxG * kGridMaxG + 1];
-    const int m = nd.m, G = nd.G, t = threadIdx.x;
+    __shared__ float s_be[D][64];
+    const int G = nd.G, t = threadIdx.x;
     int axis[3];
     node_axes<D>(quant, axis);
     const int c1 = axis[0], c2 = axis[1];
     if (t < kGridMaxG) {
         s_e1[t] = quant[c1 * kQuantFloats + t];
         s_e2[t] = c2 >= 0 ? quant[c2 * kQuantFloats + t] : __int_as_float(0x7f800000);
-        nd.e1[t] = s_e1[t];
-        nd.e2[t] = s_e2[t];
+        if (lo == 0) {
+            nd.e1[t] = s_e1[t];
+            nd.e2[t] = s_e2[t];
+        }
     }
-    if (t == 0) {
+    if (t == 0 && lo == 0) {
         node->c1 = c1;
         node->c2 = c2;
     }
+    for (int e = t; e < 64 * D; e += blockDim.x) {
+        const int c = e >> 6;
+        const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
+        s_be[c][e & 63] = quant[ax * kQuantFloats + kGridMaxG + (e & 63)];
+        if (lo == 0) nd.bedges[e] = s_be[c][e & 63];
+    }
+    __syncthreads();
+    bool bad = false;
+    for (int j = lo + t; j < hi; j += blockDim.x) {
+        float x[D];
+        unsigned bins = 0;
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
+            x[c] = __ldg(nd.x + static_cast<long long>(ax) * nd.ld + j);
+            bad |= !isfinite(x[c]);
+            bins |= static_cast<unsigned>(bin_of(s_be[c] + 1, kBitBins - 1, x[c])) << (8 * c);
+        }
+        int cell = bin_of(s_e1, G - 1, x[0]) * G;
+        if constexpr (D > 1) cell += bin_of(s_e2, G - 1, x[1]);
+        nd.cell[j] = static_cast<unsigned short>(cell);
+        if constexpr (D == 1) nd.aos[j] = x[0];
+        else if constexpr (D == 2) reinterpret_cast<float2*>(nd.aos)[j] = make_float2(x[0], x[1]);
+        else reinterpret_cast<float4*>(nd.aos)[j] = make_float4(x[0], x[1], x[2], 0.f);
+        nd.bins[j] = bins;
+    }
+    if (bad) nd.ostart[63] = 1;
+}
+
+// Counting sort of a node's frames by cell.
+template <int D>
+__device__ void node_cells(const GridNode& nd) {
+    __shared__ int s_cnt[kGridMaxG * kGridMaxG];
+    __shared__ int s_start[kGridMaxG * kGridMaxG + 1];
+    __shared__ int s_tmp1[kGridMaxG * kGridMaxG], s_tmp2[kGridMaxG * kGridMaxG + 1];
+    const int m = nd.m, G = nd.G, t = threadIdx.x;
     for (int c = t; c < G * G; c += blockDim.x) s_cnt[c] = 0;
     __syncthreads();
-    const float* x1 = nd.x + static_cast<long long>(c1) * nd.ld;
-    const float* x2 = c2 >= 0 ? nd.x + static_cast<long long>(c2) * nd.ld : nullptr;
-    for (int j = t; j < m; j += blockDim.x) {
-        const int b1 = bin_of(s_e1, G - 1, __ldg(x1 + j));
-        const int b2 = x2 ? bin_of(s_e2, G - 1, __ldg(x2 + j)) : 0;
-        const int cell = b1 * G + b2;
-        nd.cell[j] = static_cast<unsigned short>(cell);
-        atomicAdd(&s_cnt[cell], 1);
-    }
+    for (int j = t; j < m; j += blockDim.x) atomicAdd(&s_cnt[nd.cell[j]], 1);
     __syncthreads();
     block_scan(s_cnt, s_start, G * G);
     for (int c = t; c <= G * G; c += blockDim.x) nd.start[c] = s_start[c];
@@ -190,89 +226,82 @@ __device__ void node_cells(GridNode* node, const GridNode& nd, const float* quan
     build_query_order(s_cnt, G, nd.start, s_tmp1, s_tmp2);
 }
 
-// What the bitmaps are built from: frames, bins, order by c1 bin.
-template <int D>
-__device__ void node_frames(const GridNode& nd, const float* quant) {
-    __shared__ float s_be[D][64];
+// Counting sort of a node's frames by their bitmap bin of c1.
+__device__ void node_order(const GridNode& nd) {
     __shared__ int s_ocnt[64], s_ostart[65];
-    __shared__ int s_bad;
     const int m = nd.m, t = threadIdx.x;
-    int axis[3];
-    node_axes<D>(quant, axis);
-    for (int e = t; e < 64 * D; e += blockDim.x) {
-        const int c = e >> 6;
-        const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
-        const float v = quant[ax * kQuantFloats + kGridMaxG + (e & 63)];
-        s_be[c][e & 63] = v;
-        nd.bedges[e] = v;
-    }
+    if (m > kBitMaxM) return;
     if (t < 64) s_ocnt[t] = 0;
-    if (t == 0) s_bad = 0;
     __syncthreads();
-    bool bad = false;
-    for (int j = t; j < m; j += blockDim.x) {
-        float x[D];
-        unsigned bins = 0;
-#pragma unroll
-        for (int c = 0; c < D; ++c) {
-            const int ax = c == 0 ? axis[0] : c == 1 ? axis[1] : axis[2];
-            x[c] = __ldg(nd.x + static_cast<long long>(ax) * nd.ld + j);
-            bad |= !isfinite(x[c]);
-            bins |= static_cast<unsigned>(bin_of(s_be[c] + 1, kBitBins - 1, x[c])) << (8 * c);
-        }
-        if constexpr (D == 1) nd.aos[j] = x[0];
-        else if constexpr (D == 2) reinterpret_cast<float2*>(nd.aos)[j] = make_float2(x[0], x[1]);
-        else reinterpret_cast<float4*>(nd.aos)[j] = make_float4(x[0], x[1], x[2], 0.f);
-        nd.bins[j] = bins;
-        atomicAdd(&s_ocnt[bins & 0xffu], 1);
-    }
-    if (bad) s_bad = 1;
+    for (int j = t; j < m; j += blockDim.x) atomicAdd(&s_ocnt[nd.bins[j] & 0xffu], 1);
     __syncthreads();
     block_scan(s_ocnt, s_ostart, 64);
     if (t < 64) {
-        nd.ostart[t] = t < 63 ? s_ostart[t] : s_bad;
+        if (t < 63) nd.ostart[t] = s_ostart[t];
         s_ocnt[t] = 0;
     }
     __syncthreads();
-    if (m > kBitMaxM) return;
     for (int j = t; j < m; j += blockDim.x) {
         const int b = nd.bins[j] & 0xffu;
         nd.order[s_ostart[b] + atomicAdd(&s_ocnt[b], 1)] = static_cast<unsigned short>(j);
     }
 }
 
-// One CTA per node: quantiles, cells, bitmap frames.
-template <int D>
-__global__ void __launch_bounds__(kPrepThreads) grid_node_kernel(GridNode* nodes) {
-    __shared__ float s_val[kSample];
-    __shared__ float s_quant[D * kQuantFloats];
-    const GridNode nd = nodes[blockIdx.x];
-    for (int c = 0; c < D; ++c) node_quantiles(nd, c, s_val, s_quant + c * kQuantFloats);
-    node_cells<D>(nodes + blockIdx.x, nd, s_quant);
-    node_frames<D>(nd, s_quant);
+// Everything for one node by a cluster of kNodeCtas CTAs: a coordinate's
+// quantiles each, a share of the bins each, then one counting sort each in
+// two of them. One CTA doing it in sequence took 87 us for a pair's two nodes
+// at m = 10000.
+constexpr int kNodeCtas = 4;
+
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The same in three kernels for plans of many nodes: the sort waits on
-// barriers and the counting sorts on atomics, and small CTAs of one kind
-// overlap better than 1024 threads doing one after the other.
+template <int D>
+__global__ void __cluster_dims__(kNodeCtas, 1, 1) __launch_bounds__(kPrepThreads) grid_node_kernel(GridNode* nodes) {
+    __shared__ float s_val[kSample];
+    GridNode* node = nodes + blockIdx.x / kNodeCtas;
+    const int part = blockIdx.x % kNodeCtas;
+    const GridNode nd = *node;
+    if (threadIdx.x == 0 && part == 0) nd.ostart[63] = 0;
+    if (part < D) node_quantiles(nd, part, s_val, nd.quant + part * kQuantFloats);
+    cluster_wait();
+    const int share = (nd.m + kNodeCtas - 1) / kNodeCtas;
+    const int lo = min(nd.m, part * share);
+    node_bins<D>(node, nd, nd.quant, lo, min(nd.m, lo + share));
+    cluster_wait();
+    if (part == 0) node_cells<D>(nd);
+    else if (part == 1) node_order(nd);
+}
+
+// The same in four kernels for plans of many nodes: the sample sort waits on
+// barriers, the counting sorts on atomics, and the bins on binary searches;
+// small CTAs of one kind overlap better than 1024 threads doing one after the
+// other.
 constexpr int kSplitThreads = 512;
 
 __global__ void __launch_bounds__(kSplitThreads) node_quantiles_kernel(const GridNode* nodes) {
     __shared__ float s_val[kSample];
     const GridNode nd = nodes[blockIdx.x];
+    if (threadIdx.x == 0 && blockIdx.y == 0) nd.ostart[63] = 0;
     node_quantiles(nd, blockIdx.y, s_val, nd.quant + blockIdx.y * kQuantFloats);
 }
 
 template <int D>
-__global__ void __launch_bounds__(kPrepThreads) node_cells_kernel(GridNode* nodes) {
+__global__ void __launch_bounds__(kSplitThreads) node_bins_kernel(GridNode* nodes) {
     const GridNode nd = nodes[blockIdx.x];
-    node_cells<D>(nodes + blockIdx.x, nd, nd.quant);
+    const int share = (nd.m + gridDim.y - 1) / gridDim.y;
+    const int lo = blockIdx.y * share;
+    if (lo < nd.m) node_bins<D>(nodes + blockIdx.x, nd, nd.quant, lo, min(nd.m, lo + share));
 }
 
 template <int D>
-__global__ void __launch_bounds__(kSplitThreads) node_frames_kernel(const GridNode* nodes) {
-    const GridNode nd = nodes[blockIdx.x];
-    node_frames<D>(nd, nd.quant);
+__global__ void __launch_bounds__(kPrepThreads) node_cells_kernel(const GridNode* nodes) {
+    node_cells<D>(nodes[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(kSplitThreads) node_order_kernel(const GridNode* nodes) {
+    node_order(nodes[blockIdx.x]);
 }
 
 // One CTA per pair of the batch: cells over (bin of a on its c1, bin of b on
@@ -373,7 +402,7 @@ __global__ void __launch_bounds__(kPrepThreads) grid_pair_staged_kernel(const Ks
 __global__ void grid_combine_kernel(const KsgPairDesc* pairs, const int* cnt_a, const int* cnt_b,
                                     const float* psi, float* psum, int* nx_out, int* ny_out) {
     const KsgPairDesc P = pairs[blockIdx.x];
-    for (int i = threadIdx.x; i < P.m; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < P.m; i += gridDim.y * blockDim.x) {
         const long long o = P.scratch + i;
         const int nx = min(max(cnt_a[o] - 1, 0), P.m);
         const int ny = min(max(cnt_b[o] - 1, 0), P.m);
@@ -525,20 +554,6 @@ __global__ void __launch_bounds__(kOrderThreads) grid_count_order_kernel(GridArg
                     sort_low ? s_key + A.corder_ld : nullptr);
 }
 
-// Largest eps of every frame of the rank nodes over the node's variables:
-// one CTA per node and block of frames, so that eps are read in rows.
-__global__ void __launch_bounds__(256) rank_emax_kernel(GridArgs A) {
-    const RankNode rn = A.ranks[blockIdx.x];
-    const int i = blockIdx.y * blockDim.x + threadIdx.x;
-    if (i >= rn.m) return;
-    float e = 0.f;
-    for (int p = 0; p < rn.count; ++p) {
-        const long long ref = __ldg(A.refs + rn.first + p);
-        e = fmaxf(e, __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i));
-    }
-    A.rank_emax[static_cast<long long>(blockIdx.x) * A.rank_ld + i] = e;
-}
-
 // Search order: cells in kOrderBlock x kOrderBlock blocks, blocks in Z
 // order, and within a block the queries by size class. Box Z codes of the
 // estimates, which serve the counts, made the search slower (197 against
@@ -651,7 +666,7 @@ CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, 
         if (static_cast<int>(e - s) >= min_rank) {
             w.ranks.push_back({node, static_cast<int>(w.refs.size()), static_cast<int>(e - s), m});
             w.rprefix.push_back(ritems);
-            ritems += (m + kRankWarps - 1) / kRankWarps;
+            ritems += (m + kRankBlock - 1) / kRankBlock;
             for (; s < e; ++s) {
                 const int v = keyed[s].second;
                 w.refs.push_back(descs[v >> 1].scratch * 2 + (v & 1));
@@ -688,10 +703,11 @@ template <int D>
 void launch_nodes(GridNode* nodes, int nnodes, bool split, cudaStream_t st) {
     if (split) {
         node_quantiles_kernel<<<dim3(nnodes, D), kSplitThreads, 0, st>>>(nodes);
+        node_bins_kernel<D><<<dim3(nnodes, 4), kSplitThreads, 0, st>>>(nodes);
         node_cells_kernel<D><<<nnodes, kPrepThreads, 0, st>>>(nodes);
-        node_frames_kernel<D><<<nnodes, kSplitThreads, 0, st>>>(nodes);
+        node_order_kernel<<<nnodes, kSplitThreads, 0, st>>>(nodes);
     } else {
-        grid_node_kernel<D><<<nnodes, kPrepThreads, 0, st>>>(nodes);
+        grid_node_kernel<D><<<nnodes * kNodeCtas, kPrepThreads, 0, st>>>(nodes);
     }
     NSG_CUDA(cudaGetLastError());
 }
@@ -849,10 +865,6 @@ GridArgs grid_launch_count_order(const GridArgs& a, cudaStream_t st) {
     } else {
         c.corder = nullptr;
     }
-    if (c.rank_emax && c.nranks > 0) {
-        rank_emax_kernel<<<dim3(c.nranks, (c.rank_ld + 255) / 256), 256, 0, st>>>(c);
-        NSG_CUDA(cudaGetLastError());
-    }
     return c;
 }
 
@@ -865,7 +877,8 @@ void launch_counts(const GridArgs& c, int grid, cudaStream_t st) {
         NSG_CUDA(cudaGetLastError());
     }
     if (c.nranks > 0) {
-        ksg_grid_rank_kernel<D><<<c.rank_items, 32 * kRankWarps, 0, st>>>(c);
+        const int ctas = std::min(device_sms() * (40 / kRankWarps), (c.rank_items + kRankWarps - 1) / kRankWarps);
+        ksg_grid_rank_kernel<D><<<ctas, 32 * kRankWarps, 0, st>>>(c);
         NSG_CUDA(cudaGetLastError());
     }
 }
@@ -885,10 +898,12 @@ void grid_launch_counts(const GridArgs& a, int d, int grid, cudaStream_t st) {
     grid_launch_count_kernel(grid_launch_count_order(a, st), d, grid, st);
 }
 
-void grid_launch_combine(const KsgPairDesc* pairs, int npairs, const int* cnt_a, const int* cnt_b,
+void grid_launch_combine(const KsgPairDesc* pairs, int npairs, int max_m, const int* cnt_a, const int* cnt_b,
                          const float* psi, float* psum, int* nx, int* ny, cudaStream_t st) {
     if (npairs <= 0) return;
-    grid_combine_kernel<<<npairs, 256, 0, st>>>(pairs, cnt_a, cnt_b, psi, psum, nx, ny);
+    // few pairs: spread each over CTAs
+    const int parts = std::max(1, std::min((max_m + 255) / 256, 2 * device_sms() / npairs));
+    grid_combine_kernel<<<dim3(npairs, parts), 256, 0, st>>>(pairs, cnt_a, cnt_b, psi, psum, nx, ny);
     NSG_CUDA(cudaGetLastError());
 }
 

@@ -684,159 +684,203 @@ __global__ void __launch_bounds__(32 * kGridWarps, 4) ksg_grid_count_kernel(Grid
 }
 
 // ---- pass 2 by rank: nodes with many variables in the batch -------------------------
-// One warp per query of a rank node: the distances of the frames in the
-// query's box for the largest eps (the cells it overlaps, read in rows
-// straight from the grid) are listed in shared memory and counting-sorted
-// into kRankBuckets buckets of equal width; each lane then takes one
-// variable, and its count is the frames of the buckets below its eps's plus
-// those of that bucket that pass the exact comparison (the bucket index is a
-// monotone function of the distance). A few variables are counted while the
-// frames go by. A list that fills up is counted and starts again.
-constexpr int kRankList = 1024;
-constexpr int kRankBuckets = 128;
+// One warp per query of a rank node. The eps of up to kRankVars of the node's
+// variables are sorted in shared memory (by buckets of equal width, then
+// within each bucket); the frames of the query's box for the largest of them
+// (the cells it overlaps, read in rows straight from the grid) each find the
+// first eps not below their distance, from their bucket on, and count there;
+// a prefix sum turns that into every variable's count. A few variables are
+// compared one by one instead. Warps take queries in blocks of kRankBlock
+// consecutive frames, whose eps share sectors.
+constexpr int kRankVars = 256;
+constexpr int kRankBuckets = 512;
 constexpr int kRankDirect = 4;
 
 template <int D>
-__global__ void __launch_bounds__(32 * kRankWarps) ksg_grid_rank_kernel(GridArgs A) {
+__global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_rank_kernel(GridArgs A) {
     using namespace gridk;
-    __shared__ float s_list[kRankWarps][kRankList];
-    __shared__ float s_sort[kRankWarps][kRankList];
-    __shared__ __align__(16) int s_end[kRankWarps][kRankBuckets];
+    __shared__ __align__(16) int s_tab[kRankWarps][kRankBuckets + 4];
+    __shared__ __align__(16) float s_eps[kRankWarps][kRankVars];
+    __shared__ __align__(16) int s_cnt[kRankWarps][kRankVars];
+    __shared__ unsigned short s_var[kRankWarps][kRankVars];
     constexpr unsigned kFull = 0xffffffffu;
+    constexpr int kPer = kRankVars / 32;
+    static_assert(kRankBuckets == 512 && kPer == 8, "sixteen buckets and eight variables per lane");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int ri, blk;
-    item_of(A.rprefix, A.nranks, blockIdx.x, ri, blk);
-    const RankNode rn = A.ranks[ri];
-    const int i = blk * kRankWarps + wid;
-    if (i >= rn.m) return;  // whole warps; no CTA-wide waits below
-    const GridNode& nd = A.nodes[rn.node];
-    const long long* refs = A.refs + rn.first;
-    const int m = nd.m, G = nd.G, P = rn.count;
-    float q[D];
+    int* tab = s_tab[wid];
+    float* eps = s_eps[wid];
+    int* cnt = s_cnt[wid];
+    unsigned short* var = s_var[wid];
+    auto exclusive = [&](int v) {
+        int x = v;
 #pragma unroll
-    for (int c = 0; c < D; ++c) q[c] = __ldg(nd.x + static_cast<long long>(c) * nd.ld + i);
-    auto eps_of = [&](int p) {
-        const long long ref = __ldg(refs + p);
-        return __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i);
-    };
-    float emax = 0.f;  // eps are not negative
-    if (A.rank_emax) {
-        emax = __ldg(A.rank_emax + static_cast<long long>(ri) * A.rank_ld + i);
-    } else {
-        for (int p = lane; p < P; p += 32) emax = fmaxf(emax, eps_of(p));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) emax = fmaxf(emax, __shfl_xor_sync(kFull, emax, o));
-    }
-    int rlo, rhi, clo, chi;
-    bin_range(nd.e1, G, q[nd.c1], emax, rlo, rhi);
-    bin_range(nd.e2, G, nd.c2 >= 0 ? q[nd.c2] : 0.f, emax, clo, chi);
-    // row r's range of positions in lane r - rlo
-    int lo = 0, hi = 0;
-    if (lane <= rhi - rlo && clo <= chi) {
-        lo = __ldg(nd.start + (rlo + lane) * G + clo);
-        hi = __ldg(nd.start + (rlo + lane) * G + chi + 1);
-    }
-    const int nrows = clo <= chi ? rhi - rlo + 1 : 0;
-    const float* sx = nd.sx;
-    auto distance = [&](int pos) {
-        float dq[D];
-#pragma unroll
-        for (int c = 0; c < D; ++c) dq[c] = fabsf(q[c] - __ldg(sx + static_cast<long long>(c) * m + pos));
-        return max_of<D>(dq);
-    };
-    const unsigned long long scanned = __reduce_add_sync(kFull, hi - lo);
-    if (P <= kRankDirect) {
-        float e[kRankDirect];
-        int cnt[kRankDirect];
-#pragma unroll
-        for (int p = 0; p < kRankDirect; ++p) {
-            e[p] = p < P ? eps_of(p) : -inf_f();
-            cnt[p] = 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
         }
-        for (int r = 0; r < nrows; ++r) {
-            const int b = __shfl_sync(kFull, lo, r), t = __shfl_sync(kFull, hi, r);
-            for (int pos = b + lane; pos < t; pos += 32) {
-                const float dm = distance(pos);
+        return x - v;
+    };
+    unsigned long long scanned = 0, compared = 0;
+    for (;;) {
+        int item = 0;
+        if (lane == 0) item = atomicAdd(A.rank_counter, 1);
+        item = __shfl_sync(kFull, item, 0);
+        if (item >= A.rank_items) break;
+        int ri, blk;
+        item_of(A.rprefix, A.nranks, item, ri, blk);
+        const RankNode rn = A.ranks[ri];
+        const GridNode& nd = A.nodes[rn.node];
+        const long long* refs = A.refs + rn.first;
+        const int m = rn.m, G = nd.G, P = rn.count;
+        const float* __restrict__ sx = nd.sx;
+        for (int i = blk * kRankBlock; i < min(m, (blk + 1) * kRankBlock); ++i) {
+            float q[D];
 #pragma unroll
-                for (int p = 0; p < kRankDirect; ++p) cnt[p] += dm <= e[p];
-            }
-        }
+            for (int c = 0; c < D; ++c) q[c] = __ldg(nd.x + static_cast<long long>(c) * nd.ld + i);
+            const float q1 = q[nd.c1], q2 = nd.c2 >= 0 ? q[nd.c2] : 0.f;
+            auto distance = [&](int pos) {
+                float dq[D];
 #pragma unroll
-        for (int p = 0; p < kRankDirect; ++p) {
-            const int n = __reduce_add_sync(kFull, cnt[p]);
-            if (p < P && lane == 0) {
+                for (int c = 0; c < D; ++c) dq[c] = fabsf(q[c] - __ldg(sx + static_cast<long long>(c) * m + pos));
+                return max_of<D>(dq);
+            };
+            auto eps_of = [&](int p) {
+                const long long ref = __ldg(refs + p);
+                return __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i);
+            };
+            auto put = [&](int p, int n) {
                 const long long ref = __ldg(refs + p);
                 (ref & 1 ? A.cnt_b : A.cnt_a)[(ref >> 1) + i] = n;
-            }
-        }
-    } else {
-        float* list = s_list[wid];
-        float* sorted = s_sort[wid];
-        int* end = s_end[wid];
-        // bucket of a distance or eps up to emax
-        const float inv = emax > 0.f ? kRankBuckets / emax : 0.f;
-        auto bucket = [&](float v) { return min(kRankBuckets - 1, static_cast<int>(v * inv)); };
-        int n = 0;
-        bool first = true;
-        auto flush = [&]() {
-            int4* e4 = reinterpret_cast<int4*>(end);
-            static_assert(kRankBuckets == 128, "four buckets per lane");
-            e4[lane] = make_int4(0, 0, 0, 0);
-            __syncwarp();
-            for (int t = lane; t < n; t += 32) atomicAdd(end + bucket(list[t]), 1);
-            __syncwarp();
-            int4 c = e4[lane];
-            const int sum = c.x + c.y + c.z + c.w;
-            int base = sum;
+            };
+            for (int v0 = 0; v0 < P; v0 += kRankVars) {
+                const int nv = min(kRankVars, P - v0);
+                float ev[kPer];
+                float emax = 0.f;  // eps are not negative
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(kFull, base, o);
-                if (lane >= o) base += y;
-            }
-            base -= sum;
-            e4[lane] = make_int4(base, base + c.x, base + c.x + c.y, base + c.x + c.y + c.z);
-            __syncwarp();
-            for (int t = lane; t < n; t += 32) {
-                const float v = list[t];
-                sorted[atomicAdd(end + bucket(v), 1)] = v;
-            }
-            __syncwarp();
-            // end[b] is now the end of bucket b
-            for (int p = lane; p < P; p += 32) {
-                const long long ref = __ldg(refs + p);
-                const float e = __ldg((ref & 1 ? A.eps_b : A.eps_a) + (ref >> 1) + i);
-                const int b = bucket(e);
-                const int t0 = b ? end[b - 1] : 0, t1 = end[b];
-                int cnt = t0;
-                for (int t = t0; t < t1; ++t) cnt += sorted[t] <= e;
-                int* out = (ref & 1 ? A.cnt_b : A.cnt_a) + (ref >> 1) + i;
-                *out = first ? cnt : *out + cnt;
-            }
-            __syncwarp();
-            first = false;
-            n = 0;
-        };
-        for (int r = 0; r < nrows; ++r) {
-            const int b = __shfl_sync(kFull, lo, r), t = __shfl_sync(kFull, hi, r);
-            for (int p0 = b; p0 < t; p0 += 32) {
-                const int pos = p0 + lane;
-                const float dm = pos < t ? distance(pos) : inf_f();
-                const bool in = pos < t && dm <= emax;
-                const unsigned mask = __ballot_sync(kFull, in);
-                if (in) list[n + __popc(mask & ((1u << lane) - 1u))] = dm;
-                n += __popc(mask);
-                if (n > kRankList - 32) {
-                    __syncwarp();
-                    flush();
+                for (int t = 0; t < kPer; ++t) {
+                    ev[t] = 32 * t + lane < nv ? eps_of(v0 + 32 * t + lane) : 0.f;
+                    emax = fmaxf(emax, ev[t]);
                 }
+                emax = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(emax)));
+                // frames of the box, two times 32 at a time: f(distance, in)
+                int rlo, rhi, clo, chi;
+                bin_range(nd.e1, G, q1, emax, rlo, rhi);
+                bin_range(nd.e2, G, q2, emax, clo, chi);
+                // row r's range of positions in lane r - rlo
+                int lo = 0, hi = 0;
+                if (lane <= rhi - rlo && clo <= chi) {
+                    lo = __ldg(nd.start + (rlo + lane) * G + clo);
+                    hi = __ldg(nd.start + (rlo + lane) * G + chi + 1);
+                }
+                const int nrows = clo <= chi ? rhi - rlo + 1 : 0;
+                auto frames = [&](auto&& f) {
+                    for (int r = 0; r < nrows; ++r) {
+                        const int b = __shfl_sync(kFull, lo, r), t = __shfl_sync(kFull, hi, r);
+                        for (int p0 = b + lane; p0 < t; p0 += 64) {
+                            const bool two = p0 + 32 < t;
+                            const float d0 = distance(p0);
+                            const float d1 = two ? distance(p0 + 32) : inf_f();
+                            f(d0);
+                            if (two) f(d1);
+                        }
+                    }
+                };
+                const int box = __reduce_add_sync(kFull, hi - lo);
+                scanned += box;
+                compared += static_cast<unsigned long long>(box) * nv;
+                if (nv <= kRankDirect) {
+                    float e[kRankDirect];
+                    int n[kRankDirect];
+#pragma unroll
+                    for (int p = 0; p < kRankDirect; ++p) {
+                        e[p] = __shfl_sync(kFull, ev[0], p);
+                        n[p] = 0;
+                    }
+                    frames([&](float dm) {
+#pragma unroll
+                        for (int p = 0; p < kRankDirect; ++p) n[p] += dm <= e[p];
+                    });
+#pragma unroll
+                    for (int p = 0; p < kRankDirect; ++p) {
+                        n[p] = __reduce_add_sync(kFull, n[p]);
+                        if (p < nv && lane == 0) put(v0 + p, n[p]);
+                    }
+                    continue;
+                }
+                // bucket of a distance or eps up to emax: a monotone function
+                const float inv = emax > 0.f ? kRankBuckets / emax : 0.f;
+                auto bucket = [&](float v) { return min(kRankBuckets - 1, static_cast<int>(v * inv)); };
+                int4* t4 = reinterpret_cast<int4*>(tab) + 4 * lane;
+                int4* c4 = reinterpret_cast<int4*>(cnt) + 2 * lane;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) t4[g] = make_int4(0, 0, 0, 0);
+                c4[0] = c4[1] = make_int4(0, 0, 0, 0);
+                __syncwarp();
+                int slot[kPer];
+#pragma unroll
+                for (int t = 0; t < kPer; ++t)
+                    if (32 * t + lane < nv) slot[t] = atomicAdd(tab + bucket(ev[t]), 1);
+                __syncwarp();
+                {
+                    int4 w[4];
+                    int sum = 0;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        w[g] = t4[g];
+                        sum += w[g].x + w[g].y + w[g].z + w[g].w;
+                    }
+                    int base = exclusive(sum);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const int4 s = w[g];
+                        t4[g] = make_int4(base, base + s.x, base + s.x + s.y, base + s.x + s.y + s.z);
+                        base += s.x + s.y + s.z + s.w;
+                    }
+                    if (lane == 31) tab[kRankBuckets] = base;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int t = 0; t < kPer; ++t)
+                    if (32 * t + lane < nv) eps[slot[t] += tab[bucket(ev[t])]] = ev[t];
+                __syncwarp();
+#pragma unroll
+                for (int t = 0; t < kPer; ++t) {
+                    if (32 * t + lane >= nv) continue;
+                    const int b = bucket(ev[t]), first = tab[b], end = tab[b + 1];
+                    int rank = first;
+                    for (int u = first; u < end; ++u) rank += eps[u] < ev[t] || (eps[u] == ev[t] && u < slot[t]);
+                    slot[t] = rank;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int t = 0; t < kPer; ++t) {
+                    if (32 * t + lane >= nv) continue;
+                    eps[slot[t]] = ev[t];
+                    var[slot[t]] = static_cast<unsigned short>(32 * t + lane);
+                }
+                __syncwarp();
+                frames([&](float dm) {
+                    if (dm <= emax) {
+                        int u = tab[bucket(dm)];
+                        while (eps[u] < dm) ++u;  // eps[nv - 1] = emax ends it
+                        atomicAdd(cnt + u, 1);
+                    }
+                });
+                __syncwarp();
+                int n[kPer] = {c4[0].x, c4[0].y, c4[0].z, c4[0].w, c4[1].x, c4[1].y, c4[1].z, c4[1].w};
+#pragma unroll
+                for (int t = 1; t < kPer; ++t) n[t] += n[t - 1];
+                const int base = exclusive(n[kPer - 1]);
+#pragma unroll
+                for (int t = 0; t < kPer; ++t)
+                    if (kPer * lane + t < nv) put(v0 + var[kPer * lane + t], base + n[t]);
+                __syncwarp();
             }
         }
-        __syncwarp();
-        if (n > 0 || first) flush();
     }
-    if (A.evals && lane == 0) {
+    if (A.evals && lane == 0 && scanned) {
         atomicAdd(A.evals + 1, scanned);
-        atomicAdd(A.evals + 2, scanned * P);
+        atomicAdd(A.evals + 2, compared);
     }
 }
 

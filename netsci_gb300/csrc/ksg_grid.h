@@ -76,8 +76,7 @@ struct GridPair {
 //   * a few of them (up to kCountGroup) form a count group: a warp takes 16
 //     queries and compares every distance with each variable's eps;
 //   * more of them form a rank node: a warp takes one query, sorts the
-//     distances up to the largest eps into buckets once, and each lane finds
-//     the rank of one variable's eps.
+//     variables' eps, and every distance is counted at its place among them.
 constexpr int kCountGroup = 7;
 // Queries per warp in the counts: two lanes per query, each taking every
 // other frame, so the union of the warp's query boxes is that of 16 queries.
@@ -93,13 +92,14 @@ struct RankNode {
     int first, count;              // its variables in CountWork::refs
     int m;
 };
-// Queries a rank CTA takes, one per warp.
+// Consecutive queries a warp of the rank kernel takes, and its warps per CTA.
+constexpr int kRankBlock = 4;
 constexpr int kRankWarps = 4;
 struct CountWork {
     std::vector<CountGroup> groups;
     std::vector<int> gprefix;      // [groups + 1] prefix of ceil(m / kCountQueries)
     std::vector<RankNode> ranks;
-    std::vector<int> rprefix;      // [ranks + 1] prefix of ceil(m / kRankWarps)
+    std::vector<int> rprefix;      // [ranks + 1] prefix of ceil(m / kRankBlock)
     std::vector<long long> refs;   // variables of the rank nodes: scratch offset * 2 + side
 };
 
@@ -115,10 +115,7 @@ struct GridArgs {
     const int* rprefix;         // [nranks+1] prefix of their items
     const long long* refs;      // their variables
     int nranks, rank_items;
-    // [nranks][rank_ld] largest eps of each rank node's frames, filled by
-    // grid_launch_count_order; nullptr: the rank kernel finds them itself
-    float* rank_emax;
-    int rank_ld;
+    int* rank_counter;          // zero before the rank kernel
     int npairs;
     int pair_base;              // index of pairs[0] in the plan's pair array (tie entries)
     int k;
@@ -197,8 +194,8 @@ GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m, int d)
 size_t grid_pair_place(GridPair& g, size_t off, int m, int d);
 void grid_pair_rebase(GridPair& g, const void* base);
 // Node grids (nodes: device array whose x, ld, m, G and buffers are set), in
-// one kernel, or, with `split`, in three: quantiles (a CTA per node and
-// coordinate), cells, bitmap frames.
+// one kernel, or, with `split`, in four: quantiles (a CTA per node and
+// coordinate), bins (four per node), counting sorts by cell and by c1 bin.
 void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool split, cudaStream_t st);
 // Pair grids of a batch (pairs, gps: device arrays of npairs) and, when
 // `order` (the nodes carry scale estimates), their search orders. max_m: the
@@ -215,12 +212,11 @@ void grid_launch_search(const GridArgs& a, int d, int kmax, int grid, bool tie_r
 void grid_launch_search_rec(const GridArgs& a, int d, int kmax, int grid, cudaStream_t st);
 void grid_launch_counts(const GridArgs& a, int d, int grid, cudaStream_t st);
 // The two halves of grid_launch_counts: the count-order kernel (when the
-// args carry a count order and there are groups) and the rank nodes' largest
-// eps (when they carry a buffer); returns the args the count kernels take.
-// Then the group and rank kernels (each where it has work).
+// args carry a count order and there are groups; returns the args the count
+// kernels take). Then the group and rank kernels (each where it has work).
 GridArgs grid_launch_count_order(const GridArgs& a, cudaStream_t st);
 void grid_launch_count_kernel(const GridArgs& c, int d, int grid, cudaStream_t st);
-void grid_launch_combine(const KsgPairDesc* pairs, int npairs, const int* cnt_a, const int* cnt_b,
+void grid_launch_combine(const KsgPairDesc* pairs, int npairs, int max_m, const int* cnt_a, const int* cnt_b,
                          const float* psi, float* psum, int* nx, int* ny, cudaStream_t st);
 // Copies frame-mapped rows (device array of nrows); a map entry outside
 // [0, ld) sets FAULT_BAD_INDEX in *fault and reads frame 0.

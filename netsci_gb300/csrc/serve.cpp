@@ -441,7 +441,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     put(d_ranks_, work_list.ranks);
     put(d_rpre_, work_list.rprefix);
     put(d_refs_, work_list.refs);
-    NSG_CUDA(cudaMemsetAsync(d_counters_.get(), 0, sizeof(int) * 4, s));
+    NSG_CUDA(cudaMemsetAsync(d_counters_.get(), 0, sizeof(int) * 5, s));
     int* ctr = d_counters_.as<int>();
     KsgPairDesc* dp = d_pairs_.as<KsgPairDesc>();
     const int search_order = bits.ok ? 0 : grid_launch_pairs(dp, d_gpairs_.as<GridPair>(), d_gnodes_.as<GridNode>(),
@@ -460,6 +460,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     a.refs = d_refs_.as<long long>();
     a.nranks = static_cast<int>(work_list.ranks.size());
     a.rank_items = work_list.rprefix.back();
+    a.rank_counter = ctr + 4;
     a.npairs = static_cast<int>(np);
     a.pair_base = 0;
     a.k = k;
@@ -479,7 +480,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     else grid_launch_search(a, d, kmax, sms * grid_search_ctas_per_sm(d, kmax), false, s);
     a.counter = ctr + 1;
     grid_launch_counts(a, d, sms * grid_count_ctas_per_sm(d), s);
-    grid_launch_combine(dp, static_cast<int>(np), a.cnt_a, a.cnt_b, psi_->as<float>(), d_scratch_.as<float>(),
+    grid_launch_combine(dp, static_cast<int>(np), maxm, a.cnt_a, a.cnt_b, psi_->as<float>(), d_scratch_.as<float>(),
                         nullptr, nullptr, s);
     KsgTieArgs t{};
     t.pairs = dp;

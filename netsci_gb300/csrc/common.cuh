@@ -61,6 +61,13 @@ __device__ __forceinline__ float nsg_le_f32(float a, float b) {
     return r;
 }
 
+// 1.0f when a < b, else 0.0f, the same way.
+__device__ __forceinline__ float nsg_lt_f32(float a, float b) {
+    float r;
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Packed add of two float pairs (add.rn.f32x2), assembled the same way.
 __device__ __forceinline__ float2 nsg_add2(float2 a, float2 b) {
     float2 r;

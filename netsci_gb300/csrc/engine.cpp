@@ -174,8 +174,8 @@ constexpr int kGridMinSamples = 1000;
 constexpr int kGridFewPairs = 8;
 constexpr int kGridMinSamplesFew = 4000;
 // per batch: work-queue heads (two for the grid search), tie count,
-// tie-kernel counter, rank-count queue head
-constexpr int kCounters = 5;
+// tie-kernel counter, rank-count queue head, bitmap-search queue heads
+constexpr int kCounters = 5 + kBitSegments;
 }  // namespace
 
 std::shared_ptr<const DeviceBuffer> device_psi(int n) {
@@ -626,7 +626,7 @@ struct KsgPlan::GridState {
     std::vector<char> batch_order;        // whether each batch builds query orders
     bool split_nodes = false;             // an ordered batch: many nodes, four kernels
     bool node_est = false;                // a batch needs the nodes' scale estimates
-    std::vector<BitsConfig> batch_bits;   // bitmap search where ok, else the scan on pair grids
+    std::vector<std::vector<BitsSegment>> batch_bits;  // bitmap search; empty: the scan on pair grids
     int max_m = 0;
     DeviceBuffer wprefix;                 // per batch: npairs+1 prefix of ceil(m/32)
     std::vector<long long> wprefix_off;   // offset of each batch's prefix
@@ -701,8 +701,8 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
             wpre.push_back(acc);
             acc += (descs[p].m + 31) / 32;
         }
-        g->batch_bits.push_back(bits_config(d_, k_, maxm));
-        const bool bits = g->batch_bits.back().ok;
+        g->batch_bits.push_back(bits_segments(descs.data() + b.pair0, b.npairs, d_, k_));
+        const bool bits = !g->batch_bits.back().empty();
         for (int p = b.pair0; p < b.pair0 + b.npairs && !bits; ++p) off = grid_pair_place(gps[p], off, descs[p].m, d_);
         wpre.push_back(acc);
         g->batch_maxm.push_back(maxm);
@@ -785,9 +785,9 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         KsgPairDesc* bp = pairs_dev_.as<KsgPairDesc>() + b.pair0;
         GridPair* bg = g.gps.as<GridPair>() + b.pair0;
         const bool order = g.batch_order[bi] != 0;
-        const BitsConfig& bits = g.batch_bits[bi];
+        const std::vector<BitsSegment>& bits = g.batch_bits[bi];
         const int search_order =
-            bits.ok ? 0 : grid_launch_pairs(bp, bg, g.nodes.as<GridNode>(), b.npairs, g.batch_maxm[bi], d_, order, s);
+            !bits.empty() ? 0 : grid_launch_pairs(bp, bg, g.nodes.as<GridNode>(), b.npairs, g.batch_maxm[bi], d_, order, s);
         GridArgs a{};
         a.search_order = search_order;
         a.pairs = bp;
@@ -823,9 +823,8 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         a.corder_ld = g.batch_maxm[bi];
         cudaEvent_t* ev = events_.data() + kEventsPerBatch * bi;
         if (timing_) record_event(ev[0], s);
-        if (bits.ok) {
-            bits_launch_search(a, bits, g.batch_maxm[bi], d_, s);
-        } else {
+        for (size_t q = 0; q < bits.size(); ++q) bits_launch_search(a, bits[q], ctr + 5 + q, d_, s);
+        if (bits.empty()) {
             grid_launch_search(a, d_, kmax_, g.search_grid, bootstrap_, s);
         }
         if (timing_) record_event(ev[1], s);
@@ -874,16 +873,17 @@ int KsgPlan::launches() const {
     const int nb = static_cast<int>(batches_.size());
     if (search_ != 1) return 3 * nb;
     if (!nb) return 0;
-    // node grids (+ scale estimates), gather; per batch: search, combine,
+    // node grids (+ scale estimates), gather; per batch: searches, combine,
     // ties, final sums, group and rank counts (+ pair grids where the search
     // scans them; in batches with orders + search and count orders)
-    int n = 1 + (ngather_ ? 1 : 0) + 4 * nb;
+    int n = 1 + (ngather_ ? 1 : 0) + 3 * nb;
     if (grid_) {
         if (grid_->split_nodes) n += 3;
         if (grid_->node_est) ++n;
         for (size_t bi = 0; bi < grid_->batch_order.size(); ++bi) {
             const bool order = grid_->batch_order[bi] != 0, short_m = grid_->batch_maxm[bi] <= kOrderMaxM;
-            if (!grid_->batch_bits[bi].ok) n += order && short_m ? 2 : 1;
+            const int bits = static_cast<int>(grid_->batch_bits[bi].size());
+            n += bits ? bits : order && short_m ? 3 : 2;
             if (grid_->ngroups[bi]) n += order && short_m ? 2 : 1;
             if (grid_->nranks[bi]) ++n;
         }

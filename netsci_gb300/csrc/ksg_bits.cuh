@@ -18,7 +18,7 @@
 //     the rows with ballots: 2% of its time at m = 10000.
 //   * A warp takes a few queries at a time: one lane per query and
 //     coordinate finds the bins its interval reaches. Then, query by query,
-//     each lane ANDs four (or eight) words of 2d - 1 row pairs, finds the set
+//     each lane ANDs one to eight words of 2d - 1 row pairs, finds the set
 //     bit of its rank, and evaluates that frame exactly (one 16-byte gather
 //     per node); the frames within h are listed in shared memory with their
 //     distances. A lane per listed frame counts the smaller distances;
@@ -108,13 +108,31 @@ __device__ __forceinline__ int lane_prefix(int v) {
     return v;
 }
 
+// W words of a row (4 W bytes, aligned).
+template <int W>
+__device__ __forceinline__ void load_words(const unsigned* row, int x, unsigned (&w)[W]) {
+    if constexpr (W == 1) {
+        w[0] = row[x];
+    } else if constexpr (W == 2) {
+        const uint2 v = reinterpret_cast<const uint2*>(row)[x];
+        w[0] = v.x;
+        w[1] = v.y;
+    } else {
+        const uint4 v = reinterpret_cast<const uint4*>(row)[x];
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+    }
+}
+
 // Position of the bit of rank win + lane among the set bits of the lanes'
 // words (lane order, then word order): word g of a lane covers positions
 // base + 32 g for g < 4 and base + 4096 + 32 (g - 4) above. off: set bits of
-// the lanes before; cnt: of this lane; table: 32 words of shared memory.
+// the lanes before; cnt: of this lane; n: of all; table: 32 words of shared memory.
 // Lanes whose rank does not exist get an arbitrary position.
 template <int W>
-__device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int off, int cnt, int win, int lane,
+__device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int off, int cnt, int win, int n, int lane,
                                            unsigned* table) {
     // lanes with a bit in the window, in order, and where their bits start in it
     const int first = off - win;
@@ -125,20 +143,23 @@ __device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int
     __syncwarp();
     const int src = static_cast<int>(table[__popc(starts & (kFull >> (31 - lane))) - 1] & 31u);
     int r = win + lane - __shfl_sync(kFull, off, src);  // rank within the owner's words
-    unsigned bits = 0;
+    if (win + lane >= n) r = 0;
     int pos = __shfl_sync(kFull, base, src);
+    unsigned bits = __shfl_sync(kFull, w[0], src);
 #pragma unroll
-    for (int g = 0; g < W; ++g) {
+    for (int g = 1; g < W; ++g) {
+        // past the words before: the remaining rank moves on to word g
         const unsigned x = __shfl_sync(kFull, w[g], src);
-        const int c = __popc(x);
-        if (g == W - 1 || r < c) {
-            if (bits == 0) {
-                bits = x;
-                pos += 32 * (g & 3) + (g >> 2) * 4096;
-            }
+        const int c = __popc(bits);
+        if (r >= c) {
+            r -= c;
+            bits = x;
+            pos += g == 4 ? 4096 - 96 : 32;
+        } else {
+            r -= 0x10000;  // found: no later word is taken
         }
-        if (bits == 0) r -= c;
     }
+    r &= 0xffff;
     for (; r > 0; --r) bits &= bits - 1;
     __syncwarp();
     return pos + __ffs(bits) - 1;
@@ -188,24 +209,23 @@ __device__ __forceinline__ unsigned kth_lane(unsigned u, int k) {
 // v holds +inf up to the next multiple of four entries.
 template <int N>
 __device__ __forceinline__ Found select_nearest(const float* v, const float* da, const float* db, int n, int k, int lane) {
-    float x[N];
-    int less[N];
+    float x[N], less[N];
 #pragma unroll
     for (int c = 0; c < N; ++c) {
         x[c] = 32 * c + lane < n ? v[32 * c + lane] : inf_f();
-        less[c] = 0;
+        less[c] = 0.f;
     }
     for (int t = 0; t < n; t += 4) {
         const float4 y = *reinterpret_cast<const float4*>(v + t);
 #pragma unroll
         for (int c = 0; c < N; ++c)
-            less[c] += (y.x < x[c]) + (y.y < x[c]) + (y.z < x[c]) + (y.w < x[c]);
+            less[c] += (nsg_lt_f32(y.x, x[c]) + nsg_lt_f32(y.y, x[c])) + (nsg_lt_f32(y.z, x[c]) + nsg_lt_f32(y.w, x[c]));
     }
     unsigned wk = 0, ea = 0, eb = 0;
     int le = 0;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
-        const bool in = 32 * c + lane < n && less[c] <= k;
+        const bool in = 32 * c + lane < n && less[c] <= static_cast<float>(k);
         le += __popc(__ballot_sync(kFull, in));
         if (in) {
             wk = max(wk, __float_as_uint(x[c]));
@@ -341,8 +361,9 @@ __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float
 // A work item is a pair and a share of its queries (B.chunks shares per
 // pair). Dynamic shared memory: rows, node a's frame order, then per warp its
 // queries, their bins and the two lists (bits_config sizes it for the batch's
-// largest m). Up to 32 N frames within h are kept.
-template <int D, int N>
+// largest m). Up to 32 N frames within h are kept; each lane ANDs W words
+// (32 W frames), of 32 W lanes' worth or, with W = 4, of twice that.
+template <int D, int N, int W>
 __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
     using namespace bitk;
     const GridArgs& A = B.g;
@@ -365,7 +386,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
     const int R = B.rows, step = B.step, k = A.k;
     int cur_a = -1;
     float scale = 1.f;               // this warp's share in h, see the file comment
-    unsigned long long evals = 0;
+    unsigned evals = 0;
     for (;;) {
         __syncthreads();
         if (tid == 0) {
@@ -434,18 +455,17 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
         const float rank = est_rank(m);
         const float base = exp2f(__log2f(static_cast<float>(k) * m / (rank * rank)) * (0.5f / D) + 0.3f);
         __syncthreads();
-        const uint4* rows = reinterpret_cast<const uint4*>(s_dyn);
-        // bins of coordinate c of query t, packed: c = 0 the range of uint4
-        // columns, else the offsets of its two rows (in uint4)
+        // bins of coordinate c of query t, packed: c = 0 the range of columns
+        // of W words, else the offsets of its two rows in columns
         auto set_bins = [&](int t, int c) {
             int lo, hi;
             reach(s_edge[c], s_query[8 * t + (c < D ? c : 4 + c - D)], s_query[8 * t + 3], lo, hi);
             if (c == 0) {
-                lo = s_start[lo] >> 7;
-                hi = (s_start[hi] + 127) >> 7;
+                lo = s_start[lo] / (32 * W);
+                hi = (s_start[hi] + 32 * W - 1) / (32 * W);
             } else {
-                lo = ((c - 1) * R + lo) * (WS / 4);
-                hi = ((c - 1) * R + hi) * (WS / 4);
+                lo = ((c - 1) * R + lo) * (WS / W);
+                hi = ((c - 1) * R + hi) * (WS / W);
             }
             s_bins[2 * D * t + c] = static_cast<unsigned>(hi) << 16 | static_cast<unsigned>(lo);
         };
@@ -468,8 +488,6 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
             __syncwarp();
             if (lane < 2 * D * nq) set_bins(lane / (2 * D), lane % (2 * D));
             __syncwarp();
-            float ra = 0.f, rb = 0.f, rw = 0.f;  // lane t keeps query t's results
-            unsigned tmask = 0;
             for (int t = 0; t < nq; ++t) {
                 const float4 fa = *reinterpret_cast<const float4*>(s_query + 8 * t);
                 const float4 fb = *reinterpret_cast<const float4*>(s_query + 8 * t + 4);
@@ -493,26 +511,21 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                     int inside = 0;
                     int crowd = 0;
                     bool stuck = false;
-                    // the AND of the row pairs over one uint4 column
-                    auto column = [&](int x) {
-                        uint4 acc = make_uint4(0, 0, 0, 0);
+                    // the AND of the row pairs over column x
+                    auto column = [&](int x, auto& acc) {
+#pragma unroll
+                        for (int g = 0; g < W; ++g) acc[g] = 0;
                         if (x < x1) {
 #pragma unroll
                             for (int c = 0; c < NC; ++c) {
                                 const unsigned o = bins[c + 1];
-                                const uint4 u = rows[(o >> 16) + x];
-                                const uint4 v = rows[(o & 0xffffu) + x];
-                                if (c == 0) {
-                                    acc = make_uint4(u.x ^ v.x, u.y ^ v.y, u.z ^ v.z, u.w ^ v.w);
-                                } else {
-                                    acc.x &= u.x ^ v.x;
-                                    acc.y &= u.y ^ v.y;
-                                    acc.z &= u.z ^ v.z;
-                                    acc.w &= u.w ^ v.w;
-                                }
+                                unsigned u[W], v[W];
+                                load_words<W>(s_dyn, (o >> 16) + x, u);
+                                load_words<W>(s_dyn, (o & 0xffffu) + x, v);
+#pragma unroll
+                                for (int g = 0; g < W; ++g) acc[g] = c == 0 ? u[g] ^ v[g] : acc[g] & (u[g] ^ v[g]);
                             }
                         }
-                        return acc;
                     };
                     // Evaluates the frames of the set bits, 32 at a time; false: too many ties.
                     auto consume = [&](auto& w, int base, int cnt, bool last) {
@@ -529,7 +542,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                         }
                         evals += n;
                         for (int win = 0; win < n; win += 32) {
-                            const int pos = bit_of_rank(w, base, incl - cnt, cnt, win, lane, s_table);
+                            const int pos = bit_of_rank(w, base, incl - cnt, cnt, win, n, lane, s_table);
                             float da = 0.f, db = 0.f, v = inf_f();
                             if (win + lane < n) {
                                 const int j = s_perm[pos];
@@ -564,20 +577,27 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                         }
                         return true;
                     };
-                    for (int xf = x0; xf < x1 && !stuck && !crowd; xf += 64) {
+                    constexpr int kSpan = W == 4 ? 64 : 32;  // columns at a time
+                    for (int xf = x0; xf < x1 && !stuck && !crowd; xf += kSpan) {
                         const int x = xf + lane;
-                        const uint4 u = column(x);
-                        if (xf + 32 >= x1) {
-                            const unsigned w[4] = {u.x, u.y, u.z, u.w};
-                            const int cnt = __popc(u.x) + __popc(u.y) + __popc(u.z) + __popc(u.w);
-                            stuck = !consume(w, 128 * x, cnt, true);
-                        } else {
-                            const uint4 v = column(x + 32);
-                            const unsigned w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-                            int cnt = 0;
+                        const bool last = xf + kSpan >= x1;
+                        unsigned u[W];
+                        column(x, u);
+                        int cnt = 0;
 #pragma unroll
-                            for (int g = 0; g < 8; ++g) cnt += __popc(w[g]);
-                            stuck = !consume(w, 128 * x, cnt, xf + 64 >= x1);
+                        for (int g = 0; g < W; ++g) cnt += __popc(u[g]);
+                        if (W < 4 || xf + 32 >= x1) {
+                            stuck = !consume(u, 32 * W * x, cnt, last);
+                        } else {
+                            unsigned v[W], w[2 * W];
+                            column(x + 32, v);
+#pragma unroll
+                            for (int g = 0; g < W; ++g) {
+                                w[g] = u[g];
+                                w[W + g] = v[g];
+                                cnt += __popc(v[g]);
+                            }
+                            stuck = !consume(w, 32 * W * x, cnt, last);
                         }
                     }
                     if (stuck) break;
@@ -605,35 +625,21 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                     r = scan_all<D>(xa, xb, m, k, q0 + t, lane);
                     evals += m;
                 }
-                if (lane == t) {
-                    ra = r.ea;
-                    rb = r.eb;
-                    rw = r.wk;
-                }
-                if (r.tie) tmask |= 1u << t;
-            }
-            if (lane < nq) {
-                const long long o = P->scratch + q0 + lane;
-                A.eps_a[o] = ra;
-                A.eps_b[o] = rb;
-                if (A.eps_x) A.eps_x[o] = ra;
-                if (A.eps_y) A.eps_y[o] = rb;
-                if (A.kdist) A.kdist[o] = rw;
-            }
-            if (tmask) {
-                // tied samples of the block take consecutive slots of the tie list
-                int slot = 0;
-                if (lane == 0) slot = atomicAdd(A.tie_count, __popc(tmask));
-                slot = __shfl_sync(kFull, slot, 0);
-                if (tmask >> lane & 1u) {
-                    slot += __popc(tmask & ((1u << lane) - 1u));
-                    if (slot < A.tie_cap) A.ties[slot] = KsgTie{A.pair_base + p, q0 + lane};
+                const long long o = P->scratch + q0 + t;
+                if (lane < 2) (lane ? A.eps_b : A.eps_a)[o] = lane ? r.eb : r.ea;
+                if (A.eps_x && lane == 0) A.eps_x[o] = r.ea;
+                if (A.eps_y && lane == 0) A.eps_y[o] = r.eb;
+                if (A.kdist && lane == 0) A.kdist[o] = r.wk;
+                if (r.tie && lane == 0) {
+                    const int slot = atomicAdd(A.tie_count, 1);
+                    if (slot < A.tie_cap) A.ties[slot] = KsgTie{A.pair_base + p, q0 + t};
                     else atomicOr(A.fault, FAULT_TIE_OVERFLOW);
                 }
             }
         }
+        if (A.evals && lane == 0) atomicAdd(A.evals, static_cast<unsigned long long>(evals));
+        evals = 0;
     }
-    if (A.evals && lane == 0 && evals) atomicAdd(A.evals, evals);
 }
 
 // Scale estimates of one node's frames (GridNode::est), a share of them per

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "ksg_grid.h"
 
 namespace nsg {
@@ -32,6 +34,7 @@ struct BitsArgs {
 
 struct BitsConfig {
     bool ok = false;
+    int words = 0;              // words a lane ANDs at a time: 1, 2 or 4
     int keep = 0;               // frames within the search radius a query keeps, in 32s
     int threads = 0, ctas_per_sm = 0;
     int rows = 0, step = 0, rows_words = 0, perm_words = 0;
@@ -40,10 +43,20 @@ struct BitsConfig {
 // Shared-memory layout and CTA size for pairs of up to max_m frames; not ok
 // where the rows of such a pair do not fit.
 BitsConfig bits_config(int d, int k, int max_m);
+// Runs of pairs (sorted by falling m) that share a configuration, for a
+// batch whose longest pair has one: one search launch each, at most
+// kBitSegments.
+struct BitsSegment {
+    int first, npairs, max_m;
+    BitsConfig config;
+};
+constexpr int kBitSegments = 4;
+std::vector<BitsSegment> bits_segments(const KsgPairDesc* descs, int npairs, int d, int k);
 // Scale estimates of node grids (grid_launch_nodes) of up to max_m frames.
 void bits_launch_est(const GridNode* nodes, int nnodes, int max_m, int d, cudaStream_t s);
-// The search of a batch whose largest m is max_m (the nodes carry scale
-// estimates); takes what grid_launch_search takes but no pair grids.
-void bits_launch_search(const GridArgs& g, const BitsConfig& c, int max_m, int d, cudaStream_t s);
+// The search of one segment of a batch (the nodes carry scale estimates);
+// takes what grid_launch_search takes for the batch, but no pair grids, and a
+// counter of the segment's own, zero before the launch.
+void bits_launch_search(const GridArgs& g, const BitsSegment& seg, int* counter, int d, cudaStream_t s);
 
 }  // namespace nsg

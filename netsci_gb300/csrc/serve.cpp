@@ -407,8 +407,8 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
         }
     }
     h_wpre_[np] = static_cast<int>(wacc);
-    const BitsConfig bits = bits_config(d, k, maxm);
-    for (long long i = 0; i < np && !bits.ok; ++i) arena = grid_pair_place(h_gpairs_[i], arena, h_pairs_[i].m, d);
+    const BitsSegment bits{0, static_cast<int>(np), maxm, bits_config(d, k, maxm)};
+    for (long long i = 0; i < np && !bits.config.ok; ++i) arena = grid_pair_place(h_gpairs_[i], arena, h_pairs_[i].m, d);
     cudaStream_t s = ksg_stream_;
     // buffers grow on demand (by a quarter more than asked, to grow rarely)
     auto ensure = [&](DeviceBuffer& b, size_t bytes) {
@@ -422,7 +422,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     ensure(d_eps_b_, sizeof(float) * samples);
     ensure(d_cnt_a_, sizeof(int) * samples);
     ensure(d_cnt_b_, sizeof(int) * samples);
-    for (long long i = 0; i < np && !bits.ok; ++i) grid_pair_rebase(h_gpairs_[i], d_garena_.get());
+    for (long long i = 0; i < np && !bits.config.ok; ++i) grid_pair_rebase(h_gpairs_[i], d_garena_.get());
     NSG_CUDA(cudaMemcpyAsync(d_pairs_.get(), h_pairs_, sizeof(KsgPairDesc) * np, cudaMemcpyHostToDevice, s));
     NSG_CUDA(cudaMemcpyAsync(d_gpairs_.get(), h_gpairs_, sizeof(GridPair) * np, cudaMemcpyHostToDevice, s));
     NSG_CUDA(cudaMemcpyAsync(d_wpre_.get(), h_wpre_, sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
@@ -444,7 +444,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     NSG_CUDA(cudaMemsetAsync(d_counters_.get(), 0, sizeof(int) * 5, s));
     int* ctr = d_counters_.as<int>();
     KsgPairDesc* dp = d_pairs_.as<KsgPairDesc>();
-    const int search_order = bits.ok ? 0 : grid_launch_pairs(dp, d_gpairs_.as<GridPair>(), d_gnodes_.as<GridNode>(),
+    const int search_order = bits.config.ok ? 0 : grid_launch_pairs(dp, d_gpairs_.as<GridPair>(), d_gnodes_.as<GridNode>(),
                                                              static_cast<int>(np), maxm, d, order, s);
     GridArgs a{};
     a.search_order = search_order;
@@ -476,7 +476,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     a.corder = order ? d_corder_.as<int>() : nullptr;
     a.corder_ld = maxm;
     const int sms = sm_count();
-    if (bits.ok) bits_launch_search(a, bits, maxm, d, s);
+    if (bits.config.ok) bits_launch_search(a, bits, ctr, d, s);
     else grid_launch_search(a, d, kmax, sms * grid_search_ctas_per_sm(d, kmax), false, s);
     a.counter = ctr + 1;
     grid_launch_counts(a, d, sms * grid_count_ctas_per_sm(d), s);

@@ -14,6 +14,7 @@
 #include "ksg_bits.h"
 #include "ksg_grid.h"
 #include "ksg_registry.cuh"
+#include "ksg_warp.h"
 
 namespace nsg {
 
@@ -163,16 +164,18 @@ int g_forced_variant = -1;
 int g_forced_staging = -1;
 int g_forced_search = -1;
 int g_forced_orders = -1;
-// Below this many samples per pair the exhaustive kernel is used: grids of
-// a few cells per axis prune little (measured: 0.91x at m = 300, 1.08x at
-// m = 1000, 1.28x at m = 2000, whole plans of 48-node trajectories).
-constexpr int kGridMinSamples = 1000;
-// Plans of a few pairs cannot fill the GPU and wait on launch and setup
-// latency, where the grid's three extra launches cost more: one pair took
-// 0.28 ms exhaustive against 0.33 ms on grids at m = 2000, and 0.90 against
-// 0.72 ms at m = 10000.
-constexpr int kGridFewPairs = 8;
-constexpr int kGridMinSamplesFew = 4000;
+// Microseconds of a plan on cell grids and on the tiled exhaustive kernels,
+// from the times of 48 plan shapes (16, 40 and 100 nodes, m = 200 to 1500, d =
+// 1 to 3, k = 4, 6 and 20). The grids' kernels take about 110 us before they
+// are busy, then a time per sample that hardly depends on m; the tiled kernels
+// take a time per frame visit, and never less than one thread's walk over m
+// frames. 4950 pairs, d = 3, k = 6: at m = 300 1130 us tiled and 1070 on grids,
+// at m = 800 4940 and 2560; 120 pairs at m = 500: 143 and 236.
+double grid_us(int k, double samples) { return 110 + (k <= 12 ? 0.62e-3 : 0.95e-3) * samples; }
+double tiled_us(int d, int k, int max_m, double work) {
+    const double visit = (d == 1 ? 0.65e-6 : d == 2 ? 1.02e-6 : 1.17e-6) * (k <= 6 ? 1 : k <= 14 ? 2 : 3.5);
+    return 20 + std::max(0.1 * max_m, visit * work);
+}
 // per batch: work-queue heads (two for the grid search), tie count,
 // tie-kernel counter, rank-count queue head, bitmap-search queue heads
 constexpr int kCounters = 5 + kBitSegments;
@@ -294,6 +297,8 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
         maxm = std::max(maxm, q.m);
         total_samples += q.m;
     }
+    max_m_ = maxm;
+    samples_ = total_samples;
     if (kmax_ == 0) fail(NSG_ERR_UNSUPPORTED, "k > 62 is not supported by the GPU path");
     const bool per_sample = out.nx || out.ny || out.eps_x || out.eps_y || out.kdist;
 
@@ -322,12 +327,9 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     };
     std::map<RowKey, size_t> mapped;  // row -> offset (floats) of its copy
     size_t mapped_floats = 0;
-    double work = 0, work_large = 0;  // sum of m^2, and over pairs with m >= the grid's minimum
-    const int grid_min_m = npairs < kGridFewPairs ? kGridMinSamplesFew : kGridMinSamples;
+    double work = 0;  // sum of m^2
     for (const auto& q : pairs_in) {
-        const double w = static_cast<double>(q.m) * q.m;
-        work += w;
-        if (q.m >= grid_min_m) work_large += w;
+        work += static_cast<double>(q.m) * q.m;
         if (!q.fmap) continue;
         for (const float* x : {q.xa, q.xb}) {
             if (mapped.emplace(RowKey{x, q.fmap, q.m, q.ld}, mapped_floats).second) {
@@ -339,9 +341,15 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     if (search == 1 && !grid_ok) {
         fail(NSG_ERR_UNSUPPORTED, "cell-grid search: copies of the frame-mapped rows exceed 8 GiB");
     }
-    // automatic: grids when most of the work is in pairs large enough to prune
-    if (search < 0) search = (grid_ok && work_large >= 0.5 * work) ? 1 : 0;
+    // automatic: whichever is estimated faster, unless the plan is small
+    // enough for a warp per query
+    const bool warp_ok = !tile_forced && !opt.autotune && ksg_warp_fits(d, k, maxm, work);
+    if (search < 0) {
+        search = grid_ok && !warp_ok &&
+                 grid_us(k, static_cast<double>(total_samples)) < tiled_us(d, k, maxm, work) ? 1 : 0;
+    }
     search_ = search == 1 ? 1 : 0;
+    warp_ = !search_ && warp_ok;
     std::vector<nsg_ksg_pair> eff;
     if (search_ && !mapped.empty()) {
         mapped_rows_.reset(mapped_floats * sizeof(float));
@@ -448,7 +456,7 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     }
     entry_ = entry;
     variant_ = entry->variant;
-    const int qc = shape_.threads * shape_.r;
+    const int qc = warp_ ? kWarpsPerCta : shape_.threads * shape_.r;
 
     // ---- order, batches, descriptors, items ------------------------------
     std::vector<int> order(npairs);
@@ -580,8 +588,12 @@ void KsgPlan::enqueue(cudaStream_t s) {
         // and the count interval is empty.
         cudaEvent_t* ev = events_.data() + kEventsPerBatch * bi;
         if (timing_) record_event(ev[0], s);
-        entry_->launch(a, b.grid, s);
-        NSG_CUDA(cudaGetLastError());
+        if (warp_) {
+            ksg_launch_warp(a, d_, max_m_, s);
+        } else {
+            entry_->launch(a, b.grid, s);
+            NSG_CUDA(cudaGetLastError());
+        }
         if (timing_) {
             for (int j = 1; j < 5; ++j) record_event(ev[j], s);
         }
@@ -602,7 +614,7 @@ void KsgPlan::enqueue(cudaStream_t s) {
         t.dz = tie_dz_.as<float>();
         t.idx = tie_idx_.as<int>();
         t.stride = tie_stride_;
-        ksg_launch_ties(t, d_, s);
+        ksg_launch_ties(t, d_, samples_, s);
         if (timing_) record_event(ev[5], s);
         KsgFinalArgs f{};
         f.pairs = pairs_dev_.as<KsgPairDesc>() + b.pair0;
@@ -853,7 +865,7 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         t.idx = tie_idx_.as<int>();
         t.stride = tie_stride_;
         if (timing_) record_event(ev[4], s);
-        ksg_launch_ties(t, d_, s);
+        ksg_launch_ties(t, d_, samples_, s);
         if (timing_) record_event(ev[5], s);
         KsgFinalArgs f{};
         f.pairs = bp;

@@ -126,6 +126,9 @@ private:
     int tie_cap_ = 0;
     long long tie_stride_ = 0;
     int search_ = 0;
+    bool warp_ = false;                  // exhaustive, a warp per query
+    int max_m_ = 0;
+    long long samples_ = 0;              // of all pairs
     bool bootstrap_ = false;             // frame-mapped rows copied for the grid search
     DeviceBuffer mapped_rows_, gather_rows_;
     int ngather_ = 0;

@@ -105,7 +105,8 @@ void ksg_launch_counts(const KsgCountArgs& a, int d, int kmax, const KsgShape& s
 void ksg_launch_final(const KsgFinalArgs& a, cudaStream_t st);
 // Warps the tie kernel runs with (scratch rows needed).
 int ksg_tie_warps();
-void ksg_launch_ties(const KsgTieArgs& a, int d, cudaStream_t st);
+// samples: of the whole run, an upper bound on the ties.
+void ksg_launch_ties(const KsgTieArgs& a, int d, long long samples, cudaStream_t st);
 void ksg_launch_ties_ctas(const KsgTieArgs& a, int d, int ctas, cudaStream_t st);
 // One pair with all scratch in the library's static device area
 // (ksg_noalloc.cu); synchronizes s.

@@ -21,6 +21,8 @@
 // Runs between the count kernel and the finalize kernel, with a fixed grid
 // that walks the tie list through an atomic counter (an empty list costs one
 // launch that returns at once).
+#include <algorithm>
+
 #include "common.cuh"
 #include "engine.h"
 #include "ksg.cuh"
@@ -204,13 +206,12 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
     return true;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm) ksg_tie_kernel(KsgTieArgs A) {
-    __shared__ SortSegment s_stack[kWarpsPerCta][kStack];
+// The kernel body for warps of W per CTA whose rows of dz and idx lie at dz
+// and idx.
+template <int D, int W>
+__device__ __forceinline__ void resolve_ties(const KsgTieArgs& A, float* dz, int* idx) {
+    __shared__ SortSegment s_stack[W][kStack];
     const int lane = threadIdx.x & 31;
-    const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    float* dz = A.dz + warp * A.stride;
-    int* idx = A.idx + warp * A.stride;
     const int total = min(*A.tie_count, A.tie_cap);
     for (;;) {
         int e = 0;
@@ -284,23 +285,62 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm) ksg_tie_kernel(
     }
 }
 
-}  // namespace
+template <int D>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm) ksg_tie_kernel(KsgTieArgs A) {
+    const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    resolve_ties<D, kWarpsPerCta>(A, A.dz + warp * A.stride, A.idx + warp * A.stride);
+}
 
-int ksg_tie_warps() { return sm_count() * kCtasPerSm * kWarpsPerCta; }
+// The same with the rows in shared memory, for rows up to kSmemRow samples: a
+// replay is a chain of dependent reads of the row (a key behind an index), so
+// a plan with one tie waited 100 us for it at m = 1000. From kSmemRow on the
+// few warps that fit an SM resolve fewer ties at a time than the reads of the
+// global rows cost (ten samples in flight at m = 3400 against 48).
+constexpr int kSmemRow = 3400;
+constexpr int kSmemWarps = 4;
 
-void ksg_launch_ties(const KsgTieArgs& a, int d, cudaStream_t st) {
-    const int grid = sm_count() * kCtasPerSm;
-    const int threads = kWarpsPerCta * 32;
-    switch (d) {
-        case 1: ksg_tie_kernel<1><<<grid, threads, 0, st>>>(a); break;
-        case 2: ksg_tie_kernel<2><<<grid, threads, 0, st>>>(a); break;
-        case 3: ksg_tie_kernel<3><<<grid, threads, 0, st>>>(a); break;
-        default: fail(NSG_ERR_INVALID, "d must be 1, 2 or 3");
+template <int D>
+__global__ void __launch_bounds__(kSmemWarps * 32) ksg_tie_smem_kernel(KsgTieArgs A) {
+    extern __shared__ float s_rows[];
+    float* dz = s_rows + (threadIdx.x >> 5) * 2 * A.stride;
+    resolve_ties<D, kSmemWarps>(A, dz, reinterpret_cast<int*>(dz + A.stride));
+}
+
+template <int D>
+void launch_ties(const KsgTieArgs& a, long long samples, cudaStream_t st) {
+    // at most a warp per eight samples: the list is short, and empty CTAs are
+    // what the kernel costs on small plans (8 us for a pair)
+    auto ctas = [&](int warps, int per_sm) {
+        const long long most = (samples + 8 * warps - 1) / (8 * warps);
+        return static_cast<int>(std::min<long long>(sm_count() * per_sm, std::max<long long>(most, 1)));
+    };
+    if (a.stride <= kSmemRow) {
+        const size_t smem = sizeof(float) * 2 * kSmemWarps * static_cast<size_t>(a.stride);
+        // set on every launch: the attribute belongs to the current device
+        NSG_CUDA(cudaFuncSetAttribute(ksg_tie_smem_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem)));
+        const int per_sm = std::min(12, static_cast<int>((size_t(220) << 10) / (smem + 4096)));
+        ksg_tie_smem_kernel<D><<<ctas(kSmemWarps, per_sm), kSmemWarps * 32, smem, st>>>(a);
+    } else {
+        ksg_tie_kernel<D><<<ctas(kWarpsPerCta, kCtasPerSm), kWarpsPerCta * 32, 0, st>>>(a);
     }
     NSG_CUDA(cudaGetLastError());
 }
 
-// The same kernel on a caller-chosen number of CTAs (the caller's scratch
+}  // namespace
+
+int ksg_tie_warps() { return sm_count() * kCtasPerSm * kWarpsPerCta; }
+
+void ksg_launch_ties(const KsgTieArgs& a, int d, long long samples, cudaStream_t st) {
+    switch (d) {
+        case 1: launch_ties<1>(a, samples, st); break;
+        case 2: launch_ties<2>(a, samples, st); break;
+        case 3: launch_ties<3>(a, samples, st); break;
+        default: fail(NSG_ERR_INVALID, "d must be 1, 2 or 3");
+    }
+}
+
+// The kernel over global rows on a caller-chosen number of CTAs (the caller's scratch
 // holds kWarpsPerCta * ctas rows).
 void ksg_launch_ties_ctas(const KsgTieArgs& a, int d, int ctas, cudaStream_t st) {
     const int threads = kWarpsPerCta * 32;

@@ -69,8 +69,9 @@ __device__ __forceinline__ float tie_marginal(const float (&q)[D], const float* 
 // segment stack; all lanes load and vote. A segment whose depth budget runs
 // out is heapsorted by lane 0 (heap_sort_like_reference). Same result as the
 // serial routine, element for element.
+// ranked: 64 bytes of shared memory of the warp's own.
 __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortSegment* stack,
-                                 int cap, int lane) {
+                                 int cap, unsigned char* ranked, int lane) {
     if (n <= 1) return true;
     constexpr int kThreshold = 16;
     int top = 0;
@@ -150,13 +151,19 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
                 // stopper of rmask while it lies left of it; those pairs form
                 // a prefix of t and are swapped together, lane t taking pair t
                 const int npair = lend ? 0 : min(__popc(lmask), __popc(rmask));
+                // (each stopper's lane writes itself down at its rank)
+                const unsigned before = (1u << lane) - 1u;
+                if (lmask >> lane & 1u) ranked[__popc(lmask & before)] = static_cast<unsigned char>(lane);
+                if (rmask >> lane & 1u) ranked[32 + __popc(rmask & before)] = static_cast<unsigned char>(lane);
+                __syncwarp();
                 int lp = 0x7fffffff, rp = -1;
                 if (lane < npair) {
-                    lp = lchunk + static_cast<int>(__fns(lmask, 0, lane + 1));
-                    rp = rchunk - static_cast<int>(__fns(rmask, 0, lane + 1));
+                    lp = lchunk + ranked[lane];
+                    rp = rchunk - ranked[32 + lane];
                 }
                 const bool swap = lane < npair && lp < rp;
                 const int c = __popc(__ballot_sync(kFull, swap));
+                const int llast = c ? ranked[c - 1] : 0, rlast = c ? ranked[32 + c - 1] : 0;
                 if (swap) {
                     const int t = idx[lp];
                     idx[lp] = idx[rp];
@@ -166,10 +173,8 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
                 if (c > 0) prev_r = __shfl_sync(kFull, rp, c - 1);
                 if (c == npair && !lend) {
                     // every pair of the round swapped: drop them, continue
-                    for (int q = 0; q < c; ++q) {
-                        lmask &= lmask - 1;
-                        rmask &= rmask - 1;
-                    }
+                    lmask &= kFull << llast << 1;
+                    rmask &= kFull << rlast << 1;
                     continue;
                 }
                 // pair c crosses (or no left stopper is left)
@@ -189,8 +194,31 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
         if (first < T && last > prefix_end) prefix_end = last;
     }
     __syncwarp();
-    // insertion sort of [0, prefix_end) (at most a few dozen elements)
-    if (lane == 0) {
+    // The insertion sort of [0, prefix_end), a few dozen elements, is a stable
+    // sort: an element's place is the number of smaller keys plus the equal
+    // ones before it. Longer prefixes (heapsorted segments among them) are left
+    // to lane 0.
+    if (prefix_end <= 64) {
+        int v[2] = {0, 0}, place[2] = {0, 0};
+        float kv[2] = {0.f, 0.f};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = 32 * h + lane;
+            if (i < prefix_end) {
+                v[h] = idx[i];
+                kv[h] = key[v[h]];
+            }
+        }
+        for (int j = 0; j < prefix_end; ++j) {
+            const float kj = __shfl_sync(kFull, j < 32 ? kv[0] : kv[1], j & 31);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) place[h] += kj < kv[h] || (kj == kv[h] && j < 32 * h + lane);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (32 * h + lane < prefix_end) idx[place[h]] = v[h];
+    } else if (lane == 0) {
         for (int i = 1; i < prefix_end; ++i) {
             const int v = idx[i];
             const float kv = key[v];
@@ -211,6 +239,7 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
 template <int D, int W>
 __device__ __forceinline__ void resolve_ties(const KsgTieArgs& A, float* dz, int* idx) {
     __shared__ SortSegment s_stack[W][kStack];
+    __shared__ unsigned char s_ranked[W][64];
     const int lane = threadIdx.x & 31;
     const int total = min(*A.tie_count, A.tie_cap);
     for (;;) {
@@ -241,7 +270,7 @@ __device__ __forceinline__ void resolve_ties(const KsgTieArgs& A, float* dz, int
             idx[j] = j;
         }
         __syncwarp();
-        const int ok = sort_prefix_warp(dz, idx, m, A.k + 1, s_stack[threadIdx.x >> 5], kStack, lane) ? 1 : 0;
+        const int ok = sort_prefix_warp(dz, idx, m, A.k + 1, s_stack[threadIdx.x >> 5], kStack, s_ranked[threadIdx.x >> 5], lane) ? 1 : 0;
         __syncwarp();
         if (!ok) {
             if (lane == 0) atomicOr(A.fault, FAULT_TIE_UNRESOLVED);

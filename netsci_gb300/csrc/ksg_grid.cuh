@@ -678,8 +678,14 @@ __global__ void __launch_bounds__(32 * kGridWarps, 4) ksg_grid_count_kernel(Grid
         int gi, blk;
         item_of(A.gprefix, A.ngroups, t, gi, blk);
         const CountGroup& grp = A.groups[gi];
-        if (grp.nvars <= 4) count_item<D, 4>(A, grp, gi, blk, tile, lane);
-        else count_item<D, kCountGroup>(A, grp, gi, blk, tile, lane);
+        // a variable costs two instructions per frame beside five for the distance
+        switch (grp.nvars) {
+            case 1: case 2: count_item<D, 2>(A, grp, gi, blk, tile, lane); break;
+            case 3: case 4: count_item<D, 4>(A, grp, gi, blk, tile, lane); break;
+            case 5: count_item<D, 5>(A, grp, gi, blk, tile, lane); break;
+            case 6: count_item<D, 6>(A, grp, gi, blk, tile, lane); break;
+            default: count_item<D, kCountGroup>(A, grp, gi, blk, tile, lane); break;
+        }
     }
 }
 
@@ -808,8 +814,11 @@ __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_ran
                     continue;
                 }
                 // bucket of a distance or eps up to emax: a monotone function
-                const float inv = emax > 0.f ? kRankBuckets / emax : 0.f;
-                auto bucket = [&](float v) { return min(kRankBuckets - 1, static_cast<int>(v * inv)); };
+                // (rounded into the low mantissa bits of 2^23)
+                const float inv = emax > 0.f ? fminf((kRankBuckets - 1) / emax, 3e38f) : 0.f;
+                auto bucket = [&](float v) {
+                    return __float_as_int(__fmaf_rn(v, inv, 8388608.f)) & (2 * kRankBuckets - 1);
+                };
                 int4* t4 = reinterpret_cast<int4*>(tab) + 4 * lane;
                 int4* c4 = reinterpret_cast<int4*>(cnt) + 2 * lane;
 #pragma unroll

@@ -44,6 +44,7 @@
 // gives the reference's fixed point bit for bit; the automatic mode squares
 // only then (analyze_kernel checks A on the device) and runs Jacobi steps
 // otherwise.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -73,6 +74,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// S CTAs of a cluster share a tile (blockIdx.z), each reducing 1/S of k; the
+// partial minima meet in distributed shared memory, 1/S of the tile's
+// outputs per CTA. A minimum does not depend on the order, so the result is
+// the same. Matrices of few tiles leave most SMs idle otherwise: at n = 500 64
+// tiles took 25 us per step on 64 of 152 SMs.
+template <int S>
 __global__ void __launch_bounds__(kThreads, 4)
 hedetniemi_step_kernel(const float* __restrict__ X, const float* __restrict__ Ap,
                        float* __restrict__ Xn, int n, int P, int* changed, int step) {
@@ -113,11 +120,12 @@ hedetniemi_step_kernel(const float* __restrict__ X, const float* __restrict__ Ap
 #pragma unroll
         for (int v = 0; v < 4; ++v) acc[u][v] = inf;
 
-    const int nslab = P / kSlab;
-    load_slab(0, 0);
+    const int nslab = P / kSlab / S;
+    const int k_first = S > 1 ? static_cast<int>(blockIdx.z) * nslab * kSlab : 0;
+    load_slab(0, k_first);
     for (int sl = 0; sl < nslab; ++sl) {
         if (sl + 1 < nslab) {
-            load_slab((sl + 1) & 1, (sl + 1) * kSlab);
+            load_slab((sl + 1) & 1, k_first + (sl + 1) * kSlab);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
@@ -145,18 +153,41 @@ hedetniemi_step_kernel(const float* __restrict__ X, const float* __restrict__ Ap
     }
 
     bool diff = false;
+    if constexpr (S == 1) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int i = i0 + tx + 16 * u;
-        if (i >= n) continue;
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + tx + 16 * u;
+            if (i >= n) continue;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int j = j0 + ty + 16 * v;
-            if (j >= n) continue;
-            const size_t o = (size_t)j * P + i;
-            if (__float_as_int(acc[u][v]) != __float_as_int(__ldg(X + o))) diff = true;
-            Xn[o] = acc[u][v];
+            for (int v = 0; v < 4; ++v) {
+                const int j = j0 + ty + 16 * v;
+                if (j >= n) continue;
+                const size_t o = (size_t)j * P + i;
+                if (__float_as_int(acc[u][v]) != __float_as_int(__ldg(X + o))) diff = true;
+                Xn[o] = acc[u][v];
+            }
         }
+    } else {
+        static_assert(sizeof(Xs) >= sizeof(float) * kTileI * kTileJ, "a tile's partial minima fit one stage pair");
+        auto cluster = cooperative_groups::this_cluster();
+        float* part = &Xs[0][0][0];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) part[(ty + 16 * v) * kTileI + tx + 16 * u] = acc[u][v];
+        cluster.sync();
+        constexpr int kShare = kTileI * kTileJ / S;
+        for (int e = blockIdx.z * kShare + tid; e < (static_cast<int>(blockIdx.z) + 1) * kShare; e += kThreads) {
+            float m = inf;
+#pragma unroll
+            for (int r = 0; r < S; ++r) m = fminf(m, cluster.map_shared_rank(part, r)[e]);
+            const int i = i0 + e % kTileI, j = j0 + e / kTileI;
+            if (i >= n || j >= n) continue;
+            const size_t o = (size_t)j * P + i;
+            if (__float_as_int(m) != __float_as_int(__ldg(X + o))) diff = true;
+            Xn[o] = m;
+        }
+        cluster.sync();  // the others may still read this CTA's part
     }
     if (__syncthreads_or(diff) && tid == 0) changed[step] = 1;
 }
@@ -242,11 +273,34 @@ __global__ void corr_to_adj_kernel(const float* __restrict__ C, float* __restric
     A[idx] = v;
 }
 
+template <int S>
+void launch_split_step(const float* Ap, const float* X, float* Xn, int n, int P, int* changed, int step,
+                       cudaStream_t s) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(P / kTileJ, P / kTileI, S);
+    c.blockDim = dim3(kThreads);
+    c.stream = s;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim = {1, 1, S};
+    c.attrs = &a;
+    c.numAttrs = 1;
+    NSG_CUDA(cudaLaunchKernelEx(&c, hedetniemi_step_kernel<S>, X, Ap, Xn, n, P, changed, step));
+}
+
+// Up to 160 tiles (n <= 768) four CTAs a tile, up to 320 (n <= 1088) two: the
+// GPU holds 608 CTAs of this kernel.
 void launch_step(const float* Ap, const float* X, float* Xn, int n, int P, int* changed, int step,
                  cudaStream_t s) {
-    dim3 grid(P / kTileJ, P / kTileI);
-    hedetniemi_step_kernel<<<grid, kThreads, 0, s>>>(X, Ap, Xn, n, P, changed, step);
-    NSG_CUDA(cudaGetLastError());
+    const int tiles = (P / kTileJ) * (P / kTileI);
+    if (tiles <= 160) {
+        launch_split_step<4>(Ap, X, Xn, n, P, changed, step, s);
+    } else if (tiles <= 320) {
+        launch_split_step<2>(Ap, X, Xn, n, P, changed, step, s);
+    } else {
+        hedetniemi_step_kernel<1><<<dim3(P / kTileJ, P / kTileI), kThreads, 0, s>>>(X, Ap, Xn, n, P, changed, step);
+        NSG_CUDA(cudaGetLastError());
+    }
 }
 
 void launch_pad(const float* src, float* dst, int n, int P, bool transpose, cudaStream_t s) {

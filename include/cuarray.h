@@ -74,8 +74,14 @@ private:
     // copies of large arrays run at the link's speed; else new[].
     T* alloc_host(size_t count);
     void free_host();
+    // init() without the zeros, for results that overwrite all of it.
+    CuArrayError init_unset(int m, int n);
+    template <typename U>
+    friend void init_result(CuArray<U>* a, int m, int n);
     T* host_;
     T* device_;
+    T* own_ = nullptr;       // the storage alloc_host made last, and its size:
+    size_t own_count_ = 0;   // init() to the same size keeps it
     T* pinned_ = nullptr;  // host_ came from cudaHostAlloc (freed with cudaFreeHost)
     int n_{};
     int m_{};
@@ -85,6 +91,12 @@ private:
     int allocatedHost_{};
     int owner_{};
 };
+
+// Shape of a result whose every element is written next.
+template <typename U>
+void init_result(CuArray<U>* a, int m, int n) {
+    a->init_unset(m, n);
+}
 
 // Non-owning view of one row.
 template <typename T>

@@ -50,6 +50,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "apsp.h"
@@ -313,6 +315,31 @@ void launch_unpad(const float* X, float* H, int n, int P, cudaStream_t s) {
     NSG_CUDA(cudaGetLastError());
 }
 
+// The device's pool of solver workspace. The driver's default pool gives its
+// memory back at every synchronisation, so each small solve mapped its
+// matrices anew; this one keeps up to kPoolKeep bytes between solves and gives
+// them back through apsp_release_pools.
+constexpr unsigned long long kPoolKeep = 1ull << 30;
+std::mutex g_pool_mu;
+std::map<int, cudaMemPool_t> g_pools;
+
+cudaMemPool_t workspace_pool() {
+    int dev = 0;
+    NSG_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    cudaMemPool_t& pool = g_pools[dev];
+    if (!pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        NSG_CUDA(cudaMemPoolCreate(&pool, &props));
+        unsigned long long keep = kPoolKeep;
+        NSG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    return pool;
+}
+
 // Workspace allocated and freed in the order of the solver's stream, so a
 // solve does not wait for kernels on other streams.
 struct DevMem {
@@ -323,7 +350,7 @@ struct DevMem {
     }
     void alloc(size_t bytes, cudaStream_t st) {
         s = st;
-        NSG_CUDA(cudaMallocAsync(&p, bytes, st));
+        NSG_CUDA(cudaMallocFromPoolAsync(&p, bytes, workspace_pool(), st));
     }
     ~DevMem() { if (p) cudaFreeAsync(p, s); }
     DevMem(const DevMem&) = delete;
@@ -448,6 +475,12 @@ int sparse_steps(const Graph& g, const float* A, float* H, float* T, int n, int 
 }
 
 }  // namespace
+
+void apsp_release_pools() {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    for (auto& [dev, pool] : g_pools)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+}
 
 void apsp_set_method(int method) {
     if (method < -1 || method > 1) invalid("method must be -1, 0 or 1");

@@ -14,6 +14,8 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
 // for on a symmetric, zero-diagonal, non-negative A (float weights then
 // within rounding of the reference's association).
 void apsp_set_method(int method);
+// Gives the workspace kept between solves back to the driver (all devices).
+void apsp_release_pools();
 // H and paths (device, n*L*n ints) as netcalc/src/hedetniemi_gpu.cu:148-235.
 // Blocks on s.
 void apsp_paths(const float* A, float* H, int* paths, int n, int L, float tolerance,

@@ -31,17 +31,18 @@ constexpr size_t kPinnedMinBytes = size_t(16) << 20;
 template <typename T>
 T* CuArray<T>::alloc_host(size_t count) {
     if (count == 0) count = 1;
+    own_count_ = count;
     const size_t bytes = count * sizeof(T);
     if (bytes >= kPinnedMinBytes) {
         void* p = nullptr;
         if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) {
-            pinned_ = static_cast<T*>(p);
+            pinned_ = own_ = static_cast<T*>(p);
             return pinned_;
         }
         cudaGetLastError();  // no device: ordinary memory
     }
     pinned_ = nullptr;
-    return new T[count];
+    return own_ = new T[count];
 }
 
 template <typename T>
@@ -59,6 +60,8 @@ template <typename T>
 void CuArray<T>::release() {
     if (allocatedHost_ && owner_ && host_) free_host();
     pinned_ = nullptr;
+    own_ = nullptr;
+    own_count_ = 0;
     if (allocatedDevice_ && device_) cudaFree(device_);
     host_ = nullptr;
     device_ = nullptr;
@@ -67,17 +70,31 @@ void CuArray<T>::release() {
 }
 
 template <typename T>
-CuArrayError CuArray<T>::init(int m, int n) {
+CuArrayError CuArray<T>::init_unset(int m, int n) {
     if (m < 0 || n < 0) return 1;
-    release();
+    const size_t count = static_cast<size_t>(m * n);
+    if (owner_ && allocatedHost_ && host_ && host_ == own_ && own_count_ == std::max<size_t>(count, 1)) {
+        // the same size again: the storage stays (new pages would fault in one by one)
+        if (allocatedDevice_ && device_) cudaFree(device_);
+        device_ = nullptr;
+        allocatedDevice_ = 0;
+    } else {
+        release();
+        owner_ = 1;
+        host_ = alloc_host(count);
+    }
     m_ = m;
     n_ = n;
     size_ = m * n;
     bytes_ = static_cast<size_t>(size_) * sizeof(T);
-    owner_ = 1;
-    host_ = alloc_host(static_cast<size_t>(size_));
-    std::fill(host_, host_ + size_, T(0));
     allocatedHost_ = 1;
+    return 0;
+}
+
+template <typename T>
+CuArrayError CuArray<T>::init(int m, int n) {
+    if (init_unset(m, n)) return 1;
+    std::fill(host_, host_ + size_, T(0));
     return 0;
 }
 
@@ -122,11 +139,14 @@ CuArrayError CuArray<T>::fromCuArrayDeepCopy(CuArray<T>* src, int start, int end
     pinned_ = nullptr;
     T* copy = alloc_host(static_cast<size_t>(m) * n);
     T* const copy_pinned = pinned_;
+    const size_t copy_count = own_count_;
     std::copy(src->host_ + static_cast<size_t>(start) * src->n_,
               src->host_ + static_cast<size_t>(end + 1) * src->n_, copy);
     pinned_ = old_pinned;
     release();
     pinned_ = copy_pinned;
+    own_ = copy;
+    own_count_ = copy_count;
     owner_ = 1;
     m_ = m;
     n_ = n;

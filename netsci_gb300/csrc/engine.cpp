@@ -82,13 +82,31 @@ DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {
     return *this;
 }
 
+thread_local int DeviceBuffer::idle_ = 0;
+
+DeviceBuffer::IdleScope::IdleScope() : idle_(DeviceBuffer::idle_ > 0 || cudaDeviceSynchronize() == cudaSuccess) {
+    DeviceBuffer::idle_ += idle_;
+}
+DeviceBuffer::IdleScope::~IdleScope() { DeviceBuffer::idle_ -= idle_; }
+
+void DeviceBuffer::view(void* p, size_t bytes) {
+    release();
+    p_ = p;
+    bytes_ = bytes;
+}
+
 void DeviceBuffer::release() {
     if (!p_) return;
+    if (device_ < 0) {  // a view
+        p_ = nullptr;
+        bytes_ = 0;
+        return;
+    }
     BlockCache& c = block_cache();
     int cur = -1;
     cudaGetDevice(&cur);
     bool cached = false;
-    if (cur == device_ && cudaDeviceSynchronize() == cudaSuccess) {
+    if (cur == device_ && (idle_ > 0 || cudaDeviceSynchronize() == cudaSuccess)) {
         std::lock_guard<std::mutex> lock(c.mu);
         if (c.held[device_] + capacity_ <= kBlockCacheBytes) {
             c.blocks[device_].emplace(capacity_, p_);
@@ -179,6 +197,7 @@ double tiled_us(int d, int k, int max_m, double work) {
 // per batch: work-queue heads (two for the grid search), tie count,
 // tie-kernel counter, rank-count queue head, bitmap-search queue heads
 constexpr int kCounters = 5 + kBitSegments;
+size_t counter_bytes(size_t batches) { return (kCounters * batches * sizeof(int) + 7) / 8 * 8; }
 }  // namespace
 
 std::shared_ptr<const DeviceBuffer> device_psi(int n) {
@@ -275,6 +294,34 @@ long long count_items(const std::vector<nsg_ksg_pair>& pairs, int qc) {
 // Timing events per batch: search begin, search end, counts begin (after
 // the count-order kernel), counts end, tie kernel begin, tie kernel end.
 constexpr int kEventsPerBatch = 6;
+
+// Host arrays that reach the device in one copy: each add() names the buffer
+// that becomes a view of the array's place.
+class KsgPlan::Upload {
+public:
+    template <typename V>
+    void add(DeviceBuffer& to, const V& v) {
+        if (v.empty()) return;
+        const size_t off = (bytes_.size() + 255) / 256 * 256, n = v.size() * sizeof(v[0]);
+        bytes_.resize(off + n);
+        std::memcpy(bytes_.data() + off, v.data(), n);
+        places_.push_back({&to, off, n});
+    }
+    void commit(DeviceBuffer& block) {
+        block.reset(bytes_.size());
+        if (bytes_.empty()) return;
+        NSG_CUDA(cudaMemcpy(block.get(), bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice));
+        for (const Place& q : places_) q.to->view(block.as<unsigned char>() + q.off, q.n);
+    }
+
+private:
+    struct Place {
+        DeviceBuffer* to;
+        size_t off, n;
+    };
+    std::vector<unsigned char> bytes_;
+    std::vector<Place> places_;
+};
 
 KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const KsgOutputs& out,
                  const KsgPlanOptions& opt)
@@ -513,17 +560,13 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     }
 
     if (npairs) {
-        pairs_dev_.reset(descs.size() * sizeof(KsgPairDesc));
-        NSG_CUDA(cudaMemcpy(pairs_dev_.get(), descs.data(), descs.size() * sizeof(KsgPairDesc),
-                            cudaMemcpyHostToDevice));
-        if (!items.empty()) {
-            items_dev_.reset(items.size() * sizeof(KsgItem));
-            NSG_CUDA(cudaMemcpy(items_dev_.get(), items.data(), items.size() * sizeof(KsgItem),
-                                cudaMemcpyHostToDevice));
-        }
+        Upload up;
+        up.add(pairs_dev_, descs);
+        up.add(items_dev_, items);
+        up.add(fault_, std::vector<int>(1, FAULT_NONE));
         scratch_.reset(static_cast<size_t>(scratch_need) * sizeof(float));
         // per batch: work-queue head, tie count, tie-kernel work counter
-        counters_.reset(kCounters * batches_.size() * sizeof(int));
+        counters_.reset(counter_bytes(batches_.size()) + 3 * sizeof(unsigned long long));
         // Samples with an ambiguous tie are rare (about 1e-4 on trajectory
         // data), but nothing bounds them: the list holds every sample of the
         // largest batch, so it cannot overflow (8 bytes per sample, beside
@@ -537,12 +580,13 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
         tie_cap_ = static_cast<int>(std::min<long long>(std::max<long long>(1, batch_samples), 1LL << 30));
         ties_.reset(static_cast<size_t>(tie_cap_) * sizeof(KsgTie));
         tie_stride_ = maxm;
-        tie_dz_.reset(static_cast<size_t>(ksg_tie_warps()) * tie_stride_ * sizeof(float));
-        tie_idx_.reset(static_cast<size_t>(ksg_tie_warps()) * tie_stride_ * sizeof(int));
-        fault_.reset(sizeof(int));
-        NSG_CUDA(cudaMemset(fault_.get(), 0, sizeof(int)));
+        if (!ksg_ties_in_smem(maxm)) {
+            tie_dz_.reset(static_cast<size_t>(ksg_tie_warps()) * tie_stride_ * sizeof(float));
+            tie_idx_.reset(static_cast<size_t>(ksg_tie_warps()) * tie_stride_ * sizeof(int));
+        }
         psi_ = device_psi(maxm);
-        if (search_) setup_grid(descs);
+        if (search_) setup_grid(descs, up);
+        up.commit(meta_);
     }
     if (timing_) {
         events_.resize(kEventsPerBatch * batches_.size());
@@ -551,6 +595,9 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
 }
 
 KsgPlan::~KsgPlan() {
+    DeviceBuffer::IdleScope idle;  // one wait for all blocks below
+    for (DeviceBuffer* b : {&scratch_, &counters_, &ties_, &tie_dz_, &tie_idx_, &mapped_rows_, &meta_}) b->reset(0);
+    grid_.reset();
     for (auto e : events_) cudaEventDestroy(e);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (capture_stream_) cudaStreamDestroy(capture_stream_);
@@ -558,7 +605,7 @@ KsgPlan::~KsgPlan() {
 
 void KsgPlan::enqueue(cudaStream_t s) {
     if (batches_.empty()) return;
-    NSG_CUDA(cudaMemsetAsync(counters_.get(), 0, kCounters * batches_.size() * sizeof(int), s));
+    NSG_CUDA(cudaMemsetAsync(counters_.get(), 0, counters_.bytes(), s));
     if (search_) {
         enqueue_grid(s);
         return;
@@ -650,12 +697,11 @@ struct KsgPlan::GridState {
     std::vector<int> nranks, rank_items;
     DeviceBuffer corder;                  // count-query order: ngroups x largest m of a batch
     DeviceBuffer eps_a, eps_b, cnt_a, cnt_b;
-    DeviceBuffer evals;                   // 3 counters per run (see GridArgs::evals)
     int nnodes = 0;
     int search_grid = 0, count_grid = 0;
 };
 
-void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
+void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs, Upload& up) {
     auto g = std::make_shared<GridState>();
     // nodes: one per distinct (row, m, ld)
     struct Key {
@@ -697,9 +743,7 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
         nodes[i] = grid_node_at(base + node_off[i], nodes[i].x, nodes[i].ld, nodes[i].m, d_);
         g->max_m = std::max(g->max_m, nodes[i].m);
     }
-    g->nodes.reset(nodes.size() * sizeof(GridNode));
-    NSG_CUDA(cudaMemcpy(g->nodes.get(), nodes.data(), nodes.size() * sizeof(GridNode),
-                        cudaMemcpyHostToDevice));
+    up.add(g->nodes, nodes);
 
     // pair grids: every batch reuses one arena sized for the largest batch
     size_t pair_arena = 0;
@@ -756,28 +800,20 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
                 corder = std::max(corder, w.groups.size() * static_cast<size_t>(g->batch_maxm[bi]));
             }
         }
-        auto upload = [](DeviceBuffer& dst, const auto& v) {
-            if (v.empty()) return;
-            dst.reset(v.size() * sizeof(v[0]));
-            NSG_CUDA(cudaMemcpy(dst.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
-        };
         g->corder.reset(corder * sizeof(int));
-        upload(g->groups, groups);
-        upload(g->gprefix, gpre);
-        upload(g->ranks, ranks);
-        upload(g->rprefix, rpre);
-        upload(g->refs, refs);
+        up.add(g->groups, groups);
+        up.add(g->gprefix, gpre);
+        up.add(g->ranks, ranks);
+        up.add(g->rprefix, rpre);
+        up.add(g->refs, refs);
     }
-    g->gps.reset(gps.size() * sizeof(GridPair));
-    NSG_CUDA(cudaMemcpy(g->gps.get(), gps.data(), gps.size() * sizeof(GridPair), cudaMemcpyHostToDevice));
-    g->wprefix.reset(wpre.size() * sizeof(int));
-    NSG_CUDA(cudaMemcpy(g->wprefix.get(), wpre.data(), wpre.size() * sizeof(int), cudaMemcpyHostToDevice));
+    up.add(g->gps, gps);
+    up.add(g->wprefix, wpre);
     const size_t ns = scratch_.bytes() / sizeof(float);
     g->eps_a.reset(ns * sizeof(float));
     g->eps_b.reset(ns * sizeof(float));
     g->cnt_a.reset(ns * sizeof(int));
     g->cnt_b.reset(ns * sizeof(int));
-    g->evals.reset(3 * sizeof(unsigned long long));
     g->search_grid = sm_count() * grid_search_ctas_per_sm(d_, kmax_);
     g->count_grid = sm_count() * grid_count_ctas_per_sm(d_);
     grid_ = std::move(g);
@@ -787,7 +823,6 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs) {
 
 void KsgPlan::enqueue_grid(cudaStream_t s) {
     GridState& g = *grid_;
-    NSG_CUDA(cudaMemsetAsync(g.evals.get(), 0, 3 * sizeof(unsigned long long), s));
     grid_launch_gather(gather_rows_.as<GatherRow>(), ngather_, d_, fault_.as<int>(), s);
     grid_launch_nodes(g.nodes.as<GridNode>(), g.nnodes, d_, g.split_nodes, s);
     if (g.node_est) bits_launch_est(g.nodes.as<GridNode>(), g.nnodes, g.max_m, d_, s);
@@ -827,7 +862,7 @@ void KsgPlan::enqueue_grid(cudaStream_t s) {
         a.eps_b = g.eps_b.as<float>();
         a.cnt_a = g.cnt_a.as<int>();
         a.cnt_b = g.cnt_b.as<int>();
-        a.evals = g.evals.as<unsigned long long>();
+        a.evals = evals();
         a.eps_x = out_.eps_x;
         a.eps_y = out_.eps_y;
         a.kdist = out_.kdist;
@@ -903,6 +938,10 @@ int KsgPlan::launches() const {
     return n;
 }
 
+unsigned long long* KsgPlan::evals() const {
+    return reinterpret_cast<unsigned long long*>(counters_.as<unsigned char>() + counter_bytes(batches_.size()));
+}
+
 int KsgPlan::staging() const { return entry_ ? entry_->tma : 0; }
 
 long long KsgPlan::tied_samples() const {
@@ -921,7 +960,7 @@ void KsgPlan::evaluations(unsigned long long* search, unsigned long long* counts
     if (compares) *compares = 0;
     if (!search_ || !grid_) return;
     unsigned long long h[3] = {0, 0, 0};
-    NSG_CUDA(cudaMemcpy(h, grid_->evals.get(), sizeof(h), cudaMemcpyDeviceToHost));
+    NSG_CUDA(cudaMemcpy(h, evals(), sizeof(h), cudaMemcpyDeviceToHost));
     *search = h[0];
     *counts = h[1];
     if (compares) *compares = h[2];

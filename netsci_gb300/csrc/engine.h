@@ -31,9 +31,25 @@ public:
     T* as() const { return static_cast<T*>(p_); }
     size_t bytes() const { return bytes_; }
     void reset(size_t bytes);
+    // Points at memory that another buffer owns.
+    void view(void* p, size_t bytes);
+    // Releases within the scope find the device idle: it waits once instead
+    // of once per block. Only for blocks that nothing enqueued after the
+    // scope's begin uses.
+    class IdleScope {
+    public:
+        IdleScope();
+        ~IdleScope();
+        IdleScope(const IdleScope&) = delete;
+        IdleScope& operator=(const IdleScope&) = delete;
+
+    private:
+        bool idle_ = false;
+    };
 
 private:
     void release();
+    static thread_local int idle_;  // open IdleScopes of this thread
     void* p_ = nullptr;
     size_t bytes_ = 0;     // requested
     size_t capacity_ = 0;  // size of the block
@@ -110,7 +126,9 @@ private:
     };
     void enqueue(cudaStream_t s);
     void enqueue_grid(cudaStream_t s);
-    void setup_grid(const std::vector<KsgPairDesc>& descs);
+    class Upload;
+    void setup_grid(const std::vector<KsgPairDesc>& descs, Upload& up);
+    unsigned long long* evals() const;
 
     int d_, k_, kmax_;
     long long npairs_ = 0;
@@ -121,7 +139,10 @@ private:
     const struct KsgKernelEntry* entry_ = nullptr;
     KsgOutputs out_;
     std::vector<Batch> batches_;
-    DeviceBuffer pairs_dev_, items_dev_, scratch_, counters_, fault_;
+    DeviceBuffer meta_;                  // one upload: descriptors, work lists, the fault word
+    DeviceBuffer pairs_dev_, items_dev_, fault_;  // views of it
+    DeviceBuffer scratch_;
+    DeviceBuffer counters_;              // counters of the batches, then three evaluation counts
     DeviceBuffer ties_, tie_dz_, tie_idx_;
     int tie_cap_ = 0;
     long long tie_stride_ = 0;

@@ -105,6 +105,8 @@ void ksg_launch_counts(const KsgCountArgs& a, int d, int kmax, const KsgShape& s
 void ksg_launch_final(const KsgFinalArgs& a, cudaStream_t st);
 // Warps the tie kernel runs with (scratch rows needed).
 int ksg_tie_warps();
+// Whether rows of m samples are replayed in shared memory (dz and idx unused).
+bool ksg_ties_in_smem(int m);
 // samples: of the whole run, an upper bound on the ties.
 void ksg_launch_ties(const KsgTieArgs& a, int d, long long samples, cudaStream_t st);
 void ksg_launch_ties_ctas(const KsgTieArgs& a, int d, int ctas, cudaStream_t st);

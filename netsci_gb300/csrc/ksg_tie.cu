@@ -358,6 +358,8 @@ void launch_ties(const KsgTieArgs& a, long long samples, cudaStream_t st) {
 
 }  // namespace
 
+bool ksg_ties_in_smem(int m) { return m <= kSmemRow; }
+
 int ksg_tie_warps() { return sm_count() * kCtasPerSm * kWarpsPerCta; }
 
 void ksg_launch_ties(const KsgTieArgs& a, int d, long long samples, cudaStream_t st) {

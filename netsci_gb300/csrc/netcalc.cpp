@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <iostream>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -97,10 +98,13 @@ void gpu_pair_list(const DeviceBuffer& xd, int ld, int nodes, CuArray<int>* ab, 
     DeviceBuffer mi(sizeof(float) * count);
     KsgOutputs o;
     o.mi = mi.as<float>();
-    KsgPlan plan(pairs, k, d, o, KsgPlanOptions{});
-    plan.run(nullptr);
+    auto plan = std::make_unique<KsgPlan>(pairs, k, d, o, KsgPlanOptions{});
+    plan->run(nullptr);
     NSG_CUDA(cudaMemcpy(out, mi.get(), sizeof(float) * count, cudaMemcpyDeviceToHost));
-    raise_fault(plan.take_fault());
+    raise_fault(plan->take_fault());
+    DeviceBuffer::IdleScope idle;  // one wait for all of the call's blocks
+    plan.reset();
+    mi.reset(0);
 }
 
 float gpu_single_pair(CuArray<float>* Xa, CuArray<float>* Xb, int k, int n, int d) {
@@ -116,11 +120,15 @@ float gpu_single_pair(CuArray<float>* Xa, CuArray<float>* Xb, int k, int n, int 
     DeviceBuffer mi(sizeof(float));
     KsgOutputs o;
     o.mi = mi.as<float>();
-    KsgPlan plan(pairs, k, d, o, KsgPlanOptions{});
-    plan.run(nullptr);
+    auto plan = std::make_unique<KsgPlan>(pairs, k, d, o, KsgPlanOptions{});
+    plan->run(nullptr);
     float r = 0.f;
     NSG_CUDA(cudaMemcpy(&r, mi.get(), sizeof(float), cudaMemcpyDeviceToHost));
-    raise_fault(plan.take_fault());
+    raise_fault(plan->take_fault());
+    DeviceBuffer::IdleScope idle;  // one wait for all of the call's blocks
+    plan.reset();
+    mi.reset(0);
+    buf.reset(0);
     return r;
 }
 
@@ -260,6 +268,12 @@ void check_square(CuArray<float>* A) {
     if (!A || !A->allocatedHost() || !A->host()) nsg::invalid("A has no host data");
     if (A->m() != A->n()) nsg::invalid("A must be square");
 }
+
+// H as an n x n result of A: zeros only where it is A itself.
+void result_matrix(CuArray<float>* A, CuArray<float>* H, int n) {
+    if (H == A) H->init(n, n);
+    else init_result(H, n, n);
+}
 }  // namespace
 
 void hedetniemiAllShortestPaths(CuArray<float>* A, CuArray<float>* H, CuArray<int>* paths,
@@ -280,8 +294,8 @@ void hedetniemiAllShortestPathsGpu(CuArray<float>* A, CuArray<float>* H, CuArray
     if (maxPathLength < 1) nsg::invalid("maxPathLength must be >= 1");
     const int n = A->n();
     const size_t nn = static_cast<size_t>(n) * n;
-    H->init(n, n);
-    paths->init(1, n * maxPathLength * n);
+    result_matrix(A, H, n);
+    init_result(paths, 1, n * maxPathLength * n);
     nsg::DeviceBuffer a(nn * sizeof(float)), h(nn * sizeof(float));
     nsg::DeviceBuffer p(nn * maxPathLength * sizeof(int));
     NSG_CUDA(cudaMemcpy(a.get(), A->host(), nn * sizeof(float), cudaMemcpyHostToDevice));
@@ -309,7 +323,7 @@ void hedetniemiAllShortestPathLengthsGpu(CuArray<float>* A, CuArray<float>* H,
     if (maxPathLength < 0) nsg::invalid("maxPathLength must be >= 0");
     const int n = A->n();
     const size_t nn = static_cast<size_t>(n) * n;
-    H->init(n, n);
+    result_matrix(A, H, n);
     nsg::DeviceBuffer a(nn * sizeof(float)), h(nn * sizeof(float));
     NSG_CUDA(cudaMemcpy(a.get(), A->host(), nn * sizeof(float), cudaMemcpyHostToDevice));
     nsg::apsp_lengths(a.as<float>(), h.as<float>(), n, maxPathLength, nullptr);

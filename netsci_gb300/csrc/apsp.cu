@@ -390,12 +390,16 @@ struct Graph {
     bool symmetric = false;
     bool sparse = false;
     long long width = 0;
-    DevMem words, edges;  // GraphInfo, counts, slice offsets; the entries
+    DevMem words, edges;  // GraphInfo, counts, slice offsets, order, rank; the entries
     SellView rows{};
+    const int* order = nullptr;  // vertices by falling degree, where the entries are in those labels
+    const int* rank = nullptr;
 
-    // unbounded: every shortest path may be taken (maxPathLength >= n - 1)
-    Graph(const float* A, int n, bool unbounded, cudaStream_t s)
-        : words(sizeof(GraphInfo) + sizeof(int) * (2 * (size_t)n + 2), s), edges(0, nullptr) {
+    // unbounded: every shortest path may be taken (maxPathLength >= n - 1);
+    // steps: the most sparse steps whose labels are the solve's own (0 keeps
+    // the matrix's)
+    Graph(const float* A, int n, bool unbounded, int steps, cudaStream_t s)
+        : words(sizeof(GraphInfo) + sizeof(int) * (4 * (size_t)n + 2), s), edges(0, nullptr) {
         const int method = g_method.load();
         const bool may_square = method != 0 && n >= 2 && unbounded;
         GraphInfo* info = static_cast<GraphInfo*>(words.p);
@@ -418,7 +422,16 @@ struct Graph {
         sparse = n <= kSparseMaxN && sparse_step_seconds(width, n) < dense_step_seconds(n);
         if (!sparse) return;
         edges.alloc(sizeof(int2) * kSellRows * (size_t)std::max<long long>(1, width), s);
-        sparse_fill(A, n, n, ptr, static_cast<int2*>(edges.p), s);
+        if (sparse_sort_pays(width, h.entries, n, steps)) {  // shorter slices, so the entries fit
+            int* ord = ptr + n + 2;
+            sparse_sort(counts, n, ord, ord + n, s);
+            sparse_slices_sorted(counts, ord, n, info, ptr, s);
+            sparse_fill_sorted(A, n, ord, ord + n, ptr, static_cast<int2*>(edges.p), s);
+            order = ord;
+            rank = ord + n;
+        } else {
+            sparse_fill(A, n, n, ptr, static_cast<int2*>(edges.p), s);
+        }
         rows = {static_cast<const int2*>(edges.p), ptr, sell_slices(n)};
     }
 };
@@ -458,19 +471,21 @@ int ceil_log2(int v) {
     return b;
 }
 
-// Sparse Jacobi steps between H and a second matrix, the first one reading A
-// itself. Returns as run_steps; *at is the iterate after *launched steps.
+// Sparse Jacobi steps between H and T, the first one reading A (or T, if A is
+// null). Returns as run_steps; *at is the iterate after *launched steps, in T
+// where both hold it.
 int sparse_steps(const Graph& g, const float* A, float* H, float* T, int n, int most, cudaStream_t s, int* launched,
                  bool* converged, float** at) {
     DevMem changed(sizeof(int) * most, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * most, s));
     int* ch = static_cast<int*>(changed.p);
     const int steps = run_steps(most, ch, s, [&](int t) {
-        sparse_step(g.rows, t == 0 ? A : (t & 1) ? H : T, (t & 1) ? T : H, n, ch, t, false, s);
+        sparse_step(g.rows, t == 0 && A ? A : (t & 1) ? H : T, (t & 1) ? T : H, n, ch, t, false, s);
     }, launched, converged);
     // step t writes H for even t; after a step that changed nothing both
-    // matrices hold the fixed point (or H alone, if it was the first)
-    *at = *converged || (*launched & 1) ? H : T;
+    // matrices hold the fixed point (H alone, if it was the first and A not T)
+    if (*converged) *at = A ? H : T;
+    else *at = (*launched & 1) ? H : T;
     return steps;
 }
 
@@ -494,13 +509,29 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         NSG_CUDA(cudaMemcpyAsync(H, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
         return 0;
     }
-    Graph g(A, n, max_path_length >= n - 1, s);
+    const Graph g(A, n, max_path_length >= n - 1, max_path_length, s);
     const bool sparse = g.sparse && g.squaring != 2;
-    DevMem T(sparse ? nn * sizeof(float) : 0, s), copy(sparse && overlap(A, H, nn) ? nn * sizeof(float) : 0, s);
-    if (copy.p) {
+    DevMem T(sparse ? nn * sizeof(float) : 0, s);
+    DevMem copy(sparse && !g.order && overlap(A, H, nn) ? nn * sizeof(float) : 0, s);
+    const float* from = A;
+    if (g.order) {  // the steps start from the relabelled matrix in T
+        sparse_relabel(A, static_cast<float*>(T.p), n, g.order, s);
+        from = nullptr;
+    } else if (copy.p) {
         NSG_CUDA(cudaMemcpyAsync(copy.p, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
-        A = static_cast<const float*>(copy.p);
+        from = static_cast<const float*>(copy.p);
     }
+    auto deliver = [&](float* at) {  // into H, in the matrix's own labels
+        if (g.order) {
+            if (at == H) {
+                at = static_cast<float*>(T.p);
+                NSG_CUDA(cudaMemcpyAsync(at, H, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            }
+            sparse_restore(at, H, n, g.order, g.rank, s);
+        } else if (at != H) {
+            NSG_CUDA(cudaMemcpyAsync(H, at, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        }
+    };
     int launched = 0, first = 0;
     bool converged = false;
     float* at = nullptr;
@@ -516,13 +547,14 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
             const int most = ceil_log2(n);
             while (first < most && ((2 << first) - 1) * step <= (first + 1) * product) ++first;
             if (first > 0) {
-                const int h = sparse_steps(g, A, H, static_cast<float*>(T.p), n, (1 << first) - 1, s, &launched,
+                const int h = sparse_steps(g, from, H, static_cast<float*>(T.p), n, (1 << first) - 1, s, &launched,
                                            &converged, &at);
+                deliver(at);
                 if (converged) {
                     NSG_CUDA(cudaStreamSynchronize(s));
                     return ceil_log2(h) + 1;
                 }
-                A = at;  // A^(2^first)
+                A = H;  // A^(2^first)
             }
         }
         Iterates it(A, n, s);
@@ -549,9 +581,9 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         return first + q + 1;
     }
     if (sparse) {
-        const int steps = sparse_steps(g, A, H, static_cast<float*>(T.p), n, max_path_length, s, &launched,
+        const int steps = sparse_steps(g, from, H, static_cast<float*>(T.p), n, max_path_length, s, &launched,
                                        &converged, &at);
-        if (at != H) NSG_CUDA(cudaMemcpyAsync(H, at, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        deliver(at);
         NSG_CUDA(cudaStreamSynchronize(s));
         return steps;
     }
@@ -574,7 +606,7 @@ void apsp_paths(const float* A, float* H, int* paths, int n, int L, float tolera
     const size_t nn = (size_t)n * n;
     NSG_CUDA(cudaMemsetAsync(paths, 0xff, sizeof(int) * nn * L, s));  // -1
     if (n == 0) return;
-    Graph g(A, n, false, s);
+    Graph g(A, n, false, 0, s);
     DevMem snaps(nn * (L + 1) * sizeof(float), s);  // H before each step, and after the last
     DevMem changed(sizeof(int) * L, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * L, s));

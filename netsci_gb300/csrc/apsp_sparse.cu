@@ -70,17 +70,22 @@ __global__ void count_kernel(const float* __restrict__ A, int ld, int n, int* co
 
 // Slice widths (the longest row of each slice, in whole groups of
 // kSellUnroll) and their exclusive prefix; one CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ counts, int n, int nslices, int* ptr,
-                                                     GraphInfo* info) {
+// order: the vertex of each row, or null for the matrix's own order.
+__global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ counts, const int* __restrict__ order,
+                                                     int n, int nslices, int* ptr, GraphInfo* info) {
     __shared__ int s_warp[32];
     const int t = threadIdx.x, lane = t & 31;
-    int base = 0;
+    int base = 0, entries = 0;
     for (int s0 = 0; s0 < nslices; s0 += 1024) {
         const int s = s0 + t;
         int w = 0;
         for (int r = 0; r < kSellRows; ++r) {
             const int row = s * kSellRows + r;
-            if (s < nslices && row < n) w = max(w, counts[row]);
+            if (s < nslices && row < n) {
+                const int c = counts[order ? order[row] : row];
+                w = max(w, c);
+                entries += c;
+            }
         }
         w = (w + kSellUnroll - 1) / kSellUnroll * kSellUnroll;
         int x = w;
@@ -100,6 +105,10 @@ __global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ cou
         base = all;
         __syncthreads();
     }
+    if (!order) {  // the second pass over the same counts adds nothing new
+        entries = __reduce_add_sync(0xffffffffu, entries);
+        if (lane == 0) atomicAdd(&info->entries, entries);
+    }
     if (t == 0) {
         ptr[nslices] = base;
         info->width = base;
@@ -107,28 +116,63 @@ __global__ void __launch_bounds__(1024) slice_kernel(const int* __restrict__ cou
 }
 
 // One warp per row (of whole slices): its entries in ascending columns, then
-// the padding up to the slice's width.
-__global__ void fill_kernel(const float* __restrict__ A, int ld, int n, int nslices, const int* __restrict__ ptr,
-                            int2* __restrict__ edges) {
+// the padding up to the slice's width. With order and rank, row r is vertex
+// order[r]'s and columns are ranks.
+__global__ void fill_kernel(const float* __restrict__ A, int ld, int n, int nslices, const int* __restrict__ order,
+                            const int* __restrict__ rank, const int* __restrict__ ptr, int2* __restrict__ edges) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (row >= nslices * kSellRows) return;
     const int s = row / kSellRows, r = row % kSellRows;
     const int end = ptr[s + 1];
     int e = ptr[s];
     if (row < n) {
+        const int vertex = order ? order[row] : row;
         for (int k0 = 0; k0 < n; k0 += 32) {
             const int k = k0 + lane;
-            const float a = k < n ? __ldg(A + (size_t)row * ld + k) : __int_as_float(kInfBits);
+            const float a = k < n ? __ldg(A + (size_t)vertex * ld + k) : __int_as_float(kInfBits);
             const bool keep = __float_as_int(a) != kInfBits;
             const unsigned mask = __ballot_sync(0xffffffffu, keep);
             if (keep) {
                 const int at = e + __popc(mask & ((1u << lane) - 1u));
-                edges[(size_t)at * kSellRows + r] = make_int2(k, __float_as_int(a));
+                edges[(size_t)at * kSellRows + r] = make_int2(rank ? rank[k] : k, __float_as_int(a));
             }
             e += __popc(mask);
         }
     }
     for (int p = e + lane; p < end; p += 32) edges[(size_t)p * kSellRows + r] = make_int2(0, kInfBits);
+}
+
+// Rank of every vertex by falling count, ties in index order: a thread per
+// vertex compares it with all others (n^2 compares from shared memory).
+__global__ void __launch_bounds__(256) sort_kernel(const int* __restrict__ counts, int n, int* order, int* rank) {
+    __shared__ int s_c[1024];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int mine = i < n ? counts[i] : 0;
+    int r = 0;
+    for (int base = 0; base < n; base += 1024) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < 1024; q += blockDim.x) s_c[q] = base + q < n ? counts[base + q] : -1;
+        __syncthreads();
+        for (int q = 0; q < min(1024, n - base); ++q) r += s_c[q] > mine || (s_c[q] == mine && base + q < i);
+    }
+    if (i < n) {
+        rank[i] = r;
+        order[r] = i;
+    }
+}
+
+// One row per CTA through shared memory: row to[r] of out takes the elements
+// pick[c] of row from[r] (null: the row or element itself).
+__global__ void __launch_bounds__(256) pick_kernel(const float* __restrict__ A, float* __restrict__ out, int n,
+                                                   const int* __restrict__ from, const int* __restrict__ to,
+                                                   const int* __restrict__ pick) {
+    extern __shared__ float s_row[];
+    const int r = blockIdx.x;
+    const float* src = A + (size_t)(from ? from[r] : r) * n;
+    float* dst = out + (size_t)(to ? to[r] : r) * n;
+    for (int c = threadIdx.x; c < n; c += blockDim.x) s_row[c] = __ldg(src + c);
+    __syncthreads();
+    for (int c = threadIdx.x; c < n; c += blockDim.x) dst[c] = s_row[pick[c]];
 }
 
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem, int bytes16) {
@@ -314,20 +358,56 @@ static_assert(kMax16 * 16 * 4 <= 224 << 10 && kMax8 * 8 * 4 <= 224 << 10 && kSpa
 void sparse_analyze(const float* A, int n, GraphInfo* info, int* counts, int* ptr, cudaStream_t s) {
     const int t = (n + 31) / 32;
     analyze_kernel<<<dim3(t, t), dim3(32, 8), 0, s>>>(A, n, info, counts);
-    slice_kernel<<<1, 1024, 0, s>>>(counts, n, sell_slices(n), ptr, info);
+    slice_kernel<<<1, 1024, 0, s>>>(counts, nullptr, n, sell_slices(n), ptr, info);
     NSG_CUDA(cudaGetLastError());
 }
 
 void sparse_count(const float* A, int ld, int n, GraphInfo* info, int* counts, int* ptr, cudaStream_t s) {
     count_kernel<<<(n + 7) / 8, 256, 0, s>>>(A, ld, n, counts);
-    slice_kernel<<<1, 1024, 0, s>>>(counts, n, sell_slices(n), ptr, info);
+    slice_kernel<<<1, 1024, 0, s>>>(counts, nullptr, n, sell_slices(n), ptr, info);
     NSG_CUDA(cudaGetLastError());
 }
 
 void sparse_fill(const float* A, int ld, int n, const int* ptr, int2* edges, cudaStream_t s) {
     const int ns = sell_slices(n);
-    fill_kernel<<<ns, 32 * kSellRows, 0, s>>>(A, ld, n, ns, ptr, edges);
+    fill_kernel<<<ns, 32 * kSellRows, 0, s>>>(A, ld, n, ns, nullptr, nullptr, ptr, edges);
     NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_sort(const int* counts, int n, int* order, int* rank, cudaStream_t s) {
+    sort_kernel<<<(n + 255) / 256, 256, 0, s>>>(counts, n, order, rank);
+    NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_slices_sorted(const int* counts, const int* order, int n, GraphInfo* info, int* ptr, cudaStream_t s) {
+    slice_kernel<<<1, 1024, 0, s>>>(counts, order, n, sell_slices(n), ptr, info);
+    NSG_CUDA(cudaGetLastError());
+}
+
+void sparse_fill_sorted(const float* A, int n, const int* order, const int* rank, const int* ptr, int2* edges,
+                        cudaStream_t s) {
+    const int ns = sell_slices(n);
+    fill_kernel<<<ns, 32 * kSellRows, 0, s>>>(A, n, n, ns, order, rank, ptr, edges);
+    NSG_CUDA(cudaGetLastError());
+}
+
+namespace {
+void launch_pick(const float* A, float* out, int n, const int* from, const int* to, const int* pick, cudaStream_t s) {
+    const size_t smem = sizeof(float) * n;
+    // set on every launch: the attribute belongs to the current device
+    NSG_CUDA(cudaFuncSetAttribute(pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(float) * kSparseMaxN)));
+    pick_kernel<<<n, 256, smem, s>>>(A, out, n, from, to, pick);
+    NSG_CUDA(cudaGetLastError());
+}
+}  // namespace
+
+void sparse_relabel(const float* A, float* out, int n, const int* order, cudaStream_t s) {
+    launch_pick(A, out, n, order, nullptr, order, s);
+}
+
+void sparse_restore(const float* A, float* out, int n, const int* order, const int* rank, cudaStream_t s) {
+    launch_pick(A, out, n, nullptr, order, rank, s);
 }
 
 void sparse_step(const SellView& g, const float* H, float* Hn, int n, int* changed, int step, bool fill,
@@ -339,6 +419,20 @@ void sparse_step(const SellView& g, const float* H, float* Hn, int n, int* chang
 
 double sparse_step_seconds(long long width, int n) {
     return 3e-6 + 8.0 * static_cast<double>(width) * n / 6e12;
+}
+
+// Sorted slices hold the entries and about two of padding per row group (their
+// widths are rounded up to kSellUnroll). Measured per solve: the sort, the
+// slices and the fill 25 us, the two passes over the matrix 2.7 TB/s. Random
+// geometric graphs of mean degree 12, without -> with: n = 1200 350 -> 353 us
+// after 16 steps (not taken), n = 2000 602 -> 587 us after 16 and 2.00 ->
+// 1.81 ms after 61, n = 8000 9.42 -> 8.72 ms after 16. A ring of degree 6 has
+// nothing to gain: n = 4000 1.55 -> 1.65 ms (not taken).
+bool sparse_sort_pays(long long width, long long entries, int n, int steps) {
+    const long long sorted = entries / kSellRows + (kSellUnroll / 2) * sell_slices(n);
+    if (sorted >= width) return false;
+    const double saved = sparse_step_seconds(width, n) - sparse_step_seconds(sorted, n);
+    return std::min(steps, 16) * saved > 25e-6 + 16.0 * n * n / 2.7e12;
 }
 
 void sparse_walk(const SellView& cols, const float* H, const float* Hi, int* paths, float tolerance, int n, int L,

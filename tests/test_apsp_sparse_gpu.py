@@ -75,3 +75,30 @@ def test_long_chain_ends_in_products(n):
     H, products = device.apsp_lengths(dev, n, H=dev)  # in place
     assert np.array_equal(H.cpu().numpy(), np.abs(at[:, None] - at[None, :]))
     assert products == int(np.ceil(np.log2(max(1, n - 1)))) + 1
+
+
+@pytest.mark.parametrize("n,L", [(1800, 3), (1801, 4), (2600, 17), (2601, 2601)])
+@pytest.mark.parametrize("integer", [False, True])
+@pytest.mark.parametrize("alias", [False, True])
+def test_relabelled_steps_match_row_steps(n, L, integer, alias):
+    """Vertices sorted by degree (degrees from 1 to 160, so that the slices of
+    the matrix's own order are mostly padding): every parity of the last step,
+    converged or not, and the result over its own input."""
+    from netsci_gb300 import device
+    rng = np.random.default_rng(n)
+    A = np.full((n, n), np.inf, np.float32)
+    i = np.arange(1, n)
+    j = rng.integers(0, i)                       # a random tree
+    A[i, j] = A[j, i] = rng.integers(1, 50, n - 1) if integer else rng.random(n - 1) + np.float32(0.25)
+    for hub in rng.choice(n, n // 16, replace=False):
+        j = rng.choice(n, 160, replace=False)
+        w = rng.integers(1, 50, 160) if integer else rng.random(160) + 0.25
+        A[hub, j] = w
+        A[j, hub] = w
+    np.fill_diagonal(A, 0.0)
+    want, steps = _jacobi(A, L)
+    a = torch.from_numpy(A).cuda()
+    H, got = device.apsp_lengths(a, L, a if alias else None)
+    if L < n - 1 or not integer:  # otherwise repeated squaring counts products
+        assert got == steps
+    assert np.array_equal(H.cpu().numpy(), want)

@@ -187,13 +187,19 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem, int bytes
 // four columns each, so 32/(C/4) rows are reduced per warp at a time and the
 // entries of a slice arrive as one 64-byte load per entry index. Results go
 // out transposed (Hn[i][j], j along the lanes). The compare against H stops
-// reading H once a difference was seen in the CTA.
+// reading H once a difference was seen in the CTA. The entries' latency and
+// the conflicts of the row reads (64-byte rows, two to a shared-memory line)
+// bound it: the next group of entries loads while one is reduced, across the
+// slices of a warp, their offsets from shared memory (n = 2000, degree 12:
+// 1.81 -> 1.73 ms for 61 steps, n = 8000 32.0 -> 30.2 ms for 64; two groups
+// ahead 1.74 and 30.6 ms, three 1.78 and 31.7 ms: the registers run out).
 template <int C>
 __global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const float* __restrict__ H,
                                                            float* __restrict__ Hn, int n, int per_split, int vec,
                                                            int* changed, int step, int fill) {
     extern __shared__ __align__(16) float hs[];
     __shared__ int s_diff;
+    int* s_ptr = reinterpret_cast<int*>(hs + (size_t)n * C);  // offsets of this CTA's slices
     constexpr int kLanes = C / 4;           // lanes per row
     constexpr int kRows = 32 / kLanes;      // rows per warp
     constexpr int kSlices = kRows / kSellRows;
@@ -224,6 +230,7 @@ __global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const flo
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int idx = tid; idx <= last - first; idx += blockDim.x) s_ptr[idx] = __ldg(g.ptr + first + idx);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const float4* h4 = reinterpret_cast<const float4*>(hs);
@@ -234,18 +241,34 @@ __global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const flo
     float* out = Hn + (size_t)(i0 + 4 * q) * n;
     const float* old = H + (size_t)(i0 + 4 * q) * n;
     bool diff = false;
-    for (int s0 = first + (tid >> 5) * kSlices; s0 < last; s0 += stride) {
-        const int s = s0 + rw / kSellRows;
-        if (s >= last) continue;
-        const int e0 = __ldg(g.ptr + s);
-        int groups = (__ldg(g.ptr + s + 1) - e0) / kSellUnroll;
-        float acc[4] = {inf, inf, inf, inf};
-        const int2* ed = g.edges + (size_t)e0 * kSellRows + r;
-        int2 p[kSellUnroll];
-        if (groups > 0) {
-#pragma unroll
-            for (int e = 0; e < kSellUnroll; ++e) p[e] = __ldg(ed + e * kSellRows);
+    int s = first + (tid >> 5) * kSlices + rw / kSellRows;
+    // a group of entries is loaded while the one before it is reduced, on into the next slice
+    int ls = s, left = 0;
+    const int2* ed = nullptr;
+    auto open = [&] {  // first slice from ls on that has entries
+        for (; ls < last; ls += stride) {
+            const int e0 = s_ptr[ls - first];
+            left = (s_ptr[ls - first + 1] - e0) / kSellUnroll;
+            ed = g.edges + (size_t)e0 * kSellRows + r;
+            if (left > 0) return;
         }
+    };
+    open();
+    int2 p[kSellUnroll];
+    auto load = [&] {
+        if (left == 0) return;
+#pragma unroll
+        for (int e = 0; e < kSellUnroll; ++e) p[e] = __ldg(ed + e * kSellRows);
+        ed += kSellUnroll * kSellRows;
+        if (--left == 0) {
+            ls += stride;
+            open();
+        }
+    };
+    load();
+    for (; s < last; s += stride) {
+        int groups = (s_ptr[s - first + 1] - s_ptr[s - first]) / kSellUnroll;
+        float acc[4] = {inf, inf, inf, inf};
         for (; groups > 0; --groups) {
             float4 v[kSellUnroll];
             float a[kSellUnroll];
@@ -254,11 +277,7 @@ __global__ void __launch_bounds__(1024) sparse_step_kernel(SellView g, const flo
                 v[e] = h4[p[e].x * kLanes + q];
                 a[e] = __int_as_float(p[e].y);
             }
-            ed += kSellUnroll * kSellRows;
-            if (groups > 1) {  // the next entries load while these are reduced
-#pragma unroll
-                for (int e = 0; e < kSellUnroll; ++e) p[e] = __ldg(ed + e * kSellRows);
-            }
+            load();
 #pragma unroll
             for (int e = 0; e < kSellUnroll; e += 2) {
                 acc[0] = nsg_min3(acc[0], __fadd_rn(a[e], v[e].x), __fadd_rn(a[e + 1], v[e + 1].x));
@@ -328,30 +347,33 @@ int sm_count_now() {
     return sms;
 }
 
+// Columns per CTA: 16 while n rows of them fit in shared memory, then 8 and 4.
+constexpr int kMax16 = 3500, kMax8 = 7000;
+constexpr int kStepSmem = 227 * 1024 - 64;
+constexpr int step_smem(int n, int columns, int slices) { return 4 * (n * columns + slices + 1); }
+static_assert(step_smem(kMax16, 16, kMax16 / 8 + 1) <= kStepSmem && step_smem(kMax8, 8, kMax8 / 8 + 1) <= kStepSmem &&
+                  step_smem(kSparseMaxN, 4, kSparseMaxN / 8 + 1) <= kStepSmem,
+              "a column block fits in shared memory");
+
 template <int C>
 void launch_step(const SellView& g, const float* H, float* Hn, int n, int* changed, int step, bool fill,
                  cudaStream_t s) {
     static_assert(C % 4 == 0 && 32 / (C / 4) >= kSellRows, "whole slices per warp");
     constexpr int kSlices = 32 / (C / 4) / kSellRows;
-    const size_t smem = (size_t)n * C * sizeof(float);
-    // set on every launch: the attribute belongs to the current device
-    NSG_CUDA(cudaFuncSetAttribute(sparse_step_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
     const int blocks = (n + C - 1) / C;
     // slices split over CTAs until there is one per SM, at least one warp's worth each
     const int splits = std::max(1, std::min(sm_count_now() / blocks, g.nslices / (4 * kSlices)));
     const int per = (g.nslices + splits - 1) / splits;
     const int warps = std::min(32, std::max(4, (per + kSlices - 1) / kSlices));
     const int vec = (n % 4 == 0) && (reinterpret_cast<uintptr_t>(H) % 16 == 0);
+    // set on every launch: the attribute belongs to the current device. One
+    // value for all sizes: another thread may set it before this launch.
+    NSG_CUDA(cudaFuncSetAttribute(sparse_step_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
+    const int smem = step_smem(n, C, per);
     sparse_step_kernel<C><<<dim3(blocks, (g.nslices + per - 1) / per), 32 * warps, smem, s>>>(
         g, H, Hn, n, per, vec, changed, step, fill ? 1 : 0);
     NSG_CUDA(cudaGetLastError());
 }
-
-// Columns per CTA: 16 while n rows of them fit in shared memory, then 8 and 4.
-constexpr int kMax16 = 3500, kMax8 = 7000;
-static_assert(kMax16 * 16 * 4 <= 224 << 10 && kMax8 * 8 * 4 <= 224 << 10 && kSparseMaxN * 4 * 4 <= 224 << 10,
-              "a column block fits in shared memory");
 
 }  // namespace
 

@@ -9,11 +9,12 @@
 
 namespace nsg {
 
+// Shared memory of an SM, and what a CTA takes beside its dynamic part.
+static constexpr size_t kSm = 228 << 10, kStatic = 2048, kReserved = 1024;
+
 BitsConfig bits_config(int d, int k, int max_m) {
     BitsConfig c;
     if (d < 1 || d > 3 || max_m < 1 || max_m > kBitMaxM) return c;
-    // Shared memory of an SM, and what a CTA takes beside its dynamic part.
-    constexpr size_t kSm = 228 << 10, kStatic = 2048, kReserved = 1024;
     const int nc = 2 * d - 1, ws = bit_row_words(max_m);
     c.keep = k <= 12 ? 1 : 3;
     // The first coordinate's interval covers about (k/m)^(1/2d) of the frames,
@@ -57,9 +58,10 @@ namespace {
 
 template <int D, int N, int W>
 void launch(const BitsArgs& a, const BitsConfig& c, int grid, cudaStream_t s) {
-    // set on every launch: the attribute belongs to the current device
+    // set on every launch: the attribute belongs to the current device. One
+    // value for all plans: another thread may set it before this launch.
     NSG_CUDA(cudaFuncSetAttribute(ksg_bits_search_kernel<D, N, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(c.smem)));
+                                  static_cast<int>(kSm - kStatic - kReserved)));
     ksg_bits_search_kernel<D, N, W><<<grid, c.threads, c.smem, s>>>(a);
     NSG_CUDA(cudaGetLastError());
 }

@@ -345,9 +345,10 @@ void launch_ties(const KsgTieArgs& a, long long samples, cudaStream_t st) {
     };
     if (a.stride <= kSmemRow) {
         const size_t smem = sizeof(float) * 2 * kSmemWarps * static_cast<size_t>(a.stride);
-        // set on every launch: the attribute belongs to the current device
+        // set on every launch: the attribute belongs to the current device. One
+        // value for all plans: another thread may set it before this launch.
         NSG_CUDA(cudaFuncSetAttribute(ksg_tie_smem_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
+                                      static_cast<int>(sizeof(float) * 2 * kSmemWarps * kSmemRow)));
         const int per_sm = std::min(12, static_cast<int>((size_t(220) << 10) / (smem + 4096)));
         ksg_tie_smem_kernel<D><<<ctas(kSmemWarps, per_sm), kSmemWarps * 32, smem, st>>>(a);
     } else {

@@ -23,6 +23,7 @@ namespace nsg {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr size_t kMaxSmem = 200 << 10;
 constexpr int kList = 96;  // frames within the bound a query keeps
 
 template <int D>
@@ -181,9 +182,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) ksg_warp_kernel(KsgCountArg
 
 template <int D>
 void launch(const KsgCountArgs& a, size_t smem, cudaStream_t st) {
-    // set on every launch: the attribute belongs to the current device
+    // set on every launch: the attribute belongs to the current device. One
+    // value for all plans: another thread may set it before this launch.
     NSG_CUDA(cudaFuncSetAttribute(ksg_warp_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
+                                  static_cast<int>(kMaxSmem)));
     ksg_warp_kernel<D><<<a.nitems, 32 * kWarpsPerCta, smem, st>>>(a);
     NSG_CUDA(cudaGetLastError());
 }
@@ -198,7 +200,7 @@ size_t smem_bytes(int d, int max_m) {
 bool ksg_warp_fits(int d, int k, int max_m, double work) {
     const double us = (0.8 + 0.7 * d) * work * 1e-6;
     // the bound comes from 32 lane minima
-    return k <= 30 && us <= 120 && smem_bytes(d, max_m) <= (size_t(200) << 10);
+    return k <= 30 && us <= 120 && smem_bytes(d, max_m) <= kMaxSmem;
 }
 
 void ksg_launch_warp(const KsgCountArgs& a, int d, int max_m, cudaStream_t st) {

@@ -83,7 +83,8 @@ struct Found {
 };
 
 // The first part of [q - h, q + h] and one past its last among the parts
-// that 63 ascending edges e (padded with +inf) cut an axis into.
+// that 63 ascending edges e (padded with +inf) cut an axis into. With an
+// infinite h, hi passes the last part: such bins are never used.
 __device__ __forceinline__ void reach(const float* e, float q, float h, int& lo, int& hi) {
     lo = hi = 0;
 #pragma unroll
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
             reach(s_edge[c], s_query[8 * t + (c < D ? c : 4 + c - D)], s_query[8 * t + 3], lo, hi);
             if (c == 0) {
                 lo = s_start[lo] / (32 * W);
-                hi = (s_start[hi] + 32 * W - 1) / (32 * W);
+                hi = (s_start[min(hi, kBitBins)] + 32 * W - 1) / (32 * W);
             } else {
                 lo = ((c - 1) * R + lo) * (WS / W);
                 hi = ((c - 1) * R + hi) * (WS / W);
@@ -723,7 +724,7 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
                     if (__fsub_rn(x, s_whole[c][a + s - 1]) > est) a += s;
                     if (__fsub_rn(s_whole[c][b + s - 1], x) <= est) b += s;
                 }
-                ++b;
+                b = min(b + 1, R - 1);  // an infinite estimate reaches past the padded edges
                 if (c == 0) {
                     a = s_start[min(a * step, kBitBins)] >> 5;
                     b = (s_start[min(b * step, kBitBins)] + 31) >> 5;

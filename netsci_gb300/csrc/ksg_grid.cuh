@@ -618,7 +618,10 @@ __device__ __forceinline__ void count_item(const GridArgs& A, const CountGroup& 
     // each query's box of rows [qrlo, qrhi] and columns [qclo, qchi];
     // a row is scanned over the columns of the queries whose box holds it
     int qrlo = G, qrhi = -1, qclo = G, qchi = -1;
-    if (valid) {
+    if (nd.ostart[63]) {  // coordinates that are not finite lie in no cell of theirs
+        qrlo = qclo = 0;
+        qrhi = qchi = G - 1;
+    } else if (valid) {
         bin_range(nd.e1, G, q1, emax, qrlo, qrhi);
         bin_range(nd.e2, G, q2, emax, qclo, qchi);
     }
@@ -738,6 +741,7 @@ __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_ran
         const GridNode& nd = A.nodes[rn.node];
         const long long* refs = A.refs + rn.first;
         const int m = rn.m, G = nd.G, P = rn.count;
+        const bool odd = nd.ostart[63] != 0;  // coordinates that are not finite lie in no cell of theirs
         const float* __restrict__ sx = nd.sx;
         for (int i = blk * kRankBlock; i < min(m, (blk + 1) * kRankBlock); ++i) {
             float q[D];
@@ -762,16 +766,24 @@ __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_ran
                 const int nv = min(kRankVars, P - v0);
                 float ev[kPer];
                 float emax = 0.f;  // eps are not negative
+                bool plain = true;
 #pragma unroll
                 for (int t = 0; t < kPer; ++t) {
                     ev[t] = 32 * t + lane < nv ? eps_of(v0 + 32 * t + lane) : 0.f;
                     emax = fmaxf(emax, ev[t]);
+                    plain &= ev[t] < inf_f();
                 }
+                // an infinite eps (or a NaN) has no bucket
+                plain = __all_sync(kFull, plain);
                 emax = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(emax)));
                 // frames of the box, two times 32 at a time: f(distance, in)
                 int rlo, rhi, clo, chi;
                 bin_range(nd.e1, G, q1, emax, rlo, rhi);
                 bin_range(nd.e2, G, q2, emax, clo, chi);
+                if (odd) {
+                    rlo = clo = 0;
+                    rhi = chi = G - 1;
+                }
                 // row r's range of positions in lane r - rlo
                 int lo = 0, hi = 0;
                 if (lane <= rhi - rlo && clo <= chi) {
@@ -794,22 +806,24 @@ __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_ran
                 const int box = __reduce_add_sync(kFull, hi - lo);
                 scanned += box;
                 compared += static_cast<unsigned long long>(box) * nv;
-                if (nv <= kRankDirect) {
-                    float e[kRankDirect];
-                    int n[kRankDirect];
+                if (nv <= kRankDirect || !plain) {
+                    for (int p0 = 0; p0 < nv; p0 += kRankDirect) {
+                        float e[kRankDirect];
+                        int n[kRankDirect];
 #pragma unroll
-                    for (int p = 0; p < kRankDirect; ++p) {
-                        e[p] = __shfl_sync(kFull, ev[0], p);
-                        n[p] = 0;
-                    }
-                    frames([&](float dm) {
+                        for (int p = 0; p < kRankDirect; ++p) {
+                            e[p] = p0 + p < nv ? eps_of(v0 + p0 + p) : 0.f;
+                            n[p] = 0;
+                        }
+                        frames([&](float dm) {
 #pragma unroll
-                        for (int p = 0; p < kRankDirect; ++p) n[p] += dm <= e[p];
-                    });
+                            for (int p = 0; p < kRankDirect; ++p) n[p] += dm <= e[p];
+                        });
 #pragma unroll
-                    for (int p = 0; p < kRankDirect; ++p) {
-                        n[p] = __reduce_add_sync(kFull, n[p]);
-                        if (p < nv && lane == 0) put(v0 + p, n[p]);
+                        for (int p = 0; p < kRankDirect; ++p) {
+                            n[p] = __reduce_add_sync(kFull, n[p]);
+                            if (p0 + p < nv && lane == 0) put(v0 + p0 + p, n[p]);
+                        }
                     }
                     continue;
                 }

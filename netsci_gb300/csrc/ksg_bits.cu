@@ -91,8 +91,19 @@ void bits_launch_est(const GridNode* nodes, int nnodes, int max_m, int d, cudaSt
         smem = sizeof(unsigned) * (d - 1) * ((kBitBins + step - 1) / step + 1) * static_cast<size_t>(bit_row_words(max_m));
         if (smem <= most) break;
     }
-    // a node's frames split over CTAs until there are two per SM
-    const int parts = std::max(1, std::min((2 * sm_count() + nnodes - 1) / nnodes, max_m / 256));
+    // A node's frames split over CTAs (one per SM: 1024 threads of 57
+    // registers), 256 frames at a time in each; every share builds the rows
+    // again, two rounds' worth.
+    const int sms = sm_count();
+    int parts = 1, best = 1 << 30;
+    for (int p = 1; p <= std::max(1, max_m / 256); ++p) {
+        const int waves = (nnodes * p + sms - 1) / sms;
+        const int cost = waves * ((max_m / p + 255) / 256 + 2);
+        if (cost < best) {
+            best = cost;
+            parts = p;
+        }
+    }
     const dim3 grid(nnodes, parts);
     switch (d) {
         case 1: bits_est_kernel<1><<<grid, kEstThreads, 0, s>>>(nodes, step); break;

@@ -128,6 +128,22 @@ def test_ties_around_the_longest_shared_row(oracle_mod, m, d):
     assert float(out["mi"].item()) == mi
 
 
+@pytest.mark.parametrize("m", [17, 401, 2450, 2500, 5150, 5200, 20480])
+@pytest.mark.parametrize("d,k", [(1, 3), (3, 40)])
+def test_ties_match_the_kernel_for_long_rows(m, d, k):
+    """A pair of longer rows in the plan sends every tie to that kernel."""
+    from netsci_gb300 import device
+    if k >= m:
+        k = m - 2
+    X, _ = device.pack_trajectory(_walk(2, d, m, m + d, 0.5), d)
+    L, _ = device.pack_trajectory(_walk(2, d, 20481, 1, 1.0), d)
+    own = device.make_pairs(X, m, [(0, 1)])
+    mi = torch.empty(3, device="cuda")
+    device.ksg_pairs(own, k, d, mi=mi[:1])
+    device.ksg_pairs(own + device.make_pairs(L, 20481, [(0, 1)]), k, d, mi=mi[1:])
+    assert _bits(mi[0:1]) == _bits(mi[1:2])
+
+
 @pytest.mark.parametrize("m", [7, 8, 9, 511, 512, 513, 1023, 1024, 1025, 2049, 4100])
 def test_sums_at_chunk_edges(oracle_mod, m):
     """The serial sum over the samples, in its chunks of 512."""

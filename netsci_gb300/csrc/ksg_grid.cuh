@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_ran
                         int n[kRankDirect];
 #pragma unroll
                         for (int p = 0; p < kRankDirect; ++p) {
-                            e[p] = p0 + p < nv ? eps_of(v0 + p0 + p) : 0.f;
+                            e[p] = p0 == 0 ? __shfl_sync(kFull, ev[0], p) : p0 + p < nv ? eps_of(v0 + p0 + p) : 0.f;
                             n[p] = 0;
                         }
                         frames([&](float dm) {

@@ -109,17 +109,18 @@ __device__ __forceinline__ int lane_prefix(int v) {
     return v;
 }
 
-// W words of a row (4 W bytes, aligned).
+// W words at a byte offset (a multiple of 4 W).
 template <int W>
-__device__ __forceinline__ void load_words(const unsigned* row, int x, unsigned (&w)[W]) {
+__device__ __forceinline__ void load_words(const unsigned* rows, unsigned at, unsigned (&w)[W]) {
+    const char* p = reinterpret_cast<const char*>(rows) + at;
     if constexpr (W == 1) {
-        w[0] = row[x];
+        w[0] = *reinterpret_cast<const unsigned*>(p);
     } else if constexpr (W == 2) {
-        const uint2 v = reinterpret_cast<const uint2*>(row)[x];
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
         w[0] = v.x;
         w[1] = v.y;
     } else {
-        const uint4 v = reinterpret_cast<const uint4*>(row)[x];
+        const uint4 v = *reinterpret_cast<const uint4*>(p);
         w[0] = v.x;
         w[1] = v.y;
         w[2] = v.z;
@@ -128,12 +129,12 @@ __device__ __forceinline__ void load_words(const unsigned* row, int x, unsigned 
 }
 
 // Position of the bit of rank win + lane among the set bits of the lanes'
-// words (lane order, then word order): word g of a lane covers positions
-// base + 32 g for g < 4 and base + 4096 + 32 (g - 4) above. off: set bits of
+// words (lane order, then word order): word g of lane l covers positions
+// base + l span + 32 g for g < 4 and 4096 - 128 more above. off: set bits of
 // the lanes before; cnt: of this lane; n: of all; table: 32 words of shared memory.
 // Lanes whose rank does not exist get an arbitrary position.
 template <int W>
-__device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int off, int cnt, int win, int n, int lane,
+__device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int span, int off, int cnt, int win, int n, int lane,
                                            unsigned* table) {
     // lanes with a bit in the window, in order, and where their bits start in it
     const int first = off - win;
@@ -145,7 +146,7 @@ __device__ __forceinline__ int bit_of_rank(const unsigned (&w)[W], int base, int
     const int src = static_cast<int>(table[__popc(starts & (kFull >> (31 - lane))) - 1] & 31u);
     int r = win + lane - __shfl_sync(kFull, off, src);  // rank within the owner's words
     if (win + lane >= n) r = 0;
-    int pos = __shfl_sync(kFull, base, src);
+    int pos = base + span * src;
     unsigned bits = __shfl_sync(kFull, w[0], src);
 #pragma unroll
     for (int g = 1; g < W; ++g) {
@@ -222,23 +223,24 @@ __device__ __forceinline__ Found select_nearest(const float* v, const float* da,
         for (int c = 0; c < N; ++c)
             less[c] += (nsg_lt_f32(y.x, x[c]) + nsg_lt_f32(y.y, x[c])) + (nsg_lt_f32(y.z, x[c]) + nsg_lt_f32(y.w, x[c]));
     }
-    unsigned wk = 0, ea = 0, eb = 0;
+    unsigned ea = 0, eb = 0;
     int le = 0;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
         const bool in = 32 * c + lane < n && less[c] <= static_cast<float>(k);
         le += __popc(__ballot_sync(kFull, in));
         if (in) {
-            wk = max(wk, __float_as_uint(x[c]));
             ea = max(ea, __float_as_uint(da[32 * c + lane]));
             eb = max(eb, __float_as_uint(db[32 * c + lane]));
         }
     }
     Found r;
-    wk = __reduce_max_sync(kFull, wk);
+    ea = __reduce_max_sync(kFull, ea);
+    eb = __reduce_max_sync(kFull, eb);
+    const unsigned wk = max(ea, eb);  // a joint distance is the larger of its marginals
     r.wk = __uint_as_float(wk);
-    r.ea = __uint_as_float(__reduce_max_sync(kFull, ea));
-    r.eb = __uint_as_float(__reduce_max_sync(kFull, eb));
+    r.ea = __uint_as_float(ea);
+    r.eb = __uint_as_float(eb);
     r.tie = false;
     if (le > k + 1 && wk != 0) {
         unsigned alo = kFull, ahi = 0, blo = kFull, bhi = 0;
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
     float* s_da = s_v + kKeep + 4;
     float* s_db = s_da + kKeep;
     unsigned* s_bins = reinterpret_cast<unsigned*>(s_db + kKeep);
-    unsigned* s_table = s_bins + Q * 2 * D;
+    unsigned* s_table = s_bins + Q * 4 * D;
     const int R = B.rows, step = B.step, k = A.k;
     int cur_a = -1;
     float scale = 1.f;               // this warp's share in h, see the file comment
@@ -456,8 +458,8 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
         const float rank = est_rank(m);
         const float base = exp2f(__log2f(static_cast<float>(k) * m / (rank * rank)) * (0.5f / D) + 0.3f);
         __syncthreads();
-        // bins of coordinate c of query t, packed: c = 0 the range of columns
-        // of W words, else the offsets of its two rows in columns
+        // bins of coordinate c of query t: c = 0 the range of columns of W
+        // words, else the byte offsets of its two rows
         auto set_bins = [&](int t, int c) {
             int lo, hi;
             reach(s_edge[c], s_query[8 * t + (c < D ? c : 4 + c - D)], s_query[8 * t + 3], lo, hi);
@@ -465,10 +467,10 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                 lo = s_start[lo] / (32 * W);
                 hi = (s_start[min(hi, kBitBins)] + 32 * W - 1) / (32 * W);
             } else {
-                lo = ((c - 1) * R + lo) * (WS / W);
-                hi = ((c - 1) * R + hi) * (WS / W);
+                lo = ((c - 1) * R + lo) * WS * 4;
+                hi = ((c - 1) * R + hi) * WS * 4;
             }
-            s_bins[2 * D * t + c] = static_cast<unsigned>(hi) << 16 | static_cast<unsigned>(lo);
+            *reinterpret_cast<int2*>(s_bins + 4 * D * t + 2 * c) = make_int2(lo, hi);
         };
         for (;;) {
             int q0 = 0;
@@ -507,8 +509,9 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                 Found r;
                 bool done = false;
                 for (int tries = 0; tries < kBitTries && !bad && h > 0.f && h < 1e30f; ++tries) {
-                    const unsigned* bins = s_bins + 2 * D * t;
-                    const int x0 = bins[0] & 0xffffu, x1 = bins[0] >> 16;
+                    const uint4* bins = reinterpret_cast<const uint4*>(s_bins + 4 * D * t);
+                    const uint4 b0 = bins[0];
+                    const int x0 = static_cast<int>(b0.x), x1 = static_cast<int>(b0.y);
                     int inside = 0;
                     int crowd = 0;
                     bool stuck = false;
@@ -517,14 +520,20 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
 #pragma unroll
                         for (int g = 0; g < W; ++g) acc[g] = 0;
                         if (x < x1) {
-#pragma unroll
-                            for (int c = 0; c < NC; ++c) {
-                                const unsigned o = bins[c + 1];
+                            const unsigned at = 4 * W * x;
+                            auto rows_of = [&](bool start, unsigned lo, unsigned hi) {
                                 unsigned u[W], v[W];
-                                load_words<W>(s_dyn, (o >> 16) + x, u);
-                                load_words<W>(s_dyn, (o & 0xffffu) + x, v);
+                                load_words<W>(s_dyn, hi + at, u);
+                                load_words<W>(s_dyn, lo + at, v);
 #pragma unroll
-                                for (int g = 0; g < W; ++g) acc[g] = c == 0 ? u[g] ^ v[g] : acc[g] & (u[g] ^ v[g]);
+                                for (int g = 0; g < W; ++g) acc[g] = start ? u[g] ^ v[g] : acc[g] & (u[g] ^ v[g]);
+                            };
+                            rows_of(true, b0.z, b0.w);
+#pragma unroll
+                            for (int q = 1; q < D; ++q) {
+                                const uint4 b = bins[q];
+                                rows_of(false, b.x, b.y);
+                                rows_of(false, b.z, b.w);
                             }
                         }
                     };
@@ -543,7 +552,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                         }
                         evals += n;
                         for (int win = 0; win < n; win += 32) {
-                            const int pos = bit_of_rank(w, base, incl - cnt, cnt, win, n, lane, s_table);
+                            const int pos = bit_of_rank(w, base, 32 * W, incl - cnt, cnt, win, n, lane, s_table);
                             float da = 0.f, db = 0.f, v = inf_f();
                             if (win + lane < n) {
                                 const int j = s_perm[pos];
@@ -588,7 +597,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
 #pragma unroll
                         for (int g = 0; g < W; ++g) cnt += __popc(u[g]);
                         if (W < 4 || xf + 32 >= x1) {
-                            stuck = !consume(u, 32 * W * x, cnt, last);
+                            stuck = !consume(u, 32 * W * xf, cnt, last);
                         } else {
                             unsigned v[W], w[2 * W];
                             column(x + 32, v);
@@ -598,7 +607,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                                 w[W + g] = v[g];
                                 cnt += __popc(v[g]);
                             }
-                            stuck = !consume(w, 32 * W * x, cnt, last);
+                            stuck = !consume(w, 32 * W * xf, cnt, last);
                         }
                     }
                     if (stuck) break;

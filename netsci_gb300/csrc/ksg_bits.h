@@ -16,7 +16,7 @@ constexpr int kCrowd = 10;
 __host__ __device__ constexpr int bit_queries(int d) { return d == 3 ? 4 : 8; }
 // Shared words per warp: queries, the 32 n nearest frames' distances, bins, bit_of_rank's table.
 __host__ __device__ constexpr int bit_warp_words(int d, int n) {
-    return bit_queries(d) * 8 + 96 * n + 4 + bit_queries(d) * 2 * d + 32;
+    return bit_queries(d) * 8 + 96 * n + 4 + bit_queries(d) * 4 * d + 32;
 }
 
 // Words of one bitmap row over m frames: whole 16-byte groups, an odd number

@@ -16,17 +16,19 @@ Lines reported (one JSON line from rank 0):
   e2e       pairs/s through the drop-in API (netcalc.generalizedCorrelation
             over host CuArrays): host->device upload of X and the pair list
             and device->host read of the results inside every step.
-  roofline  the dominant kernel (the cell-grid search) against the CUDA-core
-            issue model (SMs x 128 lanes x max SM clock) and against the
-            measured rate of its own inner loop alone (mix_ceiling); the
-            count kernel likewise under per_kernel. Operations are counted
-            from the kernels' own evaluation counters: 4d per joint distance
-            of the search; 2d-1 per one-variable distance of the counts (one
-            per query and frame, shared by the pairs of a count group) plus
-            one per eps comparison. algorithmic_pruning_gops is the rate an
-            exhaustive search would need for the same steps, 8*d*m*(m-1)
-            operations per pair: the gain of the cell grids, not a kernel
-            fraction.
+  roofline  the dominant kernel (the bitmap search) against the CUDA-core
+            issue model (SMs x 128 lanes x max SM clock): its operations are
+            lane instructions, the warp instructions per query that ncu
+            counts at this m times 32 (bitmap words, selection and the few
+            distances alike). The count kernels stand under per_kernel with
+            operations from their own evaluation counters, 2d-1 per
+            one-variable distance (one per query and frame, shared by the
+            variables of a group or a rank pass) plus one per eps comparison
+            that an unsorted count would make, and the measured rate of the
+            group kernel's inner loop alone (mix_ceiling).
+            algorithmic_pruning_gops is the rate an exhaustive search would
+            need for the same steps, 8*d*m*(m-1) operations per pair: the
+            gain of bitmaps and grids, not a kernel fraction.
   parity    GC of random pairs of the timed batches through the drop-in API
             against the reference's own CPU code (compiled unmodified into
             oracle/_ref; the oracle restatement when that is absent), bit
@@ -78,11 +80,11 @@ sys.path.insert(0, str(ROOT))
 sys.path.insert(0, str(ROOT / "netsci_gb300" / "dropin"))
 
 N_NODES, M_FRAMES, DIM, K_NN = 2000, 10000, 3, 6
-# DRAM bytes per pair of the search kernel at m = 10000, from an ncu capture
-# of a 256-pair step of this workload (profiles/ksg_grid_kernels_N2000_m10000.md:
-# 120.3 MB read + 15.8 MB written); the traffic is per pair (each pair's grid
-# copies), so it scales with the pairs.
-SEARCH_DRAM_BYTES_PER_PAIR = (120.3 + 15.8) * 1e6 / 256
+# The search kernel at m = 10000, from an ncu capture of a 256-pair step
+# (profiles/ksg_bits_kernels_m10000.md): DRAM bytes per pair (62.1 MB read and
+# 5.9 MB written) and warp instructions per query (1.610e9 over 2.56e6 queries).
+SEARCH_DRAM_BYTES_PER_PAIR = (62.1 + 5.9) * 1e6 / 256
+SEARCH_INSTRUCTIONS_PER_QUERY = 629
 SEED = 2000
 METRIC = "GC pairs/sec (batched persistent), N=2000 nodes, m=10000 frames"
 
@@ -570,7 +572,7 @@ def main():
     ops_launch = ops_per_pair(m) * B
     search = plans[args.warmup].shape["search"]
     clocks = clk.summary()
-    ceil_search, ceil_count = device.issue_ceiling(DIM)
+    _, ceil_count = device.issue_ceiling(DIM)
     search_s = statistics.mean(k[0] for k in kms) / 1000.0
     count_s = statistics.mean(k[1] for k in kms) / 1000.0
     if search == "cell-grid":
@@ -578,36 +580,36 @@ def main():
         joint = statistics.mean(e[0] for e in evs)
         one_var = statistics.mean(e[1] for e in evs)
         compares = statistics.mean(e[2] for e in evs)
-        search_ops = joint * 4 * DIM
+        search_ops = 32.0 * SEARCH_INSTRUCTIONS_PER_QUERY * m * B if m == M_FRAMES else joint * 4 * DIM
         count_ops = one_var * (2 * DIM - 1) + compares
         per_kernel = {
-            "ksg_grid_pass1_kernel": {
+            "ksg_bits_search_kernel": {
                 "ms_per_launch": 1000 * search_s, "ops_per_launch": search_ops,
-                "joint_evaluations": joint, "ops_per_evaluation": 4 * DIM,
+                "joint_evaluations": joint,
+                "ops": ("32 lanes x warp instructions per query (ncu)" if m == M_FRAMES
+                        else "4d per joint distance alone"),
                 "achieved_gops": search_ops / search_s / 1e9,
-                "frac": search_ops / search_s / 1e9 / peak_gops,
-                "mix_ceiling_gops": ceil_search,
-                "frac_of_mix_ceiling": search_ops / search_s / 1e9 / ceil_search},
-            "ksg_grid_count_kernel": {
+                "frac": search_ops / search_s / 1e9 / peak_gops},
+            "count kernels": {
                 "ms_per_launch": 1000 * count_s, "ops_per_launch": count_ops,
                 "one_variable_evaluations": one_var, "eps_comparisons": compares,
-                "ops": "2d-1 per one-variable distance + 1 per eps comparison",
+                "ops": "2d-1 per one-variable distance + 1 per (distance, variable)",
                 "achieved_gops": count_ops / count_s / 1e9,
                 "frac": count_ops / count_s / 1e9 / peak_gops,
                 "mix_ceiling_gops": ceil_count,
                 "frac_of_mix_ceiling": count_ops / count_s / 1e9 / ceil_count},
-            "ksg_tie_kernel": {
+            "ksg_tie_smem_kernel": {
                 "ms_per_launch": statistics.mean(k[2] for k in kms),
                 "tied_samples_per_launch": statistics.mean(tied),
                 "note": ("samples whose k-th distance ties between frames with different "
                          "marginals, replayed in the reference sort's order; O(m) per "
                          "sample")},
         }
-        dom = per_kernel["ksg_grid_pass1_kernel"]
-        kernel, achieved, traffic = "ksg_grid_pass1_kernel", dom["achieved_gops"], None
+        dom = per_kernel["ksg_bits_search_kernel"]
+        kernel, achieved, traffic = "ksg_bits_search_kernel", dom["achieved_gops"], None
         if m == M_FRAMES:
             traffic = SEARCH_DRAM_BYTES_PER_PAIR * B
-        mix = ceil_search
+        mix = None
     else:
         per_kernel = None
         kernel, achieved, traffic, mix = "ksg_count_kernel", ops_launch / search_s / 1e9, None, None
@@ -624,13 +626,13 @@ def main():
         "peak_source": (f"{props.multi_processor_count} SMs x 128 lanes x {sm_max:.0f} MHz "
                         "(sm_max_mhz of MEASURED_PEAKS.json; MEASURED_PEAKS.json has no "
                         "CUDA-core figure)"),
-        "mix_ceiling_source": ("nsg_measure_issue_ceiling: the kernel's own inner loop alone on a "
-                               "staged tile (no memory traffic, no range setup, no list updates), "
-                               "measured on this GPU with CUDA events"),
+        "mix_ceiling_source": ("nsg_measure_issue_ceiling: the group counts' inner loop alone on a "
+                               "staged tile (no memory traffic, no range setup), measured on this "
+                               "GPU with CUDA events"),
         "search": search, "per_kernel": per_kernel,
         "algorithmic_pruning_gops": ops_launch / (search_s + count_s) / 1e9,
         "algorithmic_pruning_note": ("8*d*m*(m-1) operations per pair (what an exhaustive "
-                                     "search does) over the two kernels' time: the cell grids' "
+                                     "search does) over the kernels' time: the pruning's "
                                      "gain, not a kernel fraction"),
     }
 
@@ -749,9 +751,11 @@ def main():
             apsp[f"{name}_schedule"] = "squaring" if products < steps_j else "jacobi"
             apsp[f"{name}_jacobi_ms"] = ms_j
             apsp[f"{name}_jacobi_steps"] = steps_j
-            # min-plus terms (one add and one min per (i, j, k)) per second of
-            # the Jacobi steps, against one term per lane per cycle (packed
-            # add + 3-input min: two instructions per two terms)
+            # min-plus terms (one add and one min per (i, j, k)) of a dense
+            # product per second of the Jacobi steps, against one term per
+            # lane per cycle (packed add + 3-input min: two instructions per
+            # two terms); the sparse steps visit only the finite entries, so
+            # the fraction passes 1
             apsp[f"{name}_terms_per_s"] = n_g ** 3 * steps_j / (ms_j / 1000)
             apsp_graphs[name] = (A_np, H.cpu().numpy(), steps_j)
         apsp["n"] = n_g

@@ -8,8 +8,10 @@
 #include <map>
 #include <mutex>
 #include <numeric>
+#include <set>
 #include <string>
 
+#include "apsp.h"
 #include "errors.h"
 #include "ksg_bits.h"
 #include "ksg_grid.h"
@@ -56,6 +58,7 @@ void release_cached_device_blocks() {
         c.held[dev] = 0;
     }
     cudaSetDevice(cur);
+    apsp_release_pools();
 }
 
 DeviceBuffer::DeviceBuffer(size_t bytes) { reset(bytes); }
@@ -182,18 +185,47 @@ int g_forced_variant = -1;
 int g_forced_staging = -1;
 int g_forced_search = -1;
 int g_forced_orders = -1;
-// Microseconds of a plan on cell grids and on the tiled exhaustive kernels,
-// from the times of 48 plan shapes (16, 40 and 100 nodes, m = 200 to 1500, d =
-// 1 to 3, k = 4, 6 and 20). The grids' kernels take about 110 us before they
-// are busy, then a time per sample that hardly depends on m; the tiled kernels
-// take a time per frame visit, and never less than one thread's walk over m
-// frames. 4950 pairs, d = 3, k = 6: at m = 300 1130 us tiled and 1070 on grids,
-// at m = 800 4940 and 2560; 120 pairs at m = 500: 143 and 236.
-double grid_us(int k, double samples) { return 110 + (k <= 12 ? 0.62e-3 : 0.95e-3) * samples; }
-double tiled_us(int d, int k, int max_m, double work) {
-    const double visit = (d == 1 ? 0.65e-6 : d == 2 ? 1.02e-6 : 1.17e-6) * (k <= 6 ? 1 : k <= 14 ? 2 : 3.5);
-    return 20 + std::max(0.1 * max_m, visit * work);
+// Microseconds of a plan on each route, from the times of 452 plan shapes
+// (lists of 5 to 55 nodes, chains and stars of up to 1000 pairs, m = 500 to
+// 5000, d = 1 to 3, k = 1, 6 and 20): the route they choose takes 0.7% more
+// than the fastest on average, 12% or more on one shape in twenty-five.
+struct PlanSize {
+    int d, k, max_m;
+    double samples, work;  // sums of m and of m^2 over the pairs
+    double rows;           // sum of m over the distinct rows, counted up to kRowsMost
+};
+constexpr double kRowsMost = 4e4;
+
+// One thread's walk over m frames, list updates, frame visits.
+double tiled_us(const PlanSize& p) {
+    const int k = p.k, few = std::min(k, 6) - 1, more = std::max(k - 6, 0);
+    return 19.2 + 0.8 * std::min(k, 20) + p.max_m * (0.02 + 0.015 * p.d + 0.002 * std::min(k, 20)) +
+           1e-3 * p.samples * (0.13 + 0.055 * few + 0.104 * more) +
+           1e-6 * p.work * (0.14 + 0.21 * p.d + 0.025 * few + 0.107 * more);
 }
+// A warp per query: 10 pairs at m = 500, d = 3: 29 us against 65 tiled; 153
+// pairs: 155 against 109.
+double warp_us(const PlanSize& p) {
+    return 19 + 1e-3 * p.samples * (0.34 + 0.033 * (p.k - 1)) + 1e-6 * p.work * (0.52 + 0.66 * p.d + 0.01 * (p.k - 1));
+}
+// The bitmap search hardly depends on m, the scan of cells visits fewer frames
+// the lower d and k are. 703 pairs at m = 1000: d = 1, k = 6 482 us scanned and
+// 633 on bitmaps; d = 3, k = 6 654 and 708; d = 3, k = 20 1976 and 1087.
+double bits_us(const PlanSize& p) {
+    const bool one = p.k <= 12;
+    return 1.1 * (45 + 9 * p.d + 1e-3 * p.samples * (one ? 0.41 : 0.78) +
+                  p.rows * (one ? 0.0045 + 0.0003 * p.d : 0.0075) + (p.d == 3 && !one ? 0.06e-6 * p.work : 0.0));
+}
+double scan_us(const PlanSize& p) {
+    const int few = std::min(p.k, 6) - 1, more = std::max(p.k - 6, 0);
+    const double visit[3] = {0.013e-6, 0.059e-6, 0.132e-6};
+    return 62 + 9 * p.d + 0.9 * std::min(p.k, 20) + 1e-3 * p.samples * (0.23 + 0.01 * few + 0.067 * more) +
+           p.work * visit[p.d - 1] * (1 + 0.13 * few + 0.25 * more) +
+           p.rows * (0.0004 + 0.0007 * p.d + 0.0004 * few + 0.0003 * more);
+}
+// Fewer samples than this leave most of the scan's warps idle (32 queries
+// each), while the bitmap search splits a pair over CTAs.
+constexpr double kScanMinSamples = 3e4;
 // per batch: work-queue heads (two for the grid search), tie count,
 // tie-kernel counter, rank-count queue head, bitmap-search queue heads
 constexpr int kCounters = 5 + kBitSegments;
@@ -388,12 +420,23 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     if (search == 1 && !grid_ok) {
         fail(NSG_ERR_UNSUPPORTED, "cell-grid search: copies of the frame-mapped rows exceed 8 GiB");
     }
-    // automatic: whichever is estimated faster, unless the plan is small
-    // enough for a warp per query
-    const bool warp_ok = !tile_forced && !opt.autotune && ksg_warp_fits(d, k, maxm, work);
+    // the route with the smallest estimate
+    PlanSize size{d, k, maxm, static_cast<double>(total_samples), work, 0};
+    {
+        std::set<std::pair<const float*, const int*>> rows;
+        const size_t most = std::min<size_t>(pairs_in.size(), 4096);
+        for (size_t p = 0; p < most && size.rows < kRowsMost; ++p) {
+            for (const float* x : {pairs_in[p].xa, pairs_in[p].xb}) {
+                if (rows.emplace(x, pairs_in[p].fmap).second) size.rows += pairs_in[p].m;
+            }
+        }
+        size.rows = std::min(size.rows, kRowsMost);
+    }
+    const bool warp_ok = !tile_forced && !opt.autotune && ksg_warp_fits(d, k, maxm) && warp_us(size) < tiled_us(size);
+    scan_ = size.samples >= kScanMinSamples && scan_us(size) < bits_us(size);
     if (search < 0) {
-        search = grid_ok && !warp_ok &&
-                 grid_us(k, static_cast<double>(total_samples)) < tiled_us(d, k, maxm, work) ? 1 : 0;
+        const double exhaustive = warp_ok ? warp_us(size) : tiled_us(size);
+        search = grid_ok && (scan_ ? scan_us(size) : bits_us(size)) < exhaustive ? 1 : 0;
     }
     search_ = search == 1 ? 1 : 0;
     warp_ = !search_ && warp_ok;
@@ -683,7 +726,7 @@ struct KsgPlan::GridState {
     DeviceBuffer gps, pair_arena;         // GridPair per plan pair; pair grids of one batch
     std::vector<int> batch_maxm;          // largest m of each batch
     std::vector<char> batch_order;        // whether each batch builds query orders
-    bool split_nodes = false;             // an ordered batch: many nodes, four kernels
+    bool split_nodes = false;             // many nodes (grid_split_pays) or an ordered batch: four kernels
     bool node_est = false;                // a batch needs the nodes' scale estimates
     std::vector<std::vector<BitsSegment>> batch_bits;  // bitmap search; empty: the scan on pair grids
     int max_m = 0;
@@ -737,6 +780,7 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs, Upload& up) {
         gps[p].b = node_id(descs[p].xb, descs[p].m, descs[p].ld);
     }
     g->nnodes = static_cast<int>(nodes.size());
+    g->split_nodes = grid_split_pays(g->nnodes, sm_count());
     g->node_arena.reset(std::max<size_t>(arena, 16));
     unsigned char* base = g->node_arena.as<unsigned char>();
     for (size_t i = 0; i < nodes.size(); ++i) {
@@ -757,7 +801,8 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs, Upload& up) {
             wpre.push_back(acc);
             acc += (descs[p].m + 31) / 32;
         }
-        g->batch_bits.push_back(bits_segments(descs.data() + b.pair0, b.npairs, d_, k_));
+        g->batch_bits.push_back(scan_ ? std::vector<BitsSegment>{}
+                                      : bits_segments(descs.data() + b.pair0, b.npairs, d_, k_));
         const bool bits = !g->batch_bits.back().empty();
         for (int p = b.pair0; p < b.pair0 + b.npairs && !bits; ++p) off = grid_pair_place(gps[p], off, descs[p].m, d_);
         wpre.push_back(acc);
@@ -781,8 +826,7 @@ void KsgPlan::setup_grid(const std::vector<KsgPairDesc>& descs, Upload& up) {
         for (size_t bi = 0; bi < batches_.size(); ++bi) {
             const Batch& b = batches_[bi];
             const bool order = g->batch_order[bi] != 0;
-            const CountWork w = count_work(gps.data() + b.pair0, descs.data() + b.pair0, b.npairs,
-                                           order ? kRankMinVars : 1);
+            const CountWork w = count_work(gps.data() + b.pair0, descs.data() + b.pair0, b.npairs, order);
             g->group_off.push_back(static_cast<long long>(groups.size()));
             g->gprefix_off.push_back(static_cast<long long>(gpre.size()));
             g->rank_off.push_back(static_cast<long long>(ranks.size()));

@@ -56,7 +56,8 @@ private:
     int device_ = -1;
 };
 
-// Return every cached block to the driver (all devices).
+// Return every cached block and the kept shortest-path workspace to the driver
+// (all devices).
 void release_cached_device_blocks();
 
 struct KsgOutputs {
@@ -148,6 +149,7 @@ private:
     long long tie_stride_ = 0;
     int search_ = 0;
     bool warp_ = false;                  // exhaustive, a warp per query
+    bool scan_ = false;                  // cell grids: the scan of pair grids instead of bitmaps
     int max_m_ = 0;
     long long samples_ = 0;              // of all pairs
     bool bootstrap_ = false;             // frame-mapped rows copied for the grid search

@@ -648,7 +648,7 @@ void launch_pass1(const GridArgs& a, int kmax, int grid, cudaStream_t st) {
 
 }  // namespace
 
-CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, int min_rank) {
+CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, bool ordered) {
     CountWork w;
     // variables by node, in first-appearance order within a node
     std::vector<std::pair<int, int>> keyed(2 * static_cast<size_t>(npairs));
@@ -658,12 +658,18 @@ CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, 
     }
     std::stable_sort(keyed.begin(), keyed.end(),
                      [](const std::pair<int, int>& x, const std::pair<int, int>& y) { return x.first < y.first; });
+    long long rows = 0;  // queries: samples of the distinct nodes
+    for (size_t s = 0; s < keyed.size(); ++s) {
+        if (s == 0 || keyed[s].first != keyed[s - 1].first) rows += descs[keyed[s].second >> 1].m;
+    }
+    const bool few = !ordered && rows <= kRankFewRows;
     int gitems = 0, ritems = 0;
     for (size_t s = 0; s < keyed.size();) {
         size_t e = s;
         while (e < keyed.size() && keyed[e].first == keyed[s].first) ++e;
         const int node = keyed[s].first, m = descs[keyed[s].second >> 1].m;
-        if (static_cast<int>(e - s) >= min_rank) {
+        const int vars = static_cast<int>(e - s);
+        if (ordered ? vars >= kRankMinVars : few && vars <= kRankDirect) {
             w.ranks.push_back({node, static_cast<int>(w.refs.size()), static_cast<int>(e - s), m});
             w.rprefix.push_back(ritems);
             ritems += (m + kRankBlock - 1) / kRankBlock;
@@ -723,6 +729,8 @@ void grid_launch_nodes(GridNode* nodes, int nnodes, int d, bool split, cudaStrea
         default: invalid("d must be 1, 2 or 3");
     }
 }
+
+bool grid_split_pays(int nnodes, int sms) { return nnodes * kNodeCtas >= sms; }
 
 bool grid_orders_pay(long long search_warps, int sms) {
     return search_warps >= static_cast<long long>(kOrderMinWaves) * 32 * sms;

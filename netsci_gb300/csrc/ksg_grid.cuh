@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, (KMAX <= 8 ? 4 : 1)) ksg_grid
         const GridNode na = A.nodes[gp.a];
         const GridNode nb = A.nodes[gp.b];
         const int m = P->m, G = na.G;
+        const bool odd = na.ostart[63] || nb.ostart[63];  // coordinates that are not finite lie in no cell of theirs
         const long long st = m;
         const int qi = blk * 32 + lane;  // query rank in the pair's search order
         const bool valid = qi < m;
@@ -442,19 +443,24 @@ __global__ void __launch_bounds__(32 * kGridWarps, (KMAX <= 8 ? 4 : 1)) ksg_grid
                     else phase = 2;
                 }
                 if (phase == 2) {
-                    const bool more_up = up < G && __any_sync(0xffffffffu, valid &&
-                        __fsub_rn(edge_at(na.e1, up - 1, G), qa1) <= u);
-                    const bool more_dn = dn >= 0 && __any_sync(0xffffffffu, valid &&
-                        __fsub_rn(qa1, edge_at(na.e1, dn, G)) <= u);
+                    const bool more_up = up < G && __any_sync(0xffffffffu, odd || (valid &&
+                        __fsub_rn(edge_at(na.e1, up - 1, G), qa1) <= u));
+                    const bool more_dn = dn >= 0 && __any_sync(0xffffffffu, odd || (valid &&
+                        __fsub_rn(qa1, edge_at(na.e1, dn, G)) <= u));
                     if (!more_up && !more_dn) break;
                     if (more_up && (prefer_up || !more_dn)) row = up++;
                     else row = dn--;
                     prefer_up = !prefer_up;
                 }
-                const bool reach = valid && bin_reaches(na.e1, row, G, qa1, u);
+                const bool reach = valid && (odd || bin_reaches(na.e1, row, G, qa1, u));
                 if (!__any_sync(0xffffffffu, reach)) continue;
                 int clo = G, chi = -1;
-                if (reach) bin_range(nb.e1, G, qb1, u, clo, chi);
+                if (odd) {
+                    clo = 0;
+                    chi = G - 1;
+                } else if (reach) {
+                    bin_range(nb.e1, G, qb1, u, clo, chi);
+                }
                 clo = __reduce_min_sync(0xffffffffu, clo);
                 chi = __reduce_max_sync(0xffffffffu, chi);
                 if (clo > chi) continue;
@@ -540,7 +546,10 @@ __global__ void __launch_bounds__(32 * kGridWarps, (KMAX <= 8 ? 4 : 1)) ksg_grid
                 // sample: every tied lane takes the range of both marginals
                 // over the frames at exactly wk.
                 int qrlo = G, qrhi = -1, qclo = G, qchi = -1;
-                if (tie) {
+                if (odd) {
+                    qrlo = qclo = 0;
+                    qrhi = qchi = G - 1;
+                } else if (tie) {
                     bin_range(na.e1, G, qa1, wk, qrlo, qrhi);
                     bin_range(nb.e1, G, qb1, wk, qclo, qchi);
                 }
@@ -703,7 +712,6 @@ __global__ void __launch_bounds__(32 * kGridWarps, 4) ksg_grid_count_kernel(Grid
 // consecutive frames, whose eps share sectors.
 constexpr int kRankVars = 256;
 constexpr int kRankBuckets = 512;
-constexpr int kRankDirect = 4;
 
 template <int D>
 __global__ void __launch_bounds__(32 * kRankWarps, 40 / kRankWarps) ksg_grid_rank_kernel(GridArgs A) {

@@ -165,6 +165,10 @@ constexpr int kOrderMaxM = 40960;
 // m = 10000 took 1.4 ms per call with them against 0.95 ms without.
 constexpr int kOrderMinWaves = 8;
 bool grid_orders_pay(long long search_warps, int sms);
+// Whether the node grids take four kernels of small CTAs: from about a wave of
+// node clusters on (a chain of 300 pairs at m = 1000: plan 590 -> 500 us; 26
+// nodes: 1% slower).
+bool grid_split_pays(int nnodes, int sms);
 
 // A frame-mapped row copied out for the cell-grid search:
 // out[c*ld_out + s] = x[c*ld + fmap[s]] for s < m, +inf up to ld_out.
@@ -176,12 +180,19 @@ struct GatherRow {
 };
 
 // The counts of npairs pairs (node indices in gps, scratch offsets and m in
-// descs): nodes with at least min_rank variables become rank nodes.
-CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, int min_rank);
-// Variables from which a node's counts are cheaper by rank: a query's ranks
-// cost about as much as six groups' distances whatever their number. Batches
-// that build no orders are latency-bound and rank every node: a warp per query.
+// descs); ordered: the batch builds query orders.
+CountWork count_work(const GridPair* gps, const KsgPairDesc* descs, int npairs, bool ordered);
+// Variables from which a node's counts are cheaper by rank in an ordered
+// batch: a query's ranks cost about as much as six groups' distances whatever
+// their number.
 constexpr int kRankMinVars = 8;
+// Batches that build no orders count in groups (18 nodes at m = 4000 894 us
+// against 950 by rank, a chain of 300 pairs at m = 1000 588 against 906),
+// except the smallest, whose groups would leave the GPU idle: up to this many
+// queries a warp serves each, and compares the few variables of its node one
+// by one.
+constexpr long long kRankFewRows = 20000;
+constexpr int kRankDirect = 4;
 
 // Cells per axis for m samples (about ten frames per cell, at most kGridMaxG).
 int grid_cells_per_axis(int m);

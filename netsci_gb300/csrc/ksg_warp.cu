@@ -12,7 +12,7 @@
 //     k nearest selected as in the bitmap search, ties included;
 //   * the marginal counts are warp sums over all frames.
 // Per query and frame that is two to three times the tiled kernels' work, so
-// it serves small plans (ksg_warp_fits), where the GPU is mostly idle
+// it serves small plans (warp_us in engine.cpp), where the GPU is mostly idle
 // otherwise.
 #include "common.cuh"
 #include "ksg_bits.cuh"
@@ -197,10 +197,8 @@ size_t smem_bytes(int d, int max_m) {
 
 }  // namespace
 
-bool ksg_warp_fits(int d, int k, int max_m, double work) {
-    const double us = (0.8 + 0.7 * d) * work * 1e-6;
-    // the bound comes from 32 lane minima
-    return k <= 30 && us <= 120 && smem_bytes(d, max_m) <= kMaxSmem;
+bool ksg_warp_fits(int d, int k, int max_m) {
+    return k <= 30 && smem_bytes(d, max_m) <= kMaxSmem;  // the bound comes from 32 lane minima
 }
 
 void ksg_launch_warp(const KsgCountArgs& a, int d, int max_m, cudaStream_t st) {

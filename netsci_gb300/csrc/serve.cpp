@@ -428,7 +428,7 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     NSG_CUDA(cudaMemcpyAsync(d_wpre_.get(), h_wpre_, sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
     // count groups and rank nodes: variables of the tick on the same node
     const bool order = grid_orders_pay(wacc, sm_count());  // query orders for this tick
-    const CountWork work_list = count_work(h_gpairs_, h_pairs_, static_cast<int>(np), order ? kRankMinVars : 1);
+    const CountWork work_list = count_work(h_gpairs_, h_pairs_, static_cast<int>(np), order);
     const auto& groups = work_list.groups;
     if (order) ensure(d_corder_, sizeof(int) * std::max<size_t>(1, groups.size() * static_cast<size_t>(maxm)));
     auto put = [&](DeviceBuffer& b, const auto& v) {

@@ -90,10 +90,11 @@ def test_not_finite_matches_exhaustive(d, m, form):
     _same_pairs(x, m, 6, d, [(0, b) for b in range(1, 10)] + [(2, 5), (3, 4)])
 
 
-def _same_pairs(x, m, k, d, ab):
+def _same_pairs(x, m, k, d, ab, fmap=None):
     from netsci_gb300 import device
     X, _ = device.pack_trajectory(x, d)
-    pairs = device.make_pairs(X, m, ab)
+    f = None if fmap is None else torch.from_numpy(fmap).cuda()
+    pairs = device.make_pairs(X, m, ab, fmap=f, m_samples=m)
 
     def run():
         mi = torch.empty(len(pairs), device="cuda")
@@ -106,12 +107,37 @@ def _same_pairs(x, m, k, d, ab):
 
 @pytest.mark.parametrize("d", [1, 2, 3])
 @pytest.mark.parametrize("partners", [1, 2, 3, 4, 5, 6, 7, 8, 9, 13, 32, 33, 255, 256, 257, 261])
-def test_counts_of_a_star_match_exhaustive(d, partners):
-    """One node in `partners` pairs: groups up to seven, ranks from eight on,
-    in passes of 256 whose last one may hold one to four variables."""
+@pytest.mark.parametrize("orders", [0, 1])
+def test_counts_of_a_star_match_exhaustive(d, partners, orders):
+    """One node in `partners` pairs: groups up to seven; with query orders
+    ranks from eight on, in passes of 256 whose last one may hold one to four
+    variables; without, direct comparisons of up to four in small batches."""
+    from netsci_gb300 import device
     m = 1025
-    _same_pairs(_walk(partners + 1, d, m, partners, 0.03125 if partners % 2 else 0.0), m, 4, d,
-                [(0, b) if b % 3 else (b, 0) for b in range(1, partners + 1)])
+    try:
+        device.set_ksg_orders(orders)
+        _same_pairs(_walk(partners + 1, d, m, partners, 0.03125 if partners % 2 else 0.0), m, 4, d,
+                    [(0, b) if b % 3 else (b, 0) for b in range(1, partners + 1)])
+    finally:
+        device.set_ksg_orders(-1)
+
+
+@pytest.mark.parametrize("d,k,m,nodes", [(1, 1, 500, 12), (1, 6, 4001, 9), (1, 9, 1000, 40), (1, 20, 1000, 40),
+                                         (2, 1, 2200, 18), (2, 6, 700, 18), (2, 6, 2200, 18), (3, 1, 1400, 18),
+                                         (3, 6, 700, 38), (3, 6, 1025, 39), (3, 30, 500, 20)])
+@pytest.mark.parametrize("step", [0.0, 0.25])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_lists_on_either_side_of_the_scan(d, k, m, nodes, step, mapped):
+    """All pairs of a few nodes, where the estimates choose between the scan of
+    cells and the bitmaps; also resampled (copies of frames)."""
+    fmap = np.random.default_rng(m).integers(0, m, m).astype(np.int32) if mapped else None
+    _same_pairs(_walk(nodes, d, m, nodes + m, step), m, k, d,
+                [(a, b) for a in range(nodes) for b in range(a + 1, nodes)], fmap)
+
+
+def test_chain_of_many_nodes():
+    """More than a wave of nodes with two variables each."""
+    _same_pairs(_walk(200, 3, 601, 9), 601, 6, 3, [(a, a + 1) for a in range(199)])
 
 
 @pytest.mark.parametrize("m", [3399, 3400, 3401])

@@ -8,7 +8,6 @@
 #include <map>
 #include <mutex>
 #include <numeric>
-#include <set>
 #include <string>
 
 #include "apsp.h"
@@ -185,20 +184,27 @@ int g_forced_variant = -1;
 int g_forced_staging = -1;
 int g_forced_search = -1;
 int g_forced_orders = -1;
-// Microseconds of a plan on each route, from the times of 452 plan shapes
+// Microseconds of a plan on each route, from the times of 632 plan shapes
 // (lists of 5 to 55 nodes, chains and stars of up to 1000 pairs, m = 500 to
-// 5000, d = 1 to 3, k = 1, 6 and 20): the route they choose takes 0.7% more
-// than the fastest on average, 12% or more on one shape in twenty-five.
+// 5000, d = 1 to 3, k = 1 to 30): the route they choose takes 1.2% more than
+// the fastest on average, a quarter more at worst.
 struct PlanSize {
     int d, k, max_m;
     double samples, work;  // sums of m and of m^2 over the pairs
     double rows;           // sum of m over the distinct rows, counted up to kRowsMost
+    double pairs;
 };
 constexpr double kRowsMost = 4e4;
 
+// Neighbour lists beyond six entries: their cost follows the list's length in
+// registers (14, 30, 62 entries) more than k.
+double long_list(int k) {
+    return k <= 6 ? 0 : k <= 14 ? 3.5 + 0.32 * (k - 10) : k <= 30 ? 14 + 0.25 * (k - 20) : 35 + 0.3 * (k - 31);
+}
 // One thread's walk over m frames, list updates, frame visits.
 double tiled_us(const PlanSize& p) {
-    const int k = p.k, few = std::min(k, 6) - 1, more = std::max(k - 6, 0);
+    const int k = p.k, few = std::min(k, 6) - 1;
+    const double more = long_list(k);
     return 19.2 + 0.8 * std::min(k, 20) + p.max_m * (0.02 + 0.015 * p.d + 0.002 * std::min(k, 20)) +
            1e-3 * p.samples * (0.13 + 0.055 * few + 0.104 * more) +
            1e-6 * p.work * (0.14 + 0.21 * p.d + 0.025 * few + 0.107 * more);
@@ -209,15 +215,16 @@ double warp_us(const PlanSize& p) {
     return 19 + 1e-3 * p.samples * (0.34 + 0.033 * (p.k - 1)) + 1e-6 * p.work * (0.52 + 0.66 * p.d + 0.01 * (p.k - 1));
 }
 // The bitmap search hardly depends on m, the scan of cells visits fewer frames
-// the lower d and k are. 703 pairs at m = 1000: d = 1, k = 6 482 us scanned and
-// 633 on bitmaps; d = 3, k = 6 654 and 708; d = 3, k = 20 1976 and 1087.
+// the lower d and k are. 703 pairs at m = 1000: d = 1, k = 6 401 us scanned and
+// 529 on bitmaps; d = 3, k = 6 656 and 708; d = 3, k = 20 2002 and 1098.
 double bits_us(const PlanSize& p) {
     const bool one = p.k <= 12;
     return 1.1 * (45 + 9 * p.d + 1e-3 * p.samples * (one ? 0.41 : 0.78) +
                   p.rows * (one ? 0.0045 + 0.0003 * p.d : 0.0075) + (p.d == 3 && !one ? 0.06e-6 * p.work : 0.0));
 }
 double scan_us(const PlanSize& p) {
-    const int few = std::min(p.k, 6) - 1, more = std::max(p.k - 6, 0);
+    const int few = std::min(p.k, 6) - 1;
+    const double more = long_list(p.k);
     const double visit[3] = {0.013e-6, 0.059e-6, 0.132e-6};
     return 62 + 9 * p.d + 0.9 * std::min(p.k, 20) + 1e-3 * p.samples * (0.23 + 0.01 * few + 0.067 * more) +
            p.work * visit[p.d - 1] * (1 + 0.13 * few + 0.25 * more) +
@@ -226,6 +233,9 @@ double scan_us(const PlanSize& p) {
 // Fewer samples than this leave most of the scan's warps idle (32 queries
 // each), while the bitmap search splits a pair over CTAs.
 constexpr double kScanMinSamples = 3e4;
+// What a pair's node and count work lists cost when a plan on grids is built
+// (1770 pairs: 493 us against 402).
+constexpr double kGridPairUs = 0.05;
 // per batch: work-queue heads (two for the grid search), tie count,
 // tie-kernel counter, rank-count queue head, bitmap-search queue heads
 constexpr int kCounters = 5 + kBitSegments;
@@ -421,14 +431,20 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
         fail(NSG_ERR_UNSUPPORTED, "cell-grid search: copies of the frame-mapped rows exceed 8 GiB");
     }
     // the route with the smallest estimate
-    PlanSize size{d, k, maxm, static_cast<double>(total_samples), work, 0};
+    PlanSize size{d, k, maxm, static_cast<double>(total_samples), work, 0, static_cast<double>(npairs)};
     {
-        std::set<std::pair<const float*, const int*>> rows;
-        const size_t most = std::min<size_t>(pairs_in.size(), 4096);
-        for (size_t p = 0; p < most && size.rows < kRowsMost; ++p) {
+        // the first pairs tell: a list of all pairs of N nodes names them in
+        // its first N - 1, and other lists reach kRowsMost soon
+        std::vector<std::pair<std::pair<const float*, const int*>, int>> rows;
+        const size_t most = std::min<size_t>(pairs_in.size(), 128);
+        for (size_t p = 0; p < most; ++p) {
             for (const float* x : {pairs_in[p].xa, pairs_in[p].xb}) {
-                if (rows.emplace(x, pairs_in[p].fmap).second) size.rows += pairs_in[p].m;
+                rows.push_back({{x, pairs_in[p].fmap}, pairs_in[p].m});
             }
+        }
+        std::sort(rows.begin(), rows.end());
+        for (size_t r = 0; r < rows.size(); ++r) {
+            if (r == 0 || rows[r].first != rows[r - 1].first) size.rows += rows[r].second;
         }
         size.rows = std::min(size.rows, kRowsMost);
     }
@@ -436,7 +452,8 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     scan_ = size.samples >= kScanMinSamples && scan_us(size) < bits_us(size);
     if (search < 0) {
         const double exhaustive = warp_ok ? warp_us(size) : tiled_us(size);
-        search = grid_ok && (scan_ ? scan_us(size) : bits_us(size)) < exhaustive ? 1 : 0;
+        const double grids = (scan_ ? scan_us(size) : bits_us(size)) + kGridPairUs * size.pairs;
+        search = grid_ok && grids < exhaustive ? 1 : 0;
     }
     search_ = search == 1 ? 1 : 0;
     warp_ = !search_ && warp_ok;

@@ -381,7 +381,7 @@ std::atomic<int> g_method{-1};
 // N = 2000), and what a step of a small matrix takes anyway.
 double dense_step_seconds(int n) {
     const double P = (n + kPad - 1) / kPad * kPad;
-    return 4e-6 + P * P * P / 16e12;
+    return 6e-6 + P * P * P / 16e12;
 }
 
 // A and how a solve of it runs.

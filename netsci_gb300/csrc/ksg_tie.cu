@@ -514,10 +514,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kCtasPerSm) ksg_tie_kernel(
 }
 
 // A CTA per sample, rows in shared memory. Few samples tie and a replay is a
-// chain of partitions, so its latency counts: a warp per sample that finds 32
-// stoppers a round takes 45 us at m = 1000 (rows in shared memory) and over a
-// millisecond at m = 10000 (rows in global memory), a CTA 12 and 35 us. Ties
-// of a 56-node list at m = 1000 49 -> 25 us, of 101 nodes 156 -> 43 us, of
+// chain of partitions, so its latency counts. From a warp per sample that
+// finds 32 stoppers a round (rows in shared memory up to m = 3400): ties of a
+// 56-node list at m = 1000 49 -> 25 us, of 101 nodes 156 -> 43 us, of
 // 8,192 pairs at m = 10000 (8,559 samples) 3.19 -> 1.21 ms, of two resamples
 // of 100 nodes 2.70 -> 0.33 ms.
 template <int D>

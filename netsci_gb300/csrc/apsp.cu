@@ -353,6 +353,12 @@ struct DevMem {
         NSG_CUDA(cudaMallocFromPoolAsync(&p, bytes, workspace_pool(), st));
     }
     ~DevMem() { if (p) cudaFreeAsync(p, s); }
+    // For what a kernel is about to write or read: a block that was not
+    // allocated ends the solve with an error.
+    float* floats() const {
+        if (!p) fail(NSG_ERR_CUDA, "shortest paths: a workspace block is not there");
+        return static_cast<float*>(p);
+    }
     DevMem(const DevMem&) = delete;
     DevMem& operator=(const DevMem&) = delete;
 };
@@ -388,7 +394,7 @@ double dense_step_seconds(int n) {
 struct Graph {
     int squaring = 0;  // repeated squaring reaches the result: 1 exactly, 2 within rounding (requested)
     bool symmetric = false;
-    bool sparse = false;
+    bool sparse = false;  // steps over the finite entries; rounded squaring takes dense products alone
     long long width = 0;
     DevMem words, edges;  // GraphInfo, counts, slice offsets, order, rank; the entries
     SellView rows{};
@@ -419,7 +425,7 @@ struct Graph {
             if (!(h.flags & 8) && static_cast<double>(wmax) * (n - 1) < 16777216.0) squaring = 1;
             else if (method == 1) squaring = 2;  // squaring requested on any weights
         }
-        sparse = n <= kSparseMaxN && sparse_step_seconds(width, n) < dense_step_seconds(n);
+        sparse = squaring != 2 && n <= kSparseMaxN && sparse_step_seconds(width, n) < dense_step_seconds(n);
         if (!sparse) return;
         edges.alloc(sizeof(int2) * kSellRows * (size_t)std::max<long long>(1, width), s);
         if (sparse_sort_pays(width, h.entries, n, steps)) {  // shorter slices, so the entries fit
@@ -510,21 +516,21 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         return 0;
     }
     const Graph g(A, n, max_path_length >= n - 1, max_path_length, s);
-    const bool sparse = g.sparse && g.squaring != 2;
+    const bool sparse = g.sparse;
     DevMem T(sparse ? nn * sizeof(float) : 0, s);
     DevMem copy(sparse && !g.order && overlap(A, H, nn) ? nn * sizeof(float) : 0, s);
     const float* from = A;
     if (g.order) {  // the steps start from the relabelled matrix in T
-        sparse_relabel(A, static_cast<float*>(T.p), n, g.order, s);
+        sparse_relabel(A, T.floats(), n, g.order, s);
         from = nullptr;
     } else if (copy.p) {
         NSG_CUDA(cudaMemcpyAsync(copy.p, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
-        from = static_cast<const float*>(copy.p);
+        from = copy.floats();
     }
     auto deliver = [&](float* at) {  // into H, in the matrix's own labels
         if (g.order) {
             if (at == H) {
-                at = static_cast<float*>(T.p);
+                at = T.floats();
                 NSG_CUDA(cudaMemcpyAsync(at, H, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
             }
             sparse_restore(at, H, n, g.order, g.rank, s);
@@ -547,7 +553,7 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
             const int most = ceil_log2(n);
             while (first < most && ((2 << first) - 1) * step <= (first + 1) * product) ++first;
             if (first > 0) {
-                const int h = sparse_steps(g, from, H, static_cast<float*>(T.p), n, (1 << first) - 1, s, &launched,
+                const int h = sparse_steps(g, from, H, T.floats(), n, (1 << first) - 1, s, &launched,
                                            &converged, &at);
                 deliver(at);
                 if (converged) {
@@ -581,7 +587,7 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         return first + q + 1;
     }
     if (sparse) {
-        const int steps = sparse_steps(g, from, H, static_cast<float*>(T.p), n, max_path_length, s, &launched,
+        const int steps = sparse_steps(g, from, H, T.floats(), n, max_path_length, s, &launched,
                                        &converged, &at);
         deliver(at);
         NSG_CUDA(cudaStreamSynchronize(s));

@@ -9,7 +9,9 @@
 //     smallest of the 32 minima bounds the k-th neighbour's (the query itself
 //     is one frame, at distance 0), and few other frames pass that bound;
 //   * the frames within it are listed with their marginal distances and the
-//     k nearest selected as in the bitmap search, ties included;
+//     k nearest selected as in the bitmap search, ties included; samples with
+//     too many ties, fewer than k finite distances or a neighbour whose
+//     marginal is not a number count their distances up instead;
 //   * the marginal counts are warp sums over all frames.
 // Per query and frame that is two to three times the tiled kernels' work, so
 // it serves small plans (warp_us in engine.cpp), where the GPU is mostly idle
@@ -73,13 +75,17 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) ksg_warp_kernel(KsgCountArg
         }
         float h = __uint_as_float(kth_lane(__float_as_uint(least), k));
         int inside = 0;
-        bool stuck = false;
-        for (int j = lane; j < mp; j += 32) {
+        bool stuck = !(h < inf_f());
+        for (int j = lane; j < mp && !stuck; j += 32) {
             float da, db;
             distances(j, da, db);
             const float v = fmaxf(da, db);
             unsigned in = __ballot_sync(kFull, v <= h);
             if (!in) continue;
+            if (__any_sync(kFull, v <= h && (da != da || db != db))) {  // the other marginal stands for both
+                stuck = true;
+                break;
+            }
             if (inside + __popc(in) > kList) {
                 if (inside > k) inside = keep_nearest<kList / 32>(s_v, s_da, s_db, inside, k, lane, &h);
                 in = __ballot_sync(kFull, v <= h);
@@ -104,8 +110,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) ksg_warp_kernel(KsgCountArg
             r = select_nearest<kList / 32>(s_v, s_da, s_db, inside, k, lane);
             __syncwarp();
         } else {
-            // every frame at or below the bound, without the list: the
-            // (k+1)-th smallest by counting up distinct distances
+            // without the list: the (k+1)-th smallest by counting up distinct distances
             float U = -1.f;
             int le = 0;
             while (le <= k) {
@@ -126,14 +131,19 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) ksg_warp_kernel(KsgCountArg
                 le = __reduce_add_sync(kFull, le);
                 if (U == inf_f()) break;
             }
+            // As the tiled kernels have it: a marginal that is not a number
+            // adds nothing to eps but differs from every other one at U, and
+            // with fewer than k finite distances the frames at +inf are no
+            // neighbours yet: any of them makes the sample a tie.
+            const bool few = U == inf_f();
             unsigned ea = 0, eb = 0, alo = kFull, ahi = 0, blo = kFull, bhi = 0;
             for (int j = lane; j < mp; j += 32) {
                 float da, db;
                 distances(j, da, db);
                 const float v = fmaxf(da, db);
-                if (v <= U) {
-                    ea = max(ea, __float_as_uint(da));
-                    eb = max(eb, __float_as_uint(db));
+                if (few ? v < U : v <= U) {
+                    ea = max(ea, __float_as_uint(fmaxf(da, 0.f)));
+                    eb = max(eb, __float_as_uint(fmaxf(db, 0.f)));
                 }
                 if (v == U) {
                     alo = min(alo, __float_as_uint(da));
@@ -149,7 +159,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) ksg_warp_kernel(KsgCountArg
             ahi = __reduce_max_sync(kFull, ahi);
             blo = __reduce_min_sync(kFull, blo);
             bhi = __reduce_max_sync(kFull, bhi);
-            r.tie = le > k + 1 && U > 0.f && (alo != ahi || blo != bhi);
+            const unsigned inf_bits = __float_as_uint(inf_f());
+            const bool mixed = alo != ahi || blo != bhi || ahi > inf_bits || bhi > inf_bits;
+            r.tie = few ? alo != kFull : le > k + 1 && U > 0.f && mixed;
         }
         float ca = 0.f, cb = 0.f;
 #pragma unroll 4

@@ -196,18 +196,21 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
     // The insertion sort of [0, prefix_end), a few dozen elements, is a stable
     // sort: an element's place is the number of smaller keys plus the equal
     // ones before it. Longer prefixes (heapsorted segments among them) are left
-    // to lane 0.
-    if (prefix_end <= 64) {
-        int v[2] = {0, 0}, place[2] = {0, 0};
-        float kv[2] = {0.f, 0.f};
+    // to lane 0, and so are those with a NaN, which no key is smaller than and
+    // none larger: where it ends up follows from the sort's steps alone.
+    int v[2] = {0, 0};
+    float kv[2] = {0.f, 0.f};
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = 32 * h + lane;
-            if (i < prefix_end) {
-                v[h] = idx[i];
-                kv[h] = key[v[h]];
-            }
+    for (int h = 0; h < 2; ++h) {
+        const int i = 32 * h + lane;
+        if (i < prefix_end) {
+            v[h] = idx[i];
+            kv[h] = key[v[h]];
         }
+    }
+    const bool odd = __any_sync(kFull, kv[0] != kv[0] || kv[1] != kv[1]);
+    if (prefix_end <= 64 && !odd) {
+        int place[2] = {0, 0};
         for (int j = 0; j < prefix_end; ++j) {
             const float kj = __shfl_sync(kFull, j < 32 ? kv[0] : kv[1], j & 31);
 #pragma unroll
@@ -219,14 +222,14 @@ __device__ bool sort_prefix_warp(const float* key, int* idx, int n, int T, SortS
             if (32 * h + lane < prefix_end) idx[place[h]] = v[h];
     } else if (lane == 0) {
         for (int i = 1; i < prefix_end; ++i) {
-            const int v = idx[i];
-            const float kv = key[v];
+            const int moved = idx[i];
+            const float km = key[moved];
             int j = i;
-            while (j > 0 && kv < key[idx[j - 1]]) {
+            while (j > 0 && km < key[idx[j - 1]]) {
                 idx[j] = idx[j - 1];
                 --j;
             }
-            idx[j] = v;
+            idx[j] = moved;
         }
     }
     __syncwarp();
@@ -378,13 +381,18 @@ __device__ bool sort_prefix_cta(const float* key, int* idx, int n, int T, TieSha
     // The insertion sort of [0, prefix_end), a few dozen elements, is a stable
     // sort: an element's place is the number of smaller keys plus the equal
     // ones before it. Longer prefixes (heapsorted segments among them) are left
-    // to thread 0.
+    // to thread 0, and so are those with a NaN (sort_prefix_warp).
     __syncthreads();
-    if (prefix_end <= nthreads) {
-        int v = 0, place = 0;
+    int v = 0;
+    float kv = 0.f;
+    if (tid < prefix_end) {
+        v = idx[tid];
+        kv = key[v];
+    }
+    const bool odd = __syncthreads_or(kv != kv);
+    if (prefix_end <= nthreads && !odd) {
+        int place = 0;
         if (tid < prefix_end) {
-            v = idx[tid];
-            const float kv = key[v];
 #pragma unroll 4
             for (int j = 0; j < prefix_end; ++j) {
                 const float kj = key[idx[j]];
@@ -395,14 +403,14 @@ __device__ bool sort_prefix_cta(const float* key, int* idx, int n, int T, TieSha
         if (tid < prefix_end) idx[place] = v;
     } else if (tid == 0) {
         for (int i = 1; i < prefix_end; ++i) {
-            const int v = idx[i];
-            const float kv = key[v];
+            const int moved = idx[i];
+            const float km = key[moved];
             int j = i;
-            while (j > 0 && kv < key[idx[j - 1]]) {
+            while (j > 0 && km < key[idx[j - 1]]) {
                 idx[j] = idx[j - 1];
                 --j;
             }
-            idx[j] = v;
+            idx[j] = moved;
         }
     }
     __syncthreads();

@@ -327,7 +327,12 @@ __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float
         }
         U = k < 32 ? __shfl_sync(kFull, l0, k) : __shfl_sync(kFull, l1, k - 32);
     }
-    float ea = 0.f, eb = 0.f, alo = inf_f(), ahi = -1.f, blo = inf_f(), bhi = -1.f;
+    // As the tiled kernels have it: a marginal that is not a number adds nothing
+    // to eps but differs from every other one at U, and with fewer than k finite
+    // distances the frames at +inf are no neighbours yet: any of them makes the
+    // sample a tie.
+    const bool few = U == inf_f();
+    unsigned ea = 0, eb = 0, alo = kFull, ahi = 0, blo = kFull, bhi = 0;
     int le = 0;
     for (int j0 = 0; j0 < m; j0 += 32) {
         const int j = j0 + lane;
@@ -336,29 +341,29 @@ __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float
         load_frame<D>(xa, j, a);
         load_frame<D>(xb, j, b);
         const float da = dist<D>(qa, a), db = dist<D>(qb, b), v = fmaxf(da, db);
-        if (v <= U) {
+        if (few ? v < U : v <= U) {
             ++le;
-            ea = fmaxf(ea, da);
-            eb = fmaxf(eb, db);
+            ea = max(ea, __float_as_uint(fmaxf(da, 0.f)));
+            eb = max(eb, __float_as_uint(fmaxf(db, 0.f)));
         }
         if (v == U) {
-            alo = fminf(alo, da);
-            ahi = fmaxf(ahi, da);
-            blo = fminf(blo, db);
-            bhi = fmaxf(bhi, db);
+            alo = min(alo, __float_as_uint(da));
+            ahi = max(ahi, __float_as_uint(da));
+            blo = min(blo, __float_as_uint(db));
+            bhi = max(bhi, __float_as_uint(db));
         }
     }
     le = __reduce_add_sync(kFull, le);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ea = fmaxf(ea, __shfl_xor_sync(kFull, ea, o));
-        eb = fmaxf(eb, __shfl_xor_sync(kFull, eb, o));
-        alo = fminf(alo, __shfl_xor_sync(kFull, alo, o));
-        ahi = fmaxf(ahi, __shfl_xor_sync(kFull, ahi, o));
-        blo = fminf(blo, __shfl_xor_sync(kFull, blo, o));
-        bhi = fmaxf(bhi, __shfl_xor_sync(kFull, bhi, o));
-    }
-    return Found{ea, eb, U, le > k + 1 && U > 0.f && (alo != ahi || blo != bhi)};
+    ea = __reduce_max_sync(kFull, ea);
+    eb = __reduce_max_sync(kFull, eb);
+    alo = __reduce_min_sync(kFull, alo);
+    ahi = __reduce_max_sync(kFull, ahi);
+    blo = __reduce_min_sync(kFull, blo);
+    bhi = __reduce_max_sync(kFull, bhi);
+    const unsigned inf_bits = __float_as_uint(inf_f());
+    const bool mixed = alo != ahi || blo != bhi || ahi > inf_bits || bhi > inf_bits;
+    return Found{__uint_as_float(ea), __uint_as_float(eb), U,
+                 few ? alo != kFull : le > k + 1 && U > 0.f && mixed};
 }
 
 }  // namespace bitk

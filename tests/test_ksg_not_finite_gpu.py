@@ -1,5 +1,6 @@
 """Coordinates that are not numbers, or infinite, in every coordinate of a
-frame: small plans (a warp per query) against the tiled kernels, bit for bit.
+frame: small plans (a warp per query) and the bitmap search, whose queries of
+such nodes scan all frames, against the tiled kernels, bit for bit.
 With one coordinate per node such a frame's marginal distance is itself not a
 number, and the joint distance is the other node's."""
 import numpy as np
@@ -75,7 +76,29 @@ def test_small_plans_match_tiled(d, k, m, step, form):
         m = m // 4 * 4  # whole groups of the tiled kernels' frames
     x = _spoil(_walk(2, d, m, 10 * m + d, step), form)
     X, _ = device.pack_trajectory(x.reshape(2, d * m), d)
-    got = _detail(X, m, k, d)
+    _same_as_tiled(X, m, k, d, -1)
+
+
+@pytest.mark.parametrize("d,k", [(1, 4), (2, 6), (3, 6), (3, 20)])
+@pytest.mark.parametrize("m", [1025, 4301])
+@pytest.mark.parametrize("step", [0.0, 0.25])
+@pytest.mark.parametrize("form", ["one_node", "both_nodes", "inf", "many", "few", "few_inf"])
+def test_bitmap_search_matches_tiled(d, k, m, step, form):
+    from netsci_gb300 import device
+    if form.startswith("few"):
+        m = m // 4 * 4
+    x = _spoil(_walk(2, d, m, 10 * m + d, step), form)
+    X, _ = device.pack_trajectory(x.reshape(2, d * m), d)
+    _same_as_tiled(X, m, k, d, 1)
+
+
+def _same_as_tiled(X, m, k, d, search):
+    from netsci_gb300 import device
+    device.set_ksg_search(search)
+    try:
+        got = _detail(X, m, k, d)
+    finally:
+        device.set_ksg_search(-1)
     device.set_ksg_shape(*_tiled_shape(X, m, k, d))
     try:
         want = _detail(X, m, k, d)

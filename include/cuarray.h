@@ -71,8 +71,16 @@ private:
     void release();
     // Host storage of `count` elements: page-locked (cudaHostAlloc) from
     // kPinnedMinBytes up when a CUDA device is present, so host<->device
-    // copies of large arrays run at the link's speed; else new[].
-    T* alloc_host(size_t count);
+    // copies of large arrays run at the link's speed; else new[]. The array
+    // itself changes only when it takes the storage: an allocation that throws
+    // leaves it as it was.
+    struct Storage {
+        T* p;
+        size_t count;
+        bool pinned;
+    };
+    static Storage alloc_host(size_t count);
+    void hold(const Storage& s);
     void free_host();
     // init() without the zeros, for results that overwrite all of it.
     CuArrayError init_unset(int m, int n);
@@ -80,7 +88,7 @@ private:
     friend void init_result(CuArray<U>* a, int m, int n);
     T* host_;
     T* device_;
-    T* own_ = nullptr;       // the storage alloc_host made last, and its size:
+    T* own_ = nullptr;       // the storage held last, and its size:
     size_t own_count_ = 0;   // init() to the same size keeps it
     T* pinned_ = nullptr;  // host_ came from cudaHostAlloc (freed with cudaFreeHost)
     int n_{};

@@ -29,20 +29,23 @@ constexpr size_t kPinnedMinBytes = size_t(16) << 20;
 }  // namespace
 
 template <typename T>
-T* CuArray<T>::alloc_host(size_t count) {
+typename CuArray<T>::Storage CuArray<T>::alloc_host(size_t count) {
     if (count == 0) count = 1;
-    own_count_ = count;
     const size_t bytes = count * sizeof(T);
     if (bytes >= kPinnedMinBytes) {
         void* p = nullptr;
-        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) {
-            pinned_ = own_ = static_cast<T*>(p);
-            return pinned_;
-        }
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return {static_cast<T*>(p), count, true};
         cudaGetLastError();  // no device: ordinary memory
     }
-    pinned_ = nullptr;
-    return own_ = new T[count];
+    return {new T[count], count, false};
+}
+
+template <typename T>
+void CuArray<T>::hold(const Storage& s) {
+    host_ = own_ = s.p;
+    own_count_ = s.count;
+    pinned_ = s.pinned ? s.p : nullptr;
+    allocatedHost_ = 1;
 }
 
 template <typename T>
@@ -81,13 +84,12 @@ CuArrayError CuArray<T>::init_unset(int m, int n) {
     } else {
         release();
         owner_ = 1;
-        host_ = alloc_host(count);
+        hold(alloc_host(count));
     }
     m_ = m;
     n_ = n;
     size_ = m * n;
     bytes_ = static_cast<size_t>(size_) * sizeof(T);
-    allocatedHost_ = 1;
     return 0;
 }
 
@@ -107,9 +109,8 @@ CuArrayError CuArray<T>::init(T* host, int m, int n) {
     size_ = m * n;
     bytes_ = static_cast<size_t>(size_) * sizeof(T);
     owner_ = 1;
-    host_ = alloc_host(static_cast<size_t>(size_));
+    hold(alloc_host(static_cast<size_t>(size_)));
     if (size_) std::copy(host, host + size_, host_);
-    allocatedHost_ = 1;
     return 0;
 }
 
@@ -135,25 +136,16 @@ CuArrayError CuArray<T>::fromCuArrayDeepCopy(CuArray<T>* src, int start, int end
     if ((end - start + 1) * src->n_ != m * n) return 1;
     // the new storage is filled before this array's own is released (src may
     // be this array)
-    T* const old_pinned = pinned_;
-    pinned_ = nullptr;
-    T* copy = alloc_host(static_cast<size_t>(m) * n);
-    T* const copy_pinned = pinned_;
-    const size_t copy_count = own_count_;
+    const Storage copy = alloc_host(static_cast<size_t>(m) * n);
     std::copy(src->host_ + static_cast<size_t>(start) * src->n_,
-              src->host_ + static_cast<size_t>(end + 1) * src->n_, copy);
-    pinned_ = old_pinned;
+              src->host_ + static_cast<size_t>(end + 1) * src->n_, copy.p);
     release();
-    pinned_ = copy_pinned;
-    own_ = copy;
-    own_count_ = copy_count;
+    hold(copy);
     owner_ = 1;
     m_ = m;
     n_ = n;
     size_ = m * n;
     bytes_ = static_cast<size_t>(size_) * sizeof(T);
-    host_ = copy;
-    allocatedHost_ = 1;
     return 0;
 }
 
@@ -179,8 +171,7 @@ CuArrayError CuArray<T>::allocatedDevice() const { return allocatedDevice_; }
 template <typename T>
 CuArrayError CuArray<T>::allocateHost() {
     if (!allocatedHost_ && owner_) {
-        host_ = alloc_host(static_cast<size_t>(size_));
-        allocatedHost_ = 1;
+        hold(alloc_host(static_cast<size_t>(size_)));
     }
     return allocatedHost_ ? 0 : 1;
 }

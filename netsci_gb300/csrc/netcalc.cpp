@@ -274,6 +274,23 @@ void result_matrix(CuArray<float>* A, CuArray<float>* H, int n) {
     if (H == A) H->init(n, n);
     else init_result(H, n, n);
 }
+
+// A result from init_result holds whatever its storage held: zeros instead,
+// unless the solve gets as far as written().
+template <typename T>
+class ZeroUnlessWritten {
+public:
+    explicit ZeroUnlessWritten(CuArray<T>* a) : a_(a) {}
+    ~ZeroUnlessWritten() {
+        if (a_ && a_->host()) std::fill(a_->host(), a_->host() + a_->size(), T(0));
+    }
+    void written() { a_ = nullptr; }
+    ZeroUnlessWritten(const ZeroUnlessWritten&) = delete;
+    ZeroUnlessWritten& operator=(const ZeroUnlessWritten&) = delete;
+
+private:
+    CuArray<T>* a_;
+};
 }  // namespace
 
 void hedetniemiAllShortestPaths(CuArray<float>* A, CuArray<float>* H, CuArray<int>* paths,
@@ -295,7 +312,9 @@ void hedetniemiAllShortestPathsGpu(CuArray<float>* A, CuArray<float>* H, CuArray
     const int n = A->n();
     const size_t nn = static_cast<size_t>(n) * n;
     result_matrix(A, H, n);
+    ZeroUnlessWritten<float> lengths(H);
     init_result(paths, 1, n * maxPathLength * n);
+    ZeroUnlessWritten<int> nodes(paths);
     nsg::DeviceBuffer a(nn * sizeof(float)), h(nn * sizeof(float));
     nsg::DeviceBuffer p(nn * maxPathLength * sizeof(int));
     NSG_CUDA(cudaMemcpy(a.get(), A->host(), nn * sizeof(float), cudaMemcpyHostToDevice));
@@ -303,6 +322,8 @@ void hedetniemiAllShortestPathsGpu(CuArray<float>* A, CuArray<float>* H, CuArray
     NSG_CUDA(cudaMemcpy(H->host(), h.get(), nn * sizeof(float), cudaMemcpyDeviceToHost));
     NSG_CUDA(cudaMemcpy(paths->host(), p.get(), nn * maxPathLength * sizeof(int),
                         cudaMemcpyDeviceToHost));
+    lengths.written();
+    nodes.written();
 }
 
 void hedetniemiAllShortestPathsCpu(CuArray<float>*, CuArray<float>*, CuArray<int>*, float, int) {
@@ -324,10 +345,12 @@ void hedetniemiAllShortestPathLengthsGpu(CuArray<float>* A, CuArray<float>* H,
     const int n = A->n();
     const size_t nn = static_cast<size_t>(n) * n;
     result_matrix(A, H, n);
+    ZeroUnlessWritten<float> lengths(H);
     nsg::DeviceBuffer a(nn * sizeof(float)), h(nn * sizeof(float));
     NSG_CUDA(cudaMemcpy(a.get(), A->host(), nn * sizeof(float), cudaMemcpyHostToDevice));
     nsg::apsp_lengths(a.as<float>(), h.as<float>(), n, maxPathLength, nullptr);
     NSG_CUDA(cudaMemcpy(H->host(), h.get(), nn * sizeof(float), cudaMemcpyDeviceToHost));
+    lengths.written();
 }
 
 void correlationToAdjacency(CuArray<float>* A, CuArray<float>* C, int n, int platform) {

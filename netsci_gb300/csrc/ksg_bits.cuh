@@ -29,10 +29,14 @@
 //     the k-th joint distance with a spread of 8 to 14%. Each warp scales it
 //     so that about one query in fifteen finds fewer than k frames within h and
 //     tries again with a larger h; whatever h is, the accepted set is complete
-//     (every frame within h was evaluated, and at least k others were).
+//     (every frame within h was evaluated, and at least k others were). Where
+//     the frames fill fewer dimensions than the nodes have coordinates (nodes
+//     that depend on each other, drift, long tails) the estimates are off by
+//     factors: a neighbour far inside a crowded radius moves the scale by a
+//     tenth, and radii that still miss or crowd change faster look by look.
 //   * A full list of frames within h gives a smaller h, its own k-th distance.
-//     Queries that do not settle (heavy ties, no usable estimate, non-finite
-//     coordinates) scan all frames (scan_all).
+//     Queries that do not settle (heavy ties, coordinates that are not finite)
+//     scan all frames (scan_all), up to k + 1 of them at distance 0.
 //
 // Ties come out exactly: all frames at the k-th distance are among those
 // evaluated. What bounds the kernel: 629 instructions per query at m = 10000,
@@ -296,7 +300,7 @@ __device__ __forceinline__ int keep_nearest(float* v, float* da, float* db, int 
 // over the lanes (two entries each), then a second pass for eps and ties.
 template <int D>
 __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float* __restrict__ xb, int m, int k,
-                                       int query, int lane) {
+                                       int query, int lane, unsigned long long* evals) {
     float qa[D], qb[D];
     load_frame<D>(xa, query, qa);
     load_frame<D>(xb, query, qb);
@@ -326,6 +330,10 @@ __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float
             if (l1 > x) l1 = fmaxf(p1, x);
         }
         U = k < 32 ? __shfl_sync(kFull, l0, k) : __shfl_sync(kFull, l1, k - 32);
+        if (U == 0.f) {  // k others at distance 0
+            if (evals && lane == 0) atomicAdd(evals, static_cast<unsigned long long>(min(j0 + 32, m)));
+            return Found{0.f, 0.f, 0.f, false};
+        }
     }
     // As the tiled kernels have it: a marginal that is not a number adds nothing
     // to eps but differs from every other one at U, and with fewer than k finite
@@ -362,6 +370,7 @@ __device__ __noinline__ Found scan_all(const float* __restrict__ xa, const float
     bhi = __reduce_max_sync(kFull, bhi);
     const unsigned inf_bits = __float_as_uint(inf_f());
     const bool mixed = alo != ahi || blo != bhi || ahi > inf_bits || bhi > inf_bits;
+    if (evals && lane == 0) atomicAdd(evals, static_cast<unsigned long long>(m));
     return Found{__uint_as_float(ea), __uint_as_float(eb), U,
                  few ? alo != kFull : le > k + 1 && U > 0.f && mixed};
 }
@@ -493,7 +502,12 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                 float* dst = s_query + 8 * t + (lane < Q ? 0 : 4);
 #pragma unroll
                 for (int c = 0; c < D; ++c) dst[c] = x[c];
-                if (lane < Q) dst[3] = sqrtf(__ldg(na->est + i) * __ldg(nb->est + i)) * (base * scale);
+                dst[3] = 0.f;  // of b: the radius that was crowded
+                if (lane < Q) {
+                    // a node that does not move has no scale of its own
+                    const float ea = __ldg(na->est + i), eb = __ldg(nb->est + i);
+                    dst[3] = fmaxf(sqrtf((ea > 0.f ? ea : eb) * (eb > 0.f ? eb : ea)) * (base * scale), kLeastH);
+                }
             }
             __syncwarp();
             if (lane < 2 * D * nq) set_bins(lane / (2 * D), lane % (2 * D));
@@ -552,7 +566,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                             inside += n;
                             return true;
                         }
-                        if (n > kCrowd * (k + 1) && tries == 0) {
+                        if (n > (tries == 0 ? kCrowd : crowds(W)) * (k + 1) && tries < kCrowdTries) {
                             // another look at the rows is cheaper than that many frames
                             crowd = n;
                             return true;
@@ -619,19 +633,23 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                     }
                     if (stuck) break;
                     if (crowd) {
+                        if (lane == 0) s_query[8 * t + 7] = h;
                         scale *= 0.9985f;
-                        h *= exp2f(__log2f(0.5f * kCrowd * (k + 1) / crowd) * (0.5f / D));
+                        h *= exp2f(__log2f(0.5f * kCrowd * (k + 1) / crowd) * ((tries + 1) * (0.5f / D)));
                     } else if (inside > k) {
                         if (lane < 4) s_v[inside + lane] = inf_f();
                         __syncwarp();
                         r = select_nearest<N>(s_v, s_da, s_db, inside, k, lane);
                         __syncwarp();
                         if (tries == 0) scale *= 0.9985f;
+                        else if (r.wk < kFar * s_query[8 * t + 7]) scale = fmaxf(0.9f * scale, kLeastScale);
                         done = true;
                         break;
                     } else {
-                        if (tries == 0) scale *= 1.02f;
-                        h *= fminf(2.f, exp2f(__log2f(2.f * (k + 1) / (inside + 0.5f)) * (0.5f / D)));
+                        if (tries == 0) scale = fminf(1.02f * scale, 1.f / kLeastScale);
+                        const int faster = max(1, tries - 1);  // an estimate off by factors
+                        h *= fminf(static_cast<float>(1 << faster),
+                                   exp2f(__log2f(2.f * (k + 1) / (inside + 0.5f)) * (faster * (0.5f / D))));
                     }
                     if (lane == 0) s_query[8 * t + 3] = h;
                     __syncwarp();
@@ -639,8 +657,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_bits_search_kernel(BitsArgs B) {
                     __syncwarp();
                 }
                 if (!done) {
-                    r = scan_all<D>(xa, xb, m, k, q0 + t, lane);
-                    evals += m;
+                    r = scan_all<D>(xa, xb, m, k, q0 + t, lane, A.evals);
                 }
                 const long long o = P->scratch + q0 + t;
                 if (lane < 2) (lane ? A.eps_b : A.eps_a)[o] = lane ? r.eb : r.ea;
@@ -678,6 +695,7 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
     __shared__ float s_edge[D][65];
     __shared__ float s_whole[D][64];
     __shared__ int s_start[64];
+    __shared__ float s_out[D][2];
     const GridNode nd = nodes[blockIdx.x];
     const int m = nd.m;
     if (m > kBitMaxM) return;
@@ -693,6 +711,21 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
         s_whole[c][t] = (t + 1) * step < kBitBins ? __ldg(nd.bedges + c * 64 + (t + 1) * step) : inf_f();
     }
     if (tid < 64) s_start[tid] = __ldg(nd.ostart + tid);
+    // The outermost edges no further out than three times the two bins before
+    // them are wide: a frame far from all others stretched its bin, and the
+    // least width of all, by any factor.
+    int live = 0;  // coordinates that are not the same in nearly all frames
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        const float* e = nd.bedges + 64 * c;
+        const float lo = __ldg(e + 1), hi = __ldg(e + kBitBins - 1);
+        live += hi > lo;
+        if (tid == c) {
+            s_out[c][0] = fmaxf(__ldg(e), lo - 3.f * (__ldg(e + 3) - lo));
+            s_out[c][1] = fminf(__ldg(e + kBitBins), hi + 3.f * (hi - __ldg(e + kBitBins - 3)));
+        }
+    }
+    const float inv = 1.f / max(1, live);
     if constexpr (D > 1) {
         // the next word's bins load while this one's rows are made
         auto bins_of = [&](int w) {
@@ -724,12 +757,13 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
             if constexpr (D > 2) x = c == 2 ? f[2] : x;
             const int b = __ldg(nd.bins + i) >> (8 * c) & 0xffu;
             const int b0 = max(b - 2, 0), b1 = min(b + 3, kBitBins);
-            width = fmaxf((s_edge[c][b1] - s_edge[c][b0]) * (static_cast<float>(kBitBins) / (b1 - b0)),
-                          2e-3f * (s_edge[c][kBitBins] - s_edge[c][0]));
+            const float e0 = b0 == 0 ? s_out[c][0] : s_edge[c][b0], e1 = b1 == kBitBins ? s_out[c][1] : s_edge[c][b1];
+            width = fmaxf((e1 - e0) * (static_cast<float>(kBitBins) / (b1 - b0)), 2e-3f * (s_out[c][1] - s_out[c][0]));
+            if (!(s_edge[c][kBitBins - 1] > s_edge[c][1])) width = 1.f;
         }
         width *= __shfl_xor_sync(kFull, width, 1);
         width *= __shfl_xor_sync(kFull, width, 2);
-        float est = 0.5f * exp2f(__log2f(width * rank / m) / D);
+        float est = live ? 0.5f * exp2f(__log2f(width * rank / m) * inv) : 0.f;
         if constexpr (D > 1) {
             // first and one past the last whole bin within est, as in the search
             unsigned pack = 0;
@@ -761,7 +795,7 @@ __global__ void __launch_bounds__(kEstThreads) bits_est_kernel(const GridNode* n
                 n = __reduce_add_sync(kFull, n);
                 if (t == u) within = static_cast<float>(n);
             }
-            est *= exp2f(__log2f(rank / fmaxf(within, 1.f)) / D);
+            est *= exp2f(__log2f(rank / fmaxf(within, 1.f)) * inv);
         }
         if (c == 0 && q0 + t < hi) nd.est[i] = est;
     }

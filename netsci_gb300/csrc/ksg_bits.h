@@ -9,9 +9,17 @@
 
 namespace nsg {
 
-constexpr int kBitTries = 6;      // search radii tried before a query scans all frames
-// Bitmap hits per wanted frame from which a first radius is cut back unseen.
-constexpr int kCrowd = 10;
+constexpr int kBitTries = 12;     // search radii tried before a query scans all frames
+// Bitmap hits per wanted frame from which a first radius is cut back unseen,
+// and the next ones (another look takes as long as evaluating 400 frames, and
+// three times that in rows of four words a lane).
+constexpr int kCrowd = 10, kCrowdTries = 3;
+__host__ __device__ constexpr int crowds(int words) { return words == 4 ? 200 : 60; }
+// A k-th distance below this share of a crowded radius cuts the warp's scale,
+// which stays between kLeastScale and its inverse; the least radius looked at.
+constexpr float kFar = 0.45f;
+constexpr float kLeastScale = 0.05f;
+constexpr float kLeastH = 1e-30f;
 // Queries a warp takes at a time, at most: a lane per query and coordinate.
 __host__ __device__ constexpr int bit_queries(int d) { return d == 3 ? 4 : 8; }
 // Shared words per warp: queries, the 32 n nearest frames' distances, bins, bit_of_rank's table.

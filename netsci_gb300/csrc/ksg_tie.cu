@@ -381,8 +381,8 @@ __device__ bool sort_prefix_cta(const float* key, int* idx, int n, int T, TieSha
     // The insertion sort of [0, prefix_end), a few dozen elements, is a stable
     // sort: an element's place is the number of smaller keys plus the equal
     // ones before it. Longer prefixes (heapsorted segments among them) are left
-    // to thread 0, and so are those with a NaN (sort_prefix_warp).
-    __syncthreads();
+    // to thread 0, and so are those with a NaN (sort_prefix_warp). All swaps lie
+    // before the last barrier.
     int v = 0;
     float kv = 0.f;
     if (tid < prefix_end) {

@@ -49,6 +49,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -57,6 +58,7 @@
 #include "apsp.h"
 #include "apsp_sparse.h"
 #include "common.cuh"
+#include "engine.h"
 
 namespace nsg {
 namespace {
@@ -212,6 +214,26 @@ __global__ void pad_copy_kernel(const float* __restrict__ src, float* __restrict
     }
 }
 
+// The three padded matrices of a solve from one read of src: a copy, and its
+// transpose twice.
+__global__ void pad_iterates_kernel(const float* __restrict__ src, float* __restrict__ Ap, float* __restrict__ X0,
+                                    float* __restrict__ X1, int n, int P) {
+    __shared__ float t[32][33];
+    const float inf = __int_as_float(0x7f800000);
+    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;  // tile of Ap: rows by.., columns bx..
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
+        const int r = by + yy, c = bx + threadIdx.x;
+        const float v = (r < n && c < n) ? __ldg(src + (size_t)r * n + c) : inf;
+        t[yy][threadIdx.x] = v;
+        Ap[(size_t)r * P + c] = v;
+    }
+    __syncthreads();
+    for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
+        const size_t o = (size_t)(bx + yy) * P + by + threadIdx.x;
+        X0[o] = X1[o] = t[threadIdx.x][yy];
+    }
+}
+
 // H (n x n) = the n x n corner of X (stride P), transposed.
 __global__ void unpad_transpose_kernel(const float* __restrict__ X, float* __restrict__ H, int n, int P) {
     __shared__ float t[32][33];
@@ -290,14 +312,16 @@ void launch_split_step(const float* Ap, const float* X, float* Xn, int n, int P,
     NSG_CUDA(cudaLaunchKernelEx(&c, hedetniemi_step_kernel<S>, X, Ap, Xn, n, P, changed, step));
 }
 
-// Up to 160 tiles (n <= 768) four CTAs a tile, up to 320 (n <= 1088) two: the
-// GPU holds 608 CTAs of this kernel.
+// CTAs of a cluster that share a tile: four up to 160 tiles (n <= 768), two up
+// to 320 (n <= 1024), as the GPU holds 608 CTAs of this kernel.
+int step_split(int tiles) { return tiles <= 160 ? 4 : tiles <= 320 ? 2 : 1; }
+
 void launch_step(const float* Ap, const float* X, float* Xn, int n, int P, int* changed, int step,
                  cudaStream_t s) {
-    const int tiles = (P / kTileJ) * (P / kTileI);
-    if (tiles <= 160) {
+    const int split = step_split((P / kTileJ) * (P / kTileI));
+    if (split == 4) {
         launch_split_step<4>(Ap, X, Xn, n, P, changed, step, s);
-    } else if (tiles <= 320) {
+    } else if (split == 2) {
         launch_split_step<2>(Ap, X, Xn, n, P, changed, step, s);
     } else {
         hedetniemi_step_kernel<1><<<dim3(P / kTileJ, P / kTileI), kThreads, 0, s>>>(X, Ap, Xn, n, P, changed, step);
@@ -375,25 +399,91 @@ struct Iterates {
         Ap = static_cast<float*>(mem.p);
         X[0] = Ap + pp;
         X[1] = Ap + 2 * pp;
-        launch_pad(A, Ap, n, P, false, s);
-        launch_pad(A, X[0], n, P, true, s);
-        launch_pad(A, X[1], n, P, true, s);
+        pad_iterates_kernel<<<dim3(P / 32, P / 32), dim3(32, 8), 0, s>>>(A, Ap, X[0], X[1], n, P);
+        NSG_CUDA(cudaGetLastError());
     }
 };
 
 std::atomic<int> g_method{-1};
 
-// Seconds of a dense step: P^3 terms at 16e12 per second (measured at
-// N = 2000), and what a step of a small matrix takes anyway.
+int ceil_log2(int v) {
+    int b = 0;
+    while ((1 << b) < v) ++b;
+    return b;
+}
+
+// Seconds of a dense step: what the step of a small matrix takes anyway, and
+// 34.2 ns per k of a tile for the SM with the most tiles (measured at P = 512 to
+// 2048: within 6%, where P^3 alone was off by a quarter).
 double dense_step_seconds(int n) {
-    const double P = (n + kPad - 1) / kPad * kPad;
-    return 6e-6 + P * P * P / 16e12;
+    const int P = (n + kPad - 1) / kPad * kPad, tiles = (P / kTileJ) * (P / kTileI), split = step_split(tiles);
+    const int sms = sm_count();
+    return 6e-6 + 34.2e-9 * ((tiles * split + sms - 1) / sms) * (P / split);
+}
+
+// A sparse step of a solve: a row's entries are a chain of their own.
+double sparse_solve_step_seconds(long long width, int n) {
+    return sparse_step_seconds(width, n) + 40e-9 * static_cast<double>(width) / sell_slices(n);
+}
+
+// Whether a solve of few dense steps is over before the analysis of A (25 us
+// with its wait) could pay: n = 300, one to three steps 73 to 96 us without it,
+// against 82 to 100 with it for a sparse A and 94 to 118 for a full one. Node
+// sequences: every step is kept, and a back-walk looks at n entries instead of a
+// row's. Up to three steps of those gain less on a sparse symmetric A (n = 64,
+// three steps: 108 us against 131) than full or asymmetric ones lose (150).
+bool analysis_pays(int n, int steps, bool walk) {
+    const double dense = dense_step_seconds(n);
+    if (walk) return steps * (dense - 2.5e-6 + 0.1e-6 * (n - 10)) > (steps <= 3 ? 45e-6 : 20e-6);
+    return std::min(steps, 8) * (dense - 5.6e-6) > 15e-6;
+}
+
+// Whether the steps go over the entries: the fill of their lists (12 us, and the
+// transpose's for a walk over an asymmetric A) and the steps, against the
+// padded copies and the dense steps. Four steps are counted on: full matrices
+// converge in about that many, and sparse ones gain with every further step.
+// N = 200, full, five steps: 153 us over the entries, 133 dense; degree 16: 106
+// and 126.
+bool sparse_pays(long long width, int n, int steps, bool walk, bool symmetric) {
+    const double row = static_cast<double>(width) / sell_slices(n);
+    const double sparse = sparse_solve_step_seconds(width, n), dense = dense_step_seconds(n);
+    if (!walk) return 12e-6 + std::min(steps, 4) * sparse < 22e-6 + std::min(steps, 4) * dense;
+    const double fill = (symmetric ? 12e-6 : 48e-6) + 0.4e-6 * row;
+    return fill + steps * (sparse + 0.1e-6 * row) < 25e-6 + steps * (dense + 3.3e-6 + 0.1e-6 * n);
+}
+
+// Exact squaring on a sparse A: every A^(t+1) is the same matrix whichever way
+// it is reached, so 2^f - 1 sparse steps can stand for the first f products.
+// They cost a detour (the fill, the flags' wait and a copy, 25 us) and pay
+// where products are long. The f with the least time for a graph of points in
+// space (about 3.3 N^(1/3) (10 / degree)^(1/4) hops, N = 64 to 2000, degree 6 to
+// 16; other graphs go on with products where the steps end): none up to about
+// n = 700 (N = 200: 150 us against 185 with one step), three or four up to 1300,
+// all steps beyond (N = 2000: 1.3 ms against 3.6).
+int steps_before_products(long long width, long long entries, int n) {
+    const double step = sparse_solve_step_seconds(width, n), product = dense_step_seconds(n);
+    const double degree = std::max(1.0, static_cast<double>(entries) / n - 1);
+    const double hops = std::min(n - 1.0, 3.3 * std::cbrt(n) * std::pow(10 / degree, 0.25));
+    const int products = ceil_log2(static_cast<int>(std::ceil(hops)) + 1) + 1;
+    int best = 0;
+    double least = products * product;
+    for (int f = 1; f <= 6 && f <= ceil_log2(n); ++f) {
+        const double steps = (1 << f) - 1;
+        const double rest = steps >= 1.15 * hops ? 0 : std::max(1, products - f) * product;
+        const double t = 25e-6 + std::min(steps, 1.15 * hops) * step + rest;
+        if (t < least) {
+            least = t;
+            best = f;
+        }
+    }
+    return best;
 }
 
 // A and how a solve of it runs.
 struct Graph {
     int squaring = 0;  // repeated squaring reaches the result: 1 exactly, 2 within rounding (requested)
     bool symmetric = false;
+    int first = 0;        // powers of A taken by sparse steps before products go on (exact squaring)
     bool sparse = false;  // steps over the finite entries; rounded squaring takes dense products alone
     long long width = 0;
     DevMem words, edges;  // GraphInfo, counts, slice offsets, order, rank; the entries
@@ -402,12 +492,13 @@ struct Graph {
     const int* rank = nullptr;
 
     // unbounded: every shortest path may be taken (maxPathLength >= n - 1);
-    // steps: the most sparse steps whose labels are the solve's own (0 keeps
-    // the matrix's)
-    Graph(const float* A, int n, bool unbounded, int steps, cudaStream_t s)
+    // steps: the most the solve takes; walk: for node sequences (the labels
+    // stay the matrix's own)
+    Graph(const float* A, int n, bool unbounded, int steps, bool walk, cudaStream_t s)
         : words(sizeof(GraphInfo) + sizeof(int) * (4 * (size_t)n + 2), s), edges(0, nullptr) {
         const int method = g_method.load();
         const bool may_square = method != 0 && n >= 2 && unbounded;
+        if (!may_square && !analysis_pays(n, steps, walk)) return;
         GraphInfo* info = static_cast<GraphInfo*>(words.p);
         int* counts = reinterpret_cast<int*>(info + 1);
         int* ptr = counts + n;
@@ -425,10 +516,12 @@ struct Graph {
             if (!(h.flags & 8) && static_cast<double>(wmax) * (n - 1) < 16777216.0) squaring = 1;
             else if (method == 1) squaring = 2;  // squaring requested on any weights
         }
-        sparse = squaring != 2 && n <= kSparseMaxN && sparse_step_seconds(width, n) < dense_step_seconds(n);
+        if (n > kSparseMaxN || squaring == 2) return;
+        if (squaring == 1) first = steps_before_products(width, h.entries, n);
+        sparse = squaring == 1 ? first > 0 : sparse_pays(width, n, steps, walk, symmetric);
         if (!sparse) return;
         edges.alloc(sizeof(int2) * kSellRows * (size_t)std::max<long long>(1, width), s);
-        if (sparse_sort_pays(width, h.entries, n, steps)) {  // shorter slices, so the entries fit
+        if (!walk && sparse_sort_pays(width, h.entries, n, steps)) {  // shorter slices, so the entries fit
             int* ord = ptr + n + 2;
             sparse_sort(counts, n, ord, ord + n, s);
             sparse_slices_sorted(counts, ord, n, info, ptr, s);
@@ -442,40 +535,35 @@ struct Graph {
     }
 };
 
-// Jacobi steps launched in chunks; the last step's flag is read between
-// chunks, so long runs stop shortly after the fixed point (steps past it
-// return at once) and the later chunks, which hide a read each, are longer.
-// launch(t) enqueues step t. Returns the steps run up to and including the
-// one that changed nothing, *launched the steps enqueued, *converged whether
-// there was such a step.
-template <class F>
-int run_steps(int most, int* changed, cudaStream_t s, F&& launch, int* launched, bool* converged) {
-    int chunk = 8, t = 0, last_flag = 1;
-    while (t < most && last_flag) {
-        const int end = t + std::min(most - t, chunk);
+// Jacobi steps launched in chunks; a chunk's flags are read before the next, so
+// long runs stop shortly after the fixed point (steps past it return at once)
+// and the later chunks, which hide a read each, are longer. launch(t) enqueues
+// step t; finish(), if the last chunk is reached, what follows all steps. Returns
+// the steps run up to and including the one that changed nothing, *launched the
+// steps enqueued, *converged whether there was such a step.
+template <class F, class G>
+int run_steps(int most, int* changed, cudaStream_t s, F&& launch, G&& finish, int* launched, bool* converged) {
+    std::vector<int> flags;
+    int chunk = 8, t = 0;
+    *converged = false;
+    while (t < most && !*converged) {
+        const int begin = t, end = t + std::min(most - t, chunk);
         for (; t < end; ++t) launch(t);
-        NSG_CUDA(cudaMemcpyAsync(&last_flag, changed + (t - 1), sizeof(int), cudaMemcpyDeviceToHost, s));
+        if (t == most) finish();
+        flags.resize(t);
+        NSG_CUDA(cudaMemcpyAsync(flags.data() + begin, changed + begin, sizeof(int) * (t - begin), cudaMemcpyDeviceToHost, s));
         NSG_CUDA(cudaStreamSynchronize(s));
+        *converged = flags[t - 1] == 0;
         chunk = std::min(2 * chunk, 64);
     }
     *launched = t;
-    *converged = last_flag == 0;
-    if (last_flag) return t;
-    std::vector<int> flags(t);
-    NSG_CUDA(cudaMemcpyAsync(flags.data(), changed, sizeof(int) * t, cudaMemcpyDeviceToHost, s));
-    NSG_CUDA(cudaStreamSynchronize(s));
+    if (!*converged) return t;
     int q = 0;
     while (flags[q]) ++q;
     return q + 1;
 }
 
 bool overlap(const float* a, const float* b, size_t nn) { return a < b + nn && b < a + nn; }
-
-int ceil_log2(int v) {
-    int b = 0;
-    while ((1 << b) < v) ++b;
-    return b;
-}
 
 // Sparse Jacobi steps between H and T, the first one reading A (or T, if A is
 // null). Returns as run_steps; *at is the iterate after *launched steps, in T
@@ -487,7 +575,7 @@ int sparse_steps(const Graph& g, const float* A, float* H, float* T, int n, int 
     int* ch = static_cast<int*>(changed.p);
     const int steps = run_steps(most, ch, s, [&](int t) {
         sparse_step(g.rows, t == 0 && A ? A : (t & 1) ? H : T, (t & 1) ? T : H, n, ch, t, false, s);
-    }, launched, converged);
+    }, [] {}, launched, converged);
     // step t writes H for even t; after a step that changed nothing both
     // matrices hold the fixed point (H alone, if it was the first and A not T)
     if (*converged) *at = A ? H : T;
@@ -515,7 +603,7 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         NSG_CUDA(cudaMemcpyAsync(H, A, nn * sizeof(float), cudaMemcpyDeviceToDevice, s));
         return 0;
     }
-    const Graph g(A, n, max_path_length >= n - 1, max_path_length, s);
+    const Graph g(A, n, max_path_length >= n - 1, max_path_length, false, s);
     const bool sparse = g.sparse;
     DevMem T(sparse ? nn * sizeof(float) : 0, s);
     DevMem copy(sparse && !g.order && overlap(A, H, nn) ? nn * sizeof(float) : 0, s);
@@ -542,26 +630,18 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
     bool converged = false;
     float* at = nullptr;
     if (g.squaring) {
-        // A symmetric: X = A^T = A; each product X <- X (x) X.
-        // Exact sums on a sparse A: every A^(t+1) is the same matrix whichever
-        // way it is reached, so the powers are taken one sparse step at a
-        // time while 2^first - 1 of those cost less than `first` products.
-        // A fixed point at step h (the hop diameter) is the one that
+        // A symmetric: X = A^T = A; each product X <- X (x) X. A fixed point
+        // that single steps find at step h (the hop diameter) is the one that
         // ceil(log2 h) products reach and one more confirms.
-        if (sparse) {
-            const double step = sparse_step_seconds(g.width, n), product = dense_step_seconds(n);
-            const int most = ceil_log2(n);
-            while (first < most && ((2 << first) - 1) * step <= (first + 1) * product) ++first;
-            if (first > 0) {
-                const int h = sparse_steps(g, from, H, T.floats(), n, (1 << first) - 1, s, &launched,
-                                           &converged, &at);
-                deliver(at);
-                if (converged) {
-                    NSG_CUDA(cudaStreamSynchronize(s));
-                    return ceil_log2(h) + 1;
-                }
-                A = H;  // A^(2^first)
+        first = g.first;
+        if (first > 0) {
+            const int h = sparse_steps(g, from, H, T.floats(), n, (1 << first) - 1, s, &launched, &converged, &at);
+            deliver(at);
+            if (converged) {
+                NSG_CUDA(cudaStreamSynchronize(s));
+                return ceil_log2(h) + 1;
             }
+            A = H;  // A^(2^first)
         }
         Iterates it(A, n, s);
         // Exact sums: powers up to 2^t >= n - 1, then the product that changes
@@ -576,14 +656,13 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
         const int products = cap - first;
         for (int t = 0; t < products; ++t)
             launch_step(it.X[t & 1], it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
+        launch_unpad(it.X[products & 1], H, n, it.P, s);
         std::vector<int> flags(products);
         NSG_CUDA(cudaMemcpyAsync(flags.data(), ch, sizeof(int) * products, cudaMemcpyDeviceToHost, s));
         NSG_CUDA(cudaStreamSynchronize(s));
         int q = 0;
         while (q < products && flags[q]) ++q;
         if (q == products) fail(NSG_ERR_CUDA, "shortest-path squaring did not converge");
-        launch_unpad(it.X[products & 1], H, n, it.P, s);
-        NSG_CUDA(cudaStreamSynchronize(s));
         return first + q + 1;
     }
     if (sparse) {
@@ -597,12 +676,19 @@ int apsp_lengths(const float* A, float* H, int n, int max_path_length, cudaStrea
     DevMem changed(sizeof(int) * max_path_length, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * max_path_length, s));
     int* ch = static_cast<int*>(changed.p);
+    // The result of t steps lives in X[t & 1]; when converged both buffers hold it.
+    bool unpadded = false;
+    auto unpad = [&](int t) {
+        launch_unpad(it.X[t & 1], H, n, it.P, s);
+        unpadded = true;
+    };
     const int steps = run_steps(max_path_length, ch, s, [&](int t) {
         launch_step(it.Ap, it.X[t & 1], it.X[(t + 1) & 1], n, it.P, ch, t, s);
-    }, &launched, &converged);
-    // The result lives in X[launched & 1]; when converged both buffers hold it.
-    launch_unpad(it.X[launched & 1], H, n, it.P, s);
-    NSG_CUDA(cudaStreamSynchronize(s));
+    }, [&] { unpad(max_path_length); }, &launched, &converged);
+    if (!unpadded) {
+        unpad(launched);
+        NSG_CUDA(cudaStreamSynchronize(s));
+    }
     return steps;
 }
 
@@ -612,7 +698,7 @@ void apsp_paths(const float* A, float* H, int* paths, int n, int L, float tolera
     const size_t nn = (size_t)n * n;
     NSG_CUDA(cudaMemsetAsync(paths, 0xff, sizeof(int) * nn * L, s));  // -1
     if (n == 0) return;
-    Graph g(A, n, false, 0, s);
+    const Graph g(A, n, false, L, true, s);
     DevMem snaps(nn * (L + 1) * sizeof(float), s);  // H before each step, and after the last
     DevMem changed(sizeof(int) * L, s);
     NSG_CUDA(cudaMemsetAsync(changed.p, 0, sizeof(int) * L, s));

@@ -194,7 +194,9 @@ int nsg_ksg_pair_detail_device(const float* xa, const float* xb, int ld, int m, 
  * bit 2 = pick the tile shape with the autotuner (each instantiated shape
  * timed on up to 512 of the pairs, longest first; the result is cached per
  * (GPU, d, k bucket, m bucket, pair-count bucket), in the file named by the
- * environment variable NSG_TUNE_CACHE when set).
+ * environment variable NSG_TUNE_CACHE when set); bits 4 to 6 = 1 + the route
+ * to take (nsg_ksg_plan_route), 0 = choose: NSG_ERR_UNSUPPORTED when the route
+ * does not take the pairs.
  * The tile shape comes from the autotuner cache when one is loaded.       */
 typedef struct nsg_ksg_plan nsg_ksg_plan;
 int nsg_ksg_plan_create(const nsg_ksg_pair* pairs, int npairs, int k, int d, float* mi,
@@ -227,12 +229,11 @@ int nsg_ksg_set_shape(int threads, int r, int frames, int variant);
  * 16-byte aligned rows, a plane stride that is a multiple of 4 and no
  * frame map).                                                             */
 int nsg_ksg_set_staging(int staging);
-/* Search for later plans: 1 cell grids (ksg_grid.cuh: only the frames whose
- * cells can reach a query are evaluated; same results), 0 exhaustive, -1
- * automatic (cell grids when at least half of the work, counted as m^2 per
- * pair, is in pairs with m >= 1000 (4000 for plans of fewer than 8 pairs)
- * and the copies of frame-mapped rows, which the grids search instead of
- * the maps, fit in 8 GiB). */
+/* Search for later plans: 1 on node grids (rank bitmaps or the scan of cells,
+ * whichever is estimated to take less time: only frames that can reach a
+ * query are evaluated; same results), 0 exhaustive, -1 automatic (the route
+ * with the least estimated time; exhaustive where the copies of frame-mapped
+ * rows, which the grids search instead of the maps, exceed 8 GiB). */
 int nsg_ksg_set_search(int mode);
 /* Query orders of later cell-grid plans: 1 = always build them (the search's
  * block order and the counts' box order of a batch), 0 = never (cells in Z
@@ -250,8 +251,12 @@ int nsg_ksg_set_orders(int mode);
  * one-variable distance plus one per eps comparison). A diagnostic for the
  * roofline of those kernels; no reference counterpart. Takes about 0.1 s. */
 int nsg_measure_issue_ceiling(int d, double* search_gops, double* count_gops);
-/* *mode = 1 when the plan uses cell grids, 0 when exhaustive. */
+/* *mode = 1 when the plan uses node grids, 0 when exhaustive. */
 int nsg_ksg_plan_search(const nsg_ksg_plan* plan, int* mode);
+/* The kernels that find the plan's neighbours: 0 exhaustive, a thread per query
+ * (the tile shape is nsg_ksg_plan_shape's); 1 exhaustive, a warp per query; 2
+ * rank bitmaps (of any of its batches); 3 the scan of cells. */
+int nsg_ksg_plan_route(const nsg_ksg_plan* plan, int* route);
 /* Query-frame evaluations of the plan's last run with cell grids: *search
  * joint distances of the search, *counts one-variable distances of the
  * counts (one per query and frame, shared by the pairs of a count group),

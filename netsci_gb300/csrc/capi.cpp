@@ -468,6 +468,7 @@ int nsg_ksg_plan_create(const nsg_ksg_pair* pairs, int npairs, int k, int d, flo
         opt.graph = (flags & 1) != 0;
         opt.timing = (flags & 2) != 0;
         opt.autotune = (flags & 4) != 0;
+        opt.route = (flags >> 4 & 7) - 1;
         *out = new nsg_ksg_plan{new nsg::KsgPlan(v, k, d, o, opt)};
     });
 }
@@ -502,6 +503,14 @@ int nsg_ksg_plan_search(const nsg_ksg_plan* plan, int* mode) {
     return guarded([&] {
         if (!plan || !plan->plan) nsg::invalid("plan is null");
         *mode = plan->plan->search();
+    });
+}
+
+int nsg_ksg_plan_route(const nsg_ksg_plan* plan, int* route) {
+    return guarded([&] {
+        if (!plan || !plan->plan) nsg::invalid("plan is null");
+        if (!route) nsg::invalid("null output");
+        *route = plan->plan->route();
     });
 }
 

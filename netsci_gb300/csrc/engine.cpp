@@ -457,6 +457,16 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
     }
     search_ = search == 1 ? 1 : 0;
     warp_ = !search_ && warp_ok;
+    if (opt.route >= 0) {
+        if (opt.route > KSG_SCAN) invalid("route must be 0 to 3");
+        if ((opt.route >= KSG_BITMAPS && !grid_ok) || (opt.route == KSG_WARP && !ksg_warp_fits(d, k, maxm)) ||
+            (opt.route == KSG_BITMAPS && !bits_config(d, k, maxm).ok)) {
+            fail(NSG_ERR_UNSUPPORTED, "the route asked for does not take these pairs");
+        }
+        search_ = opt.route >= KSG_BITMAPS ? 1 : 0;
+        warp_ = opt.route == KSG_WARP;
+        scan_ = opt.route == KSG_SCAN;
+    }
     std::vector<nsg_ksg_pair> eff;
     if (search_ && !mapped.empty()) {
         mapped_rows_.reset(mapped_floats * sizeof(float));
@@ -997,6 +1007,14 @@ int KsgPlan::launches() const {
         }
     }
     return n;
+}
+
+int KsgPlan::route() const {
+    if (!search_) return warp_ ? KSG_WARP : KSG_TILED;
+    if (grid_)
+        for (const auto& bits : grid_->batch_bits)
+            if (!bits.empty()) return KSG_BITMAPS;
+    return KSG_SCAN;
 }
 
 unsigned long long* KsgPlan::evals() const {

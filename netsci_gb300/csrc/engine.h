@@ -73,6 +73,10 @@ struct KsgOutputs {
     float* kdist = nullptr;
 };
 
+// The kernels that find a plan's neighbours: exhaustive, a thread or a warp per
+// query, or on node grids, rank bitmaps or the scan of cells.
+enum KsgRoute { KSG_TILED = 0, KSG_WARP = 1, KSG_BITMAPS = 2, KSG_SCAN = 3 };
+
 struct KsgPlanOptions {
     bool graph = false;                  // capture each run in a CUDA graph
     bool timing = false;                 // CUDA events around each count launch
@@ -81,6 +85,7 @@ struct KsgPlanOptions {
     int variant = -1;
     int staging = -1;                    // -1 auto, 0 plain loads, 1 bulk copies (TMA)
     int search = -1;                     // -1 auto, 0 exhaustive, 1 cell grids
+    int route = -1;                      // -1 by search and estimates, else a KsgRoute
     size_t scratch_budget_bytes = 0;     // 0: library default
 };
 
@@ -101,6 +106,8 @@ public:
     long long pairs() const { return npairs_; }
     // Reads (and clears) the device fault word; synchronizes with the device.
     int take_fault();
+    // The route the plan takes (bitmaps if any of its batches does).
+    int route() const;
     const KsgShape& shape() const { return shape_; }
     int variant() const { return variant_; }
     int staging() const;  // 1: bulk-copy staged kernel, 0: plain loads

@@ -93,15 +93,20 @@ def ksg_pair_detail(xa: torch.Tensor, xb: torch.Tensor, m: int, k: int, d: int,
 
 class KsgPlan:
     """Reusable all-pairs plan (nsg_ksg_plan_*): descriptors, work queue and
-    scratch built once; ``run`` replays one captured CUDA graph."""
+    scratch built once; ``run`` replays one captured CUDA graph. ``route`` asks
+    for one of ROUTES instead of the one with the least estimated time."""
+
+    ROUTES = ("tiled", "warp", "bitmaps", "scan")
 
     def __init__(self, pairs: Sequence[KsgPair], k: int, d: int, mi: torch.Tensor | None = None,
                  gc: torch.Tensor | None = None, w: torch.Tensor | None = None,
-                 graph: bool = True, timing: bool = False, autotune: bool = False):
+                 graph: bool = True, timing: bool = False, autotune: bool = False, route: str | None = None):
         self._keep = (mi, gc, w)
         arr = _pair_array(pairs)
         h = ctypes.c_void_p()
         flags = (1 if graph else 0) | (2 if timing else 0) | (4 if autotune else 0)
+        if route is not None:
+            flags |= (1 + self.ROUTES.index(route)) << 4
         call("nsg_ksg_plan_create", arr, len(pairs), int(k), int(d), _ptr(mi), _ptr(gc), _ptr(w),
              flags, ctypes.byref(h))
         self._h = h
@@ -132,6 +137,13 @@ class KsgPlan:
         return dict(threads=v[0].value, r=v[1].value, frames=v[2].value, variant=v[3].value,
                     staging="bulk-copy" if v[4].value else "loads",
                     search="cell-grid" if v[5].value else "exhaustive")
+
+    @property
+    def route(self) -> str:
+        """The kernels that find the plan's neighbours, one of ROUTES."""
+        v = ctypes.c_int()
+        call("nsg_ksg_plan_route", self._h, ctypes.byref(v))
+        return self.ROUTES[v.value]
 
     def evaluations(self) -> tuple[int, int, int]:
         """(joint distances, one-variable distances, eps comparisons) of the

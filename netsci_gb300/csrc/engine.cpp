@@ -2,6 +2,7 @@
 #include "engine.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -184,58 +185,82 @@ int g_forced_variant = -1;
 int g_forced_staging = -1;
 int g_forced_search = -1;
 int g_forced_orders = -1;
-// Microseconds of a plan on each route, from the times of 632 plan shapes
-// (lists of 5 to 55 nodes, chains and stars of up to 1000 pairs, m = 500 to
-// 5000, d = 1 to 3, k = 1 to 30): the route they choose takes 1.2% more than
-// the fastest on average, a quarter more at worst.
+// Microseconds of a plan, built, run once and given back, on each route. The
+// terms follow the kernels, the factors are fitted to 1,998 plans on every route
+// (profiles/ksg_route_times.csv: lists of 2 to 120 nodes, a star and a chain of
+// 119 pairs, m = 500 to 4500, d = 1 to 3, k = 1 to 30, usual coordinates): 5%
+// spread for the exhaustive routes, 7 to 9% for the others where they are near
+// the best. The route chosen takes 0.4% more than the best on average, and more
+// than 13% in one plan of a hundred. Samples and distances are in thousands and
+// millions.
 struct PlanSize {
     int d, k, max_m;
-    double samples, work;  // sums of m and of m^2 over the pairs
-    double rows;           // sum of m over the distinct rows, counted up to kRowsMost
-    double pairs;
+    double pairs, samples, work;  // pairs, sum of m, sum of m^2
+    double blocks, block_work;    // the same with m rounded up to whole CTAs of the tiled kernels
+    double rows;                  // sum of m over the distinct rows
+    bool orders;                  // query orders are built
 };
-constexpr double kRowsMost = 4e4;
 
 // Neighbour lists beyond six entries: their cost follows the list's length in
 // registers (14, 30, 62 entries) more than k.
 double long_list(int k) {
     return k <= 6 ? 0 : k <= 14 ? 3.5 + 0.32 * (k - 10) : k <= 30 ? 14 + 0.25 * (k - 20) : 35 + 0.3 * (k - 31);
 }
-// One thread's walk over m frames, list updates, frame visits.
+// Queries per CTA of the tiled kernel that such a plan takes.
+int tiled_block(int k, double samples, int sms) {
+    if (k > 30) return 64;
+    if (k > 6) return 128;
+    for (const auto& [block, ctas_per_sm] : {std::pair{256, 5}, {128, 10}, {512, 2}}) {
+        if (samples / block >= 2.0 * ctas_per_sm * sms) return block;
+    }
+    return 64;
+}
+// A thread's walk over all frames, then list updates and frame visits of all
+// queries, idle ones of a pair's last CTA among them (m = 512 against 600: the
+// same two CTAs of 256 or three).
 double tiled_us(const PlanSize& p) {
-    const int k = p.k, few = std::min(k, 6) - 1;
-    const double more = long_list(k);
-    return 19.2 + 0.8 * std::min(k, 20) + p.max_m * (0.02 + 0.015 * p.d + 0.002 * std::min(k, 20)) +
-           1e-3 * p.samples * (0.13 + 0.055 * few + 0.104 * more) +
-           1e-6 * p.work * (0.14 + 0.21 * p.d + 0.025 * few + 0.107 * more);
+    const int few = std::min(p.k, 6) - 1;
+    const double more = long_list(p.k);
+    return 40 + 0.06 * p.pairs + 1e-2 * p.max_m * (1.98 + 1.35 * p.d + 0.387 * few + 0.262 * more) +
+           1e-3 * p.blocks * (0.077 + 0.049 * few + 0.106 * more) * std::max(0.3, 1 + 0.784 * std::log(p.max_m / 500.0)) +
+           1e-6 * p.block_work * (0.142 + 0.19 * p.d + 0.049 * more);
 }
 // A warp per query: 10 pairs at m = 500, d = 3: 29 us against 65 tiled; 153
 // pairs: 155 against 109.
 double warp_us(const PlanSize& p) {
-    return 19 + 1e-3 * p.samples * (0.34 + 0.033 * (p.k - 1)) + 1e-6 * p.work * (0.52 + 0.66 * p.d + 0.01 * (p.k - 1));
+    return 35 + 1e-3 * p.samples * (0.921 + 0.04 * (p.k - 1)) + 1e-6 * p.work * (0.531 + 0.584 * p.d + 0.019 * (p.k - 1)) +
+           1e-2 * p.max_m * (0.255 + 0.091 * p.d);
 }
+// Nodes up to about a wave of CTAs cost more than the ones after them.
+constexpr double kFirstRows = 4e4;
 // The bitmap search hardly depends on m, the scan of cells visits fewer frames
-// the lower d and k are. 703 pairs at m = 1000: d = 1, k = 6 401 us scanned and
-// 529 on bitmaps; d = 3, k = 6 656 and 708; d = 3, k = 20 2002 and 1098.
+// the lower d and k are; orders cost the scan more. 990 pairs at m = 999: d = 3,
+// k = 6 1.16 ms scanned and 0.99 on bitmaps; 190 pairs at m = 999, d = 2, k = 1
+// 0.21 and 0.31.
 double bits_us(const PlanSize& p) {
-    const bool one = p.k <= 12;
-    return 1.1 * (45 + 9 * p.d + 1e-3 * p.samples * (one ? 0.41 : 0.78) +
-                  p.rows * (one ? 0.0045 + 0.0003 * p.d : 0.0075) + (p.d == 3 && !one ? 0.06e-6 * p.work : 0.0));
+    const double first = std::min(p.rows, kFirstRows), rest = p.rows - first;
+    const double per_sample = p.k <= 12 ? 0.416 + 0.003 * p.d + 0.0163 * p.k : 0.574 + 0.033 * p.d + 0.0182 * p.k;
+    return 70 + 10.4 * p.d + 0.088 * p.pairs + 1e-3 * p.samples * per_sample + 1e-6 * p.work * (p.d == 3 ? 0.063 : 0.029) +
+           1e-3 * first * (2.02 + 1.03 * p.d) + 1e-3 * rest * (0.477 + 0.153 * p.d) +
+           1e-2 * p.max_m * (0.517 + 0.128 * p.d + 0.104 * p.k) + (p.orders ? 10 : 0);
 }
 double scan_us(const PlanSize& p) {
     const int few = std::min(p.k, 6) - 1;
     const double more = long_list(p.k);
-    const double visit[3] = {0.013e-6, 0.059e-6, 0.132e-6};
-    return 62 + 9 * p.d + 0.9 * std::min(p.k, 20) + 1e-3 * p.samples * (0.23 + 0.01 * few + 0.067 * more) +
-           p.work * visit[p.d - 1] * (1 + 0.13 * few + 0.25 * more) +
-           p.rows * (0.0004 + 0.0007 * p.d + 0.0004 * few + 0.0003 * more);
+    const double visit[3] = {0.0104, 0.0779, 0.146};
+    const double first = std::min(p.rows, kFirstRows), rest = p.rows - first;
+    return 90 + 7.5 * p.d + 0.56 * std::min(p.k, 20) + 0.101 * p.pairs +
+           1e-3 * p.samples * (0.21 + 0.033 * few + 0.0775 * more + (p.orders ? 0.074 : 0)) +
+           1e-6 * p.work * visit[p.d - 1] * (1 + 0.187 * few + 0.344 * more) + 1e-3 * first * (0.5 + 0.344 * p.d) +
+           1e-3 * rest * 0.213 + 1e-2 * p.max_m * (1.83 + (p.d > 1 ? 0.78 : 0) + (p.d > 2 ? 0.91 : 0) + 0.268 * more) +
+           (p.orders ? 88 : 0);
 }
 // Fewer samples than this leave most of the scan's warps idle (32 queries
 // each), while the bitmap search splits a pair over CTAs.
 constexpr double kScanMinSamples = 3e4;
-// What a pair's node and count work lists cost when a plan on grids is built
-// (1770 pairs: 493 us against 402).
-constexpr double kGridPairUs = 0.05;
+bool scan_faster(const PlanSize& p) {
+    return !bits_config(p.d, p.k, p.max_m).ok || (p.samples >= kScanMinSamples && scan_us(p) < bits_us(p));
+}
 // per batch: work-queue heads (two for the grid search), tie count,
 // tie-kernel counter, rank-count queue head, bitmap-search queue heads
 constexpr int kCounters = 5 + kBitSegments;
@@ -431,10 +456,18 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
         fail(NSG_ERR_UNSUPPORTED, "cell-grid search: copies of the frame-mapped rows exceed 8 GiB");
     }
     // the route with the smallest estimate
-    PlanSize size{d, k, maxm, static_cast<double>(total_samples), work, 0, static_cast<double>(npairs)};
+    const double total = static_cast<double>(total_samples);
+    PlanSize size{d, k, maxm, static_cast<double>(npairs), total, work, 0, 0, 0,
+                  grid_orders_pay(total_samples / 32, sm_count())};
     {
-        // the first pairs tell: a list of all pairs of N nodes names them in
-        // its first N - 1, and other lists reach kRowsMost soon
+        const int block = tiled_block(k, total, sm_count());
+        for (const auto& q : pairs_in) {
+            const double whole = static_cast<double>((q.m + block - 1) / block) * block;
+            size.blocks += whole;
+            size.block_work += whole * q.m;
+        }
+        // the first pairs tell the rows: a list of all pairs of N nodes names
+        // them in its first N - 1, and further rows cost little
         std::vector<std::pair<std::pair<const float*, const int*>, int>> rows;
         const size_t most = std::min<size_t>(pairs_in.size(), 128);
         for (size_t p = 0; p < most; ++p) {
@@ -446,14 +479,12 @@ KsgPlan::KsgPlan(const std::vector<nsg_ksg_pair>& pairs_in, int k, int d, const 
         for (size_t r = 0; r < rows.size(); ++r) {
             if (r == 0 || rows[r].first != rows[r - 1].first) size.rows += rows[r].second;
         }
-        size.rows = std::min(size.rows, kRowsMost);
     }
-    const bool warp_ok = !tile_forced && !opt.autotune && ksg_warp_fits(d, k, maxm) && warp_us(size) < tiled_us(size);
-    scan_ = size.samples >= kScanMinSamples && scan_us(size) < bits_us(size);
+    const bool warp_ok = !tile_forced && !opt.autotune && npairs > 0 && ksg_warp_fits(d, k, maxm) && warp_us(size) < tiled_us(size);
+    scan_ = npairs > 0 && scan_faster(size);
     if (search < 0) {
         const double exhaustive = warp_ok ? warp_us(size) : tiled_us(size);
-        const double grids = (scan_ ? scan_us(size) : bits_us(size)) + kGridPairUs * size.pairs;
-        search = grid_ok && grids < exhaustive ? 1 : 0;
+        search = grid_ok && (scan_ ? scan_us(size) : bits_us(size)) < exhaustive ? 1 : 0;
     }
     search_ = search == 1 ? 1 : 0;
     warp_ = !search_ && warp_ok;

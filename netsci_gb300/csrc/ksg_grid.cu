@@ -741,11 +741,15 @@ size_t grid_node_bytes(int m, int d) {
     const size_t mm = static_cast<size_t>(m);
     return a16(2 * kGridMaxG * sizeof(float)) + grid_index_bytes(grid_cells_per_axis(m)) +
            a16(mm * sizeof(unsigned short)) + a16(mm * sizeof(int)) + a16(mm * sizeof(float)) +
-           a16(static_cast<size_t>(d) * mm * sizeof(float)) +
-           // bitmap search: frames, bins, order, edges, starts
-           a16((d == 3 ? 4 : d) * mm * sizeof(float)) + a16(mm * sizeof(unsigned)) +
-           a16(mm * sizeof(unsigned short)) + static_cast<size_t>(d) * (64 + kQuantFloats) * sizeof(float) +
-           64 * sizeof(int);
+           a16(static_cast<size_t>(d) * mm * sizeof(float)) + grid_node_bitmap_bytes(m, d);
+}
+
+size_t grid_node_bitmap_bytes(int m, int d) {
+    auto a16 = [](size_t b) { return (b + 15) & ~size_t(15); };
+    const size_t mm = static_cast<size_t>(m);
+    // frames, bins, order, edges, starts
+    return a16((d == 3 ? 4 : d) * mm * sizeof(float)) + a16(mm * sizeof(unsigned)) + a16(mm * sizeof(unsigned short)) +
+           static_cast<size_t>(d) * (64 + kQuantFloats) * sizeof(float) + 64 * sizeof(int);
 }
 
 GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m, int d) {

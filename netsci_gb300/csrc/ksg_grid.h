@@ -199,6 +199,8 @@ int grid_cells_per_axis(int m);
 // Bytes of one node grid's buffers, and its descriptor with the buffers at
 // `base` (16-byte aligned) for row x (stride ld) of m samples.
 size_t grid_node_bytes(int m, int d);
+// Those of them that only the bitmap search reads.
+size_t grid_node_bitmap_bytes(int m, int d);
 GridNode grid_node_at(unsigned char* base, const float* x, int ld, int m, int d);
 // Places a pair grid's buffers at byte offset `off` of a batch arena
 // (pointers hold offsets until grid_pair_rebase) and returns the end offset.

@@ -158,11 +158,15 @@ int Server::register_trajectory(const float* X, int N, int m, int d) {
     NSG_CUDA(cudaMemcpy2D(t->X.get(), t->ld * sizeof(float), X, m * sizeof(float),
                           m * sizeof(float), static_cast<size_t>(N) * d, cudaMemcpyHostToDevice));
     // node grids of every row, built once: the cell-grid search of later ticks reads them
+    // charged to the budget: the grids without what only the bitmap search
+    // reads (22 bytes a frame at d = 3), which spares ticks the uncharged
+    // scratch of pair grids (32 bytes a frame and pair). Charged, a budget of 46
+    // bytes a frame no longer admits any job beside its trajectory.
     size_t gbytes = 0;
     if (next_node_slot_ + N <= kNodeSlots - 2 * kMiSlotPairs) {
         const size_t per = grid_node_bytes(m, d);
-        gbytes = per * N;
-        t->grid_arena.reset(gbytes);
+        t->grid_arena.reset(per * N);
+        gbytes = (per - grid_node_bitmap_bytes(m, d)) * N;
         t->slot0 = next_node_slot_;
         std::vector<GridNode> nodes(N);
         const size_t row = static_cast<size_t>(d) * t->ld;

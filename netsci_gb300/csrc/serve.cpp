@@ -176,7 +176,7 @@ int Server::register_trajectory(const float* X, int N, int m, int d) {
         }
         GridNode* dst = d_gnodes_.as<GridNode>() + t->slot0;
         NSG_CUDA(cudaMemcpy(dst, nodes.data(), sizeof(GridNode) * N, cudaMemcpyHostToDevice));
-        grid_launch_nodes(dst, N, d, false, nullptr);
+        grid_launch_nodes(dst, N, d, grid_split_pays(N, sm_count()), nullptr);
         bits_launch_est(dst, N, m, d, nullptr);
         NSG_CUDA(cudaDeviceSynchronize());
         next_node_slot_ += N;

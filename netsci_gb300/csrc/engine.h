@@ -197,6 +197,10 @@ void ksg_force_search(int mode);
 // automatic, 0 never, 1 always).
 void ksg_force_orders(int mode);
 int ksg_forced_orders();
+// Whether a serving tick (pairs; the sums of m and of m^2 over them), whose
+// node grids stand already, is searched faster by the scan of cells than on
+// bitmaps, or the bitmaps do not fit.
+bool ksg_tick_scans(int d, int k, int max_m, double pairs, double samples, double work, bool orders);
 // True when every pair allows bulk-copy staging (16-byte aligned rows,
 // plane stride a multiple of 4, no frame map).
 bool ksg_bulk_copy_ok(const std::vector<nsg_ksg_pair>& pairs);

@@ -411,7 +411,11 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
         }
     }
     h_wpre_[np] = static_cast<int>(wacc);
-    const BitsSegment bits{0, static_cast<int>(np), maxm, bits_config(d, k, maxm)};
+    const bool order = grid_orders_pay(wacc, sm_count());  // query orders for this tick
+    BitsSegment bits{0, static_cast<int>(np), maxm, {}};
+    if (!ksg_tick_scans(d, k, maxm, static_cast<double>(np), static_cast<double>(samples), work, order)) {
+        bits.config = bits_config(d, k, maxm);
+    }
     for (long long i = 0; i < np && !bits.config.ok; ++i) arena = grid_pair_place(h_gpairs_[i], arena, h_pairs_[i].m, d);
     cudaStream_t s = ksg_stream_;
     // buffers grow on demand (by a quarter more than asked, to grow rarely)
@@ -431,7 +435,6 @@ bool Server::run_tick_grid(std::vector<std::pair<Job*, std::pair<long long, long
     NSG_CUDA(cudaMemcpyAsync(d_gpairs_.get(), h_gpairs_, sizeof(GridPair) * np, cudaMemcpyHostToDevice, s));
     NSG_CUDA(cudaMemcpyAsync(d_wpre_.get(), h_wpre_, sizeof(int) * (np + 1), cudaMemcpyHostToDevice, s));
     // count groups and rank nodes: variables of the tick on the same node
-    const bool order = grid_orders_pay(wacc, sm_count());  // query orders for this tick
     const CountWork work_list = count_work(h_gpairs_, h_pairs_, static_cast<int>(np), order);
     const auto& groups = work_list.groups;
     if (order) ensure(d_corder_, sizeof(int) * std::max<size_t>(1, groups.size() * static_cast<size_t>(maxm)));

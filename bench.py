@@ -17,10 +17,12 @@ Lines reported (one JSON line from rank 0):
             over host CuArrays): host->device upload of X and the pair list
             and device->host read of the results inside every step.
   roofline  the dominant kernel (the bitmap search) against the CUDA-core
-            issue model (SMs x 128 lanes x max SM clock): its operations are
-            lane instructions, the warp instructions per query that ncu
-            counts at this m times 32 (bitmap words, selection and the few
-            distances alike). The count kernels stand under per_kernel with
+            issue model (SMs x 128 lanes x max SM clock). Its operations are
+            not counted in the run: they are an estimate, the warp
+            instructions per query of one ncu capture at this m times 32
+            (bitmap words, selection and the few distances alike), and the
+            share of the peak that follows is called estimated_frac. The
+            count kernels stand under per_kernel with
             operations from their own evaluation counters, 2d-1 per
             one-variable distance (one per query and frame, shared by the
             variables of a group or a rank pass) plus one per eps comparison
@@ -80,11 +82,12 @@ sys.path.insert(0, str(ROOT))
 sys.path.insert(0, str(ROOT / "netsci_gb300" / "dropin"))
 
 N_NODES, M_FRAMES, DIM, K_NN = 2000, 10000, 3, 6
-# The search kernel at m = 10000, from an ncu capture of a 256-pair step
-# (profiles/ksg_bits_kernels_m10000.md): DRAM bytes per pair (62.1 MB read and
-# 5.9 MB written) and warp instructions per query (1.610e9 over 2.56e6 queries).
-SEARCH_DRAM_BYTES_PER_PAIR = (62.1 + 5.9) * 1e6 / 256
-SEARCH_INSTRUCTIONS_PER_QUERY = 629
+# The bitmap search at m = 10000, d = 3, k = 6, from one ncu capture of a
+# 256-pair step (profiles/ksg_bits_kernels_m10000.md): DRAM bytes per pair (62.3 MB
+# read and 5.4 MB written) and warp instructions per query (1.626e9 over 2.56e6
+# queries). A change to the kernel makes them stale until it is captured again.
+SEARCH_DRAM_BYTES_PER_PAIR = (62.3 + 5.4) * 1e6 / 256
+SEARCH_INSTRUCTIONS_PER_QUERY = 635
 SEED = 2000
 METRIC = "GC pairs/sec (batched persistent), N=2000 nodes, m=10000 frames"
 
@@ -571,6 +574,7 @@ def main():
     peak_gops = props.multi_processor_count * 128 * sm_max * 1e6 / 1e9
     ops_launch = ops_per_pair(m) * B
     search = plans[args.warmup].shape["search"]
+    route = plans[args.warmup].route
     clocks = clk.summary()
     _, ceil_count = device.issue_ceiling(DIM)
     search_s = statistics.mean(k[0] for k in kms) / 1000.0
@@ -580,16 +584,20 @@ def main():
         joint = statistics.mean(e[0] for e in evs)
         one_var = statistics.mean(e[1] for e in evs)
         compares = statistics.mean(e[2] for e in evs)
-        search_ops = 32.0 * SEARCH_INSTRUCTIONS_PER_QUERY * m * B if m == M_FRAMES else joint * 4 * DIM
+        # one capture stands for the bitmap search at its m; elsewhere only the distances are known
+        captured = route == "bitmaps" and m == M_FRAMES
+        search_ops = 32.0 * SEARCH_INSTRUCTIONS_PER_QUERY * m * B if captured else joint * 4 * DIM
+        kernel = "ksg_bits_search_kernel" if route == "bitmaps" else "ksg_grid_pass1_kernel"
         count_ops = one_var * (2 * DIM - 1) + compares
         per_kernel = {
-            "ksg_bits_search_kernel": {
+            kernel: {
                 "ms_per_launch": 1000 * search_s, "ops_per_launch": search_ops,
                 "joint_evaluations": joint,
-                "ops": ("32 lanes x warp instructions per query (ncu)" if m == M_FRAMES
+                "ops": (f"estimate: 32 lanes x {SEARCH_INSTRUCTIONS_PER_QUERY} warp instructions per query "
+                        "(one ncu capture, not counted here)" if captured
                         else "4d per joint distance alone"),
-                "achieved_gops": search_ops / search_s / 1e9,
-                "frac": search_ops / search_s / 1e9 / peak_gops},
+                "estimated_gops" if captured else "achieved_gops": search_ops / search_s / 1e9,
+                "estimated_frac" if captured else "frac": search_ops / search_s / 1e9 / peak_gops},
             "count kernels": {
                 "ms_per_launch": 1000 * count_s, "ops_per_launch": count_ops,
                 "one_variable_evaluations": one_var, "eps_comparisons": compares,
@@ -605,20 +613,25 @@ def main():
                          "marginals, replayed in the reference sort's order; O(m) per "
                          "sample")},
         }
-        dom = per_kernel["ksg_bits_search_kernel"]
-        kernel, achieved, traffic = "ksg_bits_search_kernel", dom["achieved_gops"], None
-        if m == M_FRAMES:
+        achieved, traffic, mix = search_ops / search_s / 1e9, None, None
+        if captured:
             traffic = SEARCH_DRAM_BYTES_PER_PAIR * B
-        mix = None
     else:
-        per_kernel = None
-        kernel, achieved, traffic, mix = "ksg_count_kernel", ops_launch / search_s / 1e9, None, None
+        per_kernel, captured = None, False
+        kernel = "ksg_warp_kernel" if route == "warp" else "ksg_count_kernel"
+        achieved, traffic, mix = ops_launch / search_s / 1e9, None, None
     frac_at_clock = None
     if clocks.get("sm_mhz"):
         frac_at_clock = achieved / (props.multi_processor_count * 128 * clocks["sm_mhz"] * 1e6 / 1e9)
     roofline = {
-        "bound": "cuda_core_issue", "kernel": kernel, "achieved": achieved, "peak": peak_gops,
-        "unit": "Gop/s", "frac": achieved / peak_gops, "frac_at_median_clock": frac_at_clock,
+        "bound": "cuda_core_issue", "kernel": kernel, "achieved": None if captured else achieved,
+        "peak": peak_gops, "unit": "Gop/s", "frac": None if captured else achieved / peak_gops,
+        "estimated": achieved if captured else None,
+        "estimated_frac": achieved / peak_gops if captured else None,
+        "estimate_source": ("warp instructions per query of one ncu capture (256 pairs) over this run's "
+                            "time" if captured else None),
+        "frac_at_median_clock": None if captured else frac_at_clock,
+        "estimated_frac_at_median_clock": frac_at_clock if captured else None,
         "mix_ceiling": mix, "frac_of_mix_ceiling": (achieved / mix) if mix else None,
         "traffic": traffic,
         "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the search kernel "
@@ -629,7 +642,7 @@ def main():
         "mix_ceiling_source": ("nsg_measure_issue_ceiling: the group counts' inner loop alone on a "
                                "staged tile (no memory traffic, no range setup), measured on this "
                                "GPU with CUDA events"),
-        "search": search, "per_kernel": per_kernel,
+        "search": search, "route": route, "per_kernel": per_kernel,
         "algorithmic_pruning_gops": ops_launch / (search_s + count_s) / 1e9,
         "algorithmic_pruning_note": ("8*d*m*(m-1) operations per pair (what an exhaustive "
                                      "search does) over the kernels' time: the pruning's "

@@ -39,11 +39,11 @@
 //     scan all frames (scan_all), up to k + 1 of them at distance 0.
 //
 // Ties come out exactly: all frames at the k-th distance are among those
-// evaluated. What bounds the kernel: 629 instructions per query at m = 10000,
-// 0.76 of the issue slots with the one CTA of 1024
-// threads that the rows leave room for, and about 110 shared-memory wavefronts
-// beside the gathers. 8192 pairs at m = 10000: 53.8 ms, against 175 ms for the
-// cell-grid scan, which spent about 2000 instructions per query.
+// evaluated. What bounds the kernel: 635 instructions per query at m = 10000,
+// about 0.76 of the issue slots with the one CTA of 1024 threads that the rows
+// leave room for, and about 110 shared-memory wavefronts beside the gathers.
+// 8192 pairs at m = 10000: 54.1 ms, against 175 ms for the cell-grid scan, which
+// spent about 2000 instructions per query.
 #pragma once
 
 #include "common.cuh"

@@ -190,9 +190,9 @@ int g_forced_orders = -1;
 // (profiles/ksg_route_times.csv: lists of 2 to 120 nodes, a star and a chain of
 // 119 pairs, m = 500 to 4500, d = 1 to 3, k = 1 to 30, usual coordinates): 5%
 // spread for the exhaustive routes, 7 to 9% for the others where they are near
-// the best. The route chosen takes 0.4% more than the best on average, and more
-// than 13% in one plan of a hundred. Samples and distances are in thousands and
-// millions.
+// the best. The route chosen takes 0.6% more than the best on average, more than
+// 18% in one plan of a hundred, 39% at worst. Samples and distances are in
+// thousands and millions.
 struct PlanSize {
     int d, k, max_m;
     double pairs, samples, work;  // pairs, sum of m, sum of m^2
